@@ -17,6 +17,7 @@ LIB_PATH = os.environ.get("DBMP_LIBRARY") or os.path.join(HERE, "libdbmp.so")
 DBMP_OK, DBMP_ERR_INVALID, DBMP_ERR_CUDA, DBMP_ERR_CAPACITY, DBMP_ERR_UNSUPPORTED = range(5)
 ATLAS_F32, ATLAS_F32_QUAD, ATLAS_F16_QUAD, ATLAS_BF16_QUAD, ATLAS_F16_PAIR, ATLAS_BF16_PAIR = range(6)
 BIN_CONTENT, BIN_CULL, BIN_CONTENT_REF = 0, 1, 2
+EXTENDED_ATLAS = 0x41545845    # Canvas.reserved of calls that pass an extended atlas
 
 # Every symbol include/dbmp.h declares, with (restype, argtypes).
 _vp, _i, _ll, _sz, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_size_t, ctypes.c_float
@@ -60,6 +61,8 @@ SIGNATURES = {
     "dbmp_atlas_pack": (_i, [_vp, _i, _i, _i, _i, _vp, _vp]),
     "dbmp_template_blur": (_i, [_vp, _i, _i, _i, _f, _vp, _vp]),
     "dbmp_atlas_bytes": (_sz, [_i, _i, _i, _i]),
+    "dbmp_atlas_extended_bytes": (_sz, [_i, _i, _i, _i]),
+    "dbmp_atlas_pack_extended": (_i, [_vp, _i, _i, _i, _i, _vp, _vp]),
     "dbmp_bin_workspace_bytes": (_sz, [_CP, _ll]),
     "dbmp_prim_info_bytes": (_sz, [_i]),
     "dbmp_prepare": (_i, [_CP, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),

@@ -500,54 +500,81 @@ size_t atlas_bytes(int P, int Ht, int Wt, int kind) {
   return atlas_grid_offset(P, Ht, Wt, kind) + (size_t)P * gx * gy;
 }
 
-// Clearance grid (layout in dbmp_internal.cuh), one CTA per (cell column,
-// template).  Separable: per template row the x-distance from the column's
-// range to the nearest support texel of that row, then per cell the minimum
-// over rows of max(row distance, y-distance).  Texels further than kGridCap-1
-// beyond the cell cannot lower a capped value and are not visited.
+// Clearance grid and, with SOLID, the solid grid of the same cells (layouts in
+// dbmp_internal.cuh), one CTA per (cell column, template).  Separable: per
+// template row the x-distance from the column's range to the nearest bounding
+// texel of that row, then per cell the minimum over rows of max(row distance,
+// y-distance).  Bounding texels are the support texels, respectively the
+// texels other than exactly 1 (NaN counts as either).  Texels further than
+// kGridCap-1 beyond the cell cannot lower a capped value and are not visited.
+template <bool SOLID>
 __global__ void atlas_grid_kernel(const float* __restrict__ tmpl, int Ht, int Wt, int gsx, int gsy, int Gx, int Gy,
-                                  unsigned char* __restrict__ grid) {
-  extern __shared__ unsigned char s_row[];   // Ht row distances
+                                  unsigned char* __restrict__ grid, unsigned char* __restrict__ solid) {
+  extern __shared__ unsigned char s_row[];   // Ht row distances (clearance), then Ht more (solid)
   const int ix = blockIdx.x, p = blockIdx.y;
   const float* t = tmpl + (size_t)p * Ht * Wt;
   const int lo = ix << gsx, hi = min((ix + 1) << gsx, Wt - 1);
   const int xa = max(0, lo - (kGridCap - 1)), xb = min(Wt - 1, hi + (kGridCap - 1));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int y = warp; y < Ht; y += nwarps) {
-    int best = kGridCap;
+    int best = kGridCap, sbest = kGridCap;
     const float* row = t + (size_t)y * Wt;
     for (int x = xa + lane; x <= xb; x += 32) {
       const float v = row[x];
-      if (!(v <= kGridSupport)) best = min(best, max(0, max(lo - x, x - hi)));
+      const int d = max(0, max(lo - x, x - hi));
+      if (!(v <= kGridSupport)) best = min(best, d);
+      if (SOLID && !(v == 1.f)) sbest = min(sbest, d);
     }
     best = __reduce_min_sync(0xffffffffu, best);
-    if (lane == 0) s_row[y] = (unsigned char)best;
+    if (SOLID) sbest = __reduce_min_sync(0xffffffffu, sbest);
+    if (lane == 0) {
+      s_row[y] = (unsigned char)best;
+      if (SOLID) s_row[Ht + y] = (unsigned char)sbest;
+    }
   }
   __syncthreads();
   for (int iy = threadIdx.x; iy < Gy; iy += blockDim.x) {
     const int ylo = iy << gsy, yhi = min((iy + 1) << gsy, Ht - 1);
     const int ya = max(0, ylo - (kGridCap - 1)), yb = min(Ht - 1, yhi + (kGridCap - 1));
-    int best = kGridCap;
-    for (int y = ya; y <= yb; ++y) best = min(best, max((int)s_row[y], max(0, max(ylo - y, y - yhi))));
-    grid[((size_t)p * Gy + iy) * Gx + ix] = (unsigned char)best;
+    int best = kGridCap, sbest = kGridCap;
+    for (int y = ya; y <= yb; ++y) {
+      const int d = max(0, max(ylo - y, y - yhi));
+      best = min(best, max((int)s_row[y], d));
+      if (SOLID) sbest = min(sbest, max((int)s_row[Ht + y], d));
+    }
+    const size_t cell = ((size_t)p * Gy + iy) * Gx + ix;
+    grid[cell] = (unsigned char)best;
+    if (SOLID) solid[cell] = (unsigned char)sbest;
   }
 }
 
-int launch_atlas_grid(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st) {
+// The grids of a packed atlas of kind `kind` at `out`; solid_off: the solid grid's byte offset there (0: none).
+static int launch_grids(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, size_t solid_off,
+                        cudaStream_t st) {
   int sx, sy, gx, gy;
   grid_shape(Wt, &sx, &gx);
   grid_shape(Ht, &sy, &gy);
   unsigned char* grid = static_cast<unsigned char*>(out) + atlas_grid_offset(P, Ht, Wt, kind);
-  if (Ht > 48 * 1024) {   // row distances do not fit the shared buffer: clearance 0 never skips
-    cudaError_t e = cudaMemsetAsync(grid, 0, (size_t)P * gx * gy, st);
+  unsigned char* solid = solid_off ? static_cast<unsigned char*>(out) + solid_off : nullptr;
+  // row distances that do not fit the shared buffer: distance 0 never skips
+  if (solid && Ht > 24 * 1024) {
+    const cudaError_t e = cudaMemsetAsync(solid, 0, (size_t)P * gx * gy, st);
+    if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(solid)");
+    solid = nullptr;
+  }
+  if (Ht > 48 * 1024) {
+    const cudaError_t e = cudaMemsetAsync(grid, 0, (size_t)P * gx * gy, st);
     return e == cudaSuccess ? DBMP_OK : cuda_status(e, "cudaMemsetAsync(grid)");
   }
-  atlas_grid_kernel<<<dim3(gx, P), 256, Ht, st>>>(tmpl, Ht, Wt, sx, sy, gx, gy, grid);
+  if (solid) atlas_grid_kernel<true><<<dim3(gx, P), 256, 2 * Ht, st>>>(tmpl, Ht, Wt, sx, sy, gx, gy, grid, solid);
+  else atlas_grid_kernel<false><<<dim3(gx, P), 256, Ht, st>>>(tmpl, Ht, Wt, sx, sy, gx, gy, grid, nullptr);
   DBMP_CHECK_LAUNCH("atlas_grid_kernel");
   return DBMP_OK;
 }
 
-int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st) {
+// Packs the records and grids of a packed kind; solid_off as in launch_grids.
+static int pack_records(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, size_t solid_off,
+                        cudaStream_t st) {
   const long long total = (long long)P * (Ht + 1) * Wt;
   if (total == 0) return DBMP_OK;
   const int blocks = (int)((total + 255) / 256 < 148 * 32 ? (total + 255) / 256 : 148 * 32);
@@ -560,7 +587,21 @@ int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* 
     default: set_error("dbmp_atlas_pack: kind %d is not a packed kind", kind); return DBMP_ERR_INVALID;
   }
   DBMP_CHECK_LAUNCH("atlas_pack_kernel");
-  return launch_atlas_grid(tmpl, P, Ht, Wt, kind, out, st);
+  return launch_grids(tmpl, P, Ht, Wt, kind, out, solid_off, st);
+}
+
+int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st) {
+  return pack_records(tmpl, P, Ht, Wt, kind, out, 0, st);
+}
+
+int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st) {
+  if (P == 0) return DBMP_OK;
+  const AtlasExt x = atlas_ext(P, Ht, Wt, kind);
+  if (x.rec_off != 0 && tmpl != out) {   // DBMP_ATLAS_F32: the plain templates come first
+    const cudaError_t e = cudaMemcpyAsync(out, tmpl, sizeof(float) * (size_t)P * Ht * Wt, cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return cuda_status(e, "cudaMemcpyAsync(templates)");
+  }
+  return pack_records(tmpl, P, Ht, Wt, x.kind, static_cast<unsigned char*>(out) + x.rec_off, x.solid_off, st);
 }
 
 // Gaussian blur of the templates (pydiffbmp/util/utils.py:22-67,

@@ -27,6 +27,7 @@ size_t atlas_bytes(int P, int Ht, int Wt, int kind);
 int launch_template_bboxes(const float* tmpl, int P, int Ht, int Wt, float* out, cudaStream_t st);
 int launch_template_blur(const float* in, int P, int Ht, int Wt, float sigma, float* out, cudaStream_t st);
 int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
+int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
 int launch_prepare(const Geom& g, const float* means2D, const float* radii, const float* rot, const float* opac,
                    const float* colors, const int* sel, PrimInfo* out, cudaStream_t st);
 int launch_bin(const Geom& g, int bin_mode, const float* means2D, const float* radii, const float* rot,
@@ -123,6 +124,13 @@ int make_geom(const dbmp_canvas* cv, Geom* g, const char* who) {
   }
   grid_shape(cv->tmpl_w, &g->gsx, &g->gGx);
   grid_shape(cv->tmpl_h, &g->gsy, &g->gGy);
+  g->solid_off = g->rec_off = 0;
+  if (cv->reserved == DBMP_CANVAS_EXTENDED_ATLAS) {
+    const AtlasExt x = atlas_ext(g->P, g->Ht, g->Wt, g->kind);
+    g->kind = x.kind;
+    g->rec_off = (long long)x.rec_off;
+    g->solid_off = (long long)x.solid_off;
+  }
   g->grid_off = (long long)atlas_grid_offset(g->P, g->Ht, g->Wt, g->kind);
   return DBMP_OK;
 }
@@ -169,6 +177,19 @@ int dbmp_atlas_pack(const float* templates, int P, int Ht, int Wt, int kind, voi
 size_t dbmp_atlas_bytes(int P, int Ht, int Wt, int kind) {
   if (P < 0 || Ht < 1 || Wt < 1) return 0;
   return atlas_bytes(P, Ht, Wt, kind);
+}
+
+size_t dbmp_atlas_extended_bytes(int P, int Ht, int Wt, int kind) {
+  if (P < 0 || Ht < 1 || Wt < 1 || kind < DBMP_ATLAS_F32 || kind > DBMP_ATLAS_BF16_PAIR) return 0;
+  return atlas_ext(P, Ht, Wt, kind).total;
+}
+
+int dbmp_atlas_pack_extended(const float* templates, int P, int Ht, int Wt, int kind, void* out, void* stream) {
+  REQUIRE(P >= 0 && Ht >= 1 && Wt >= 1, "dbmp_atlas_pack_extended: bad atlas shape %dx%dx%d", P, Ht, Wt);
+  REQUIRE(kind >= DBMP_ATLAS_F32 && kind <= DBMP_ATLAS_BF16_PAIR, "dbmp_atlas_pack_extended: kind %d unknown", kind);
+  REQUIRE(P == 0 || (templates && out), "dbmp_atlas_pack_extended: null pointer");
+  REQUIRE(((uintptr_t)out & 255) == 0, "dbmp_atlas_pack_extended: out must be 256-byte aligned");
+  return launch_atlas_extended(templates, P, Ht, Wt, kind, out, (cudaStream_t)stream);
 }
 
 size_t dbmp_bin_workspace_bytes(const dbmp_canvas* cv, long long capacity) {
@@ -221,7 +242,7 @@ int dbmp_forward(const dbmp_canvas* cv, const void* prim_info, const void* atlas
   REQUIRE(atlas && tile_offsets && tile_indices && out_color && out_alpha && T_last && last_pos,
           "dbmp_forward: null pointer");
   REQUIRE(g.N == 0 || prim_info, "dbmp_forward: prim_info is null");
-  return launch_forward(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices, out_color,
+  return launch_forward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, out_color,
                         out_alpha, T_last, last_pos, (cudaStream_t)stream);
 }
 
@@ -242,7 +263,7 @@ int dbmp_backward(const dbmp_canvas* cv, const void* prim_info, const void* atla
     cudaError_t e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N, st);
     if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(grad_accum)");
   }
-  rc = launch_backward(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices, T_last,
+  rc = launch_backward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, T_last,
                        last_pos, grad_color, grad_alpha, grad_accum, st);
   if (rc) return rc;
   return launch_finalize(g, radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii,
@@ -274,7 +295,7 @@ int dbmp_forward_blend(const dbmp_canvas* cv, const void* prim_info, const void*
   REQUIRE(g.N == 0 || prim_info, "dbmp_forward_blend: prim_info is null");
   REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_forward_blend: c_blend %g outside [0, 1]", (double)c_blend);
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_forward_blend: colors_orig is null with c_blend > 0");
-  return launch_forward_blend(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices,
+  return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream, 1,
                               0, 0);
 }
@@ -300,7 +321,7 @@ int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void
     cudaError_t e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N, st);
     if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(grad_accum)");
   }
-  rc = launch_backward_blend(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices,
+  rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0);
   if (rc) return rc;
   return launch_finalize(g, radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii,
@@ -322,7 +343,7 @@ int dbmp_forward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, 
   REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_forward_batch: c_blend %g outside [0, 1]", (double)c_blend);
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_forward_batch: colors_orig is null with c_blend > 0");
   REQUIRE(((uintptr_t)prim_info & 15) == 0, "dbmp_forward_batch: prim_info must be 16-byte aligned");
-  return launch_forward_blend(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices,
+  return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream,
                               batch, index_stride, colors_orig_stride);
 }
@@ -351,7 +372,7 @@ int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info,
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N * batch, st);
   if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(grad_accum)");
-  rc = launch_backward_blend(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices,
+  rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, batch,
                              index_stride, colors_orig_stride);
   if (rc) return rc;
@@ -376,7 +397,7 @@ int dbmp_count(const dbmp_canvas* cv, const void* prim_info, const void* atlas, 
   REQUIRE(g.N == 0 || prim_info, "dbmp_count: prim_info is null");
   cudaError_t e = cudaMemsetAsync(counts, 0, 10 * sizeof(unsigned long long), (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(counts)");
-  return launch_count(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices, counts,
+  return launch_count(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, counts,
                       (cudaStream_t)stream);
 }
 
@@ -392,7 +413,7 @@ int dbmp_fused_fwd_bwd(const dbmp_canvas* cv, const void* prim_info, const void*
   cudaError_t e = cudaMemsetAsync(loss_out, 0, sizeof(double), st);
   if (e == cudaSuccess && g.N > 0) e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N, st);
   if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(fused outputs)");
-  return launch_fused(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices, target,
+  return launch_fused(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, target,
                       background, out_image, grad_accum, loss_out, skip_flag, st);
 }
 

@@ -103,6 +103,42 @@ __host__ __device__ inline size_t atlas_grid_offset(int P, int Ht, int Wt, int k
   return (atlas_record_bytes(P, Ht, Wt, kind) + 255) & ~(size_t)255;
 }
 
+// Extended atlas (dbmp_atlas_pack_extended; canvases with reserved =
+// DBMP_CANVAS_EXTENDED_ATLAS).  After the bytes that dbmp_atlas_bytes counts,
+// at 256-byte boundaries:
+//   packed kinds: the solid grid;
+//   ATLAS_F32: an F32_QUAD atlas of the same templates (records, clearance
+//   grid) and its solid grid, which the walks read in place of the reference
+//   layout (same values: the differences are the ones it takes after the loads).
+// The solid grid has the clearance grid's cells.  A cell stores the
+// L-infinity distance, capped at kGridCap, to the nearest texel other than
+// exactly 1.  Where a warp footprint (half extent e in texels, plus the
+// bilinear reach of 1) stays within that distance and inside the template, every
+// texel it reads is 1 with zero differences in every storage kind, so its
+// mask is exactly 1 and the mask's gradient exactly 0, and the walk needs
+// neither texel coordinates nor texels.
+struct AtlasExt {
+  int kind;          // the kind the walks read
+  size_t rec_off;    // byte offset of its records from the atlas pointer
+  size_t solid_off;  // byte offset of the solid grid from those records
+  size_t total;      // bytes of the whole extended atlas
+};
+__host__ __device__ inline size_t atlas_grid_bytes(int P, int Ht, int Wt) {
+  int sx, sy, gx, gy;
+  grid_shape(Wt, &sx, &gx);
+  grid_shape(Ht, &sy, &gy);
+  return (size_t)P * gx * gy;
+}
+__host__ __device__ inline AtlasExt atlas_ext(int P, int Ht, int Wt, int kind) {
+  AtlasExt x;
+  x.kind = kind == ATLAS_F32 ? ATLAS_F32_QUAD : kind;
+  x.rec_off = kind == ATLAS_F32 ? atlas_grid_offset(P, Ht, Wt, ATLAS_F32) : 0;
+  const size_t grid = atlas_grid_bytes(P, Ht, Wt);
+  x.solid_off = (atlas_grid_offset(P, Ht, Wt, x.kind) + grid + 255) & ~(size_t)255;
+  x.total = x.rec_off + x.solid_off + grid;
+  return x;
+}
+
 // Thread layout of the tile walk: one CTA per TS x TS tile, NP pixels per
 // thread, each warp owning an FW x FH footprint.
 // DBMP_SQUARE_FOOTPRINT: with 2 pixels per thread, an 8x8 warp footprint
@@ -119,6 +155,10 @@ struct Layout {
   static constexpr int WPR = TS / FW;              // warps per footprint row
   static constexpr int NW = (TS / FW) * (TS / FH);
   static constexpr int NT = NW * 32;
+  // texel coordinates of the second pixel: from its own offset to the centre
+  // (16-pixel tiles) or from the first pixel's by a multiple of a column of
+  // the inverse affine (one rounding apart)
+  static constexpr bool kDirect = TS == 16;
   static __host__ __device__ __forceinline__ int ox(int p) { return kSq ? 0 : 8 * (p & 1); }
   static __host__ __device__ __forceinline__ int oy(int p) { return kSq ? 4 * p : 4 * (p >> 1); }
 };
@@ -129,7 +169,7 @@ template <int TS> struct DefaultNP;
 #define DBMP_NP32 2
 #endif
 template <> struct DefaultNP<32> { static constexpr int v = DBMP_NP32; };
-template <> struct DefaultNP<16> { static constexpr int v = 1; };
+template <> struct DefaultNP<16> { static constexpr int v = 2; };
 
 struct Geom {
   // operand pairs of the packed pixel-pair arithmetic (both halves equal)
@@ -150,6 +190,12 @@ struct Geom {
   int gsx, gsy;        // clearance grid: log2 of the cell size in texels
   int gGx, gGy;        // clearance grid: cells per template row / column
   long long grid_off;  // byte offset of the clearance grid in a packed atlas
+  long long solid_off; // byte offset of the solid grid in an extended atlas (0: none)
+  long long rec_off;   // byte offset of the records the walks read (host side only)
+  // the walks' atlas: the caller's pointer advanced to the records they read
+  const void* records(const void* atlas) const {
+    return atlas ? static_cast<const char*>(atlas) + rec_off : nullptr;
+  }
 };
 
 // Bilinear neighbours of texel (x0, y0) in difference form: v00, d01 =

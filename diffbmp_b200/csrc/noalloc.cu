@@ -130,7 +130,7 @@ extern "C" int dbmp_backward_noalloc(const dbmp_canvas* cv, const void* prim_inf
     cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(double) * 8 * (size_t)g.N, st);
     if (e != cudaSuccess) return cuda_status(e, "dbmp_backward_noalloc: cudaMemsetAsync");
   }
-  rc = launch_backward(g, cv->atlas_kind, (const PrimInfo*)prim_info, atlas, tile_offsets, tile_indices, T_last,
+  rc = launch_backward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, T_last,
                        last_pos, grad_color, grad_alpha, scratch, st);
   if (rc) return rc;
   return launch_finalize(g, radii, rotations, opacities, colors, scratch, grad_means2D, grad_radii, grad_rotations,

@@ -43,20 +43,21 @@ __device__ __forceinline__ bool footprint_inside(const float4& g0, float x0, flo
          (g0.y + g0.w >= y1 + 1.f);
 }
 
-// Warp-uniform: true when the template's clearance grid shows that no pixel
-// of the warp footprint (centre (cx, cy)) can get a fragment from this
-// primitive.  The footprint centre's texel coordinate is clamped into the
-// template (clamping only shortens distances to its texels), and its cell's
-// clearance is compared with the primitive's requirement gext.
-__device__ __forceinline__ bool grid_clear(const Geom& g, const unsigned char* __restrict__ grid, const float4& g0,
-                                           const float4& g1, int goff, int gext, float cx, float cy) {
+// Grid cell (within the template's cells) of the warp footprint's centre
+// (cx, cy): its texel coordinate clamped into the template, which only
+// shortens distances to the template's texels.  The cell's clearance compared
+// with the primitive's requirement gext tells, warp-uniformly, that no pixel
+// of the footprint can get a fragment (clearance grid), or that every pixel's
+// mask is exactly 1 (solid grid, for a footprint whose texel box lies inside
+// the template).
+__device__ __forceinline__ int grid_cell(const Geom& g, const float4& g0, const float4& g1, float cx, float cy) {
   const float dx = cx - g0.x, dy = cy - g0.y;
   const float tx = fminf(fmaxf(fmaf(g1.x, dx, fmaf(g1.y, dy, g.hx)), 0.f), g.wm1);
   const float ty = fminf(fmaxf(fmaf(g1.z, dx, fmaf(g1.w, dy, g.hy)), 0.f), g.hm1);
   float unused;
   const int ix = floor_small(tx, &unused) >> g.gsx;
   const int iy = floor_small(ty, &unused) >> g.gsy;
-  return (int)__ldg(grid + goff + iy * g.gGx + ix) >= gext;
+  return iy * g.gGx + ix;
 }
 
 // Texel coordinates, sampling position and fetched neighbours of one pixel.
@@ -305,6 +306,7 @@ struct ChunkMasks {
   unsigned todo;     // entries the warp composites
   unsigned inside;   // footprint entirely inside the entry's cull square
   unsigned fast;     // ... and its texel-space box inside the template
+  unsigned solid;    // ... and its mask exactly 1 everywhere (solid grid)
   unsigned clear;    // clearance grid shows no fragment (skipped unless counting)
   unsigned miss;     // footprint misses the cull square
 };
@@ -342,6 +344,7 @@ struct TileWalker {
   static __device__ __forceinline__ int rec_toff(const Rec& r) { return __float_as_int(r[kRec - 1].x); }
 
   int warp, lw, lane, start, end;   // warp: index within the tile, lw: within the CTA
+  int solid_delta;                  // solid grid minus clearance grid (0: no solid grid)
   const float* cmap = nullptr;
   float cblend = 0.f;
 
@@ -363,6 +366,7 @@ struct TileWalker {
     lw = threadIdx.x >> 5;
     warp = part * cta_warps + lw;
     lane = threadIdx.x & 31;
+    solid_delta = g.solid_off ? (int)(g.solid_off - g.grid_off) : 0;
     const int tx = tile % g.tilesX, ty = tile / g.tilesX;
     start = __ldg(offs + tile);
     end = __ldg(offs + tile + 1);
@@ -398,7 +402,7 @@ struct TileWalker {
   __device__ __forceinline__ ChunkMasks stage(const Geom& g, const PrimInfo* __restrict__ prims,
                                               const int* __restrict__ idx, const unsigned char* __restrict__ grid,
                                               int base, int stop, Rec* w, int* my_id) {
-    bool keep = false, inside = false, fast = false, clear = false, miss = false;
+    bool keep = false, inside = false, fast = false, clear = false, solid = false, miss = false;
     int id = -1;
     __syncwarp();   // every lane is done with the previous chunk's records
     const int pos = base + lane;
@@ -413,8 +417,12 @@ struct TileWalker {
           const int toff = __float_as_int(q.x);
           if (toff != kNoFrag) {
             const float4 g1 = __ldg(r + 1);
-            if (kGrid)
-              clear = grid_clear(g, grid, g0, g1, __float_as_int(q.y), __float_as_int(q.z), fcx, fcy);
+            if (kGrid) {
+              const unsigned char* cell = grid + __float_as_int(q.y) + grid_cell(g, g0, g1, fcx, fcy);
+              const int need = __float_as_int(q.z);
+              clear = (int)__ldg(cell) >= need;
+              if (solid_delta != 0) solid = (int)__ldg(cell + solid_delta) >= need;
+            }
             keep = KEEP_CLEAR || !clear;
             if (keep) {
               inside = footprint_inside(g0, fx0, fx1, fy0, fy1);
@@ -428,6 +436,7 @@ struct TileWalker {
                 const float ey = fmaf(fabsf(g1.z), g.fhx, fmaf(fabsf(g1.w), g.fhy, 0.05f));
                 fast = cx - ex >= 0.f && cx + ex <= g.wm1 && cy - ey >= 0.f && cy + ey <= g.hm1;
               }
+              solid = solid && fast;
               float4 g2 = __ldg(r + 2);
               if (half_record(KIND)) {   // FP16 (alpha0, r) and (g, b) pairs
                 const float2 ar = h2f(__float_as_uint(g2.x)), gb = h2f(__float_as_uint(g2.y));
@@ -455,6 +464,7 @@ struct TileWalker {
     m.todo = __ballot_sync(kFull, keep);
     m.inside = __ballot_sync(kFull, inside);
     m.fast = __ballot_sync(kFull, fast);
+    m.solid = __ballot_sync(kFull, solid && keep);
     m.clear = KEEP_CLEAR ? __ballot_sync(kFull, clear) : 0u;
     m.miss = KEEP_CLEAR ? __ballot_sync(kFull, miss) : 0u;
     return m;
@@ -487,6 +497,36 @@ struct TileWalker {
     if (lane < 8 && acc[0] != 0.f) atomicAdd(dst + kidx, (double)acc[0]);
   }
 
+  // warp_add for a solid entry: acc holds sums 4..7 (the mask-gradient sums
+  // 0..3 are 0), reduced in the same order with 6 shuffles.  A sum that is
+  // not finite (an infinite or NaN gradient or colour) makes 0..3 NaN, as
+  // the product of such a term with the zero mask gradient does.
+  __device__ __forceinline__ void warp_add4(float (&acc)[4], double* __restrict__ dst) const {
+    const bool b0 = lane & 1, b1 = lane & 2;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float send = b0 ? acc[k] : acc[k + 2];
+      const float keep = b0 ? acc[k + 2] : acc[k];
+      acc[k] = keep + __shfl_xor_sync(kFull, send, 1);
+    }
+    {
+      const float send = b1 ? acc[0] : acc[1];
+      const float keep = b1 ? acc[1] : acc[0];
+      acc[0] = keep + __shfl_xor_sync(kFull, send, 2);
+    }
+    acc[0] += __shfl_xor_sync(kFull, acc[0], 4);
+    acc[0] += __shfl_xor_sync(kFull, acc[0], 8);
+    acc[0] += __shfl_xor_sync(kFull, acc[0], 16);
+    if (lane < 4 && acc[0] != 0.f) {
+      const int k = 2 * (lane & 1) + ((lane >> 1) & 1);
+      atomicAdd(dst + 4 + k, (double)acc[0]);
+      if (k == 3 && !(fabsf(acc[0]) < INFINITY)) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) atomicAdd(dst + j, (double)NAN);
+      }
+    }
+  }
+
   // Phase 1 of a forward entry for a pixel pair: coordinates and texel loads.
   __device__ __forceinline__ void pair_issue(const Geom& g, const void* __restrict__ atlas, const Rec* w, int e,
                                              const ChunkMasks& cm, const bool (&live)[2], PairPre<KIND>& p) const {
@@ -505,18 +545,13 @@ struct TileWalker {
     bool live[2];
   };
 
-  // Phase 2 of a forward entry: blend the loaded texels and composite.
-  // Returns true when every pixel of the warp has stopped.
-  __device__ __forceinline__ bool pair_composite(const Geom& g, const Rec* w, int e, int pos, const PairPre<KIND>& p,
-                                                 PairFwd& f, bool vote = true) const {
+  // Composites masks m of entry e (fragments f0, f1) onto the pixel pair.
+  // Returns true when every pixel of the warp has stopped (if vote).
+  __device__ __forceinline__ bool pair_over(const Geom& g, const Rec* w, int e, int pos, float2 m, bool f0, bool f1,
+                                            PairFwd& f, bool vote) const {
     const float4 c0 = w[e][2];
     const float4 c1 = w[e][3];
-    PairSample s;
-    pair_unpack<KIND>(g, p, s);
-    const float2 m = pair_blend<false, false>(g, s, nullptr, nullptr);
-    // a pixel may have stopped since the loads were issued
-    const bool f0 = s.ok0 && f.live[0] && m.x > 1e-6f, f1 = s.ok1 && f.live[1] && m.y > 1e-6f;
-    float2 a = make_float2(f0 ? c0.x * m.x : 0.f, f1 ? c0.y * m.y : 0.f);
+    const float2 a = make_float2(f0 ? c0.x * m.x : 0.f, f1 ? c0.y * m.y : 0.f);
     const float2 wt = make_float2(f.t.x * a.x, f.t.y * a.y);
     f.cr = make_float2(fmaf(wt.x, c0.z, f.cr.x), fmaf(wt.y, c0.w, f.cr.y));
     f.cg = make_float2(fmaf(wt.x, c1.x, f.cg.x), fmaf(wt.y, c1.y, f.cg.y));
@@ -533,10 +568,25 @@ struct TileWalker {
     return vote && __all_sync(kFull, !f.live[0] && !f.live[1]);
   }
 
+  // Phase 2 of a forward entry: blend the loaded texels and composite.
+  __device__ __forceinline__ bool pair_composite(const Geom& g, const Rec* w, int e, int pos, const PairPre<KIND>& p,
+                                                 PairFwd& f, bool vote = true) const {
+    PairSample s;
+    pair_unpack<KIND>(g, p, s);
+    const float2 m = pair_blend<false, false>(g, s, nullptr, nullptr);
+    // a pixel may have stopped since the loads were issued
+    const bool f0 = s.ok0 && f.live[0] && m.x > 1e-6f, f1 = s.ok1 && f.live[1] && m.y > 1e-6f;
+    return pair_over(g, w, e, pos, m, f0, f1, f, vote);
+  }
+
   // Forward walk of the pixel-pair form: the walk of forward() with both
-  // pixels' sampling, blending and compositing as packed pairs.  Entries go
-  // two at a time: the texel loads of both are issued before either is
-  // composited, so their latencies overlap.
+  // pixels' sampling, blending and compositing as packed pairs.  Entries that
+  // are sampled go two at a time: the texel loads of both are issued before
+  // either is composited, so their latencies overlap.  Solid entries (mask 1 on
+  // the whole footprint) are composited straight from their record: they need
+  // a third of the instructions of a sampled one, and at 2048x2048, N=20000,
+  // 256x256 bitmaps with soft rims they are 44 % of the entries (forward walk
+  // 244 -> 218 us, backward 432 -> 361, fused kernel 637 -> 548).
   __device__ __forceinline__ void forward_pair(const Geom& g, const PrimInfo* __restrict__ prims,
                                                const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
                                                float (&C)[2][3], float (&T)[2], float (&Tl)[2], int (&lp)[2]) {
@@ -555,9 +605,16 @@ struct TileWalker {
       while (todo) {
         const int e1 = __ffs(todo) - 1;
         todo &= todo - 1;
-        const bool two = todo != 0;
-        const int e2 = two ? __ffs(todo) - 1 : e1;   // e1 again when it is the chunk's last
-        todo &= todo - 1;
+        if ((cm.solid >> e1) & 1u) {   // every live pixel of the warp has mask 1: nothing to sample
+          if (pair_over(g, w, e1, base - start + e1, make_float2(1.f, 1.f), f.live[0], f.live[1], f, true)) {
+            warp_done = true;
+            break;
+          }
+          continue;
+        }
+        const bool two = todo != 0 && !((cm.solid >> (__ffs(todo) - 1)) & 1u);
+        const int e2 = two ? __ffs(todo) - 1 : e1;   // e1 again when no sampled entry follows it
+        if (two) todo &= todo - 1;
         PairPre<KIND> p1, p2;
         pair_issue(g, atlas, w, e1, cm, f.live, p1);
         pair_issue(g, atlas, w, e2, cm, f.live, p2);
@@ -603,6 +660,30 @@ struct TileWalker {
         const float4 c1 = w[e][3];
         const int toff = rec_toff(w[e]);
         const bool live[2] = {pos <= lp[0], pos <= lp[1]};
+        if ((cm.solid >> e) & 1u) {
+          // mask 1 with gradient 0 on the whole footprint: the operations below
+          // with m = 1 and gx = gy = 0, which leave the colour and opacity sums
+          const float2 a = make_float2(live[0] ? c0.x : 0.f, live[1] ? c0.y : 0.f);
+          const float2 om = make_float2(__saturatef(1.f - a.x), __saturatef(1.f - a.y));
+          const float2 tk = make_float2((pos == lp[0]) ? ts.x : __fdividef(ts.x, om.x),
+                                        (pos == lp[1]) ? ts.y : __fdividef(ts.y, om.y));
+          ts = tk;
+          const float2 gcc = make_float2(fmaf(gcr.x, c0.z, fmaf(gcg.x, c1.x, gcb.x * c1.z)),
+                                         fmaf(gcr.y, c0.w, fmaf(gcg.y, c1.y, gcb.y * c1.w)));
+          float2 dlda;
+          if (kQuad) dlda = make_float2(tk.x * fmaf(ga.x, bt.x, gcc.x - h.x), tk.y * fmaf(ga.y, bt.y, gcc.y - h.y));
+          else dlda = mul2(tk, fma2(ga, bt, sub2(g, gcc, h)));
+          const float2 wt = mul2(a, tk);
+          float acc[4];
+          acc[0] = fmaf(gcr.y, wt.y, gcr.x * wt.x);
+          acc[1] = fmaf(gcg.y, wt.y, gcg.x * wt.x);
+          acc[2] = fmaf(gcb.y, wt.y, gcb.x * wt.x);
+          acc[3] = fmaf(dlda.y, a.y, dlda.x * a.x);
+          h = make_float2(fmaf(om.x, h.x, a.x * gcc.x), fmaf(om.y, h.y, a.y * gcc.y));
+          bt = make_float2(bt.x * om.x, bt.y * om.y);
+          warp_add4(acc, gacc + (size_t)id * 8);
+          continue;
+        }
         PairSample s;
         const bool inside = (cm.inside >> e) & 1u;
         if ((cm.fast >> e) & 1u) pair_sample<L, KIND, true>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, s);

@@ -294,8 +294,8 @@ class ImageFitter:
         a = self.atlas
         call("dbmp_template_blur_scheduled", _ptr(a.templates), a.P, a.Ht, a.Wt, ctypes.byref(self.blur),
              _ptr(self.step_count), _ptr(self._blurred), st)
-        if a.kind != _lib.ATLAS_F32:
-            call("dbmp_atlas_pack", _ptr(self._blurred), a.P, a.Ht, a.Wt, a.kind, _ptr(a.data), st)
+        if a.extended:
+            a.pack(self._blurred, st)
 
     def _enqueue(self):
         st = _stream()

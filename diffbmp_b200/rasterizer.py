@@ -23,7 +23,7 @@ import torch
 
 from . import _lib
 from ._lib import (ATLAS_BF16_PAIR, ATLAS_BF16_QUAD, ATLAS_F16_PAIR, ATLAS_F16_QUAD, ATLAS_F32, ATLAS_F32_QUAD,
-                   BIN_CONTENT, BIN_CONTENT_REF, BIN_CULL, Canvas, DbmpError, call, lib)
+                   BIN_CONTENT, BIN_CONTENT_REF, BIN_CULL, EXTENDED_ATLAS, Canvas, DbmpError, call, lib)
 
 # Atlas storage kinds: "f32" is the reference layout; the precision form
 # stores half / bfloat16 texels as horizontal pairs ("f16", "bf16", two 4-byte
@@ -74,12 +74,23 @@ class Atlas:
             call("dbmp_template_blur", _ptr(self.templates), self.P, self.Ht, self.Wt, ctypes.c_float(self.sigma),
                  _ptr(blurred), st)
             self.templates = blurred
-        if self.kind == ATLAS_F32:
-            self.data = self.templates
+        self.extended = self.kind != ATLAS_F32
+        if self.extended:
+            self._alloc()
+            self.pack(self.templates, st)
         else:
-            nbytes = int(lib.dbmp_atlas_bytes(self.P, self.Ht, self.Wt, self.kind))
-            self.data = torch.empty(nbytes, dtype=torch.uint8, device=t.device)
-            call("dbmp_atlas_pack", _ptr(self.templates), self.P, self.Ht, self.Wt, self.kind, _ptr(self.data), st)
+            self.data = self.templates
+
+    def _alloc(self):
+        """The extended atlas's buffer; data is the part dbmp_atlas_bytes counts."""
+        total = int(lib.dbmp_atlas_extended_bytes(self.P, self.Ht, self.Wt, self.kind))
+        buf = torch.empty(total, dtype=torch.uint8, device=self.templates.device)
+        self.data = buf[:int(lib.dbmp_atlas_bytes(self.P, self.Ht, self.Wt, self.kind))]
+
+    def pack(self, templates: torch.Tensor, st=None):
+        """Fills the buffer from (P,Ht,Wt) f32 templates (extended atlases)."""
+        call("dbmp_atlas_pack_extended", _ptr(templates), self.P, self.Ht, self.Wt, self.kind, _ptr(self.data),
+             st if st is not None else _stream())
 
     def private_copy(self) -> "Atlas":
         """An atlas of the same kind, templates and content bboxes with its own
@@ -88,7 +99,11 @@ class Atlas:
         a = Atlas.__new__(Atlas)
         a.templates, a.sigma, a.bbox = self.templates, self.sigma, self.bbox
         a.P, a.Ht, a.Wt, a.kind = self.P, self.Ht, self.Wt, self.kind
-        a.data = torch.empty_like(self.data)
+        a.extended = self.extended
+        if a.extended:
+            a._alloc()
+        else:
+            a.data = torch.empty_like(self.data)
         return a
 
     def with_kind(self, kind) -> "Atlas":
@@ -180,7 +195,7 @@ class Rasterizer:
 
     def canvas(self, N: int, atlas: Atlas) -> Canvas:
         return Canvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
-                      self.alpha_max, self.t_stop, 0)
+                      self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.extended else 0)
 
     # -- binning -----------------------------------------------------------
     def _ensure(self, cv: Canvas, cap: int):

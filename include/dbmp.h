@@ -70,8 +70,12 @@ typedef struct {
   int32_t bin_mode;           /* DBMP_BIN_* */
   float alpha_max;            /* alpha_upper_bound (finite, >= 0) */
   float t_stop;               /* early-termination transmittance, in [1e-30, 1) */
-  int32_t reserved;
+  int32_t reserved;           /* 0, or DBMP_CANVAS_EXTENDED_ATLAS */
 } dbmp_canvas;
+
+/* dbmp_canvas.reserved: the atlas pointers passed with this canvas are
+ * extended atlases (dbmp_atlas_pack_extended).  Any other value means plain ones. */
+#define DBMP_CANVAS_EXTENDED_ATLAS 0x41545845
 
 const char* dbmp_last_error(void);
 int dbmp_version(void);
@@ -114,6 +118,20 @@ int dbmp_template_blur(const float* templates, int P, int Ht, int Wt, float sigm
  * counterpart (storage format of the precision form). */
 size_t dbmp_atlas_bytes(int P, int Ht, int Wt, int kind);
 int dbmp_atlas_pack(const float* templates, int P, int Ht, int Wt, int kind, void* out, void* stream);
+
+/* Extended atlas: the atlas of a kind (its first dbmp_atlas_bytes bytes: as
+ * dbmp_atlas_pack writes it, or for DBMP_ATLAS_F32 the plain (P,Ht,Wt) templates),
+ * followed by what lets the walks skip work without changing a result.  For
+ * every kind that is a solid grid: per cell of the clearance grid the
+ * L-infinity distance to the nearest texel other than exactly 1; where a
+ * warp footprint stays within it the mask is 1 and its gradient 0, and no
+ * texel is read.  DBMP_ATLAS_F32 also gets f32 quads with their clearance
+ * grid, which the walks then read.  `out` is 256-byte aligned and
+ * dbmp_atlas_extended_bytes large; for DBMP_ATLAS_F32 it may be `templates`
+ * itself.  Calls that are passed such an atlas say so in dbmp_canvas.reserved.
+ * No reference counterpart. */
+size_t dbmp_atlas_extended_bytes(int P, int Ht, int Wt, int kind);
+int dbmp_atlas_pack_extended(const float* templates, int P, int Ht, int Wt, int kind, void* out, void* stream);
 
 /* Scratch bytes that dbmp_bin needs (per primitive and per tile; the
  * capacity argument is accepted for compatibility and does not change it). */
