@@ -501,73 +501,145 @@ size_t atlas_bytes(int P, int Ht, int Wt, int kind) {
 }
 
 // Clearance grid and, with SOLID, the solid grid of the same cells (layouts in
-// dbmp_internal.cuh), one CTA per (cell column, template).  Separable: per
-// template row the x-distance from the column's range to the nearest bounding
-// texel of that row, then per cell the minimum over rows of max(row distance,
-// y-distance).  Bounding texels are the support texels, respectively the
-// texels other than exactly 1 (NaN counts as either).  Texels further than
-// kGridCap-1 beyond the cell cannot lower a capped value and are not visited.
+// dbmp_internal.cuh), one CTA per (strip of cell rows, template).
+// Bounding texels are the support texels, respectively the texels other than
+// exactly 1 (NaN counts as either).  First a warp takes each template row that
+// can matter to the strip (up to kGridCap-1 rows beyond it): ballots turn the
+// row into bit masks, and each cell column's distance to the row's nearest
+// bounding texel comes from the 64-bit windows left and right of the cell.
+// Then each cell takes the minimum over rows of max(row distance, y-distance),
+// going outwards until the y-distance alone reaches its minimum.  1024 templates
+// of 256x256 take 1.4 ms; scanning every texel within reach of a cell column for
+// each row, as one CTA per (cell column, template), took 4.6 ms.  With few
+// templates the kernel is latency-bound (8 of 128x128: 20 us).
+constexpr int kGridThreads = 1024;   // latency-bound: a warp's rows and a thread's cells run in series
+
+struct GridArgs {
+  int Ht, Wt, gsx, gsy, Gx, Gy;
+  int strip;   // cell rows of a CTA
+  int words;   // 32-bit words of a row's mask: Wt bits, rounded up, and 5 zero words (2 before, 3 after)
+  int rows;    // template rows of a strip at most
+  unsigned char* grid;
+  unsigned char* solid;
+};
+
+// Bits [pos, pos + 64) of a mask with two zero words before bit 0 (pos >= -64).
+__device__ __forceinline__ unsigned long long mask_window(const unsigned* m, int pos) {
+  const int q = pos + 64, w = q >> 5, s = q & 31;
+  const unsigned a = __funnelshift_r(m[w], m[w + 1], s), b = __funnelshift_r(m[w + 1], m[w + 2], s);
+  return ((unsigned long long)b << 32) | a;
+}
+
+// Distance of the cell range [lo, hi] to the nearest set bit, capped at kGridCap.
+__device__ __forceinline__ int mask_distance(const unsigned* m, int lo, int hi) {
+  for (int x = lo; x <= hi; x += 64) {
+    unsigned long long v = mask_window(m, x);
+    if (hi - x < 63) v &= (2ull << (hi - x)) - 1ull;
+    if (v) return 0;
+  }
+  const unsigned long long l = mask_window(m, lo - 64), r = mask_window(m, hi + 1);
+  const int dl = l ? __clzll((long long)l) + 1 : kGridCap, dr = r ? __ffsll((long long)r) : kGridCap;
+  return min(min(dl, dr), kGridCap);
+}
+
 template <bool SOLID>
-__global__ void atlas_grid_kernel(const float* __restrict__ tmpl, int Ht, int Wt, int gsx, int gsy, int Gx, int Gy,
-                                  unsigned char* __restrict__ grid, unsigned char* __restrict__ solid) {
-  extern __shared__ unsigned char s_row[];   // Ht row distances (clearance), then Ht more (solid)
-  const int ix = blockIdx.x, p = blockIdx.y;
-  const float* t = tmpl + (size_t)p * Ht * Wt;
-  const int lo = ix << gsx, hi = min((ix + 1) << gsx, Wt - 1);
-  const int xa = max(0, lo - (kGridCap - 1)), xb = min(Wt - 1, hi + (kGridCap - 1));
+__global__ void __launch_bounds__(kGridThreads) atlas_grid_kernel(const float* __restrict__ tmpl, GridArgs a) {
+  extern __shared__ unsigned s_mem[];
+  constexpr int K = SOLID ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  for (int y = warp; y < Ht; y += nwarps) {
-    int best = kGridCap, sbest = kGridCap;
-    const float* row = t + (size_t)y * Wt;
-    for (int x = xa + lane; x <= xb; x += 32) {
-      const float v = row[x];
-      const int d = max(0, max(lo - x, x - hi));
-      if (!(v <= kGridSupport)) best = min(best, d);
-      if (SOLID && !(v == 1.f)) sbest = min(sbest, d);
+  unsigned* mask = s_mem + (size_t)warp * K * a.words;                             // this warp's row masks
+  unsigned char* dist = reinterpret_cast<unsigned char*>(s_mem + (size_t)nwarps * K * a.words);   // K x rows x Gx
+  const int p = blockIdx.y;
+  const float* t = tmpl + (size_t)p * a.Ht * a.Wt;
+  const int c0 = blockIdx.x * a.strip, c1 = min(c0 + a.strip, a.Gy);
+  const int y0 = max(0, (c0 << a.gsy) - (kGridCap - 1)), y1 = min(a.Ht - 1, (c1 << a.gsy) + (kGridCap - 1));
+  for (int i = lane; i < K * a.words; i += 32) mask[i] = 0u;
+  __syncwarp();
+  for (int y = y0 + warp; y <= y1; y += nwarps) {
+    const float* row = t + (size_t)y * a.Wt;
+#pragma unroll 4
+    for (int x0 = 0; x0 < a.Wt; x0 += 32) {
+      const bool in = x0 + lane < a.Wt;
+      const float v = in ? row[x0 + lane] : 0.f;
+      const unsigned b = __ballot_sync(0xffffffffu, in && !(v <= kGridSupport));
+      const unsigned c = SOLID ? __ballot_sync(0xffffffffu, in && !(v == 1.f)) : 0u;
+      if (lane == 0) {
+        mask[2 + (x0 >> 5)] = b;
+        if (SOLID) mask[a.words + 2 + (x0 >> 5)] = c;
+      }
     }
-    best = __reduce_min_sync(0xffffffffu, best);
-    if (SOLID) sbest = __reduce_min_sync(0xffffffffu, sbest);
-    if (lane == 0) {
-      s_row[y] = (unsigned char)best;
-      if (SOLID) s_row[Ht + y] = (unsigned char)sbest;
+    __syncwarp();
+    for (int ix = lane; ix < a.Gx; ix += 32) {
+      const int lo = ix << a.gsx, hi = min((ix + 1) << a.gsx, a.Wt - 1);
+      dist[(size_t)(y - y0) * a.Gx + ix] = (unsigned char)mask_distance(mask, lo, hi);
+      if (SOLID) dist[(size_t)(a.rows + y - y0) * a.Gx + ix] = (unsigned char)mask_distance(mask + a.words, lo, hi);
     }
+    __syncwarp();   // the masks are rewritten for the next row
   }
   __syncthreads();
-  for (int iy = threadIdx.x; iy < Gy; iy += blockDim.x) {
-    const int ylo = iy << gsy, yhi = min((iy + 1) << gsy, Ht - 1);
-    const int ya = max(0, ylo - (kGridCap - 1)), yb = min(Ht - 1, yhi + (kGridCap - 1));
-    int best = kGridCap, sbest = kGridCap;
-    for (int y = ya; y <= yb; ++y) {
-      const int d = max(0, max(ylo - y, y - yhi));
-      best = min(best, max((int)s_row[y], d));
-      if (SOLID) sbest = min(sbest, max((int)s_row[Ht + y], d));
+  for (int i = threadIdx.x; i < K * (c1 - c0) * a.Gx; i += blockDim.x) {
+    const int k = i / ((c1 - c0) * a.Gx), j = i - k * (c1 - c0) * a.Gx;
+    const int iy = c0 + j / a.Gx, ix = j % a.Gx;
+    const int ylo = iy << a.gsy, yhi = min((iy + 1) << a.gsy, a.Ht - 1);
+    const unsigned char* d = dist + (size_t)k * a.rows * a.Gx + ix;
+    int best = kGridCap;
+    for (int y = ylo; y <= yhi; ++y) best = min(best, (int)d[(size_t)(y - y0) * a.Gx]);
+    for (int e = 1; e < best; ++e) {
+      int m = kGridCap;
+      if (ylo - e >= y0) m = d[(size_t)(ylo - e - y0) * a.Gx];
+      if (yhi + e <= y1) m = min(m, (int)d[(size_t)(yhi + e - y0) * a.Gx]);
+      best = min(best, max(m, e));
     }
-    const size_t cell = ((size_t)p * Gy + iy) * Gx + ix;
-    grid[cell] = (unsigned char)best;
-    if (SOLID) solid[cell] = (unsigned char)sbest;
+    (k == 0 ? a.grid : a.solid)[((size_t)p * a.Gy + iy) * a.Gx + ix] = (unsigned char)best;
   }
 }
 
 // The grids of a packed atlas of kind `kind` at `out`; solid_off: the solid grid's byte offset there (0: none).
 static int launch_grids(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, size_t solid_off,
                         cudaStream_t st) {
-  int sx, sy, gx, gy;
-  grid_shape(Wt, &sx, &gx);
-  grid_shape(Ht, &sy, &gy);
-  unsigned char* grid = static_cast<unsigned char*>(out) + atlas_grid_offset(P, Ht, Wt, kind);
-  unsigned char* solid = solid_off ? static_cast<unsigned char*>(out) + solid_off : nullptr;
-  // row distances that do not fit the shared buffer: distance 0 never skips
-  if (solid && Ht > 24 * 1024) {
-    const cudaError_t e = cudaMemsetAsync(solid, 0, (size_t)P * gx * gy, st);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(solid)");
-    solid = nullptr;
+  GridArgs a;
+  a.Ht = Ht;
+  a.Wt = Wt;
+  grid_shape(Wt, &a.gsx, &a.Gx);
+  grid_shape(Ht, &a.gsy, &a.Gy);
+  a.grid = static_cast<unsigned char*>(out) + atlas_grid_offset(P, Ht, Wt, kind);
+  a.solid = solid_off ? static_cast<unsigned char*>(out) + solid_off : nullptr;
+  a.words = (Wt + 31) / 32 + 5;
+  const int k = a.solid ? 2 : 1;
+  const size_t row_bytes = (size_t)k * a.words * 4;
+  constexpr size_t kSmem = 224 * 1024;
+  // strips of 32 cell rows, or fewer while the grid has less than two CTAs per
+  // SM (a shorter strip scans more rows beyond it per row of its own) or the
+  // row distances do not fit
+  size_t smem = 0;
+  int warps = kGridThreads / 32;
+  for (a.strip = 32;; a.strip >>= 1) {
+    const long long rows = ((long long)a.strip << a.gsy) + 2 * kGridCap;
+    a.rows = (int)(rows < Ht ? rows : Ht);
+    const size_t dist_bytes = (size_t)k * a.rows * a.Gx;
+    smem = warps * row_bytes + dist_bytes;
+    if (a.strip > 8 && (long long)((a.Gy + a.strip - 1) / a.strip) * P < 296) continue;
+    if (smem <= kSmem || a.strip == 1) {
+      while (warps > 1 && smem > kSmem) {
+        warps >>= 1;
+        smem = warps * row_bytes + dist_bytes;
+      }
+      break;
+    }
   }
-  if (Ht > 48 * 1024) {
-    const cudaError_t e = cudaMemsetAsync(grid, 0, (size_t)P * gx * gy, st);
+  if (smem > kSmem) {   // a side of tens of thousands of texels: distance 0 never skips
+    cudaError_t e = cudaMemsetAsync(a.grid, 0, atlas_grid_bytes(P, Ht, Wt), st);
+    if (e == cudaSuccess && a.solid) e = cudaMemsetAsync(a.solid, 0, atlas_grid_bytes(P, Ht, Wt), st);
     return e == cudaSuccess ? DBMP_OK : cuda_status(e, "cudaMemsetAsync(grid)");
   }
-  if (solid) atlas_grid_kernel<true><<<dim3(gx, P), 256, 2 * Ht, st>>>(tmpl, Ht, Wt, sx, sy, gx, gy, grid, solid);
-  else atlas_grid_kernel<false><<<dim3(gx, P), 256, Ht, st>>>(tmpl, Ht, Wt, sx, sy, gx, gy, grid, nullptr);
+  const dim3 ctas((a.Gy + a.strip - 1) / a.strip, P);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = a.solid ? cudaFuncSetAttribute(atlas_grid_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem)
+                                  : cudaFuncSetAttribute(atlas_grid_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(atlas_grid_kernel)");
+  }
+  if (a.solid) atlas_grid_kernel<true><<<ctas, warps * 32, smem, st>>>(tmpl, a);
+  else atlas_grid_kernel<false><<<ctas, warps * 32, smem, st>>>(tmpl, a);
   DBMP_CHECK_LAUNCH("atlas_grid_kernel");
   return DBMP_OK;
 }

@@ -240,7 +240,7 @@ class ImageFitter:
                 raise ValueError(f"blur must be one of {sorted(BLUR_MODES)}, not {cfg.blur!r}")
             if cfg.blur == "adaptive" and cfg.num_iterations < 1:
                 raise ValueError("the adaptive blur schedule needs FitConfig.num_iterations")
-            self.atlas = atlas.private_copy()
+            self.atlas = atlas.private_copy(self.H * self.W)
             self.cv = self.rz.canvas(self.N, self.atlas)
             self.blur = _lib.BlurSchedule(BLUR_MODES[cfg.blur], cfg.blur_sigma, cfg.blur_sigma_start,
                                           cfg.blur_sigma_end, int(cfg.num_iterations))
@@ -370,6 +370,7 @@ class ImageFitter:
 
     def step(self):
         """Enqueues one fit iteration (no host synchronisation)."""
+        self.atlas.refresh()
         if self.graph is not None:
             self.graph.replay()
         else:

@@ -31,6 +31,14 @@ from ._lib import (ATLAS_BF16_PAIR, ATLAS_BF16_QUAD, ATLAS_F16_PAIR, ATLAS_F16_Q
 KIND_NAMES = {"f32": ATLAS_F32, "f32q": ATLAS_F32_QUAD, "f16q": ATLAS_F16_QUAD, "bf16q": ATLAS_BF16_QUAD,
               "f16": ATLAS_F16_PAIR, "bf16": ATLAS_BF16_PAIR}
 
+# An "f32" atlas also holds its templates as f32 quads (16 bytes a texel) up to
+# this many bytes.  The walks are as fast on quads far beyond the L2 as inside it
+# (2048x2048, N=20000, 1024 templates of 256x256, 1 GiB of quads: forward 257 us,
+# backward 384, against 549 and 810 on the reference layout; with 16 templates 239
+# and 363 against 537 and 800), so the limit only bounds their memory and the time
+# to pack them (1.6 ms per GiB).
+MAX_F32_QUAD_BYTES = 1 << 30
+
 DEFAULT_T_STOP = 1e-6   # image error <= t_stop * max colour, well inside the 1e-5 parity bar
 
 
@@ -74,10 +82,16 @@ class Atlas:
             call("dbmp_template_blur", _ptr(self.templates), self.P, self.Ht, self.Wt, ctypes.c_float(self.sigma),
                  _ptr(blurred), st)
             self.templates = blurred
-        self.extended = self.kind != ATLAS_F32
+        # an extended atlas (dbmp_atlas_pack_extended) holds the grids, and for
+        # "f32" the quads, that let the walks skip work
+        self.extended = self.kind != ATLAS_F32 or (self.templates.numel() * 16 <= MAX_F32_QUAD_BYTES
+                                                   and not self.templates.is_inference())
+        self._followed = None
         if self.extended:
             self._alloc()
             self.pack(self.templates, st)
+            if self.kind == ATLAS_F32:
+                self._followed = self.templates._version
         else:
             self.data = self.templates
 
@@ -86,24 +100,39 @@ class Atlas:
         total = int(lib.dbmp_atlas_extended_bytes(self.P, self.Ht, self.Wt, self.kind))
         buf = torch.empty(total, dtype=torch.uint8, device=self.templates.device)
         self.data = buf[:int(lib.dbmp_atlas_bytes(self.P, self.Ht, self.Wt, self.kind))]
+        if self.kind == ATLAS_F32:
+            self.data = self.data.view(torch.float32).view(self.P, self.Ht, self.Wt)
+
+    def refresh(self):
+        """Repacks an "f32" atlas whose templates tensor was changed in place
+        since it was packed: that kind renders the caller's tensor as it is."""
+        if self._followed is not None and self._followed != self.templates._version:
+            self.pack(self.templates)
+            self._followed = self.templates._version
 
     def pack(self, templates: torch.Tensor, st=None):
         """Fills the buffer from (P,Ht,Wt) f32 templates (extended atlases)."""
         call("dbmp_atlas_pack_extended", _ptr(templates), self.P, self.Ht, self.Wt, self.kind, _ptr(self.data),
              st if st is not None else _stream())
 
-    def private_copy(self) -> "Atlas":
+    def private_copy(self, pixels: Optional[int] = None) -> "Atlas":
         """An atlas of the same kind, templates and content bboxes with its own
-        texel buffer (filled by the caller), for a job that re-derives its
-        texels every step (the fit loop's blur schedule)."""
+        texel buffer (filled by the caller), for a job on a canvas of `pixels`
+        that re-derives its texels every step (the fit loop's blur schedule).
+        Such a job repacks an extended atlas every step, which an "f32" one
+        only does where the walks gain more than that takes: 23 us for 8
+        templates of 128x128 against 33 us of a 512x512 step (N=600), but 50 us
+        for 16 of 256x256 against 10 us of a 300x300 step (N=300)."""
         a = Atlas.__new__(Atlas)
         a.templates, a.sigma, a.bbox = self.templates, self.sigma, self.bbox
         a.P, a.Ht, a.Wt, a.kind = self.P, self.Ht, self.Wt, self.kind
-        a.extended = self.extended
+        a.extended = self.extended and (a.kind != ATLAS_F32 or pixels is None
+                                        or pixels >= max(2 * self.templates.numel(), 1 << 18))
+        a._followed = None
         if a.extended:
             a._alloc()
         else:
-            a.data = torch.empty_like(self.data)
+            a.data = torch.empty_like(self.templates)
         return a
 
     def with_kind(self, kind) -> "Atlas":
@@ -194,6 +223,7 @@ class Rasterizer:
         self._small = torch.zeros(2, dtype=torch.int32, device=self.device)   # total L, overflow flag
 
     def canvas(self, N: int, atlas: Atlas) -> Canvas:
+        atlas.refresh()
         return Canvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
                       self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.extended else 0)
 

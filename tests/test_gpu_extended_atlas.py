@@ -30,15 +30,15 @@ def binary_templates(rng, P, Ht, Wt):
     return T
 
 
-def solid_bruteforce(t, cap=64, max_cells=128):
-    """Per cell of the clearance grid: L-infinity distance from its coordinate range to the nearest texel != 1."""
+def grid_bruteforce(t, free, cap=64, max_cells=128):
+    """Per cell: L-infinity distance from its coordinate range to the nearest texel that is not free, capped."""
     def shape(n):
         s = 0
         while -(-n // (1 << s)) > max_cells:
             s += 1
         return s, -(-n // (1 << s))
     (Ht, Wt), (sx, gx), (sy, gy) = t.shape, shape(t.shape[1]), shape(t.shape[0])
-    ys, xs = np.nonzero(~(t == 1))
+    ys, xs = np.nonzero(~free)
     out = np.full((gy, gx), cap, np.int64)
     for iy in range(gy):
         dy = np.maximum(0, np.maximum((iy << sy) - ys, ys - min((iy + 1) << sy, Ht - 1)))
@@ -50,18 +50,21 @@ def solid_bruteforce(t, cap=64, max_cells=128):
 
 
 @pytest.mark.parametrize("kind", ["f16", "bf16q"])
-@pytest.mark.parametrize("Ht,Wt", [(2, 2), (40, 72), (130, 130), (300, 20)])
+@pytest.mark.parametrize("Ht,Wt", [(2, 2), (40, 72), (130, 130), (300, 20), (33, 1030), (4100, 31), (257, 129)])
 def test_solid_grid_matches_definition_gpu(kind, Ht, Wt):
     T = binary_templates(np.random.default_rng(0), 3, Ht, Wt)
     T[1, Ht // 2, Wt // 2] = np.nan
     atlas = R.Atlas(torch.from_numpy(T).cuda(), kind)
     raw = torch.as_strided(atlas.data, (int(R.lib.dbmp_atlas_extended_bytes(3, Ht, Wt, atlas.kind)),), (1,))
     raw = raw.cpu().numpy()
-    want = [solid_bruteforce(t) for t in T]
+    want = [grid_bruteforce(t, t == 1) for t in T]
+    clear = [grid_bruteforce(t, t <= 5e-7) for t in T]
     off = raw.size - sum(w.size for w in want)
     assert off % 256 == 0 and off >= atlas.data.numel()
     for p, w in enumerate(want):
         assert np.array_equal(raw[off + p * w.size: off + (p + 1) * w.size].reshape(w.shape), w), p
+        at = atlas.data.numel() + (p - 3) * w.size      # the clearance grid ends the plain atlas
+        assert np.array_equal(raw[at: at + w.size].reshape(w.shape), clear[p]), p
 
 
 def walk(atlas, extended, d, N, H, W, ts, gc, ga):
@@ -105,3 +108,41 @@ def test_walks_equal_the_plain_atlas_gpu(kind, H, W, ts, N, Ht, Wt, bad):
         fin = torch.isfinite(b)
         assert torch.equal(fin, torch.isfinite(a))
         assert (a - b)[fin].norm() <= 1e-6 * b[fin].norm()
+
+
+def test_f32_atlas_follows_its_templates_gpu():
+    """An "f32" atlas renders the caller's tensor as it is, also after an in-place change."""
+    rng = np.random.default_rng(3)
+    T = torch.from_numpy(binary_templates(rng, 2, 48, 48)).cuda()
+    d = [torch.tensor([[30.0, 30.0], [50.0, 40.0]]).cuda(), torch.tensor([25.0, 30.0]).cuda(), torch.zeros(2).cuda(),
+         torch.zeros(2).cuda(), torch.zeros(2, 3).cuda(), torch.tensor([0, 1], dtype=torch.int32).cuda()]
+    rz = R.Rasterizer(64, 80)
+    atlas = R.Atlas(T, "f32")
+    before = rz.forward(*d, atlas)[0]
+    T.mul_(0.5)
+    after = rz.forward(*d, atlas)[0]
+    assert torch.equal(after, rz.forward(*d, R.Atlas(T, "f32"))[0])
+    assert not torch.equal(before, after)
+
+
+@pytest.mark.parametrize("H,W,ts", [(64, 48, 32), (130, 77, 16)])
+def test_f32_quads_equal_the_reference_layout_gpu(H, W, ts, monkeypatch):
+    """The walks of an extended "f32" atlas (quads) against those on the plain templates."""
+    rng = np.random.default_rng(H)
+    cu = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    N = 80
+    d = [cu(rng.uniform(0, [W, H], (N, 2))), cu(rng.uniform(4, 50, N)), cu(rng.uniform(0, 7, N)),
+         cu(rng.normal(0, 2, N)), cu(rng.normal(0, 1, (N, 3))), torch.from_numpy(rng.integers(0, 3, N).astype(np.int32)).cuda()]
+    T = cu(binary_templates(rng, 3, 70, 51) * rng.uniform(0.5, 1, (3, 70, 51)))
+    gc, ga = cu(rng.normal(0, 1, (H, W, 3))), cu(rng.normal(0, 1, (H, W)))
+    res = []
+    for limit in (1 << 30, 0):
+        monkeypatch.setattr(R, "MAX_F32_QUAD_BYTES", limit)
+        atlas, rz = R.Atlas(T, "f32"), R.Rasterizer(H, W, ts)
+        assert atlas.extended == (limit > 0)
+        c, a, st = rz.forward(*d, atlas)
+        res.append(([c, a, st.T_last, st.last_pos], rz.backward(st, gc, ga, *d[1:5], atlas)))
+    for a, b in zip(*(r[0] for r in res)):
+        assert torch.equal(a, b)
+    for a, b in zip(*(r[1] for r in res)):
+        assert (a - b).norm() <= 1e-6 * b.norm()
