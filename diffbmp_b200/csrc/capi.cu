@@ -115,21 +115,17 @@ int make_geom(const dbmp_canvas* cv, Geom* g, const char* who) {
   g->kind = cv->atlas_kind;
   g->alpha_max = cv->alpha_max;
   g->t_stop = cv->t_stop;
-  if (cv->tile_size == 32) {
-    using L = Layout<32, DefaultNP<32>::v>;
-    g->fhx = 0.5f * (float)(L::FW - 1); g->fhy = 0.5f * (float)(L::FH - 1);
-  } else {
-    using L = Layout<16, DefaultNP<16>::v>;
-    g->fhx = 0.5f * (float)(L::FW - 1); g->fhy = 0.5f * (float)(L::FH - 1);
-  }
+  g->fhx = 0.5f * (float)(Layout<32>::FW - 1);   // both tile sizes have the same footprint
+  g->fhy = 0.5f * (float)(Layout<32>::FH - 1);
   grid_shape(cv->tmpl_w, &g->gsx, &g->gGx);
   grid_shape(cv->tmpl_h, &g->gsy, &g->gGy);
-  g->solid_off = g->rec_off = 0;
+  g->solid_delta = 0;
+  g->rec_off = 0;
   if (cv->reserved == DBMP_CANVAS_EXTENDED_ATLAS) {
     const AtlasExt x = atlas_ext(g->P, g->Ht, g->Wt, g->kind);
     g->kind = x.kind;
     g->rec_off = (long long)x.rec_off;
-    g->solid_off = (long long)x.solid_off;
+    g->solid_delta = (int)(x.solid_off - atlas_grid_offset(g->P, g->Ht, g->Wt, x.kind));
   }
   g->grid_off = (long long)atlas_grid_offset(g->P, g->Ht, g->Wt, g->kind);
   return DBMP_OK;

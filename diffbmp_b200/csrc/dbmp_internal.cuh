@@ -139,37 +139,19 @@ __host__ __device__ inline AtlasExt atlas_ext(int P, int Ht, int Wt, int kind) {
   return x;
 }
 
-// Thread layout of the tile walk: one CTA per TS x TS tile, NP pixels per
-// thread, each warp owning an FW x FH footprint.
-// DBMP_SQUARE_FOOTPRINT: with 2 pixels per thread, an 8x8 warp footprint
-// (the second pixel 4 rows below the first) instead of 16x4.
-#ifndef DBMP_SQUARE_FOOTPRINT
-#define DBMP_SQUARE_FOOTPRINT 1
-#endif
-template <int TS, int NP>
+// Thread layout of the tile walk: a TS x TS tile is covered by 8x8 warp
+// footprints, two pixels per thread, the second kStep rows below the first.
+template <int TS>
 struct Layout {
-  static_assert(NP == 1 || NP == 2 || NP == 4, "pixels per thread");
-  static constexpr bool kSq = DBMP_SQUARE_FOOTPRINT && NP == 2;
-  static constexpr int FW = kSq ? 8 : (NP >= 2 ? 16 : 8);     // warp footprint
-  static constexpr int FH = kSq ? 8 : (NP == 4 ? 8 : 4);
+  static constexpr int FW = 8, FH = 8;             // warp footprint
+  static constexpr int kStep = 4;
   static constexpr int WPR = TS / FW;              // warps per footprint row
   static constexpr int NW = (TS / FW) * (TS / FH);
-  static constexpr int NT = NW * 32;
   // texel coordinates of the second pixel: from its own offset to the centre
-  // (16-pixel tiles) or from the first pixel's by a multiple of a column of
-  // the inverse affine (one rounding apart)
+  // (16-pixel tiles) or from the first pixel's (32-pixel tiles), one rounding
+  // apart
   static constexpr bool kDirect = TS == 16;
-  static __host__ __device__ __forceinline__ int ox(int p) { return kSq ? 0 : 8 * (p & 1); }
-  static __host__ __device__ __forceinline__ int oy(int p) { return kSq ? 4 * p : 4 * (p >> 1); }
 };
-
-// Pixels per thread of each tile size (tuned on B200).
-template <int TS> struct DefaultNP;
-#ifndef DBMP_NP32
-#define DBMP_NP32 2
-#endif
-template <> struct DefaultNP<32> { static constexpr int v = DBMP_NP32; };
-template <> struct DefaultNP<16> { static constexpr int v = 2; };
 
 struct Geom {
   // operand pairs of the packed pixel-pair arithmetic (both halves equal)
@@ -190,7 +172,7 @@ struct Geom {
   int gsx, gsy;        // clearance grid: log2 of the cell size in texels
   int gGx, gGy;        // clearance grid: cells per template row / column
   long long grid_off;  // byte offset of the clearance grid in a packed atlas
-  long long solid_off; // byte offset of the solid grid in an extended atlas (0: none)
+  int solid_delta;     // solid grid minus clearance grid, in bytes (0: no extended atlas)
   long long rec_off;   // byte offset of the records the walks read (host side only)
   // the walks' atlas: the caller's pointer advanced to the records they read
   const void* records(const void* atlas) const {
@@ -215,14 +197,10 @@ template <> struct AtlasFetch<ATLAS_F32> {
     return make_float4(__ldg(t), xr ? __ldg(t + 1) : 0.f, yr ? __ldg(t + Wt) : 0.f,
                        (xr && yr) ? __ldg(t + Wt + 1) : 0.f);
   }
-  static __device__ __forceinline__ Quad get(const void* atlas, int off, int Ht, int Wt, int x0, int y0) {
-    const float4 v = get_raw(atlas, off, Ht, Wt, x0, y0);
-    return Quad{v.x, v.y - v.x, v.z, v.w - v.z};
-  }
 };
 
 // Packed kinds: load() fetches record i (= off + y0 Wt + x0; int or unsigned)
-// as stored, unpack() turns it into a Quad, at() does both.
+// as stored, unpack() turns it into a Quad.
 template <> struct AtlasFetch<ATLAS_F32_QUAD> {
   using Raw = float4;
   template <typename I>
@@ -230,11 +208,6 @@ template <> struct AtlasFetch<ATLAS_F32_QUAD> {
     return __ldg(static_cast<const float4*>(atlas) + i);
   }
   static __device__ __forceinline__ Quad unpack(const Raw& v) { return Quad{v.x, v.y, v.z, v.w}; }
-  template <typename I>
-  static __device__ __forceinline__ Quad at(const void* atlas, I i, int Wt) { return unpack(load(atlas, i, Wt)); }
-  static __device__ __forceinline__ Quad get(const void* atlas, int off, int Ht, int Wt, int x0, int y0) {
-    return at(atlas, off + y0 * Wt + x0, Wt);
-  }
 };
 
 __device__ __forceinline__ float2 h2f(unsigned u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
@@ -252,11 +225,6 @@ template <> struct AtlasFetch<ATLAS_F16_QUAD> {
     const float2 a = h2f(r.x), b = h2f(r.y);
     return Quad{a.x, a.y, b.x, b.y};
   }
-  template <typename I>
-  static __device__ __forceinline__ Quad at(const void* atlas, I i, int Wt) { return unpack(load(atlas, i, Wt)); }
-  static __device__ __forceinline__ Quad get(const void* atlas, int off, int Ht, int Wt, int x0, int y0) {
-    return at(atlas, off + y0 * Wt + x0, Wt);
-  }
 };
 
 template <> struct AtlasFetch<ATLAS_BF16_QUAD> {
@@ -268,11 +236,6 @@ template <> struct AtlasFetch<ATLAS_BF16_QUAD> {
   static __device__ __forceinline__ Quad unpack(const Raw& r) {
     const float2 a = b2f(r.x), b = b2f(r.y);
     return Quad{a.x, a.y, b.x, b.y};
-  }
-  template <typename I>
-  static __device__ __forceinline__ Quad at(const void* atlas, I i, int Wt) { return unpack(load(atlas, i, Wt)); }
-  static __device__ __forceinline__ Quad get(const void* atlas, int off, int Ht, int Wt, int x0, int y0) {
-    return at(atlas, off + y0 * Wt + x0, Wt);
   }
 };
 
@@ -287,11 +250,6 @@ template <> struct AtlasFetch<ATLAS_F16_PAIR> {
     const float2 a = h2f(r.x), b = h2f(r.y);
     return Quad{a.x, a.y, b.x, b.y};
   }
-  template <typename I>
-  static __device__ __forceinline__ Quad at(const void* atlas, I i, int Wt) { return unpack(load(atlas, i, Wt)); }
-  static __device__ __forceinline__ Quad get(const void* atlas, int off, int Ht, int Wt, int x0, int y0) {
-    return at(atlas, off + y0 * Wt + x0, Wt);
-  }
 };
 
 template <> struct AtlasFetch<ATLAS_BF16_PAIR> {
@@ -304,11 +262,6 @@ template <> struct AtlasFetch<ATLAS_BF16_PAIR> {
   static __device__ __forceinline__ Quad unpack(const Raw& r) {
     const float2 a = b2f(r.x), b = b2f(r.y);
     return Quad{a.x, a.y, b.x, b.y};
-  }
-  template <typename I>
-  static __device__ __forceinline__ Quad at(const void* atlas, I i, int Wt) { return unpack(load(atlas, i, Wt)); }
-  static __device__ __forceinline__ Quad get(const void* atlas, int off, int Ht, int Wt, int x0, int y0) {
-    return at(atlas, off + y0 * Wt + x0, Wt);
   }
 };
 

@@ -1,25 +1,25 @@
 // Forward / backward / fused tile compositing kernels.
 //
-// A tile of TS x TS pixels is walked by NW warps (one or more CTAs); each thread owns NP pixels
-// (NP = 4, 2 or 1) of a compact warp footprint (16x8, 8x8 or 8x4 pixels) so
-// that a primitive's square cull is mostly warp-uniform and the warp's texel
+// A tile of TS x TS pixels is walked by NW warps (one or more CTAs); each thread
+// owns 2 pixels (4 rows apart) of a compact 8x8 warp footprint, so that a
+// primitive's square cull is mostly warp-uniform and the warp's texel
 // fetches stay close together in the atlas.
 //
 // Every warp walks the tile's primitive list on its own, without CTA
 // barriers: it stages 32 list entries at a time into a warp-private shared
-// buffer (lane i loads entry i's 64-byte PrimInfo record and runs the
-// warp-footprint cull and the clearance-grid test for it), and a ballot of
-// the survivors gives the entries the warp composites, in list order in the
+// buffer (lane i loads entry i's 64-byte PrimInfo record, runs the
+// warp-footprint cull and the grid tests for it, and stores it behind the
+// survivors before it), and composites the survivors, in list order in the
 // forward walk and in reverse order in the backward walk.  Per entry a thread
 // first computes the texel coordinates of all its pixels and issues their
 // texel loads (addresses of pixels without a fragment are redirected to texel
 // 0 of the template, so every load is in bounds), then composites them
 // branch-free.  A warp stops when all its pixels are below t_stop; the
 // backward walk of a warp starts at its own last contributor and adds its
-// warp-reduced per-primitive sums straight into the FP64 accumulator.  With 2
-// pixels per thread (32x32 tiles) both pixels go through the arithmetic as one
-// float2 of packed FP32x2 instructions, and the forward walk issues the
-// texel loads of two entries before compositing either.
+// warp-reduced per-primitive sums straight into the FP64 accumulator.  A
+// thread's two pixels go through the arithmetic as one float2 of packed FP32x2
+// instructions, and the forward walk issues the texel loads of two entries
+// before compositing either.
 #include "dbmp_internal.cuh"
 
 namespace dbmp {
@@ -27,20 +27,24 @@ namespace dbmp {
 constexpr int kChunk = 32;   // list entries staged per warp at a time (one per lane)
 constexpr unsigned kFull = 0xffffffffu;
 
+// A warp footprint reaches 3.5 pixels from its centre (cx, cy); the cull tests
+// of whole footprints take 1 px more for rounding.
+constexpr float kReach = 4.5f;
+
 // Conservative warp-uniform rejection: true when the primitive's cull square
 // misses every pixel of the warp footprint (1 px margin for rounding; NaN
 // never rejects, matching the reference's cull).
-__device__ __forceinline__ bool footprint_miss(const float4& g0, float x0, float x1, float y0, float y1) {
-  return (g0.x - g0.z > x1 + 1.f) || (g0.x + g0.z < x0 - 1.f) || (g0.y - g0.w > y1 + 1.f) ||
-         (g0.y + g0.w < y0 - 1.f);
+__device__ __forceinline__ bool footprint_miss(const float4& g0, float cx, float cy) {
+  return (g0.x - g0.z > cx + kReach) || (g0.x + g0.z < cx - kReach) || (g0.y - g0.w > cy + kReach) ||
+         (g0.y + g0.w < cy - kReach);
 }
 
 // Warp-uniform: true when every pixel of the warp footprint passes the
 // primitive's square cull with a 1 px margin, so the per-pixel cull can be
 // skipped (false for NaN geometry, which then takes the per-pixel path).
-__device__ __forceinline__ bool footprint_inside(const float4& g0, float x0, float x1, float y0, float y1) {
-  return (g0.x - g0.z <= x0 - 1.f) && (g0.x + g0.z >= x1 + 1.f) && (g0.y - g0.w <= y0 - 1.f) &&
-         (g0.y + g0.w >= y1 + 1.f);
+__device__ __forceinline__ bool footprint_inside(const float4& g0, float cx, float cy) {
+  return (g0.x - g0.z <= cx - kReach) && (g0.x + g0.z >= cx + kReach) && (g0.y - g0.w <= cy - kReach) &&
+         (g0.y + g0.w >= cy + kReach);
 }
 
 // Grid cell (within the template's cells) of the warp footprint's centre
@@ -60,31 +64,38 @@ __device__ __forceinline__ int grid_cell(const Geom& g, const float4& g0, const 
   return iy * g.gGx + ix;
 }
 
-// Texel coordinates, sampling position and fetched neighbours of one pixel.
-struct Sample {
-  float tx, ty, wx, wy;
+// Texel coordinates of one pixel.
+struct Coord {
+  float tx, ty;
   bool ok;    // pixel live, inside the cull square and inside [0,W-1]x[0,H-1]
-  Quad q;
 };
 
-// Phase 1 of an entry: texel coordinates of every pixel of the thread (the
-// inverse affine is linear, so pixel p is pixel 0 plus a multiple of a column
-// of A) and whether the pixel can yield a fragment (live, inside the cull
-// square, inside [0,W-1]x[0,H-1]).
+// Texel coordinates of a thread's two pixels for an entry, and whether each
+// can yield a fragment (live, inside the cull square, inside
+// [0,W-1]x[0,H-1]).  The second pixel's come from the first's, since the inverse
+// affine is linear (32-pixel tiles), or from its own offset (16-pixel tiles).
 // FAST: the warp footprint lies inside the cull square and its texel-space
 // box inside the template (with margin), so every pixel passes both tests.
-template <int NP, class L, bool FAST>
+template <class L, bool FAST>
 __device__ __forceinline__ void entry_coords(const Geom& g, const float4& g0, const float4& g1, bool inside,
-                                             const float (&pxf)[NP], const float (&pyf)[NP],
-                                             const bool (&live)[NP], Sample (&s)[NP]) {
+                                             const float (&pxf)[2], const float (&pyf)[2], const bool (&live)[2],
+                                             Coord (&s)[2]) {
   const float dx0 = pxf[0] - g0.x, dy0 = pyf[0] - g0.y;
   const float tx0 = fmaf(g1.x, dx0, fmaf(g1.y, dy0, g.hx));
   const float ty0 = fmaf(g1.z, dx0, fmaf(g1.w, dy0, g.hy));
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {
+  for (int p = 0; p < 2; ++p) {
     float tx = tx0, ty = ty0;
-    if (L::ox(p)) { tx = fmaf((float)L::ox(p), g1.x, tx); ty = fmaf((float)L::ox(p), g1.z, ty); }
-    if (L::oy(p)) { tx = fmaf((float)L::oy(p), g1.y, tx); ty = fmaf((float)L::oy(p), g1.w, ty); }
+    if (p == 1) {
+      if (L::kDirect) {
+        const float dy = pyf[1] - g0.y;
+        tx = fmaf(g1.x, dx0, fmaf(g1.y, dy, g.hx));
+        ty = fmaf(g1.z, dx0, fmaf(g1.w, dy, g.hy));
+      } else {
+        tx = fmaf((float)L::kStep, g1.y, tx);
+        ty = fmaf((float)L::kStep, g1.w, ty);
+      }
+    }
     if (FAST) {
       s[p].ok = live[p];
     } else {
@@ -96,55 +107,6 @@ __device__ __forceinline__ void entry_coords(const Geom& g, const float4& g0, co
     s[p].tx = tx;
     s[p].ty = ty;
   }
-}
-
-// Phase 2 for one pixel: sampling position and texel fetch (texel 0 of the
-// template when the pixel cannot yield a fragment, so the load is in bounds).
-template <int KIND, bool FAST>
-__device__ __forceinline__ void entry_fetch(const Geom& g, const void* __restrict__ atlas, int toff, Sample& s) {
-  // FAST: every pixel's coordinate lies inside the template, no redirection needed
-  const float tx = (FAST || s.ok) ? s.tx : 0.f, ty = (FAST || s.ok) ? s.ty : 0.f;
-  float fx, fy;
-  const int x0 = floor_small(tx, &fx);
-  const int y0 = floor_small(ty, &fy);
-  s.wx = tx - fx;
-  s.wy = ty - fy;
-  s.q = AtlasFetch<KIND>::get(atlas, toff, g.Ht, g.Wt, x0, y0);
-}
-
-// Texel coordinates and texel fetches of all pixels of the thread for one
-// entry (fast: the entry's warp-uniform interior bit).
-template <int NP, class L, int KIND>
-__device__ __forceinline__ void entry_sample(const Geom& g, const void* __restrict__ atlas, int toff,
-                                             const float4& g0, const float4& g1, bool inside, bool fast,
-                                             const float (&pxf)[NP], const float (&pyf)[NP],
-                                             const bool (&live)[NP], Sample (&s)[NP]) {
-  if (fast) {
-    entry_coords<NP, L, true>(g, g0, g1, inside, pxf, pyf, live, s);
-#pragma unroll
-    for (int p = 0; p < NP; ++p) entry_fetch<KIND, true>(g, atlas, toff, s[p]);
-  } else {
-    entry_coords<NP, L, false>(g, g0, g1, inside, pxf, pyf, live, s);
-#pragma unroll
-    for (int p = 0; p < NP; ++p) entry_fetch<KIND, false>(g, atlas, toff, s[p]);
-  }
-}
-
-// Bilinear mask and, with GRAD, its texel-space gradient.  The reference
-// clamps the mask to [0,1] (tile_forward.cu:271, NaN -> 1); only the upper
-// clamp is applied here, since every caller discards masks failing the
-// fragment test mask > 1e-6, which the lower clamp cannot change.
-template <bool GRAD>
-__device__ __forceinline__ float blend(const Sample& s, float* gx, float* gy) {
-  const float dt = s.q.d01, db = s.q.d11;
-  const float top = fmaf(s.wx, dt, s.q.v00);
-  const float bot = fmaf(s.wx, db, s.q.v10);
-  const float m = fmaf(s.wy, bot - top, top);
-  if (GRAD) {
-    *gx = fmaf(s.wy, db - dt, dt);
-    *gy = bot - top;
-  }
-  return fminf(1.f, m);
 }
 
 // ---------------------------------------------------------------------------
@@ -168,7 +130,7 @@ struct PairSample {
   float2 tx, ty;             // texel coordinates (not redirected)
   float2 wx, wy;             // bilinear weights of the fetched texel
   float2 v00, d01, v10, d11;  // neighbours in difference form (Quad)
-  bool ok0, ok1;             // pixel can yield a fragment (as Sample::ok)
+  bool ok0, ok1;             // pixel can yield a fragment (as Coord::ok)
 };
 
 // A pixel pair's sample with its texel loads issued but not yet consumed.
@@ -177,6 +139,7 @@ struct PairPre {
   float2 wx, wy;
   typename AtlasFetch<KIND>::Raw r0, r1;   // the two pixels' records as loaded
   bool ok0, ok1;
+  float2 tx, ty;                           // texel coordinates (colour-map walks only)
 };
 
 // Coordinates, weights and texel loads of both pixels for one entry; tx, ty
@@ -186,8 +149,8 @@ __device__ __forceinline__ void pair_prep(const Geom& g, const void* __restrict_
                                           const float4& g0, const float4& g1, bool inside, const float (&pxf)[2],
                                           const float (&pyf)[2], const bool (&live)[2], PairPre<KIND>& s,
                                           float2* ptx = nullptr, float2* pty = nullptr) {
-  Sample c[2];
-  entry_coords<2, L, FAST>(g, g0, g1, inside, pxf, pyf, live, c);
+  Coord c[2];
+  entry_coords<L, FAST>(g, g0, g1, inside, pxf, pyf, live, c);
   s.ok0 = c[0].ok;
   s.ok1 = c[1].ok;
   if (ptx) {
@@ -250,9 +213,11 @@ __device__ __forceinline__ void pair_sample(const Geom& g, const void* __restric
   pair_unpack<KIND>(g, p, s);
 }
 
-// Bilinear mask of both pixels (upper-clamped as in blend()) and, with GRAD, its texel-space
-// gradient: the operations of blend() on pairs.  PACKED: as FP32x2 instructions;
-// otherwise as scalar ones (same roundings).
+// Bilinear mask of both pixels and, with GRAD, its texel-space gradient.
+// PACKED: as FP32x2 instructions; otherwise as scalar ones (same roundings).
+// The reference clamps the mask to [0,1] (tile_forward.cu:271, NaN -> 1); only
+// the upper clamp is applied here, since every caller discards masks failing
+// the fragment test mask > 1e-6, which the lower clamp cannot change.
 template <bool GRAD, bool PACKED = true>
 __device__ __forceinline__ float2 pair_blend(const Geom& g, const PairSample& s, float2* gx, float2* gy) {
   if (!PACKED) {
@@ -301,63 +266,69 @@ __device__ __forceinline__ float3 sample_cmap(const float* __restrict__ cm, int 
 }
 
 // ---------------------------------------------------------------------------
-// Ballots of one staged chunk (bit j = entry base + j).
-struct ChunkMasks {
-  unsigned todo;     // entries the warp composites
+// A staged chunk: its n surviving entries sit at w[0..n-1] in list order; bit j
+// of each mask belongs to entry w[j].
+struct Chunk {
+  int n;             // entries the warp composites
   unsigned inside;   // footprint entirely inside the entry's cull square
   unsigned fast;     // ... and its texel-space box inside the template
   unsigned solid;    // ... and its mask exactly 1 everywhere (solid grid)
-  unsigned clear;    // clearance grid shows no fragment (skipped unless counting)
-  unsigned miss;     // footprint misses the cull square
+  unsigned clear;    // clearance grid shows no fragment (counting walk only: skipped otherwise)
+  unsigned miss;     // list entries whose cull square the footprint misses (counting walk only)
 };
+constexpr unsigned kInside = 1u, kFast = 2u, kSolid = 4u, kClear = 8u;
+
+// Staged record: [0] (mx, my, hw, hh)  [1] A  [2] (op, r, g, b)
+// [3] (toff, flags, position in the tile's list, primitive id).
+using Rec = float4[4];
+
+// a / b for 2^-126 <= b <= 1, as a times the approximate reciprocal.
+__device__ __forceinline__ float div_unit(float a, float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return a * r;
+}
 
 // CB: fragment colours blend a per-primitive colour map (cmap, (N,Ht,Wt,3))
 // with weight cblend, (1 - cblend) sigmoid(c) + cblend c_o (tile_forward.cu:316-330).
-#ifndef DBMP_PACKED_PAIRS
-#define DBMP_PACKED_PAIRS 1
-#endif
-
-
-template <int TS, int NP, int KIND, bool CB = false>
+template <int TS, int KIND, bool CB = false>
 struct TileWalker {
-  using L = Layout<TS, NP>;
-  static constexpr int NT = L::NT;
-  static constexpr int NW = L::NW;
+  static constexpr int NP = 2;      // pixels of a thread
+  using L = Layout<TS>;
   static constexpr bool kGrid = KIND != ATLAS_F32;   // packed atlases carry a clearance grid
   static constexpr bool kQuad = KIND == ATLAS_F32_QUAD || KIND == ATLAS_F16_QUAD || KIND == ATLAS_BF16_QUAD;
-  // Pixel-pair walk (2 pixels per thread, fixed colours).  Its staged record
-  // holds the opacity and colours as duplicated pairs:
-  //   [0] (mx, my, hw, hh)  [1] A  [2] (op, op, r, r)  [3] (g, g, b, b)  [4] (toff, goff, gext, -)
-  // otherwise the PrimInfo record as is: [0] [1] A [2] (op, r, g, b) [3] (toff, goff, gext, -).
-  static constexpr bool kPair = DBMP_PACKED_PAIRS && NP == 2 && !CB;
-  static constexpr int kRec = kPair ? 5 : 4;
-  using Rec = float4[kRec];
-
-  // (op, r, g, b) and the atlas offset of a staged record.
-  static __device__ __forceinline__ float4 rec_g2(const Rec& r) {
-    if (kPair) {
-      const float4 a = r[2], b = r[3];
-      return make_float4(a.x, a.z, b.x, b.z);
-    }
-    return r[2];
-  }
-  static __device__ __forceinline__ int rec_toff(const Rec& r) { return __float_as_int(r[kRec - 1].x); }
 
   int warp, lw, lane, start, end;   // warp: index within the tile, lw: within the CTA
-  int solid_delta;                  // solid grid minus clearance grid (0: no solid grid)
   const float* cmap = nullptr;
   float cblend = 0.f;
-
-  // Fragment colour of pixel sample s for primitive id (g2.yzw = sigmoid(c)).
-  __device__ __forceinline__ float3 frag_colour(const Geom& g, const float4& g2, int id, const Sample& s) const {
-    if (!CB) return make_float3(g2.y, g2.z, g2.w);
-    const float3 co = sample_cmap(cmap + (size_t)id * g.Ht * g.Wt * 3, g.Ht, g.Wt, s.tx, s.ty);
-    const float k = 1.f - cblend;
-    return make_float3(k * g2.y + cblend * co.x, k * g2.z + cblend * co.y, k * g2.w + cblend * co.z);
-  }
   float pxf[NP], pyf[NP];
   bool valid[NP];
-  float fx0, fx1, fy0, fy1, fcx, fcy;
+  float fcx, fcy;   // centre of the warp footprint
+
+  // Colours of the pixel pair for an entry (g2.yzw = sigmoid(c)); with CB, the
+  // map is sampled at the texel coordinates of the pixels with a fragment.
+  __device__ __forceinline__ void pair_colour(const Geom& g, const float4& g2, int id, float2 tx, float2 ty, bool f0,
+                                              bool f1, float2& r, float2& gr, float2& b) const {
+    r = make_float2(g2.y, g2.y);
+    gr = make_float2(g2.z, g2.z);
+    b = make_float2(g2.w, g2.w);
+    if constexpr (CB) {
+      const float* cm = cmap + (size_t)id * g.Ht * g.Wt * 3;
+      const float k = 1.f - cblend;
+      if (f0) {
+        const float3 co = sample_cmap(cm, g.Ht, g.Wt, tx.x, ty.x);
+        r.x = k * g2.y + cblend * co.x;
+        gr.x = k * g2.z + cblend * co.y;
+        b.x = k * g2.w + cblend * co.z;
+      }
+      if (f1) {
+        const float3 co = sample_cmap(cm, g.Ht, g.Wt, tx.y, ty.y);
+        r.y = k * g2.y + cblend * co.x;
+        gr.y = k * g2.z + cblend * co.y;
+        b.y = k * g2.w + cblend * co.z;
+      }
+    }
+  }
 
   // tile: the CTA's tile; part: which group of warps of the tile the CTA runs
   // (a CTA holds kCtaWarps of the tile's NW warps).
@@ -366,67 +337,68 @@ struct TileWalker {
     lw = threadIdx.x >> 5;
     warp = part * cta_warps + lw;
     lane = threadIdx.x & 31;
-    solid_delta = g.solid_off ? (int)(g.solid_off - g.grid_off) : 0;
     const int tx = tile % g.tilesX, ty = tile / g.tilesX;
     start = __ldg(offs + tile);
     end = __ldg(offs + tile + 1);
-    const int bx = px(tile, g, 0), by = py(tile, g, 0);
+    const int bx = px(tile, g), by = py(tile, g, 0);
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      pxf[p] = (float)(bx + L::ox(p));
-      pyf[p] = (float)(by + L::oy(p));
-      valid[p] = bx + L::ox(p) < g.W && by + L::oy(p) < g.H;
+      pxf[p] = (float)bx;
+      pyf[p] = (float)(by + p * L::kStep);
+      valid[p] = bx < g.W && by + p * L::kStep < g.H;
     }
-    fx0 = (float)(tx * TS + (warp % L::WPR) * L::FW);
-    fx1 = fx0 + (float)(L::FW - 1);
-    fy0 = (float)(ty * TS + (warp / L::WPR) * L::FH);
-    fy1 = fy0 + (float)(L::FH - 1);
-    fcx = fx0 + 0.5f * (float)(L::FW - 1);
-    fcy = fy0 + 0.5f * (float)(L::FH - 1);
+    fcx = (float)(tx * TS + (warp % L::WPR) * L::FW) + 0.5f * (float)(L::FW - 1);
+    fcy = (float)(ty * TS + (warp / L::WPR) * L::FH) + 0.5f * (float)(L::FH - 1);
   }
 
   // Pixel coordinates of pixel p of this thread.
-  __device__ __forceinline__ int px(int tile, const Geom& g, int p) const {
-    return (tile % g.tilesX) * TS + (warp % L::WPR) * L::FW + (lane & 7) + L::ox(p);
+  __device__ __forceinline__ int px(int tile, const Geom& g) const {
+    return (tile % g.tilesX) * TS + (warp % L::WPR) * L::FW + (lane & 7);
   }
   __device__ __forceinline__ int py(int tile, const Geom& g, int p) const {
-    return (tile / g.tilesX) * TS + (warp / L::WPR) * L::FH + (lane >> 3) + L::oy(p);
+    return (tile / g.tilesX) * TS + (warp / L::WPR) * L::FH + (lane >> 3) + p * L::kStep;
   }
 
   // Stages list positions [base, min(base + 32, stop)) into the warp's buffer
-  // w (lane i: position base + i) and returns the chunk's ballots.  With
-  // KEEP_CLEAR, entries the clearance grid rules out stay in `todo` (the
+  // w: lane i tests position base + i, and the survivors' records go to
+  // w[0..n-1].  With KEEP_CLEAR, entries the clearance grid rules out stay (the
   // counting walk checks them).  Out-of-range primitive ids never yield a
-  // fragment (tile_forward.cu:184-185).  my_id: this lane's primitive id.
+  // fragment (tile_forward.cu:184-185).  Compacted records let the walks step
+  // through the buffer by constant offsets instead of searching a bit mask
+  // for each entry, and carry the entry's position and id (2048x2048, N=20000,
+  // FP16 quads: backward walk 319 -> 288 M instructions, 365 -> 348 us, fused
+  // kernel 551 -> 535).  The tests load a record's parts as they need them, and
+  // the survivors' loads are repeated after the ballot: holding the record, or
+  // the next chunk's ids, in registers spills the walk's state (fused 565 us).
   template <bool KEEP_CLEAR>
-  __device__ __forceinline__ ChunkMasks stage(const Geom& g, const PrimInfo* __restrict__ prims,
-                                              const int* __restrict__ idx, const unsigned char* __restrict__ grid,
-                                              int base, int stop, Rec* w, int* my_id) {
-    bool keep = false, inside = false, fast = false, clear = false, solid = false, miss = false;
-    int id = -1;
-    __syncwarp();   // every lane is done with the previous chunk's records
+  __device__ __forceinline__ Chunk stage(const Geom& g, const PrimInfo* __restrict__ prims,
+                                         const int* __restrict__ idx, const unsigned char* __restrict__ grid,
+                                         int base, int stop, Rec* w) const {
+    bool keep = false, miss = false;
+    unsigned flags = 0u;
+    int id = -1, toff = kNoFrag;
     const int pos = base + lane;
     if (pos < stop) {
       id = __ldg(idx + pos);
       if (id >= 0 && id < g.N) {
         const float4* r = reinterpret_cast<const float4*>(prims + id);
         const float4 g0 = __ldg(r);
-        miss = footprint_miss(g0, fx0, fx1, fy0, fy1);
+        miss = footprint_miss(g0, fcx, fcy);
         if (!miss) {
           const float4 q = __ldg(r + 3);
-          const int toff = __float_as_int(q.x);
+          toff = __float_as_int(q.x);
           if (toff != kNoFrag) {
             const float4 g1 = __ldg(r + 1);
+            bool clear = false, solid = false;
             if (kGrid) {
               const unsigned char* cell = grid + __float_as_int(q.y) + grid_cell(g, g0, g1, fcx, fcy);
               const int need = __float_as_int(q.z);
               clear = (int)__ldg(cell) >= need;
-              if (solid_delta != 0) solid = (int)__ldg(cell + solid_delta) >= need;
+              if (g.solid_delta != 0) solid = (int)__ldg(cell + g.solid_delta) >= need;
             }
             keep = KEEP_CLEAR || !clear;
             if (keep) {
-              inside = footprint_inside(g0, fx0, fx1, fy0, fy1);
-              if (inside) {
+              if (footprint_inside(g0, fcx, fcy)) {
                 // texel box of the footprint: centre +- |A| (half extents), plus
                 // 0.05 texel for the rounding of the per-pixel coordinates
                 const float dx = fcx - g0.x, dy = fcy - g0.y;
@@ -434,40 +406,42 @@ struct TileWalker {
                 const float cy = fmaf(g1.z, dx, fmaf(g1.w, dy, g.hy));
                 const float ex = fmaf(fabsf(g1.x), g.fhx, fmaf(fabsf(g1.y), g.fhy, 0.05f));
                 const float ey = fmaf(fabsf(g1.z), g.fhx, fmaf(fabsf(g1.w), g.fhy, 0.05f));
-                fast = cx - ex >= 0.f && cx + ex <= g.wm1 && cy - ey >= 0.f && cy + ey <= g.hm1;
+                const bool fast = cx - ex >= 0.f && cx + ex <= g.wm1 && cy - ey >= 0.f && cy + ey <= g.hm1;
+                flags = kInside | (fast ? kFast | (solid ? kSolid : 0u) : 0u);
               }
-              solid = solid && fast;
-              float4 g2 = __ldg(r + 2);
-              if (half_record(KIND)) {   // FP16 (alpha0, r) and (g, b) pairs
-                const float2 ar = h2f(__float_as_uint(g2.x)), gb = h2f(__float_as_uint(g2.y));
-                g2 = make_float4(ar.x, ar.y, gb.x, gb.y);
-              }
-              w[lane][0] = g0;
-              w[lane][1] = g1;
-              if (kPair) {
-                w[lane][2] = make_float4(g2.x, g2.x, g2.y, g2.y);
-                w[lane][3] = make_float4(g2.z, g2.z, g2.w, g2.w);
-              } else {
-                w[lane][2] = g2;
-              }
-              w[lane][kRec - 1] = q;
+              if (KEEP_CLEAR && clear) flags |= kClear;
             }
           }
         }
-      } else {
-        id = -1;
       }
     }
+    const unsigned todo = __ballot_sync(kFull, keep);
+    __syncwarp();   // every lane is done with the previous chunk's records
+    if (keep) {
+      // reads the record again (L1) rather than holding it across the ballot
+      const float4* r = reinterpret_cast<const float4*>(prims + id);
+      float4* d = w[__popc(todo & ((1u << lane) - 1u))];
+      float4 g2 = __ldg(r + 2);
+      if (half_record(KIND)) {   // FP16 (alpha0, r) and (g, b) pairs
+        const float2 ar = h2f(__float_as_uint(g2.x)), gb = h2f(__float_as_uint(g2.y));
+        g2 = make_float4(ar.x, ar.y, gb.x, gb.y);
+      }
+      d[0] = __ldg(r);
+      d[1] = __ldg(r + 1);
+      d[2] = g2;
+      d[3] = make_float4(__int_as_float(toff), __uint_as_float(flags), __int_as_float(pos - start),
+                         __int_as_float(id));
+    }
     __syncwarp();   // the records are visible to every lane
-    *my_id = id;
-    ChunkMasks m;
-    m.todo = __ballot_sync(kFull, keep);
-    m.inside = __ballot_sync(kFull, inside);
-    m.fast = __ballot_sync(kFull, fast);
-    m.solid = __ballot_sync(kFull, solid && keep);
-    m.clear = KEEP_CLEAR ? __ballot_sync(kFull, clear) : 0u;
-    m.miss = KEEP_CLEAR ? __ballot_sync(kFull, miss) : 0u;
-    return m;
+    Chunk c;
+    c.n = __popc(todo);
+    const unsigned f = lane < c.n ? __float_as_uint(w[lane][3].y) : 0u;
+    c.inside = __ballot_sync(kFull, f & kInside);
+    c.fast = __ballot_sync(kFull, f & kFast);
+    c.solid = __ballot_sync(kFull, f & kSolid);
+    c.clear = KEEP_CLEAR ? __ballot_sync(kFull, f & kClear) : 0u;
+    c.miss = KEEP_CLEAR ? __ballot_sync(kFull, miss) : 0u;
+    return c;
   }
 
   // Adds the warp's 8 per-primitive sums (acc, one set per lane) to dst[0..7]:
@@ -527,15 +501,16 @@ struct TileWalker {
     }
   }
 
-  // Phase 1 of a forward entry for a pixel pair: coordinates and texel loads.
-  __device__ __forceinline__ void pair_issue(const Geom& g, const void* __restrict__ atlas, const Rec* w, int e,
-                                             const ChunkMasks& cm, const bool (&live)[2], PairPre<KIND>& p) const {
-    const int toff = rec_toff(w[e]);
-    const float4 g0 = w[e][0];
-    const float4 g1 = w[e][1];
-    const bool inside = (cm.inside >> e) & 1u;
-    if ((cm.fast >> e) & 1u) pair_prep<L, KIND, true>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, p);
-    else pair_prep<L, KIND, false>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, p);
+  // Phase 1 of a forward entry: coordinates and texel loads of the pixel pair.
+  __device__ __forceinline__ void pair_issue(const Geom& g, const void* __restrict__ atlas, const Rec& r, bool inside,
+                                             bool fast, const bool (&live)[2], PairPre<KIND>& p) const {
+    const int toff = __float_as_int(r[3].x);
+    const float4 g0 = r[0];
+    const float4 g1 = r[1];
+    float2* tx = CB ? &p.tx : nullptr;
+    float2* ty = CB ? &p.ty : nullptr;
+    if (fast) pair_prep<L, KIND, true>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, p, tx, ty);
+    else pair_prep<L, KIND, false>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, p, tx, ty);
   }
 
   // Forward state of a pixel pair.
@@ -545,22 +520,27 @@ struct TileWalker {
     bool live[2];
   };
 
-  // Composites masks m of entry e (fragments f0, f1) onto the pixel pair.
-  // Returns true when every pixel of the warp has stopped (if vote).
-  __device__ __forceinline__ bool pair_over(const Geom& g, const Rec* w, int e, int pos, float2 m, bool f0, bool f1,
-                                            PairFwd& f, bool vote) const {
-    const float4 c0 = w[e][2];
-    const float4 c1 = w[e][3];
-    const float2 a = make_float2(f0 ? c0.x * m.x : 0.f, f1 ? c0.y * m.y : 0.f);
+  // Composites masks m of a staged entry (fragments f0, f1; CB: texel
+  // coordinates tx, ty) onto the pixel pair.  Returns true when every pixel of
+  // the warp has stopped (if vote).
+  __device__ __forceinline__ bool pair_over(const Geom& g, const Rec& r, float2 m, bool f0, bool f1, float2 tx,
+                                            float2 ty, PairFwd& f, bool vote) const {
+    const float4 g2 = r[2];
+    const int pos = __float_as_int(r[3].z);
+    float2 cr, cg, cb;
+    pair_colour(g, g2, CB ? __float_as_int(r[3].w) : 0, tx, ty, f0, f1, cr, cg, cb);
+    const float2 a = make_float2(f0 ? g2.x * m.x : 0.f, f1 ? g2.x * m.y : 0.f);
     const float2 wt = make_float2(f.t.x * a.x, f.t.y * a.y);
-    f.cr = make_float2(fmaf(wt.x, c0.z, f.cr.x), fmaf(wt.y, c0.w, f.cr.y));
-    f.cg = make_float2(fmaf(wt.x, c1.x, f.cg.x), fmaf(wt.y, c1.y, f.cg.y));
-    f.cb = make_float2(fmaf(wt.x, c1.z, f.cb.x), fmaf(wt.y, c1.w, f.cb.y));
+    f.cr = make_float2(fmaf(wt.x, cr.x, f.cr.x), fmaf(wt.y, cr.y, f.cr.y));
+    f.cg = make_float2(fmaf(wt.x, cg.x, f.cg.x), fmaf(wt.y, cg.y, f.cg.y));
+    f.cb = make_float2(fmaf(wt.x, cb.x, f.cb.x), fmaf(wt.y, cb.y, f.cb.y));
     f.tl.x = f0 ? f.t.x : f.tl.x;
     f.tl.y = f1 ? f.t.y : f.tl.y;
     f.lp0 = f0 ? pos : f.lp0;
     f.lp1 = f1 ? pos : f.lp1;
-    // T (1 - a) as in forward(), saturated per pixel (no packed form)
+    // T (1 - a); 0 when a > 1 (alpha_max > 1).  a >= 0 (alpha_max >= 0), so
+    // T stays <= 1 and saturating equals max(., 0), NaN included (per pixel:
+    // saturation has no packed form).
     f.t.x = __saturatef(fmaf(-f.t.x, a.x, f.t.x));
     f.t.y = __saturatef(fmaf(-f.t.y, a.y, f.t.y));
     f.live[0] = f.live[0] && !(f.t.x < g.t_stop);
@@ -569,27 +549,26 @@ struct TileWalker {
   }
 
   // Phase 2 of a forward entry: blend the loaded texels and composite.
-  __device__ __forceinline__ bool pair_composite(const Geom& g, const Rec* w, int e, int pos, const PairPre<KIND>& p,
-                                                 PairFwd& f, bool vote = true) const {
+  __device__ __forceinline__ bool pair_composite(const Geom& g, const Rec& r, const PairPre<KIND>& p, PairFwd& f,
+                                                 bool vote) const {
     PairSample s;
     pair_unpack<KIND>(g, p, s);
     const float2 m = pair_blend<false, false>(g, s, nullptr, nullptr);
     // a pixel may have stopped since the loads were issued
     const bool f0 = s.ok0 && f.live[0] && m.x > 1e-6f, f1 = s.ok1 && f.live[1] && m.y > 1e-6f;
-    return pair_over(g, w, e, pos, m, f0, f1, f, vote);
+    return pair_over(g, r, m, f0, f1, p.tx, p.ty, f, vote);
   }
 
-  // Forward walk of the pixel-pair form: the walk of forward() with both
-  // pixels' sampling, blending and compositing as packed pairs.  Entries that
-  // are sampled go two at a time: the texel loads of both are issued before
-  // either is composited, so their latencies overlap.  Solid entries (mask 1 on
-  // the whole footprint) are composited straight from their record: they need
-  // a third of the instructions of a sampled one, and at 2048x2048, N=20000,
-  // 256x256 bitmaps with soft rims they are 44 % of the entries (forward walk
-  // 244 -> 218 us, backward 432 -> 361, fused kernel 637 -> 548).
-  __device__ __forceinline__ void forward_pair(const Geom& g, const PrimInfo* __restrict__ prims,
-                                               const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
-                                               float (&C)[2][3], float (&T)[2], float (&Tl)[2], int (&lp)[2]) {
+  // Forward walk.  Entries that are sampled go two at a time: the texel loads
+  // of both are issued before either is composited, so their latencies
+  // overlap.  Solid entries (mask 1 on the whole footprint) are composited
+  // straight from their record: they need a third of the instructions of a
+  // sampled one, and at 2048x2048, N=20000, 256x256 bitmaps with soft rims they
+  // are 44 % of the entries (forward walk 244 -> 218 us, backward 432 -> 361,
+  // fused kernel 637 -> 548).
+  __device__ __forceinline__ void forward(const Geom& g, const PrimInfo* __restrict__ prims,
+                                          const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
+                                          float (&C)[2][3], float (&T)[2], float (&Tl)[2], int (&lp)[2]) const {
     const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
     PairFwd f;
     f.cr = f.cg = f.cb = make_float2(0.f, 0.f);
@@ -599,29 +578,28 @@ struct TileWalker {
     f.live[1] = valid[1];
     bool warp_done = __all_sync(kFull, !f.live[0] && !f.live[1]);
     for (int base = start; base < end && !warp_done; base += kChunk) {
-      int my_id;
-      const ChunkMasks cm = stage<false>(g, prims, idx, grid, base, end, w, &my_id);
-      unsigned todo = cm.todo;
-      while (todo) {
-        const int e1 = __ffs(todo) - 1;
-        todo &= todo - 1;
-        if ((cm.solid >> e1) & 1u) {   // every live pixel of the warp has mask 1: nothing to sample
-          if (pair_over(g, w, e1, base - start + e1, make_float2(1.f, 1.f), f.live[0], f.live[1], f, true)) {
+      const Chunk c = stage<false>(g, prims, idx, grid, base, end, w);
+      for (int j = 0; j < c.n;) {
+        if ((c.solid >> j) & 1u) {   // every live pixel of the warp has mask 1: nothing to sample
+          float2 tx, ty;
+          if constexpr (CB) pair_coords(g, w[j], tx, ty);
+          if (pair_over(g, w[j], make_float2(1.f, 1.f), f.live[0], f.live[1], tx, ty, f, true)) {
             warp_done = true;
             break;
           }
+          ++j;
           continue;
         }
-        const bool two = todo != 0 && !((cm.solid >> (__ffs(todo) - 1)) & 1u);
-        const int e2 = two ? __ffs(todo) - 1 : e1;   // e1 again when no sampled entry follows it
-        if (two) todo &= todo - 1;
+        const bool two = j + 1 < c.n && !((c.solid >> (j + 1)) & 1u);
+        const int j2 = two ? j + 1 : j;   // j again when no sampled entry follows it
         PairPre<KIND> p1, p2;
-        pair_issue(g, atlas, w, e1, cm, f.live, p1);
-        pair_issue(g, atlas, w, e2, cm, f.live, p2);
-        // one termination vote per pair: a pixel that stops at e1 has live
-        // false, so e2 composites nothing for it
-        if (pair_composite(g, w, e1, base - start + e1, p1, f, !two)) { warp_done = true; break; }
-        if (two && pair_composite(g, w, e2, base - start + e2, p2, f)) { warp_done = true; break; }
+        pair_issue(g, atlas, w[j], (c.inside >> j) & 1u, (c.fast >> j) & 1u, f.live, p1);
+        pair_issue(g, atlas, w[j2], (c.inside >> j2) & 1u, (c.fast >> j2) & 1u, f.live, p2);
+        // one termination vote per pair: a pixel that stops at the first has live
+        // false, so the second composites nothing for it
+        if (pair_composite(g, w[j], p1, f, !two)) { warp_done = true; break; }
+        if (two && pair_composite(g, w[j2], p2, f, true)) { warp_done = true; break; }
+        j = j2 + 1;
       }
     }
     C[0][0] = f.cr.x; C[0][1] = f.cg.x; C[0][2] = f.cb.x;
@@ -631,45 +609,58 @@ struct TileWalker {
     lp[0] = f.lp0; lp[1] = f.lp1;
   }
 
-  // Reverse walk of the pixel-pair form (the walk of backward() with both
-  // pixels' arithmetic as packed pairs; each per-primitive sum adds the two
-  // pixels' terms before the warp reduction).
-  __device__ __forceinline__ void backward_pair(const Geom& g, const PrimInfo* __restrict__ prims,
-                                                const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
-                                                const float (&gC)[2][3], const float (&gA)[2], float (&Ts)[2],
-                                                const int (&lp)[2], double* __restrict__ gacc) {
+  // Texel coordinates of the pixel pair alone (solid entries of a colour-map walk).
+  __device__ __forceinline__ void pair_coords(const Geom& g, const Rec& r, float2& tx, float2& ty) const {
+    const bool live[2] = {true, true};
+    Coord s[2];
+    entry_coords<L, true>(g, r[0], r[1], true, pxf, pyf, live, s);
+    tx = make_float2(s[0].tx, s[1].tx);
+    ty = make_float2(s[0].ty, s[1].ty);
+  }
+
+  // Reverse walk.  gC/gA: upstream gradients per pixel; Ts: T entering each
+  // pixel's last contributor (lp).  H = gC . R and B = prod(1 - a) over the
+  // fragments behind the current one, where R is their colour composited from
+  // T = 1; both obey X_{k-1} = (1 - a_k) X_k + a_k x_k, so
+  // dL/da_k = T_k (gC.c_k - H + gA B).  Per entry the warp reduces its
+  // per-primitive partial sums (each lane's two pixels added first) and lanes
+  // 0..7 add them to gacc (N,8) f64 (layout documented at finalize_kernel).
+  __device__ __forceinline__ void backward(const Geom& g, const PrimInfo* __restrict__ prims,
+                                           const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
+                                           const float (&gC)[2][3], const float (&gA)[2], const float (&Ts)[2],
+                                           const int (&lp)[2], double* __restrict__ gacc) const {
     const int warp_max = __reduce_max_sync(kFull, max(lp[0], lp[1]));
     if (warp_max < 0) return;
     const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
+    // sum index that lane l < 8 holds after the recursive-halving reduction
     const int kidx = 4 * (lane & 1) + 2 * ((lane >> 1) & 1) + ((lane >> 2) & 1);
     const float2 gcr = make_float2(gC[0][0], gC[1][0]), gcg = make_float2(gC[0][1], gC[1][1]),
                  gcb = make_float2(gC[0][2], gC[1][2]), ga = make_float2(gA[0], gA[1]);
     float2 h = make_float2(0.f, 0.f), bt = make_float2(1.f, 1.f), ts = make_float2(Ts[0], Ts[1]);
     for (int cb = (warp_max / kChunk) * kChunk; cb >= 0; cb -= kChunk) {
-      int my_id;
-      const ChunkMasks cm = stage<false>(g, prims, idx, grid, start + cb, start + warp_max + 1, w, &my_id);
-      unsigned todo = cm.todo;
-      while (todo) {
-        const int e = 31 - __clz(todo);
-        todo &= ~(1u << e);
-        const int pos = cb + e;
-        const int id = __shfl_sync(kFull, my_id, e);
-        const float4 g0 = w[e][0];
-        const float4 g1 = w[e][1];
-        const float4 c0 = w[e][2];
-        const float4 c1 = w[e][3];
-        const int toff = rec_toff(w[e]);
+      const Chunk c = stage<false>(g, prims, idx, grid, start + cb, start + warp_max + 1, w);
+      for (int j = c.n - 1; j >= 0; --j) {
+        const Rec& r = w[j];
+        const float4 g2 = r[2];
+        const float4 q = r[3];
+        const int pos = __float_as_int(q.z);
+        const int id = __float_as_int(q.w);
         const bool live[2] = {pos <= lp[0], pos <= lp[1]};
-        if ((cm.solid >> e) & 1u) {
+        float2 col_r, col_g, col_b;
+        if ((c.solid >> j) & 1u) {
           // mask 1 with gradient 0 on the whole footprint: the operations below
           // with m = 1 and gx = gy = 0, which leave the colour and opacity sums
-          const float2 a = make_float2(live[0] ? c0.x : 0.f, live[1] ? c0.y : 0.f);
-          const float2 om = make_float2(__saturatef(1.f - a.x), __saturatef(1.f - a.y));
-          const float2 tk = make_float2((pos == lp[0]) ? ts.x : __fdividef(ts.x, om.x),
-                                        (pos == lp[1]) ? ts.y : __fdividef(ts.y, om.y));
+          float2 tx, ty;
+          if constexpr (CB) pair_coords(g, r, tx, ty);
+          pair_colour(g, g2, id, tx, ty, live[0], live[1], col_r, col_g, col_b);
+          const float om1 = __saturatef(1.f - g2.x);
+          const float2 a = make_float2(live[0] ? g2.x : 0.f, live[1] ? g2.x : 0.f);
+          const float2 om = make_float2(live[0] ? om1 : 1.f, live[1] ? om1 : 1.f);
+          const float2 td = make_float2(div_unit(ts.x, om1), div_unit(ts.y, om1));
+          const float2 tk = make_float2(pos < lp[0] ? td.x : ts.x, pos < lp[1] ? td.y : ts.y);
           ts = tk;
-          const float2 gcc = make_float2(fmaf(gcr.x, c0.z, fmaf(gcg.x, c1.x, gcb.x * c1.z)),
-                                         fmaf(gcr.y, c0.w, fmaf(gcg.y, c1.y, gcb.y * c1.w)));
+          const float2 gcc = make_float2(fmaf(gcr.x, col_r.x, fmaf(gcg.x, col_g.x, gcb.x * col_b.x)),
+                                         fmaf(gcr.y, col_r.y, fmaf(gcg.y, col_g.y, gcb.y * col_b.y)));
           float2 dlda;
           if (kQuad) dlda = make_float2(tk.x * fmaf(ga.x, bt.x, gcc.x - h.x), tk.y * fmaf(ga.y, bt.y, gcc.y - h.y));
           else dlda = mul2(tk, fma2(ga, bt, sub2(g, gcc, h)));
@@ -685,25 +676,32 @@ struct TileWalker {
           continue;
         }
         PairSample s;
-        const bool inside = (cm.inside >> e) & 1u;
-        if ((cm.fast >> e) & 1u) pair_sample<L, KIND, true>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, s);
-        else pair_sample<L, KIND, false>(g, atlas, toff, g0, g1, inside, pxf, pyf, live, s);
+        const bool inside = (c.inside >> j) & 1u;
+        if ((c.fast >> j) & 1u)
+          pair_sample<L, KIND, true>(g, atlas, __float_as_int(q.x), r[0], r[1], inside, pxf, pyf, live, s);
+        else
+          pair_sample<L, KIND, false>(g, atlas, __float_as_int(q.x), r[0], r[1], inside, pxf, pyf, live, s);
         float2 gx, gy;
         const float2 m = pair_blend<true>(g, s, &gx, &gy);
         const float2 tx = s.tx, ty = s.ty;
         const bool f0 = s.ok0 && m.x > 1e-6f, f1 = s.ok1 && m.y > 1e-6f;
-        float2 a = make_float2(f0 ? c0.x * m.x : 0.f, f1 ? c0.y * m.y : 0.f);
-        const float2 om = make_float2(__saturatef(1.f - a.x), __saturatef(1.f - a.y));
-        // T entering this fragment (see backward())
-        const float2 tk = make_float2((pos == lp[0]) ? ts.x : __fdividef(ts.x, om.x),
-                                      (pos == lp[1]) ? ts.y : __fdividef(ts.y, om.y));
+        pair_colour(g, g2, id, tx, ty, f0, f1, col_r, col_g, col_b);
+        const float2 a = make_float2(f0 ? g2.x * m.x : 0.f, f1 ? g2.x * m.y : 0.f);
+        const float2 om = make_float2(__saturatef(1.f - a.x), __saturatef(1.f - a.y));   // max(1 - a, 0) for a >= 0
+        // T entering this fragment: stored for the last contributor, else undo
+        // the forward product (om >= t_stop > 0 for every earlier fragment, so the
+        // approximate division is well conditioned; om = 1 leaves ts unchanged
+        // where there is no fragment)
+        const float2 tk = make_float2((pos == lp[0]) ? ts.x : div_unit(ts.x, om.x),
+                                      (pos == lp[1]) ? ts.y : div_unit(ts.y, om.y));
         ts = tk;
-        const float2 col_r = make_float2(c0.z, c0.w), col_g = make_float2(c1.x, c1.y),
-                     col_b = make_float2(c1.z, c1.w);
         const float2 gcc = make_float2(fmaf(gcr.x, col_r.x, fmaf(gcg.x, col_g.x, gcb.x * col_b.x)),
                                        fmaf(gcr.y, col_r.y, fmaf(gcg.y, col_g.y, gcb.y * col_b.y)));
         // dL/da and the mask-gradient terms: scalar for the quad layouts, packed
-        // for the others (each measured faster on B200)
+        // for the others (each measured faster on B200).  A pixel without a
+        // fragment contributes nothing: a = 0 zeroes its colour and opacity terms,
+        // and its mask gradient (from a redirected texel, possibly NaN) is
+        // replaced by 0 rather than multiplied by 0.
         float2 dlda, u, v;
         if (kQuad) {
           dlda = make_float2(tk.x * fmaf(ga.x, bt.x, gcc.x - h.x), tk.y * fmaf(ga.y, bt.y, gcc.y - h.y));
@@ -720,12 +718,12 @@ struct TileWalker {
         acc[0] = u.x + u.y;
         acc[1] = v.x + v.y;
         {
-          const float2 r = fma2(u, ex, mul2(v, ey));
-          acc[2] = r.x + r.y;
+          const float2 e = fma2(u, ex, mul2(v, ey));
+          acc[2] = e.x + e.y;
         }
         {
-          const float2 r = fma2(mul2(u, g.rxy2), ey, mul2(mul2(v, g.nryx2), ex));
-          acc[3] = r.x + r.y;
+          const float2 e = fma2(mul2(u, g.rxy2), ey, mul2(mul2(v, g.nryx2), ex));
+          acc[3] = e.x + e.y;
         }
         acc[4] = fmaf(gcr.y, wt.y, gcr.x * wt.x);
         acc[5] = fmaf(gcg.y, wt.y, gcg.x * wt.x);
@@ -736,217 +734,68 @@ struct TileWalker {
         if (__any_sync(kFull, f0 || f1)) warp_add(acc, kidx, gacc + (size_t)id * 8);
       }
     }
-    Ts[0] = ts.x;
-    Ts[1] = ts.y;
   }
 
-  // Forward walk.  STATS: counts (pixel, primitive) pairs that pass the cull
+  // Counting walk (diagnostics): (pixel, primitive) pairs that pass the cull
   // and fragments composited, both before termination, plus walk statistics;
   // it evaluates the clearance-grid test without skipping and counts the
   // warp entries it would skip and, among them, those with a fragment (a
   // correct grid gives 0).
-  template <bool STATS = false>
-  __device__ __forceinline__ void forward(const Geom& g, const PrimInfo* __restrict__ prims,
-                                          const void* __restrict__ atlas, const int* __restrict__ idx,
-                                          Rec* w,
-                                          float (&C)[NP][3], float (&T)[NP], float (&Tl)[NP], int (&lp)[NP],
-                                          unsigned long long* cnt = nullptr) {
-    if constexpr (kPair && !STATS) {
-      forward_pair(g, prims, atlas, idx, w, C, T, Tl, lp);
-      return;
-    }
+  __device__ __forceinline__ void count(const Geom& g, const PrimInfo* __restrict__ prims,
+                                        const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
+                                        unsigned long long* cnt) const {
+    const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
     unsigned long long n_cand = 0, n_frag = 0, n_went = 0, n_slots = 0, n_miss = 0, n_empty = 0, n_clear = 0,
                        n_bad = 0;
-    unsigned n_depth[NP];
-    const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
-    bool live[NP];
-    bool all_done = true;
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      C[p][0] = C[p][1] = C[p][2] = 0.f;
-      T[p] = 1.f; Tl[p] = 1.f; lp[p] = -1;
-      live[p] = valid[p];
-      n_depth[p] = 0;
-      all_done = all_done && !live[p];
-    }
-    bool warp_done = __all_sync(kFull, all_done);
+    unsigned n_depth[NP] = {0u, 0u};
+    float T[NP] = {1.f, 1.f};
+    bool live[NP] = {valid[0], valid[1]};
+    bool warp_done = __all_sync(kFull, !live[0] && !live[1]);
     for (int base = start; base < end && !warp_done; base += kChunk) {
-      int my_id;
-      const ChunkMasks cm = stage<STATS>(g, prims, idx, grid, base, end, w, &my_id);
-      unsigned todo = cm.todo;
-      if (STATS) n_miss += __popc(cm.miss);
-      while (todo) {
-        const int e = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const float4 g0 = w[e][0];
-        const float4 g1 = w[e][1];
-        const float4 g2 = rec_g2(w[e]);
-        const int toff = rec_toff(w[e]);
-        const int pos = base - start + e;
-        const bool clear = (cm.clear >> e) & 1u;
-        if (STATS) {
-          ++n_went;
-          n_clear += clear;
+      const Chunk c = stage<true>(g, prims, idx, grid, base, end, w);
+      n_miss += __popc(c.miss);
+      for (int j = 0; j < c.n; ++j) {
+        const float4 g0 = w[j][0];
+        const float op = w[j][2].x;
+        const bool clear = (c.clear >> j) & 1u;
+        ++n_went;
+        n_clear += clear;
 #pragma unroll
-          for (int p = 0; p < NP; ++p) n_slots += __popc(__ballot_sync(kFull, live[p]));
-        }
-        Sample s[NP];
-        float m[NP];
-        entry_sample<NP, L, KIND>(g, atlas, toff, g0, g1, (cm.inside >> e) & 1u, (cm.fast >> e) & 1u, pxf, pyf,
-                                  live, s);
+        for (int p = 0; p < NP; ++p) n_slots += __popc(__ballot_sync(kFull, live[p]));
+        PairPre<KIND> pre;
+        PairSample s;
+        pair_issue(g, atlas, w[j], (c.inside >> j) & 1u, (c.fast >> j) & 1u, live, pre);
+        pair_unpack<KIND>(g, pre, s);
+        const float2 m2 = pair_blend<false, false>(g, s, nullptr, nullptr);
+        const float m[NP] = {m2.x, m2.y};
+        const bool ok[NP] = {s.ok0, s.ok1};
+        const bool anyf = __any_sync(kFull, (ok[0] && m[0] > 1e-6f) || (ok[1] && m[1] > 1e-6f));
+        n_empty += !anyf;
+        n_bad += clear && anyf;
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-          m[p] = blend<false>(s[p], nullptr, nullptr);
-          if (STATS) {
-            const bool c = live[p] && !(fabsf(pxf[p] - g0.x) > g0.z || fabsf(pyf[p] - g0.y) > g0.w);
-            n_cand += c;
-          }
-        }
-        if (STATS) {
-          bool anyf = false;
-#pragma unroll
-          for (int p = 0; p < NP; ++p) anyf = anyf || (s[p].ok && m[p] > 1e-6f);
-          anyf = __any_sync(kFull, anyf);
-          n_empty += !anyf;
-          n_bad += clear && anyf;
-        }
-        bool local_done = true;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const bool frag = s[p].ok && m[p] > 1e-6f;
-          if (STATS) { n_frag += frag; n_depth[p] += frag; }
-          const float a = frag ? g2.x * m[p] : 0.f;
-          const float wt = T[p] * a;
-          if (CB) {
-            const float3 col = frag_colour(g, g2, __shfl_sync(kFull, my_id, e), s[p]);
-            C[p][0] = fmaf(wt, col.x, C[p][0]);
-            C[p][1] = fmaf(wt, col.y, C[p][1]);
-            C[p][2] = fmaf(wt, col.z, C[p][2]);
-          } else {
-            C[p][0] = fmaf(wt, g2.y, C[p][0]);
-            C[p][1] = fmaf(wt, g2.z, C[p][1]);
-            C[p][2] = fmaf(wt, g2.w, C[p][2]);
-          }
-          Tl[p] = frag ? T[p] : Tl[p];
-          lp[p] = frag ? pos : lp[p];
-          // T (1 - a); 0 when a > 1 (alpha_max > 1).  a >= 0 (alpha_max >= 0), so
-          // T stays <= 1 and saturating equals max(., 0), NaN included.
+          n_cand += live[p] && !(fabsf(pxf[p] - g0.x) > g0.z || fabsf(pyf[p] - g0.y) > g0.w);
+          const bool frag = ok[p] && m[p] > 1e-6f;
+          n_frag += frag;
+          n_depth[p] += frag;
+          const float a = frag ? op * m[p] : 0.f;
           T[p] = __saturatef(fmaf(-T[p], a, T[p]));
           live[p] = live[p] && !(T[p] < g.t_stop);
-          local_done = local_done && !live[p];
         }
-        if (__all_sync(kFull, local_done)) { warp_done = true; break; }
+        if (__all_sync(kFull, !live[0] && !live[1])) { warp_done = true; break; }
       }
     }
-    if (STATS) {
-      atomicAdd(cnt + 0, n_cand);
-      atomicAdd(cnt + 1, n_frag);
-      unsigned dmax = 0;
-#pragma unroll
-      for (int p = 0; p < NP; ++p) dmax = max(dmax, n_depth[p]);
-      dmax = __reduce_max_sync(kFull, dmax);
-      if (lane == 0) {
-        atomicAdd(cnt + 3, n_went);
-        atomicAdd(cnt + 4, n_slots);
-        atomicAdd(cnt + 5, n_miss);
-        atomicMax(cnt + 6, (unsigned long long)dmax);
-        atomicAdd(cnt + 7, n_empty);
-        atomicAdd(cnt + 8, n_clear);
-        atomicAdd(cnt + 9, n_bad);
-      }
-    }
-  }
-
-  // Reverse walk.  gC/gA: upstream gradients per pixel; Ts: on entry the T
-  // entering each pixel's last contributor (lp).  Per entry the warp reduces
-  // its per-primitive partial sums and lanes 0..7 add them to gacc (N,8) f64
-  // (layout documented at finalize_kernel).
-  __device__ __forceinline__ void backward(const Geom& g, const PrimInfo* __restrict__ prims,
-                                           const void* __restrict__ atlas, const int* __restrict__ idx,
-                                           Rec* w, const float (&gC)[NP][3], const float (&gA)[NP],
-                                           float (&Ts)[NP], const int (&lp)[NP], double* __restrict__ gacc) {
-    if constexpr (kPair) {
-      backward_pair(g, prims, atlas, idx, w, gC, gA, Ts, lp, gacc);
-      return;
-    }
-    int my_max = -1;
-#pragma unroll
-    for (int p = 0; p < NP; ++p) my_max = max(my_max, lp[p]);
-    const int warp_max = __reduce_max_sync(kFull, my_max);
-    if (warp_max < 0) return;
-    const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
-    // sum index that lane l < 8 holds after the recursive-halving reduction
-    const int kidx = 4 * (lane & 1) + 2 * ((lane >> 1) & 1) + ((lane >> 2) & 1);
-
-    // H = gC . R and B = prod(1 - a) over the fragments behind the current
-    // one, where R is their colour composited from T = 1; both obey
-    // X_{k-1} = (1 - a_k) X_k + a_k x_k, so dL/da_k = T_k (gC.c_k - H + gA B).
-    float H[NP], B[NP];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      H[p] = 0.f;
-      B[p] = 1.f;
-    }
-    for (int cb = (warp_max / kChunk) * kChunk; cb >= 0; cb -= kChunk) {
-      int my_id;
-      const ChunkMasks cm = stage<false>(g, prims, idx, grid, start + cb, start + warp_max + 1, w, &my_id);
-      unsigned todo = cm.todo;
-      while (todo) {
-        const int e = 31 - __clz(todo);
-        todo &= ~(1u << e);
-        const int pos = cb + e;
-        const int id = __shfl_sync(kFull, my_id, e);
-        const float4 g0 = w[e][0];
-        const float4 g1 = w[e][1];
-        const float4 g2 = rec_g2(w[e]);
-        const int toff = rec_toff(w[e]);
-        float acc[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = 0.f;
-        bool any = false;
-        bool live[NP];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) live[p] = pos <= lp[p];
-        Sample s[NP];
-        float m[NP], gx[NP], gy[NP];
-        entry_sample<NP, L, KIND>(g, atlas, toff, g0, g1, (cm.inside >> e) & 1u, (cm.fast >> e) & 1u, pxf, pyf,
-                                  live, s);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) m[p] = blend<true>(s[p], &gx[p], &gy[p]);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const bool frag = s[p].ok && m[p] > 1e-6f;
-          const float a = frag ? g2.x * m[p] : 0.f;
-          const float om = __saturatef(1.f - a);   // max(1 - a, 0) for a >= 0
-          // T entering this fragment: stored for the last contributor, else
-          // undo the forward product (om >= t_stop > 0 for every earlier
-          // fragment, so the fast division is well conditioned; om = 1 and
-          // Ts is unchanged when there is no fragment).
-          const float Tk = (pos == lp[p]) ? Ts[p] : __fdividef(Ts[p], om);
-          Ts[p] = Tk;
-          const float3 col = frag_colour(g, g2, id, s[p]);
-          const float gCc = fmaf(gC[p][0], col.x, fmaf(gC[p][1], col.y, gC[p][2] * col.z));
-          // a pixel without a fragment contributes nothing: a = 0 zeroes its colour
-          // and opacity terms, and its mask gradient (from a redirected texel,
-          // possibly NaN) is replaced by 0 rather than multiplied by 0
-          const float dLda = Tk * (gCc - H[p] + gA[p] * B[p]);
-          const float u = dLda * (frag ? gx[p] : 0.f), v = dLda * (frag ? gy[p] : 0.f);
-          const float ex = s[p].tx - g.hx, ey = s[p].ty - g.hy;
-          acc[0] += u;
-          acc[1] += v;
-          acc[2] = fmaf(u, ex, fmaf(v, ey, acc[2]));
-          acc[3] = fmaf(u * g.rxy, ey, fmaf(-v * g.ryx, ex, acc[3]));
-          const float wt = a * Tk;
-          acc[4] = fmaf(gC[p][0], wt, acc[4]);
-          acc[5] = fmaf(gC[p][1], wt, acc[5]);
-          acc[6] = fmaf(gC[p][2], wt, acc[6]);
-          acc[7] = fmaf(dLda, a, acc[7]);
-          H[p] = fmaf(om, H[p], a * gCc);
-          B[p] *= om;
-          any = any || frag;
-        }
-        if (__any_sync(kFull, any)) warp_add(acc, kidx, gacc + (size_t)id * 8);
-      }
+    atomicAdd(cnt + 0, n_cand);
+    atomicAdd(cnt + 1, n_frag);
+    const unsigned dmax = __reduce_max_sync(kFull, max(n_depth[0], n_depth[1]));
+    if (lane == 0) {
+      atomicAdd(cnt + 3, n_went);
+      atomicAdd(cnt + 4, n_slots);
+      atomicAdd(cnt + 5, n_miss);
+      atomicMax(cnt + 6, (unsigned long long)dmax);
+      atomicAdd(cnt + 7, n_empty);
+      atomicAdd(cnt + 8, n_clear);
+      atomicAdd(cnt + 9, n_bad);
     }
   }
 };
@@ -968,7 +817,7 @@ struct TileWalker {
 #ifndef DBMP_WARPS_PER_SM_F32
 #define DBMP_WARPS_PER_SM_F32 32
 #endif
-template <int TS> constexpr int kTileWarps() { return Layout<TS, DefaultNP<TS>::v>::NW; }
+template <int TS> constexpr int kTileWarps() { return Layout<TS>::NW; }
 template <int TS> constexpr int kCtaWarps() {
   return kTileWarps<TS>() < DBMP_CTA_WARPS ? kTileWarps<TS>() : DBMP_CTA_WARPS;
 }
@@ -986,9 +835,9 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
     const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
     long long idx_stride, long long cmap_stride) {
-  constexpr int NP = DefaultNP<TS>::v;
-  using TW = TileWalker<TS, NP, KIND, CB>;
-  __shared__ typename TW::Rec s_pi[kCtaWarps<TS>()][kChunk];
+  constexpr int NP = 2;
+  using TW = TileWalker<TS, KIND, CB>;
+  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
   // a batch of candidates is one grid over all their tiles: candidate b's
   // records, lists and images follow candidate b-1's
   const int gt = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
@@ -1008,7 +857,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     if (!tw.valid[p]) continue;
-    const size_t q = (size_t)tw.py(tile, g, p) * g.W + tw.px(tile, g, p);
+    const size_t q = (size_t)tw.py(tile, g, p) * g.W + tw.px(tile, g);
     out_color[3 * q + 0] = C[p][0];
     out_color[3 * q + 1] = C[p][1];
     out_color[3 * q + 2] = C[p][2];
@@ -1026,15 +875,12 @@ __global__ void __launch_bounds__(kThreadsOf<TS>()) count_kernel(Geom g, const P
                                                                  const int* __restrict__ offs,
                                                                  const int* __restrict__ idx,
                                                                  unsigned long long* __restrict__ cnt) {
-  constexpr int NP = DefaultNP<TS>::v;
-  using TW = TileWalker<TS, NP, KIND>;
-  __shared__ typename TW::Rec s_pi[kCtaWarps<TS>()][kChunk];
+  using TW = TileWalker<TS, KIND>;
+  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
   TW tw;
   const int tile = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
   tw.init(g, tile, part, kCtaWarps<TS>(), offs);
-  float C[NP][3], T[NP], Tl[NP];
-  int lp[NP];
-  tw.template forward<true>(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp, cnt);
+  tw.count(g, prims, atlas, idx, s_pi[tw.lw], cnt);
   if (threadIdx.x == 0 && part == 0) atomicAdd(cnt + 2, (unsigned long long)(tw.end - tw.start));
 }
 
@@ -1044,9 +890,9 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
     const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
     const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
     const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride) {
-  constexpr int NP = DefaultNP<TS>::v;
-  using TW = TileWalker<TS, NP, KIND, CB>;
-  __shared__ typename TW::Rec s_pi[kCtaWarps<TS>()][kChunk];
+  constexpr int NP = 2;
+  using TW = TileWalker<TS, KIND, CB>;
+  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
   const int gt = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;     // candidate and tile (see forward_kernel)
   const size_t pix = (size_t)b * g.H * g.W;
@@ -1065,7 +911,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     if (tw.valid[p]) {
-      const size_t q = (size_t)tw.py(tile, g, p) * g.W + tw.px(tile, g, p);
+      const size_t q = (size_t)tw.py(tile, g, p) * g.W + tw.px(tile, g);
       gC[p][0] = grad_color[3 * q + 0];
       gC[p][1] = grad_color[3 * q + 1];
       gC[p][2] = grad_color[3 * q + 2];
@@ -1139,9 +985,9 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fu
     float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
     const int* __restrict__ skip_flag) {
   if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
-  constexpr int NP = DefaultNP<TS>::v;
-  using TW = TileWalker<TS, NP, KIND>;
-  __shared__ typename TW::Rec s_pi[kCtaWarps<TS>()][kChunk];
+  constexpr int NP = 2;
+  using TW = TileWalker<TS, KIND>;
+  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
   __shared__ float s_loss[kCtaWarps<TS>()];
   __shared__ unsigned s_arrived;
   if (threadIdx.x == 0) s_arrived = 0u;
@@ -1159,7 +1005,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fu
     gA[p] = 0.f;
     gC[p][0] = gC[p][1] = gC[p][2] = 0.f;
     if (!tw.valid[p]) continue;
-    const size_t q = (size_t)tw.py(tile, g, p) * g.W + tw.px(tile, g, p);
+    const size_t q = (size_t)tw.py(tile, g, p) * g.W + tw.px(tile, g);
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) {
       const float bg = background ? background[3 * q + ch] : 0.f;
