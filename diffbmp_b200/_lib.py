@@ -64,6 +64,8 @@ SIGNATURES = {
     "dbmp_atlas_extended_bytes": (_sz, [_i, _i, _i, _i]),
     "dbmp_atlas_pack_extended": (_i, [_vp, _i, _i, _i, _i, _vp, _vp]),
     "dbmp_bin_workspace_bytes": (_sz, [_CP, _ll]),
+    "dbmp_bin_batch_workspace_bytes": (_sz, [_CP, _i]),
+    "dbmp_bin_batch": (_i, [_CP, _i] + [_vp] * 6 + [_ll] + [_vp] * 4 + [_ll, _ll, _vp, _vp, _sz, _vp]),
     "dbmp_prim_info_bytes": (_sz, [_i]),
     "dbmp_prepare": (_i, [_CP, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "dbmp_bin": (_i, [_CP, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _sz, _vp]),

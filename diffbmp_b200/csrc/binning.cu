@@ -147,11 +147,24 @@ __device__ __forceinline__ int2 tile_span_cull(float m, float h, int ts, int ext
   return make_int2(a / ts, b / ts);
 }
 
+// blockIdx.y: the candidate of a batch, whose inputs and outputs follow those
+// of the one before (sel: sel_stride apart).  row_total (tilesY per candidate)
+// is zeroed for counts_kernel.
 __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const float* __restrict__ radii,
                                const float* __restrict__ rot, const float* __restrict__ opac,
-                               const float* __restrict__ colors, const int* __restrict__ sel,
+                               const float* __restrict__ colors, const int* __restrict__ sel, long long sel_stride,
                                const float* __restrict__ tbbox, int bin_mode, PrimInfo* __restrict__ out,
-                               int4* __restrict__ rects, int* __restrict__ diff, int span) {
+                               int4* __restrict__ rects, unsigned long long* __restrict__ row_total) {
+  grid_dependency();
+  const size_t b = blockIdx.y, bn = b * g.N;
+  means2D += 2 * bn; radii += bn; rot += bn; opac += bn; colors += 3 * bn;
+  sel += b * sel_stride;
+  out += bn;
+  if (rects != nullptr) {
+    rects += bn;
+    if (blockIdx.x == 0)
+      for (int i = threadIdx.x; i < g.tilesY; i += blockDim.x) row_total[b * g.tilesY + i] = 0ull;
+  }
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= g.N) return;
   const float mx = means2D[2 * n], my = means2D[2 * n + 1];
@@ -226,34 +239,29 @@ __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const 
     }
   }
   rects[n] = make_int4(sx.x, sx.y, sy.x, sy.y);
-  if (diff != nullptr && sx.x <= sx.y && sy.x <= sy.y) {
-    // the rectangle's corners in its slice's 2-D difference array of
-    // (tilesY+1) x (tilesX+1) counters; its 2-D prefix sum is the number of
-    // the slice's rectangles covering each tile
-    const int gw = g.tilesX + 1;
-    int* d = diff + (size_t)(n / span) * (g.tilesY + 1) * gw;
-    atomicAdd(d + sy.x * gw + sx.x, 1);
-    atomicAdd(d + sy.x * gw + sx.y + 1, -1);
-    atomicAdd(d + (sy.y + 1) * gw + sx.x, -1);
-    atomicAdd(d + (sy.y + 1) * gw + sx.y + 1, 1);
-  }
 }
 
-// Tile lists.  Counts: per primitive slice, prepare_kernel marks each
-// rectangle's corners in a 2-D difference array and counts_kernel prefix-sums
-// it into counts[t * S + slice], the number of the slice's rectangles covering
-// tile t.  The exclusive scan of the counts is tile-major and slice-minor.
+// Tile lists, four launches (prepare, counts, offsets, rows).  Counts: one CTA per
+// primitive slice marks its rectangles' corners in a 2-D difference array in
+// shared memory and prefix-sums it into counts[t * S + part], the number of
+// the slice's rectangles covering tile t (S counting slices), and adds each tile row's sum to
+// row_total.
 // Write: one CTA per (tile row, group of kBinGroup tiles, primitive slice),
-// kBinTPW tiles per warp (warp w: tiles w + k kBinWarps of the group); the
-// CTA walks the primitives of its slice in index order in chunks of
+// kBinTPW tiles per warp (warp w: tiles w + k kBinWarps of the group).  The CTA
+// walks the primitives of its slice in index order in chunks of
 // kBinThreads, compacts those whose rectangle covers its row and overlaps its
 // tile group, and each warp writes the ids of the compacted rectangles
-// containing each of its tiles from offs[t * S + slice] on, so a tile's
-// entries come out in ascending primitive order.  Two tiles per warp halve
-// the per-tile share of the row filter, compaction and count scan (write
-// pass 39.8 -> 29.4 us at 2048x2048, N=20000 on a B200).  The write pass also
-// publishes tile_offsets, L and the overflow flag, and leaves the outputs
-// untouched when L exceeds the capacity.
+// containing each of its tiles, so a tile's entries come out in ascending
+// primitive order.  Two tiles per warp halve the per-tile share of the row
+// filter, compaction and count scan (write pass 39.8 -> 29.4 us at 2048x2048,
+// N=20000 on a B200).  The write pass also publishes tile_offsets, L and the
+// overflow flag, and leaves the outputs untouched when L exceeds the capacity.
+// The write loop is bound by its instructions: write positions are pointers and
+// the compaction buffer is padded, so that it holds neither 64-bit index sums nor
+// bounds tests.  Replayed from a graph: 16.5 -> 10.5 us at 256x256, N=512;
+// 20.5 -> 14.1 at 1024x1024, N=5000; 49.0 -> 45.3 at 2048x2048, N=20000; 487 ->
+// 439 at 4096x4096, N=100000 (against a memset, a difference array in global
+// memory and a library scan of all counts, six launches).
 constexpr int kBinThreads = 512;
 constexpr int kBinWarps = kBinThreads / 32;
 constexpr int kBinTPW = 2;                       // tiles per warp
@@ -263,6 +271,8 @@ struct BinGrid {
   int groups;   // tile groups per row
   int slices;   // primitive slices
   int span;     // primitives per slice (multiple of kBinThreads)
+  int subs;     // counting slices per slice
+  int cspan;    // primitives per counting slice
   long long ctas;
 };
 
@@ -278,87 +288,180 @@ static inline BinGrid bin_grid(int N, int tilesX, int tilesY) {
   const int per = (chunks + b.slices - 1) / b.slices;
   b.span = per * kBinThreads;
   b.slices = N > 0 ? (N + b.span - 1) / b.span : 1;
+  // counted in up to 64 finer slices: a counting CTA's shared-memory adds run at
+  // about one rectangle per 30 cycles (100,000 rectangles: 3 CTAs take 110 us, 49
+  // take 9), but every writing CTA sums the counts left of its tiles
+  int cspan = (N + 63) / 64 > kBinThreads ? (N + 63) / 64 : kBinThreads;
+  if (cspan > b.span) cspan = b.span;
+  b.subs = (b.span + cspan - 1) / cspan;
+  b.cspan = (b.span + b.subs - 1) / b.subs;
   b.ctas = base * b.slices;
   return b;
 }
 
-// One CTA per slice: 2-D inclusive prefix sum of the slice's difference array
-// (rows, then columns), written as counts[t * S + slice]; counts[T * S] = 0.
-// SMEM: the array is staged in shared memory (it fits for canvases up to
-// about 3500 x 3500 pixels at tile 32); otherwise it is scanned in place.
-// Rows are scanned by whole warps (shuffle scans over 32-column chunks),
-// columns by one thread each.
-template <bool SMEM>
-__global__ void __launch_bounds__(1024) counts_kernel(Geom g, BinGrid bg, int* __restrict__ diff,
-                                                      long long* __restrict__ counts) {
+// One CTA per (counting slice, candidate); slice s has counting slices s subs to
+// s subs + subs - 1.  The difference array of (tilesY+1) x
+// (tilesX+1) counters sits in dynamic shared memory, or, for canvases beyond
+// about 7500 x 7500 pixels at tile 32, in the slice's own part of scratch.
+// Rows are scanned by whole warps (shuffle scans over 32-column chunks), then
+// columns the same way.
+__global__ void __launch_bounds__(1024) counts_kernel(Geom g, BinGrid bg, const int4* __restrict__ rects,
+                                                      int* __restrict__ scratch, int* __restrict__ counts,
+                                                      unsigned long long* __restrict__ row_total) {
   extern __shared__ int s_diff[];
-  const int slice = blockIdx.x;
+  grid_dependency();
+  const int part = blockIdx.x, parts = gridDim.x;   // counting slice
+  const size_t b = blockIdx.y;
   const int gw = g.tilesX + 1;
   const int cells = (g.tilesY + 1) * gw;
-  int* src = diff + (size_t)slice * cells;
-  int* d = SMEM ? s_diff : src;
-  if (SMEM) {
-    for (int i = threadIdx.x; i < cells; i += blockDim.x) s_diff[i] = src[i];
-    __syncthreads();
+  int* d = scratch ? scratch + (b * parts + part) * cells : s_diff;
+  rects += b * g.N;
+  counts += b * g.T * parts;
+  row_total += b * g.tilesY;
+  for (int i = threadIdx.x; i < cells; i += blockDim.x) d[i] = 0;
+  __syncthreads();
+  // the rectangles' corners; the array's 2-D prefix sum is the number of
+  // rectangles covering each tile
+  const int slice = part / bg.subs, sub = part - slice * bg.subs;
+  const int lo = slice * bg.span + sub * bg.cspan;
+  const int hi = min(g.N, min(lo + bg.cspan, (slice + 1) * bg.span));
+  for (int n = lo + threadIdx.x; n < hi; n += blockDim.x) {
+    const int4 rc = rects[n];
+    if (rc.x <= rc.y && rc.z <= rc.w) {
+      atomicAdd(d + rc.z * gw + rc.x, 1);
+      atomicAdd(d + rc.z * gw + rc.y + 1, -1);
+      atomicAdd(d + (rc.w + 1) * gw + rc.x, -1);
+      atomicAdd(d + (rc.w + 1) * gw + rc.y + 1, 1);
+    }
   }
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  for (int y = warp; y < g.tilesY; y += nwarps) {
+  auto scan = [&](int* p, int len, int stride) {   // inclusive prefix sum of p[0], p[stride], ... by one warp
     int carry = 0;
-    for (int x0 = 0; x0 < g.tilesX; x0 += 32) {
-      const int x = x0 + lane;
-      int v = x < g.tilesX ? d[y * gw + x] : 0;
+    for (int i0 = 0; i0 < len; i0 += 32) {
+      const int i = i0 + lane;
+      int v = i < len ? p[(size_t)i * stride] : 0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += u;
       }
       v += carry;
-      if (x < g.tilesX) d[y * gw + x] = v;
+      if (i < len) p[(size_t)i * stride] = v;
       carry = __shfl_sync(0xffffffffu, v, 31);
     }
-  }
+  };
+  for (int y = warp; y < g.tilesY; y += nwarps) scan(d + y * gw, g.tilesX, 1);
   __syncthreads();
-  for (int x = threadIdx.x; x < g.tilesX; x += blockDim.x) {
-    long long acc = 0;
-    for (int y = 0; y < g.tilesY; ++y) {
-      acc += d[y * gw + x];
-      counts[((long long)y * g.tilesX + x) * bg.slices + slice] = acc;
+  for (int x = warp; x < g.tilesX; x += nwarps) scan(d + x, g.tilesY, gw);
+  __syncthreads();
+  for (int y = warp; y < g.tilesY; y += nwarps) {
+    unsigned long long sum = 0;
+    for (int x = lane; x < g.tilesX; x += 32) {
+      const int v = d[y * gw + x];
+      counts[((size_t)y * g.tilesX + x) * parts + part] = v;
+      sum += (unsigned long long)v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && sum) atomicAdd(row_total + y, sum);
+  }
+}
+
+// One CTA per (tile row, candidate): the list position of each (tile, writing
+// slice) of the row, offs[t * S + slice] (tile-major, slice-minor over the
+// canvas), from the totals of the rows above and a scan over the row's counts.
+// The last row's CTA also writes offs[T * S] = L.
+constexpr int kOffsThreads = 512;
+
+__global__ void __launch_bounds__(kOffsThreads) offsets_kernel(Geom g, BinGrid bg, const int* __restrict__ counts,
+                                                               const unsigned long long* __restrict__ row_total,
+                                                               long long* __restrict__ offs) {
+  __shared__ long long s_base;
+  __shared__ int s_warp[kOffsThreads / 32];
+  grid_dependency();
+  const int ty = blockIdx.x;
+  const size_t cand = blockIdx.y;
+  const int parts = bg.slices * bg.subs;
+  counts += (cand * g.T + (size_t)ty * g.tilesX) * parts;
+  row_total += cand * g.tilesY;
+  offs += cand * ((size_t)g.T * bg.slices + 1) + (size_t)ty * g.tilesX * bg.slices;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {
+    long long above = 0;
+    for (int y = lane; y < ty; y += 32) above += (long long)row_total[y];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
+    if (lane == 0) {
+      s_base = above;
+      if (ty == g.tilesY - 1) offs[(size_t)g.tilesX * bg.slices] = above + (long long)row_total[ty];
     }
   }
-  if (slice == 0 && threadIdx.x == 0) counts[(long long)g.T * bg.slices] = 0;
+  const int len = g.tilesX * parts;
+  long long carry = 0;
+  for (int i0 = 0; i0 < len; i0 += kOffsThreads) {
+    const int i = i0 + threadIdx.x;
+    const int own = i < len ? counts[i] : 0;
+    int v = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) s_warp[warp] = v;
+    __syncthreads();
+    int w = lane < kOffsThreads / 32 ? s_warp[lane] : 0;   // inclusive prefix of the warps' sums, one per lane
+#pragma unroll
+    for (int o = 1; o < kOffsThreads / 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    const int before = warp > 0 ? __shfl_sync(0xffffffffu, w, warp - 1) : 0;
+    const int total = __shfl_sync(0xffffffffu, w, kOffsThreads / 32 - 1);
+    if (i < len && i % bg.subs == 0) offs[i / bg.subs] = s_base + carry + before + v - own;
+    carry += total;
+    __syncthreads();   // s_warp is rewritten by the next round
+  }
 }
 
 __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGrid bg,
                                                                   const int4* __restrict__ rects,
                                                                   const long long* __restrict__ offs, long long cap,
-                                                                  int* __restrict__ indices,
+                                                                  int* __restrict__ indices, long long index_stride,
                                                                   int* __restrict__ tile_offsets,
                                                                   int* __restrict__ total_out,
-                                                                  int* __restrict__ overflow_out) {
+                                                                  int* __restrict__ overflow_out,
+                                                                  long long flag_stride) {
   // Two compaction buffers: chunk c is compacted into buffer c & 1 while the
   // warps may still read chunk c - 1 from the other one, so one barrier per
   // chunk orders everything (see the loop).
   __shared__ int s_id[2][kBinThreads];
   __shared__ int2 s_xr[2][kBinThreads];   // the rectangle's tile columns x0, x1
   __shared__ int s_wcnt[2][kBinWarps];
+  grid_dependency();
+  const size_t cand = blockIdx.y;   // candidate of a batch
+  const long long nslots = (long long)g.T * bg.slices;
+  rects += cand * g.N;
+  offs += cand * (nslots + 1);
+  indices += cand * index_stride;
+  tile_offsets += cand * (g.T + 1);
   const int slice = blockIdx.x % bg.slices;
   const int rg = blockIdx.x / bg.slices;
   const int ty = rg / bg.groups;
   const int gx0 = (rg - ty * bg.groups) * kBinGroup, gx1 = min(gx0 + kBinGroup - 1, g.tilesX - 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long nslots = (long long)g.T * bg.slices;
   const unsigned lt = (1u << lane) - 1u;
   // this warp's tiles gx0 + warp + k kBinWarps: the column a rectangle must
   // reach (INT_MAX for a tile past the canvas, which no rectangle contains)
   // and the next write position of each
   int col[kBinTPW];
-  long long cur[kBinTPW];
+  int* cur[kBinTPW];
   {
     const long long L = offs[nslots];
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
     if (first) {
-      if (total_out) *total_out = (int)min(L, (long long)INT_MAX);
-      if (overflow_out) *overflow_out = (L > cap) ? 1 : 0;
+      if (total_out) total_out[cand * flag_stride] = (int)min(L, (long long)INT_MAX);
+      if (overflow_out) overflow_out[cand * flag_stride] = (L > cap) ? 1 : 0;
     }
     if (L > cap) return;   // uniform over the CTA
     if (first) tile_offsets[g.T] = (int)L;
@@ -366,12 +469,13 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
     for (int k = 0; k < kBinTPW; ++k) {
       const int tx = gx0 + warp + k * kBinWarps;
       col[k] = INT_MAX;
-      cur[k] = 0;
+      cur[k] = indices;
       if (tx <= gx1) {
         const int t = ty * g.tilesX + tx;
+        const long long at = offs[(long long)t * bg.slices + slice];
         col[k] = tx;
-        cur[k] = offs[(long long)t * bg.slices + slice];
-        if (lane == 0 && slice == 0) tile_offsets[t] = (int)cur[k];
+        cur[k] = indices + at;
+        if (lane == 0 && slice == 0) tile_offsets[t] = (int)at;
       }
     }
   }
@@ -404,6 +508,9 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
       s_id[buf][p] = n;
       s_xr[buf][p] = make_int2(rc.x, rc.y);
     }
+    // pad the last group of 32 with rectangles that contain no column
+    const int padded = (total + 31) & ~31;
+    if ((int)threadIdx.x >= total && (int)threadIdx.x < padded) s_xr[buf][threadIdx.x] = make_int2(1, 0);
     // (2) test and count the next chunk, and load the one after it
     n += kBinThreads;
     rc = rn;
@@ -417,14 +524,14 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
     // barrier), and s_wcnt[buf], last read in (1) above (before this barrier).
     __syncthreads();
     // (3) each warp writes the compacted rectangles that contain its tiles
-    for (int j = lane; j < ((total + 31) & ~31); j += 32) {
-      const int2 xr = j < total ? s_xr[buf][j] : make_int2(1, 0);
-      const int id = j < total ? s_id[buf][j] : 0;
+    for (int j = lane; j < padded; j += 32) {
+      const int2 xr = s_xr[buf][j];
+      const int id = s_id[buf][j];   // (not set in the padding, nor used there)
 #pragma unroll
       for (int k = 0; k < kBinTPW; ++k) {
         const bool in = xr.x <= col[k] && col[k] <= xr.y;
         const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (in) indices[cur[k] + __popc(m & lt)] = id;
+        if (in) cur[k][__popc(m & lt)] = id;
         cur[k] += __popc(m);
       }
     }
@@ -433,55 +540,46 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
 
 // ---------------------------------------------------------------------------
 struct BinWorkspace {
-  int4* rects;         // N tile rectangles (x0, x1, y0, y1)
-  long long* counts;   // T*S+1 entries per (tile, primitive slice)
-  long long* offs;     // exclusive prefix of counts
-  int* diff;           // S difference arrays of (tilesY+1) x (tilesX+1)
-  size_t diff_bytes;
-  void* cub_tmp;
-  size_t cub_bytes;
-  size_t total;
+  int4* rects;                     // N tile rectangles (x0, x1, y0, y1) per candidate
+  int* counts;                     // (tile, counting slice) entries per candidate
+  long long* offs;                 // list positions per (tile, writing slice), and L, per candidate
+  unsigned long long* row_total;   // tilesY list lengths of the tile rows per candidate
+  int* scratch;                    // difference arrays that do not fit shared memory (null otherwise)
 };
 
 static inline size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
 
-static BinWorkspace layout_ws(void* base, int N, int T, long long nslots, size_t diff_bytes, bool query,
-                              size_t* needed) {
-  BinWorkspace w{};
-  size_t scan_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (long long*)nullptr, (long long*)nullptr, nslots + 1);
-  w.cub_bytes = align_up(scan_bytes);
+constexpr size_t kCountsSmem = 200 * 1024;
+
+static inline size_t diff_cells_bytes(int tilesX, int tilesY) {
+  return sizeof(int) * (size_t)(tilesY + 1) * (tilesX + 1);
+}
+
+// Lays the workspace out from base and returns its size.
+static size_t layout_ws(void* base, int batch, int N, int T, int tilesX, int tilesY, const BinGrid& bg,
+                        BinWorkspace* w) {
+  const size_t B = batch, parts = (size_t)bg.slices * bg.subs;
   size_t off = 0;
-  auto take = [&](size_t bytes) { size_t o = off; off += align_up(bytes); return o; };
-  const size_t o_rects = take(sizeof(int4) * (size_t)(N > 0 ? N : 1));
-  const size_t o_counts = take(sizeof(long long) * (size_t)(nslots + 1));
-  const size_t o_offs = take(sizeof(long long) * (size_t)(nslots + 1));
-  const size_t o_cub = take(w.cub_bytes);
-  const size_t o_diff = take(diff_bytes);
-  w.diff_bytes = diff_bytes;
-  w.total = off;
-  if (needed) *needed = off;
-  if (!query) {
+  auto take = [&](size_t bytes) { const size_t o = off; off += align_up(bytes); return o; };
+  const size_t o_rects = take(sizeof(int4) * B * (N > 0 ? N : 1));
+  const size_t o_counts = take(sizeof(int) * 2 * (B * T * parts + 1));
+  const size_t o_offs = take(sizeof(long long) * B * ((size_t)T * bg.slices + 1));
+  const size_t o_rows = take(sizeof(unsigned long long) * B * tilesY);
+  const size_t cells = diff_cells_bytes(tilesX, tilesY);
+  const size_t o_scratch = cells > kCountsSmem ? take(cells * B * parts) : 0;
+  if (w) {
     char* b = static_cast<char*>(base);
-    w.rects = reinterpret_cast<int4*>(b + o_rects);
-    w.counts = reinterpret_cast<long long*>(b + o_counts);
-    w.offs = reinterpret_cast<long long*>(b + o_offs);
-    w.cub_tmp = b + o_cub;
-    w.diff = reinterpret_cast<int*>(b + o_diff);
+    w->rects = reinterpret_cast<int4*>(b + o_rects);
+    w->counts = reinterpret_cast<int*>(b + o_counts);
+    w->offs = reinterpret_cast<long long*>(b + o_offs);
+    w->row_total = reinterpret_cast<unsigned long long*>(b + o_rows);
+    w->scratch = cells > kCountsSmem ? reinterpret_cast<int*>(b + o_scratch) : nullptr;
   }
-  return w;
+  return off;
 }
 
-static inline size_t diff_bytes_of(const BinGrid& bg, int tilesX, int tilesY) {
-  return sizeof(int) * (size_t)bg.slices * (tilesY + 1) * (tilesX + 1);
-}
-
-size_t bin_workspace_bytes(int N, int T, int tilesX, int tilesY, long long cap) {
-  (void)cap;   // the row binning needs no scratch per list entry
-  const BinGrid bg = bin_grid(N, tilesX, tilesY);
-  size_t need = 0;
-  layout_ws(nullptr, N, T, (long long)T * bg.slices, diff_bytes_of(bg, tilesX, tilesY), true, &need);
-  return need;
+size_t bin_workspace_bytes(int batch, int N, int T, int tilesX, int tilesY) {
+  return layout_ws(nullptr, batch, N, T, tilesX, tilesY, bin_grid(N, tilesX, tilesY), nullptr);
 }
 
 int launch_template_bboxes(const float* tmpl, int P, int Ht, int Wt, float* out, cudaStream_t st) {
@@ -794,47 +892,52 @@ int launch_template_blur_sched(const float* in, int P, int Ht, int Wt, const dbm
   return DBMP_OK;
 }
 
+// Threads per CTA of prepare_kernel: a primitive is one long chain of double
+// and float functions, so few primitives are spread over many SMs.
+constexpr int kPrepThreads = 64;
+
 int launch_prepare(const Geom& g, const float* means2D, const float* radii, const float* rot, const float* opac,
                    const float* colors, const int* sel, PrimInfo* out, cudaStream_t st) {
   if (g.N == 0) return DBMP_OK;
-  prepare_kernel<<<(g.N + 255) / 256, 256, 0, st>>>(g, means2D, radii, rot, opac, colors, sel, nullptr, 0,
-                                                    out, nullptr, nullptr, 1);
-  DBMP_CHECK_LAUNCH("prepare_kernel");
-  return DBMP_OK;
+  return launch_chained("prepare_kernel", prepare_kernel, dim3((g.N + kPrepThreads - 1) / kPrepThreads), kPrepThreads, 0,
+                        st, g, means2D, radii, rot, opac, colors, sel, 0ll, (const float*)nullptr, 0, out,
+                        (int4*)nullptr, (unsigned long long*)nullptr);
 }
 
-int launch_bin(const Geom& g, int bin_mode, const float* means2D, const float* radii, const float* rot,
-               const float* opac, const float* colors, const int* sel, const float* tbbox, PrimInfo* prim_info,
-               int* tile_offsets, int* tile_indices, long long cap, int* total_out, int* overflow_out,
-               void* ws, size_t ws_bytes, cudaStream_t st) {
+int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
+               const float* opac, const float* colors, const int* sel, long long sel_stride, const float* tbbox,
+               PrimInfo* prim_info, int* tile_offsets, int* tile_indices, long long index_stride, long long cap,
+               int* total_out, int* overflow_out, long long flag_stride, void* ws, size_t ws_bytes, cudaStream_t st) {
   const BinGrid bg = bin_grid(g.N, g.tilesX, g.tilesY);
-  const long long nslots = (long long)g.T * bg.slices;
-  size_t need = 0;
-  BinWorkspace w = layout_ws(ws, g.N, g.T, nslots, diff_bytes_of(bg, g.tilesX, g.tilesY), false, &need);
+  BinWorkspace w{};
+  const size_t need = layout_ws(ws, batch, g.N, g.T, g.tilesX, g.tilesY, bg, &w);
   if (ws_bytes < need) {
     set_error("dbmp_bin: workspace of %zu bytes is smaller than the %zu bytes required", ws_bytes, need);
     return DBMP_ERR_CAPACITY;
   }
-  if (bg.ctas > 0x7fffffffll) { set_error("dbmp_bin: canvas and primitive count too large"); return DBMP_ERR_INVALID; }
-  cudaError_t e = cudaMemsetAsync(w.diff, 0, w.diff_bytes, st);
-  if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(diff)");
-  if (g.N > 0) {
-    prepare_kernel<<<(g.N + 255) / 256, 256, 0, st>>>(g, means2D, radii, rot, opac, colors, sel, tbbox, bin_mode,
-                                                      prim_info, w.rects, w.diff, bg.span);
-    DBMP_CHECK_LAUNCH("prepare_kernel");
+  if (bg.ctas > 0x7fffffffll || batch > 65535) {
+    set_error("dbmp_bin: canvas, primitive count or batch too large");
+    return DBMP_ERR_INVALID;
   }
-  const size_t cells_bytes = sizeof(int) * (size_t)(g.tilesY + 1) * (g.tilesX + 1);
-  if (cells_bytes <= 48 * 1024) counts_kernel<true><<<bg.slices, 1024, cells_bytes, st>>>(g, bg, w.diff, w.counts);
-  else counts_kernel<false><<<bg.slices, 1024, 0, st>>>(g, bg, w.diff, w.counts);
-  DBMP_CHECK_LAUNCH("counts_kernel");
-  size_t tmp = w.cub_bytes;
-  e = cub::DeviceScan::ExclusiveSum(w.cub_tmp, tmp, w.counts, w.offs, nslots + 1, st);
-  if (e != cudaSuccess) return cuda_status(e, "cub::DeviceScan::ExclusiveSum");
-  const int grid = (int)bg.ctas;   // (tile row, tile group, primitive slice) triples
-  bin_rows_kernel<<<grid, kBinThreads, 0, st>>>(g, bg, w.rects, w.offs, cap, tile_indices, tile_offsets, total_out,
-                                                overflow_out);
-  DBMP_CHECK_LAUNCH("bin_rows_kernel");
-  return DBMP_OK;
+  // prepare also runs with N = 0: it zeroes the row totals
+  const dim3 prep(g.N > 0 ? (g.N + kPrepThreads - 1) / kPrepThreads : 1, batch);
+  int rc = launch_chained("prepare_kernel", prepare_kernel, prep, kPrepThreads, 0, st, g, means2D, radii, rot, opac,
+                          colors, sel, sel_stride, tbbox, bin_mode, prim_info, w.rects, w.row_total);
+  if (rc) return rc;
+  const size_t smem = w.scratch ? 0 : diff_cells_bytes(g.tilesX, g.tilesY);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(counts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountsSmem);
+    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(counts_kernel)");
+  }
+  rc = launch_chained("counts_kernel", counts_kernel, dim3(bg.slices * bg.subs, batch), 1024, smem, st, g, bg,
+                      (const int4*)w.rects, w.scratch, w.counts, w.row_total);
+  if (rc) return rc;
+  rc = launch_chained("offsets_kernel", offsets_kernel, dim3(g.tilesY, batch), kOffsThreads, 0, st, g, bg,
+                      (const int*)w.counts, (const unsigned long long*)w.row_total, w.offs);
+  if (rc) return rc;
+  return launch_chained("bin_rows_kernel", bin_rows_kernel, dim3((unsigned)bg.ctas, batch), kBinThreads, 0, st, g, bg,
+                        (const int4*)w.rects, (const long long*)w.offs, cap, tile_indices, index_stride, tile_offsets,
+                        total_out, overflow_out, flag_stride);
 }
 
 }  // namespace dbmp

@@ -22,18 +22,19 @@ int cuda_status(cudaError_t e, const char* what) {
 }
 
 // launchers (binning.cu, raster.cu)
-size_t bin_workspace_bytes(int N, int T, int tilesX, int tilesY, long long cap);
+size_t bin_workspace_bytes(int batch, int N, int T, int tilesX, int tilesY);
 size_t atlas_bytes(int P, int Ht, int Wt, int kind);
 int launch_template_bboxes(const float* tmpl, int P, int Ht, int Wt, float* out, cudaStream_t st);
 int launch_template_blur(const float* in, int P, int Ht, int Wt, float sigma, float* out, cudaStream_t st);
 int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
 int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
+int launch_zero(double* a, long long n, double* b, cudaStream_t st);
 int launch_prepare(const Geom& g, const float* means2D, const float* radii, const float* rot, const float* opac,
                    const float* colors, const int* sel, PrimInfo* out, cudaStream_t st);
-int launch_bin(const Geom& g, int bin_mode, const float* means2D, const float* radii, const float* rot,
-               const float* opac, const float* colors, const int* sel, const float* tbbox, PrimInfo* prim_info,
-               int* tile_offsets, int* tile_indices, long long cap, int* total_out, int* overflow_out,
-               void* ws, size_t ws_bytes, cudaStream_t st);
+int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
+               const float* opac, const float* colors, const int* sel, long long sel_stride, const float* tbbox,
+               PrimInfo* prim_info, int* tile_offsets, int* tile_indices, long long index_stride, long long cap,
+               int* total_out, int* overflow_out, long long flag_stride, void* ws, size_t ws_bytes, cudaStream_t st);
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                    const int* idx, float* color, float* alpha, float* T_last, int* last_pos, cudaStream_t st);
 int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
@@ -191,8 +192,14 @@ int dbmp_atlas_pack_extended(const float* templates, int P, int Ht, int Wt, int 
 size_t dbmp_bin_workspace_bytes(const dbmp_canvas* cv, long long capacity) {
   Geom g;
   if (make_geom(cv, &g, "dbmp_bin_workspace_bytes") != DBMP_OK) return 0;
-  if (capacity < 0) capacity = 0;
-  return bin_workspace_bytes(g.N, g.T, g.tilesX, g.tilesY, capacity);
+  (void)capacity;   // the row binning needs no scratch per list entry
+  return bin_workspace_bytes(1, g.N, g.T, g.tilesX, g.tilesY);
+}
+
+size_t dbmp_bin_batch_workspace_bytes(const dbmp_canvas* cv, int batch) {
+  Geom g;
+  if (make_geom(cv, &g, "dbmp_bin_batch_workspace_bytes") != DBMP_OK || batch < 0) return 0;
+  return bin_workspace_bytes(batch, g.N, g.T, g.tilesX, g.tilesY);
 }
 
 int dbmp_prepare(const dbmp_canvas* cv, const float* means2D, const float* radii, const float* rotations,
@@ -224,9 +231,38 @@ int dbmp_bin(const dbmp_canvas* cv, const float* means2D, const float* radii, co
   REQUIRE(capacity == 0 || tile_indices, "dbmp_bin: tile_indices is null");
   REQUIRE(((uintptr_t)prim_info & 15) == 0 && ((uintptr_t)workspace & 255) == 0,
           "dbmp_bin: prim_info must be 16-byte and workspace 256-byte aligned");
-  return launch_bin(g, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, tmpl_bbox,
-                    (PrimInfo*)prim_info, tile_offsets, tile_indices, capacity, total_out, overflow_out, workspace,
-                    workspace_bytes, (cudaStream_t)stream);
+  return launch_bin(g, 1, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, 0, tmpl_bbox,
+                    (PrimInfo*)prim_info, tile_offsets, tile_indices, 0, capacity, total_out, overflow_out, 0,
+                    workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii,
+                   const float* rotations, const float* opacities, const float* colors, const int32_t* sel,
+                   long long sel_stride, const float* tmpl_bbox, void* prim_info, int32_t* tile_offsets,
+                   int32_t* tile_indices, long long index_stride, long long capacity, int32_t* total_and_overflow,
+                   void* workspace, size_t workspace_bytes, void* stream) {
+  Geom g;
+  int rc = make_geom(cv, &g, "dbmp_bin_batch");
+  if (rc) return rc;
+  REQUIRE(batch >= 0, "dbmp_bin_batch: batch %d < 0", batch);
+  if (batch == 0) return DBMP_OK;
+  REQUIRE(cv->bin_mode == DBMP_BIN_CONTENT || cv->bin_mode == DBMP_BIN_CULL || cv->bin_mode == DBMP_BIN_CONTENT_REF,
+          "dbmp_bin_batch: bin_mode %d unknown", cv->bin_mode);
+  REQUIRE(g.N == 0 || (means2D && radii && rotations && opacities && colors && sel && prim_info),
+          "dbmp_bin_batch: null pointer");
+  REQUIRE(cv->bin_mode == DBMP_BIN_CULL || tmpl_bbox,
+          "dbmp_bin_batch: tmpl_bbox is required in the DBMP_BIN_CONTENT modes");
+  REQUIRE(tile_offsets && total_and_overflow && workspace, "dbmp_bin_batch: null output or workspace");
+  REQUIRE(capacity >= 0 && capacity <= 0x7fffffffll, "dbmp_bin_batch: capacity %lld outside [0, 2^31)", capacity);
+  REQUIRE(capacity <= index_stride || batch == 1, "dbmp_bin_batch: index_stride %lld below the capacity %lld",
+          index_stride, capacity);
+  REQUIRE(capacity == 0 || tile_indices, "dbmp_bin_batch: tile_indices is null");
+  REQUIRE(sel_stride == 0 || sel_stride >= g.N, "dbmp_bin_batch: sel_stride %lld", sel_stride);
+  REQUIRE(((uintptr_t)prim_info & 15) == 0 && ((uintptr_t)workspace & 255) == 0,
+          "dbmp_bin_batch: prim_info must be 16-byte and workspace 256-byte aligned");
+  return launch_bin(g, batch, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, sel_stride, tmpl_bbox,
+                    (PrimInfo*)prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
+                    total_and_overflow + 1, 2, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int dbmp_forward(const dbmp_canvas* cv, const void* prim_info, const void* atlas, const int32_t* tile_offsets,
@@ -255,10 +291,8 @@ int dbmp_backward(const dbmp_canvas* cv, const void* prim_info, const void* atla
   REQUIRE(g.N == 0 || (grad_accum && grad_means2D && grad_radii && grad_rotations && grad_opacities && grad_colors),
           "dbmp_backward: null output");
   cudaStream_t st = (cudaStream_t)stream;
-  if (g.N > 0) {
-    cudaError_t e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N, st);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(grad_accum)");
-  }
+  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, st);
+  if (rc) return rc;
   rc = launch_backward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, T_last,
                        last_pos, grad_color, grad_alpha, grad_accum, st);
   if (rc) return rc;
@@ -313,10 +347,8 @@ int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void
   REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_backward_blend: c_blend %g outside [0, 1]", (double)c_blend);
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_backward_blend: colors_orig is null with c_blend > 0");
   cudaStream_t st = (cudaStream_t)stream;
-  if (g.N > 0) {
-    cudaError_t e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N, st);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(grad_accum)");
-  }
+  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, st);
+  if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0);
   if (rc) return rc;
@@ -366,8 +398,8 @@ int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info,
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_backward_batch: colors_orig is null with c_blend > 0");
   if (!work) return DBMP_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N * batch, st);
-  if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(grad_accum)");
+  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, st);
+  if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, batch,
                              index_stride, colors_orig_stride);
@@ -406,9 +438,8 @@ int dbmp_fused_fwd_bwd(const dbmp_canvas* cv, const void* prim_info, const void*
   REQUIRE(atlas && tile_offsets && tile_indices && target && loss_out, "dbmp_fused_fwd_bwd: null input");
   REQUIRE(g.N == 0 || (prim_info && grad_accum), "dbmp_fused_fwd_bwd: null prim_info / grad_accum");
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(loss_out, 0, sizeof(double), st);
-  if (e == cudaSuccess && g.N > 0) e = cudaMemsetAsync(grad_accum, 0, sizeof(double) * 8 * (size_t)g.N, st);
-  if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync(fused outputs)");
+  rc = launch_zero(grad_accum, 8ll * g.N, loss_out, st);
+  if (rc) return rc;
   return launch_fused(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, target,
                       background, out_image, grad_accum, loss_out, skip_flag, st);
 }

@@ -306,4 +306,32 @@ int cuda_status(cudaError_t e, const char* what);
     if (_e != cudaSuccess) return ::dbmp::cuda_status(_e, what); \
   } while (0)
 
+// Chained launches (programmatic dependent launch): a kernel of a chain starts
+// while the one before it on the stream drains, and grid_dependency(), its
+// first statement, waits until that one has completed and its writes are
+// visible; it then lets the next one start.  What a launch costs between
+// two short kernels shrinks from about 2 us to below 1 us.  After any other work
+// (a copy, another library's kernel) the launch waits as usual.
+__device__ __forceinline__ void grid_dependency() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
+template <typename... P, typename... A>
+int launch_chained(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                   A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e == cudaSuccess ? DBMP_OK : cuda_status(e, what);
+}
+
 }  // namespace dbmp

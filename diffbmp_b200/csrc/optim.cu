@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(kAdamThreads) adam_kernel(Geom g, AdamArgs a, 
                                                             float* __restrict__ colors, float* __restrict__ m1,
                                                             float* __restrict__ m2, const int* __restrict__ step_count,
                                                             const int* __restrict__ skip_flag) {
+  grid_dependency();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   // The step's scalars, once per CTA: thread k < 8 the step size of parameter
   // k, lr_k * gamma^(t-1) / (1 - beta1^t) in double as torch computes it
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(kAdamThreads) adam_kernel(Geom g, AdamArgs a, 
 }
 
 __global__ void step_increment_kernel(int* __restrict__ step_count, const int* __restrict__ skip_flag) {
+  grid_dependency();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   *step_count += 1;
 }
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(kPruneThreads) prune_kernel(Geom g, PruneArgs 
                                                               const int* __restrict__ skip_flag) {
   __shared__ int s_warp[kPruneThreads / 32];
   __shared__ int s_total;
+  grid_dependency();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   const int it = *step_count;
   // the reference's schedule (simple_tile_renderer.py:1007-1012); an iteration
@@ -197,10 +200,8 @@ int launch_prune(const Geom& g, const PruneArgs& a, const int* step_count, const
                  float* means2D, float* radii, float* rot, float* opac, float* colors, const int* skip_flag,
                  cudaStream_t st) {
   if (g.N == 0) return DBMP_OK;
-  prune_kernel<<<1, kPruneThreads, 0, st>>>(g, a, step_count, pool, state, means2D, radii, rot, opac, colors,
-                                            skip_flag);
-  DBMP_CHECK_LAUNCH("prune_kernel");
-  return DBMP_OK;
+  return launch_chained("prune_kernel", prune_kernel, dim3(1), kPruneThreads, 0, st, g, a, step_count, pool, state,
+                        means2D, radii, rot, opac, colors, skip_flag);
 }
 
 int launch_adam(const Geom& g, const AdamArgs& a, const double* gacc, float* means2D, float* radii, float* rot,
@@ -208,13 +209,11 @@ int launch_adam(const Geom& g, const AdamArgs& a, const double* gacc, float* mea
                 cudaStream_t st) {
   if (g.N > 0) {
     const int ctas = (int)(((long long)g.N + 32 * kAdamBlocks - 1) / (32 * kAdamBlocks));
-    adam_kernel<<<ctas, kAdamThreads, 0, st>>>(g, a, gacc, means2D, radii, rot, opac, colors, m1, m2, step_count,
-                                               skip_flag);
-    DBMP_CHECK_LAUNCH("adam_kernel");
+    const int rc = launch_chained("adam_kernel", adam_kernel, dim3(ctas), kAdamThreads, 0, st, g, a, gacc, means2D, radii,
+                                  rot, opac, colors, m1, m2, (const int*)step_count, skip_flag);
+    if (rc) return rc;
   }
-  step_increment_kernel<<<1, 1, 0, st>>>(step_count, skip_flag);
-  DBMP_CHECK_LAUNCH("step_increment_kernel");
-  return DBMP_OK;
+  return launch_chained("step_increment_kernel", step_increment_kernel, dim3(1), 1, 0, st, step_count, skip_flag);
 }
 
 }  // namespace dbmp

@@ -835,6 +835,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
     const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
     long long idx_stride, long long cmap_stride) {
+  grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
   __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
@@ -890,6 +891,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
     const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
     const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
     const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride) {
+  grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
   __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
@@ -943,6 +945,7 @@ __global__ void finalize_kernel(Geom g, const float* __restrict__ radii, const f
                                 const double* __restrict__ gacc, float* __restrict__ g_means,
                                 float* __restrict__ g_radii, float* __restrict__ g_rot, float* __restrict__ g_opac,
                                 float* __restrict__ g_colors) {
+  grid_dependency();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= g.N) return;
   const double* S = gacc + (size_t)n * 8;
@@ -984,6 +987,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fu
     const int* __restrict__ idx, const float* __restrict__ target, const float* __restrict__ background,
     float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
     const int* __restrict__ skip_flag) {
+  grid_dependency();
   if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND>;
@@ -1065,18 +1069,14 @@ int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const v
   const long long ctas = (long long)batch * g.T * kParts<32>();
   if (ctas > 0x7fffffffll) { set_error("forward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
   if (cmap != nullptr && cblend > 0.f) {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (forward_kernel<TSV, KD, true>
-                                                 <<<batch * g.T * kParts<TSV>(), kThreadsOf<TSV>(), 0, st>>>(
-                                                     g, prims, atlas, offs, idx, color, alpha, T_last, last_pos,
-                                                     cmap, cblend, idx_stride, cmap_stride))));
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
+        "forward_kernel", forward_kernel<TSV, KD, true>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride)));
   } else {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (forward_kernel<TSV, KD, false>
-                                                 <<<batch * g.T * kParts<TSV>(), kThreadsOf<TSV>(), 0, st>>>(
-                                                     g, prims, atlas, offs, idx, color, alpha, T_last, last_pos,
-                                                     nullptr, 0.f, idx_stride, 0))));
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
+        "forward_kernel", forward_kernel<TSV, KD, false>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll)));
   }
-  DBMP_CHECK_LAUNCH("forward_kernel");
-  return DBMP_OK;
 }
 
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
@@ -1102,18 +1102,16 @@ int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const 
   const long long ctas = (long long)batch * g.T * kParts<32>();
   if (ctas > 0x7fffffffll) { set_error("backward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
   if (cmap != nullptr && cblend > 0.f) {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (backward_kernel<TSV, KD, true>
-                                                 <<<batch * g.T * kParts<TSV>(), kThreadsOf<TSV>(), 0, st>>>(
-                                                     g, prims, atlas, offs, idx, T_last, last_pos, grad_color,
-                                                     grad_alpha, gacc, cmap, cblend, idx_stride, cmap_stride))));
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
+        "backward_kernel", backward_kernel<TSV, KD, true>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, cmap, cblend, idx_stride,
+        cmap_stride)));
   } else {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (backward_kernel<TSV, KD, false>
-                                                 <<<batch * g.T * kParts<TSV>(), kThreadsOf<TSV>(), 0, st>>>(
-                                                     g, prims, atlas, offs, idx, T_last, last_pos, grad_color,
-                                                     grad_alpha, gacc, nullptr, 0.f, idx_stride, 0))));
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
+        "backward_kernel", backward_kernel<TSV, KD, false>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, (const float*)nullptr, 0.f,
+        idx_stride, 0ll)));
   }
-  DBMP_CHECK_LAUNCH("backward_kernel");
-  return DBMP_OK;
 }
 
 int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
@@ -1123,23 +1121,36 @@ int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* 
                                nullptr, 0.f, st, 1, 0, 0);
 }
 
+// Zeroes n doubles at a and, when given, one at b: a kernel rather than
+// memsets, so that the launches around it stay chained.
+__global__ void zero_kernel(double* __restrict__ a, long long n, double* __restrict__ b) {
+  grid_dependency();
+  const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long i = i0; i < n; i += (long long)gridDim.x * blockDim.x) a[i] = 0.0;
+  if (b != nullptr && i0 == 0) *b = 0.0;
+}
+
+int launch_zero(double* a, long long n, double* b, cudaStream_t st) {
+  if (n == 0 && b == nullptr) return DBMP_OK;
+  const long long ctas = (n + 255) / 256;
+  return launch_chained("zero_kernel", zero_kernel, dim3((unsigned)(ctas < 1 ? 1 : ctas < 1184 ? ctas : 1184)), 256, 0,
+                        st, a, n, b);
+}
+
 int launch_finalize(const Geom& g, const float* radii, const float* rot, const float* opac, const float* colors,
                     const double* gacc, float* gm, float* gr, float* grot, float* go, float* gc, cudaStream_t st) {
   if (g.N == 0) return DBMP_OK;
-  finalize_kernel<<<(g.N + 255) / 256, 256, 0, st>>>(g, radii, rot, opac, colors, gacc, gm, gr, grot, go, gc);
-  DBMP_CHECK_LAUNCH("finalize_kernel");
-  return DBMP_OK;
+  return launch_chained("finalize_kernel", finalize_kernel, dim3((g.N + 63) / 64), 64, 0, st, g, radii, rot, opac,
+                        colors, gacc, gm, gr, grot, go, gc);
 }
 
 int launch_fused(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs, const int* idx,
                  const float* target, const float* background, float* out_image, double* gacc, double* loss,
                  const int* skip_flag, cudaStream_t st) {
   if (g.T == 0) return DBMP_OK;
-  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (fused_kernel<TSV, KD><<<g.T * kParts<TSV>(), kThreadsOf<TSV>(), 0, st>>>(
-                                                   g, prims, atlas, offs, idx, target, background, out_image,
-                                                   gacc, loss, skip_flag))));
-  DBMP_CHECK_LAUNCH("fused_kernel");
-  return DBMP_OK;
+  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
+      "fused_kernel", fused_kernel<TSV, KD>, dim3(g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st, g, prims, atlas, offs,
+      idx, target, background, out_image, gacc, loss, skip_flag)));
 }
 
 }  // namespace dbmp

@@ -228,14 +228,13 @@ class Rasterizer:
                       self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.extended else 0)
 
     # -- binning -----------------------------------------------------------
-    def _ensure(self, cv: Canvas, cap: int):
+    def _ensure(self, cv: Canvas, cap: int, nbytes: int = 0):
+        """Scratch for lists of `cap` entries, and nbytes of workspace at least."""
         if cap > self.capacity or self._ws is None:
             self.capacity = int(cap)
-            nbytes = int(lib.dbmp_bin_workspace_bytes(ctypes.byref(cv), self.capacity))
-            self._ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=self.device)
             self._idx = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=self.device)
-        nbytes = int(lib.dbmp_bin_workspace_bytes(ctypes.byref(cv), self.capacity))
-        if self._ws.numel() < nbytes + 256:
+        nbytes = max(nbytes, int(lib.dbmp_bin_workspace_bytes(ctypes.byref(cv), self.capacity)))
+        if self._ws is None or self._ws.numel() < nbytes + 256:
             self._ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=self.device)
 
     def _ws_ptr(self):
@@ -314,19 +313,27 @@ class Rasterizer:
         st = _stream(stream)
         prim = torch.empty((max(B * N, 1), 16), dtype=torch.float32, device=self.device)
         offsets = torch.empty((B, self.T + 1), dtype=torch.int32, device=self.device)
-        small = torch.zeros((B, 2), dtype=torch.int32, device=self.device)    # per candidate: L, overflow
-        sel2 = sel if sel.dim() == 2 else sel.unsqueeze(0).expand(B, -1)
+        small = torch.empty((B, 2), dtype=torch.int32, device=self.device)    # per candidate: L, overflow
+        sel_stride = N if sel.dim() == 2 else 0
+        if B == 0:
+            return prim, offsets, torch.empty((0, max(self.capacity, 1)), dtype=torch.int32, device=self.device)
+        # the call steps from candidate to candidate by N (candidates may come strided or expanded)
+        means2D, radii, rotations, opacities, colors, sel = (
+            t.contiguous() for t in (means2D, radii, rotations, opacities, colors, sel))
+        n = min(B, 65535)                       # candidates of one call
+        nbytes = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), n))
         for _ in range(3):
-            self._ensure(cv, self.capacity)
+            self._ensure(cv, self.capacity, nbytes)
             ws, wsb = self._ws_ptr()
             cap = max(self.capacity, 1)
             indices = torch.empty((B, cap), dtype=torch.int32, device=self.device)
-            for b in range(B):
-                call("dbmp_bin", ctypes.byref(cv), _ptr(means2D[b]), _ptr(radii[b]), _ptr(rotations[b]),
-                     _ptr(opacities[b]), _ptr(colors[b]), _ptr(sel2[b]), _ptr(atlas.bbox),
+            for b in range(0, B, n):
+                call("dbmp_bin_batch", ctypes.byref(cv), min(n, B - b), _ptr(means2D[b]), _ptr(radii[b]),
+                     _ptr(rotations[b]), _ptr(opacities[b]), _ptr(colors[b]),
+                     _ptr(sel[b]) if sel_stride else _ptr(sel), ctypes.c_longlong(sel_stride), _ptr(atlas.bbox),
                      ctypes.c_void_p(prim.data_ptr() + b * N * 64), _ptr(offsets[b]), _ptr(indices[b]),
-                     ctypes.c_longlong(self.capacity), _ptr(small[b]), ctypes.c_void_p(small[b].data_ptr() + 4),
-                     ws, ctypes.c_size_t(wsb), st)
+                     ctypes.c_longlong(cap), ctypes.c_longlong(self.capacity), _ptr(small[b]), ws,
+                     ctypes.c_size_t(wsb), st)
             Ls = small.cpu()
             if not bool(Ls[:, 1].any()):
                 return prim, offsets, indices

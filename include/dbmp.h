@@ -168,6 +168,19 @@ int dbmp_bin(const dbmp_canvas* cv, const float* means2D, const float* radii,
              int32_t* total_out, int32_t* overflow_out, void* workspace, size_t workspace_bytes,
              void* stream);
 
+/* dbmp_bin of `batch` candidates of one canvas in the launches of one:
+ * candidate b's parameters follow candidate b-1's (N each; sel sel_stride
+ * apart, 0: shared), and so do its records, its T+1 offsets, its indices
+ * (index_stride apart, `capacity` entries at most) and its two flags in
+ * total_and_overflow.  Workspace: dbmp_bin_batch_workspace_bytes. */
+size_t dbmp_bin_batch_workspace_bytes(const dbmp_canvas* cv, int batch);
+int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii,
+                   const float* rotations, const float* opacities, const float* colors,
+                   const int32_t* sel, long long sel_stride, const float* tmpl_bbox, void* prim_info,
+                   int32_t* tile_offsets, int32_t* tile_indices, long long index_stride,
+                   long long capacity, int32_t* total_and_overflow, void* workspace,
+                   size_t workspace_bytes, void* stream);
+
 /* Forward compositing.  out_color (H,W,3) f32 = sum_k T_k a_k c_k and
  * out_alpha (H,W) f32 = 1 - T_final, front to back over each tile's list,
  * stopping a pixel once T < t_stop.  Per pixel it also stores the
