@@ -14,7 +14,6 @@
 // psd_export_kernels.cu:26-55,96-195).
 #include <cstdint>
 
-#include <mutex>
 #include <type_traits>
 
 #include "dbmp_internal.cuh"
@@ -310,12 +309,13 @@ __global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float*
 // then PSDImage.save; psd_export_uint8.py:153-186, psd_exporter.py:468-501),
 // which splits it into planes and RLE-compresses them row by row on the host.
 // Here every (layer, channel, row) is encoded on the device.  Rows are taken
-// 32 at a time, one warp per group of 32 rows of a layer and one lane per
-// row; each lane runs four encoders at once, one per RGBA byte, on uchar4
-// pixels that the warp stages through shared memory 32 rows x 32 pixels at a
-// time (cp.async copies of coalesced row segments into two buffers, the next
-// chunk in flight while the current one is encoded; conflict-free reads with
-// a 36-word row pitch, four pixels per 16-byte read).
+// 32 at a time, one warp per group of 32 rows of a layer, in chunks of 32 columns.
+// The warp first looks at the chunk four rows at a time, four pixels per lane:
+// ballots of "differs from its left neighbour" give each channel's run starts as
+// bit masks.  Then each lane takes one row and visits only the set bits of its
+// four masks, so equal pixels, nearly all of a layer, cost a dozen instructions per
+// 128 of them.  (Encoders that looked at every pixel of their row took, at
+// 1024x1024, N=5000, 388 M and 510 M instructions for the two passes.)
 //
 // Encoding rule (a valid PackBits stream; a packet never crosses a row):
 //   - a maximal run of L >= 3 equal bytes becomes replicate packets
@@ -332,12 +332,12 @@ __global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float*
 // match the data can write wrong bytes but never out of bounds.
 // ---------------------------------------------------------------------------
 
-constexpr int kRleWarps = 4;      // warps per CTA (two staging buffers of 32 x 36 words each)
-// Words per staged row: 32 pixels + 4 pad.  Row starts 144 bytes apart keep
-// the staging copies (32 consecutive words of a row) and each lane's 16-byte
-// reads of its own row (8 lanes per phase on distinct 16-byte bank groups)
-// free of bank conflicts.
+constexpr int kRleWarps = 4;      // warps per CTA
+// Words per staged row: three unused, the pixel left of the chunk, the chunk's
+// 32.  Pixels start at a multiple of 16 bytes, and eight lanes' 16-byte reads of
+// a row, as the lanes' 4-byte reads of their own rows, cover distinct banks.
 constexpr int kRlePitch = 36;
+constexpr int kRleFirst = 4;      // word of the chunk's first pixel
 
 struct RleArgs {
   const uint8_t* layers;        // packed RGBA crops, row-major per layer
@@ -357,122 +357,124 @@ struct RleArgs {
   long long out_bytes;
 };
 
-// Four PackBits encoders of one row, counting output bytes only (count pass).
-// A literal segment's headers are added when the segment closes, or when 128
-// bytes are in.
+// A PackBits encoder of one channel of one row, fed with its runs in order:
+// counting output bytes only (count pass).  A literal segment's headers are
+// added when the segment closes, or when 128 bytes are in.
 struct RleCount {
-  int prev[4], run[4], lit[4];
-  long long pos[4];
+  int pos = 0, lit = 0;
 
-  __device__ __forceinline__ void close(int s) {
-    const int L = run[s];
+  __device__ __forceinline__ void run(int L, unsigned) {
     if (L >= 3) {
-      if (lit[s] > 0) pos[s] += 1 + lit[s];
-      lit[s] = 0;
-      pos[s] += 2 * ((L + 127) >> 7);
+      if (lit > 0) pos += 1 + lit;
+      lit = 0;
+      pos += 2 * ((L + 127) >> 7);
     } else {
-      lit[s] += L;
-      if (lit[s] >= 128) {
-        pos[s] += 129;
-        lit[s] -= 128;
+      lit += L;
+      if (lit >= 128) {
+        pos += 129;
+        lit -= 128;
       }
     }
   }
-  __device__ __forceinline__ void push(int s, int v) {
-    if (v == prev[s]) { ++run[s]; return; }
-    close(s);
-    prev[s] = v;
-    run[s] = 1;
-  }
-  __device__ __forceinline__ void finish(int s) {
-    close(s);
-    if (lit[s] > 0) pos[s] += 1 + lit[s];
+  __device__ __forceinline__ void finish() {
+    if (lit > 0) pos += 1 + lit;
   }
 };
 
-// Four PackBits encoders of one row that store their bytes (write pass).
-// Positions are byte offsets within the row's output of each channel slot.
-// A literal byte is stored as soon as its run closes (a run of one or two
-// bytes), at its final place: a literal packet's header position is reserved
-// when the packet opens and written when it closes (127 when 128 bytes are
-// in, the count minus one at the end of the segment), so no byte of the crop
-// is read twice.  (An earlier form re-read literal bytes from the crop when
-// their segment closed: 23.3 against 14.9 ms at 2048x2048, N=20000.  The
-// count pass keeps its own encoder: sharing this one took it from 8.0 to
-// 14.1 ms.)
+// The encoder that stores its bytes (write pass); positions are byte offsets
+// within the row's output.  A literal byte is stored as soon as its run closes
+// (a run of one or two bytes), at its final place: a literal packet's header
+// position is reserved when the packet opens and written when it closes (127
+// when 128 bytes are in, the count minus one at the end of the segment).
 struct RleWrite {
-  int prev[4], run[4], lit[4], pos[4], lim[4], hdr[4];
-  uint8_t* dst[4];   // the row's first output byte of each slot
+  int pos = 0, lit = 0, hdr = 0, lim = 0;
+  uint8_t* dst = nullptr;   // the row's first output byte
 
-  __device__ __forceinline__ void store(int s, int p, unsigned v) {
-    if (p < lim[s]) dst[s][p] = (uint8_t)v;
+  __device__ __forceinline__ void store(int p, unsigned v) {
+    if (p < lim) dst[p] = (uint8_t)v;
   }
-  __device__ __forceinline__ void put(int s, unsigned v) {
-    store(s, pos[s], v);
-    ++pos[s];
+  __device__ __forceinline__ void put(unsigned v) {
+    store(pos, v);
+    ++pos;
   }
   // Appends one byte to the open literal segment.
-  __device__ __forceinline__ void lit_byte(int s, unsigned v) {
-    if ((lit[s] & 127) == 0) hdr[s] = pos[s]++;
-    put(s, v);
-    if ((++lit[s] & 127) == 0) store(s, hdr[s], 127u);
+  __device__ __forceinline__ void lit_byte(unsigned v) {
+    if ((lit & 127) == 0) hdr = pos++;
+    put(v);
+    if ((++lit & 127) == 0) store(hdr, 127u);
   }
-  __device__ __forceinline__ void end_literal(int s) {
-    if (lit[s] & 127) store(s, hdr[s], (unsigned)((lit[s] & 127) - 1));
-    lit[s] = 0;
+  __device__ __forceinline__ void end_literal() {
+    if (lit & 127) store(hdr, (unsigned)((lit & 127) - 1));
+    lit = 0;
   }
-  // Closes the run of run[s] bytes equal to prev[s].
-  __device__ __forceinline__ void close(int s) {
-    const int L = run[s];
+  // A run of L bytes v.
+  __device__ __forceinline__ void run(int L, unsigned v) {
     if (L >= 3) {
-      end_literal(s);
+      end_literal();
       for (int rem = L; rem > 0; rem -= 128) {
         const int k = min(rem, 128);
-        put(s, k >= 2 ? (unsigned)(1 - k) & 0xFFu : 0u);
-        put(s, (unsigned)prev[s]);
+        put(k >= 2 ? (unsigned)(1 - k) & 0xFFu : 0u);
+        put(v);
       }
     } else {
-      for (int j = 0; j < L; ++j) lit_byte(s, (unsigned)prev[s]);
+      if (L >= 1) lit_byte(v);
+      if (L >= 2) lit_byte(v);
     }
   }
-  __device__ __forceinline__ void push(int s, int v) {
-    if (v == prev[s]) { ++run[s]; return; }
-    close(s);
-    prev[s] = v;
-    run[s] = 1;
-  }
-  __device__ __forceinline__ void finish(int s) {
-    close(s);
-    end_literal(s);
-  }
+  __device__ __forceinline__ void finish() { end_literal(); }
 };
 
-// One 4-byte asynchronous copy from global to shared memory (cp.async); with
-// valid false nothing is read and the word is zero-filled.
-__device__ __forceinline__ void cp_async_word(uint32_t* dst, const void* src, bool valid) {
+// One 4-byte asynchronous copy from global to shared memory (cp.async).
+__device__ __forceinline__ void cp_async_word(uint32_t* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// Largest i < n with base[i] <= g (base[0] <= g), by a whole warp: 32 probes a step.
+__device__ __forceinline__ int warp_search(const long long* __restrict__ base, int n, long long g, int lane) {
+  int lo = 0, len = n;
+  while (len > 1) {
+    const int step = (len + 31) >> 5;
+    const int at = lo + lane * step;
+    const unsigned le = __ballot_sync(0xffffffffu, lane * step < len && base[at] <= g);
+    const int k = 31 - __clz(le);   // bit 0 is set: base[lo] <= g
+    lo += k * step;
+    len = min(step, len - k * step);
+  }
+  return lo;
+}
+
+// Planes of a row's run starts (see psd_rle_kernel) to one bit per column, in
+// order: a transpose in three masked exchanges.
+__device__ __forceinline__ unsigned planes_to_columns(unsigned v) {
+  unsigned t = (v ^ (v >> 12)) & 0x0000F0F0u;
+  v ^= t ^ (t << 12);
+  t = (v ^ (v >> 6)) & 0x00CC00CCu;
+  v ^= t ^ (t << 6);
+  t = (v ^ (v >> 3)) & 0x0A0A0A0Au;
+  v ^= t ^ (t << 3);
+  return v;
+}
+
+// The registers are bounded for 36 resident warps per SM in the count pass and 28
+// in the write pass.
 template <bool WRITE>
-__global__ void __launch_bounds__(kRleWarps * 32) psd_rle_kernel(RleArgs a) {
-  // Per warp, two staging buffers of 32 rows x 32 pixels: the copies of the
-  // next 32 columns of the group's rows are in flight while the lanes encode
-  // the current ones.
-  __shared__ __align__(16) uint32_t stage[kRleWarps][2][32 * kRlePitch];
+__global__ void __launch_bounds__(kRleWarps * 32, WRITE ? 7 : 9) psd_rle_kernel(RleArgs a) {
+  // Per warp one buffer of 32 rows x (1 + 32) pixels, filled asynchronously: the
+  // count pass refills it as soon as the masks are taken.  Many warps with one
+  // buffer hide the copies better than 24 warps with two (count / write pass at
+  // 1024x1024, N=5000: 538 / 658 us with two buffers, 442 / 504 with one, 356 /
+  // 450 with one group per warp as well; 597 / 871 for encoders that look at
+  // every pixel.  At 2048x2048, N=20000, 15.8 GB: 6.2 / 8.0 -> 4.0 / 4.5 ms, 0.61
+  // and 0.55 of the copy bandwidth.)  What bounds them now is the visits to the
+  // run starts, with 28 of 32 lanes active and two fifths of the issue slots used.
+  __shared__ __align__(16) uint32_t stage[kRleWarps][32 * kRlePitch];
   const int lane = threadIdx.x & 31;
-  uint32_t(*sm)[32 * kRlePitch] = stage[threadIdx.x >> 5];
+  uint32_t* buf = stage[threadIdx.x >> 5];
   const long long nwarps = (long long)gridDim.x * kRleWarps;
   for (long long g = (long long)blockIdx.x * kRleWarps + (threadIdx.x >> 5); g < a.G; g += nwarps) {
-    int lo = 0, hi = a.N;   // largest i with group_base[i] <= g
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (a.group_base[mid] <= g) lo = mid; else hi = mid;
-    }
-    const int i = lo;
+    const int i = warp_search(a.group_base, a.N, g, lane);   // the group's layer
     const int w = a.sizes[2 * i], h = a.sizes[2 * i + 1];
     const long long off = a.layer_off[i];
     const bool ok = w >= 1 && w <= a.width_limit && h >= 1 && off >= 0 && (off & 3) == 0;
@@ -481,14 +483,12 @@ __global__ void __launch_bounds__(kRleWarps * 32) psd_rle_kernel(RleArgs a) {
     const bool active = ok && y0 + lane < h;
     const uint8_t* base = a.layers + (ok ? off : 0);
 
-    std::conditional_t<WRITE, RleWrite, RleCount> e;
+    std::conditional_t<WRITE, RleWrite, RleCount> e[4];
     unsigned short planned[4] = {0, 0, 0, 0};
     bool skip = !ok;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) e.pos[s] = 0;
     if constexpr (WRITE) {
 #pragma unroll
-      for (int s = 0; s < 4; ++s) { e.lim[s] = 0; e.hdr[s] = 0; e.dst[s] = a.out; }
+      for (int s = 0; s < 4; ++s) e[s].dst = a.out;
       if (ok && active) {
         const ushort4 rb = reinterpret_cast<const ushort4*>(a.row_bytes)[g * 32 + lane];
         planned[0] = rb.x; planned[1] = rb.y; planned[2] = rb.z; planned[3] = rb.w;
@@ -506,8 +506,8 @@ __global__ void __launch_bounds__(kRleWarps * 32) psd_rle_kernel(RleArgs a) {
         const long long gd = ok ? a.group_dst[4 * g + s] : -1;
         if (co >= 0 && gd >= 0) {   // otherwise every store of this slot is dropped
           const long long start = gd + pre;
-          e.dst[s] = a.out + start;
-          e.lim[s] = (int)max(0ll, min((long long)planned[s], a.out_bytes - start));
+          e[s].dst = a.out + start;
+          e[s].lim = (int)max(0ll, min((long long)planned[s], a.out_bytes - start));
           if (active) {   // row byte count, big-endian, in the block's table; block header on row 0
             const long long t = co + 2 + 2ll * y;
             if (t + 1 < a.out_bytes) { a.out[t] = (uint8_t)(planned[s] >> 8); a.out[t + 1] = (uint8_t)planned[s]; }
@@ -518,80 +518,107 @@ __global__ void __launch_bounds__(kRleWarps * 32) psd_rle_kernel(RleArgs a) {
       skip = skip || (a.chan_off[4 * i] < 0 && a.chan_off[4 * i + 1] < 0 && a.chan_off[4 * i + 2] < 0 &&
                       a.chan_off[4 * i + 3] < 0);
     }
-#pragma unroll
-    for (int s = 0; s < 4; ++s) { e.prev[s] = -1; e.run[s] = 0; e.lit[s] = 0; }
 
     uint32_t any_alpha = 0;
-    unsigned long long last = 1ull << 32;   // the previous pixel; no pixel equals the initial value
-    int eq = 0;                             // pixels equal to it not yet added to the four runs
     if (!skip) {   // warp-uniform: skip depends on the layer only
-      // columns x0 .. x0 + 31 of the group's 32 rows into buffer buf, one
-      // coalesced 128-byte row segment per copy instruction of the warp
-      auto stage_chunk = [&](int x0, uint32_t* buf) {
+      int from[4] = {0, 0, 0, 0};       // first column of the channel's open run
+      unsigned val[4] = {0, 0, 0, 0};   // its byte (write pass)
+      const int rows = (int)min(32ll, h - y0);
+      unsigned byte_of[4];              // channel slot -> mask of its byte in a pixel
+#pragma unroll
+      for (int s = 0; s < 4; ++s) byte_of[s] = 0xFFu << (8 * ((a.order >> (8 * s)) & 3));
+      const uint32_t* row0 = reinterpret_cast<const uint32_t*>(base) + y0 * w;
+      // columns x0 - 1 .. x0 + 31 of the group's rows (column -1 and the columns
+      // past the layer are not copied, and not looked at)
+      auto stage_chunk = [&](int x0) {
+        if (x0 > 0 && lane < rows) cp_async_word(buf + lane * kRlePitch + kRleFirst - 1, row0 + (long long)lane * w + x0 - 1);
+        if (x0 + lane < w) {
+          const uint32_t* q = row0 + x0 + lane;
+          uint32_t* d = buf + kRleFirst + lane;
 #pragma unroll 8
-        for (int r = 0; r < 32; ++r) {
-          const bool v = y0 + r < h && x0 + lane < w;
-          cp_async_word(buf + r * kRlePitch + lane, v ? base + ((y0 + r) * (long long)w + x0 + lane) * 4 : base, v);
+          for (int r = 0; r < rows; ++r, q += w, d += kRlePitch) cp_async_word(d, q);
         }
-        cp_async_commit();
       };
-      __syncwarp();   // every lane is done with both buffers (previous group)
-      stage_chunk(0, sm[0]);
-      int cur = 0;
-      for (int x0 = 0; x0 < w; x0 += 32, cur ^= 1) {
-        if (x0 + 32 < w) {
-          stage_chunk(x0 + 32, sm[cur ^ 1]);   // read by every lane in the previous iteration
-          cp_async_wait<1>();
-        } else {
-          cp_async_wait<0>();
-        }
+      __syncwarp();   // every lane is done with the buffer (previous group)
+      stage_chunk(0);
+      for (int x0 = 0; x0 < w; x0 += 32) {
+        cp_async_wait_all();
         __syncwarp();   // the lanes' copies of this chunk are visible to the whole warp
-        if (active) {
-          const int n = min(32, w - x0);
-          for (int x = 0; x < n; x += 4) {   // four pixels per 16-byte read
-            const uint4 q = *reinterpret_cast<const uint4*>(&sm[cur][lane * kRlePitch + x]);
-            // When all four bytes repeat, every run grows; such pixels are only
-            // counted, and added to the four runs when the pixel changes.  Four
-            // repeats are taken at once from one 16-byte read (2048x2048,
-            // N=20000 on a B200: count pass 12.5 -> 6.2 ms, write pass 14.7 ->
-            // 8.0 ms against a per-byte path on 4-byte reads).
-            if (x + 4 <= n && (unsigned long long)q.x == last && q.y == q.x && q.z == q.x && q.w == q.x) {
-              eq += 4;
-              continue;
-            }
-            const int k = min(4, n - x);
+        // Run starts of this lane's row per channel slot, in planes of eight bits:
+        // bit l of plane 0, 1, 2, 3 is pixel 4 l + 0, 2, 1, 3 of the chunk.
+        unsigned m[4] = {0, 0, 0, 0};
+        const int l = lane & 7, left_cols = w - x0 - 4 * l;   // columns of the layer from this lane's first on
+        const uint32_t* q = buf + (lane >> 3) * kRlePitch + kRleFirst + 4 * l;
+        const unsigned pick = (unsigned)(lane & 3);           // byte of a ballot that holds this lane's row
+        for (int k = 0; 4 * k < rows; ++k, q += 4 * kRlePitch) {
+          const bool row_in = 4 * k + (lane >> 3) < rows;
+          const uint4 p = *reinterpret_cast<const uint4*>(q);
+          uint32_t prev = __shfl_up_sync(0xffffffffu, p.w, 1);
+          if (l == 0) prev = x0 > 0 ? q[-1] : p.x;
+          uint32_t d[4] = {p.x ^ prev, p.y ^ p.x, p.z ^ p.y, p.w ^ p.z};
+          if (left_cols < 4 || !row_in) {   // columns or rows past the layer hold leftovers
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (j >= k) break;
-              const uint32_t p = j == 0 ? q.x : j == 1 ? q.y : j == 2 ? q.z : q.w;
-              if ((unsigned long long)p == last) {
-                ++eq;
-                continue;
-              }
+            for (int j = 0; j < 4; ++j)
+              if (j >= left_cols || !row_in) d[j] = 0u;
+          }
+          if (!WRITE && row_in) {
+            if (left_cols > 0) any_alpha |= p.x & 0xFF000000u;
+            if (left_cols > 1) any_alpha |= p.y & 0xFF000000u;
+            if (left_cols > 2) any_alpha |= p.z & 0xFF000000u;
+            if (left_cols > 3) any_alpha |= p.w & 0xFF000000u;
+          }
+          const uint32_t any = d[0] | d[1] | d[2] | d[3];
+          if (__any_sync(0xffffffffu, any != 0u)) {
 #pragma unroll
-              for (int s = 0; s < 4; ++s) e.run[s] += eq;
-              eq = 0;
-              last = p;
-              any_alpha |= p & 0xFF000000u;
+            for (int s = 0; s < 4; ++s) {
+              if (!__any_sync(0xffffffffu, any & byte_of[s])) continue;
+              unsigned b[4];
 #pragma unroll
-              for (int s = 0; s < 4; ++s) e.push(s, (p >> (8 * ((a.order >> (8 * s)) & 3))) & 0xFF);
+              for (int j = 0; j < 4; ++j) b[j] = __ballot_sync(0xffffffffu, d[j] & byte_of[s]);
+              const unsigned lo = __byte_perm(b[0], b[2], pick | (pick + 4) << 4);
+              const unsigned hi = __byte_perm(b[1], b[3], pick | (pick + 4) << 4);
+              if ((lane >> 2) == k) m[s] = __byte_perm(lo, hi, 0x5410);
             }
           }
         }
-        __syncwarp();   // every lane is done with this buffer before the next iteration refills it
+        if (!WRITE) {
+          __syncwarp();   // every lane is done with the buffer
+          if (x0 + 32 < w) stage_chunk(x0 + 32);
+        }
+        if (WRITE && x0 == 0) {
+          const uint32_t p = buf[lane * kRlePitch + kRleFirst];
+#pragma unroll
+          for (int s = 0; s < 4; ++s) val[s] = (p >> (8 * ((a.order >> (8 * s)) & 3))) & 0xFFu;
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          unsigned k = planes_to_columns(m[s]);
+          while (k) {
+            const int j = __ffs(k) - 1;
+            k &= k - 1;
+            const int x = x0 + j;
+            e[s].run(x - from[s], val[s]);
+            from[s] = x;
+            if (WRITE) val[s] = (buf[lane * kRlePitch + kRleFirst + j] >> (8 * ((a.order >> (8 * s)) & 3))) & 0xFFu;
+          }
+        }
+        if (WRITE) {
+          __syncwarp();   // every lane is done with the buffer
+          if (x0 + 32 < w) stage_chunk(x0 + 32);
+        }
       }
       if (active) {
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-          e.run[s] += eq;
-          e.finish(s);
+          e[s].run(w - from[s], val[s]);
+          e[s].finish();
         }
       }
     }
-    if (!WRITE) {
+    if constexpr (!WRITE) {
       int c[4];
 #pragma unroll
-      for (int s = 0; s < 4; ++s) c[s] = active && !skip ? (int)e.pos[s] : 0;
+      for (int s = 0; s < 4; ++s) c[s] = active && !skip ? e[s].pos : 0;
       reinterpret_cast<ushort4*>(a.row_bytes)[g * 32 + lane] =
           make_ushort4((unsigned short)c[0], (unsigned short)c[1], (unsigned short)c[2], (unsigned short)c[3]);
 #pragma unroll
@@ -605,26 +632,6 @@ __global__ void __launch_bounds__(kRleWarps * 32) psd_rle_kernel(RleArgs a) {
   }
 }
 
-// CTAs of psd_rle_kernel<write> resident at once on the current device,
-// computed once per (device, pass) under a lock (devices may differ).
-static int rle_resident_ctas(bool write) {
-  constexpr int kMaxDevices = 64;
-  static std::mutex mu;
-  static int resident[kMaxDevices][2] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
-  std::lock_guard<std::mutex> lock(mu);
-  int& r = resident[dev][write ? 1 : 0];
-  if (r == 0) {
-    int per_sm = 0, sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (write) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psd_rle_kernel<true>, kRleWarps * 32, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, psd_rle_kernel<false>, kRleWarps * 32, 0);
-    r = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 148);
-  }
-  return r;
-}
-
 int launch_psd_rle(bool write, const uint8_t* layers, const int* sizes, const long long* layer_off,
                    const long long* group_base, int N, long long G, unsigned order, int width_limit,
                    unsigned short* row_bytes, int* group_tot, int* alpha_any, const long long* chan_off,
@@ -632,11 +639,11 @@ int launch_psd_rle(bool write, const uint8_t* layers, const int* sizes, const lo
   if (G == 0 || N == 0) return DBMP_OK;
   const RleArgs a{layers, sizes, layer_off, group_base, G, N, order, width_limit, row_bytes, group_tot,
                   alpha_any, chan_off, group_dst, out, out_bytes};
-  // Persistent grid: as many CTAs as are resident at once (the device's SMs x
-  // the kernel's occupancy), so the grid-stride loop balances the row groups.
-  const int resident = rle_resident_ctas(write);
+  // One group per warp, so that the SMs refill as groups of uneven width finish
+  // (a persistent grid-stride loop left them a third empty on average); the loop
+  // only serves counts beyond a grid's limit.
   long long ctas = (G + kRleWarps - 1) / kRleWarps;
-  if (ctas > resident) ctas = resident;
+  if (ctas > 0x7fffffffll) ctas = 0x7fffffffll;
   if (write) psd_rle_kernel<true><<<(int)ctas, kRleWarps * 32, 0, st>>>(a);
   else psd_rle_kernel<false><<<(int)ctas, kRleWarps * 32, 0, st>>>(a);
   DBMP_CHECK_LAUNCH("psd_rle_kernel");
