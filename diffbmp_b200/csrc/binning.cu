@@ -431,7 +431,8 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
                                                                   int* __restrict__ tile_offsets,
                                                                   int* __restrict__ total_out,
                                                                   int* __restrict__ overflow_out,
-                                                                  long long flag_stride) {
+                                                                  long long flag_stride,
+                                                                  volatile int* host_flags) {
   // Two compaction buffers: chunk c is compacted into buffer c & 1 while the
   // warps may still read chunk c - 1 from the other one, so one barrier per
   // chunk orders everything (see the loop).
@@ -462,6 +463,12 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
     if (first) {
       if (total_out) total_out[cand * flag_stride] = (int)min(L, (long long)INT_MAX);
       if (overflow_out) overflow_out[cand * flag_stride] = (L > cap) ? 1 : 0;
+      if (host_flags) {   // the host polls the second word
+        host_flags[2 * cand] = (int)min(L, (long long)INT_MAX);
+        __threadfence_system();
+        host_flags[2 * cand + 1] = (L > cap) ? 1 : 0;
+        __threadfence_system();
+      }
     }
     if (L > cap) return;   // uniform over the CTA
     if (first) tile_offsets[g.T] = (int)L;
@@ -907,7 +914,8 @@ int launch_prepare(const Geom& g, const float* means2D, const float* radii, cons
 int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
                const float* opac, const float* colors, const int* sel, long long sel_stride, const float* tbbox,
                PrimInfo* prim_info, int* tile_offsets, int* tile_indices, long long index_stride, long long cap,
-               int* total_out, int* overflow_out, long long flag_stride, void* ws, size_t ws_bytes, cudaStream_t st) {
+               int* total_out, int* overflow_out, long long flag_stride, int* host_flags, void* ws, size_t ws_bytes,
+               cudaStream_t st) {
   const BinGrid bg = bin_grid(g.N, g.tilesX, g.tilesY);
   BinWorkspace w{};
   const size_t need = layout_ws(ws, batch, g.N, g.T, g.tilesX, g.tilesY, bg, &w);
@@ -937,7 +945,7 @@ int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, con
   if (rc) return rc;
   return launch_chained("bin_rows_kernel", bin_rows_kernel, dim3((unsigned)bg.ctas, batch), kBinThreads, 0, st, g, bg,
                         (const int4*)w.rects, (const long long*)w.offs, cap, tile_indices, index_stride, tile_offsets,
-                        total_out, overflow_out, flag_stride);
+                        total_out, overflow_out, flag_stride, (volatile int*)host_flags);
 }
 
 }  // namespace dbmp

@@ -1,4 +1,6 @@
 // C ABI of libdbmp.so (declarations and contracts in include/dbmp.h).
+#include <atomic>
+#include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -28,18 +30,22 @@ int launch_template_bboxes(const float* tmpl, int P, int Ht, int Wt, float* out,
 int launch_template_blur(const float* in, int P, int Ht, int Wt, float sigma, float* out, cudaStream_t st);
 int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
 int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
+int launch_convert(int n, const void* const* src, void* const* dst, const long long* counts, bool to_half,
+                   cudaStream_t st);
 int launch_zero(double* a, long long n, double* b, cudaStream_t st);
 int launch_prepare(const Geom& g, const float* means2D, const float* radii, const float* rot, const float* opac,
                    const float* colors, const int* sel, PrimInfo* out, cudaStream_t st);
 int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
                const float* opac, const float* colors, const int* sel, long long sel_stride, const float* tbbox,
                PrimInfo* prim_info, int* tile_offsets, int* tile_indices, long long index_stride, long long cap,
-               int* total_out, int* overflow_out, long long flag_stride, void* ws, size_t ws_bytes, cudaStream_t st);
+               int* total_out, int* overflow_out, long long flag_stride, int* host_flags, void* ws, size_t ws_bytes,
+               cudaStream_t st);
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                    const int* idx, float* color, float* alpha, float* T_last, int* last_pos, cudaStream_t st);
 int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                          const int* idx, float* color, float* alpha, float* T_last, int* last_pos, const float* cmap,
-                         float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride);
+                         float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride,
+                         const int* flags);
 int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                           const int* idx, const float* T_last, const int* last_pos, const float* grad_color,
                           const float* grad_alpha, double* gacc, const float* cmap, float cblend, cudaStream_t st,
@@ -233,7 +239,33 @@ int dbmp_bin(const dbmp_canvas* cv, const float* means2D, const float* radii, co
           "dbmp_bin: prim_info must be 16-byte and workspace 256-byte aligned");
   return launch_bin(g, 1, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, 0, tmpl_bbox,
                     (PrimInfo*)prim_info, tile_offsets, tile_indices, 0, capacity, total_out, overflow_out, 0,
-                    workspace, workspace_bytes, (cudaStream_t)stream);
+                    nullptr, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+static int bin_checked(const Geom& g, const char* who, const dbmp_canvas* cv, int batch, const float* means2D,
+                       const float* radii, const float* rotations, const float* opacities, const float* colors,
+                       const int32_t* sel, long long sel_stride, const float* tmpl_bbox, void* prim_info,
+                       int32_t* tile_offsets, int32_t* tile_indices, long long index_stride, long long capacity,
+                       int32_t* total_and_overflow, int32_t* host_flags, void* workspace, size_t workspace_bytes,
+                       cudaStream_t st) {
+  REQUIRE(batch >= 0, "%s: batch %d < 0", who, batch);
+  if (batch == 0) return DBMP_OK;
+  REQUIRE(cv->bin_mode == DBMP_BIN_CONTENT || cv->bin_mode == DBMP_BIN_CULL || cv->bin_mode == DBMP_BIN_CONTENT_REF,
+          "%s: bin_mode %d unknown", who, cv->bin_mode);
+  REQUIRE(g.N == 0 || (means2D && radii && rotations && opacities && colors && sel && prim_info), "%s: null pointer",
+          who);
+  REQUIRE(cv->bin_mode == DBMP_BIN_CULL || tmpl_bbox, "%s: tmpl_bbox is required in the DBMP_BIN_CONTENT modes", who);
+  REQUIRE(tile_offsets && total_and_overflow && workspace, "%s: null output or workspace", who);
+  REQUIRE(capacity >= 0 && capacity <= 0x7fffffffll, "%s: capacity %lld outside [0, 2^31)", who, capacity);
+  REQUIRE(capacity <= index_stride || batch == 1, "%s: index_stride %lld below the capacity %lld", who, index_stride,
+          capacity);
+  REQUIRE(capacity == 0 || tile_indices, "%s: tile_indices is null", who);
+  REQUIRE(sel_stride == 0 || sel_stride >= g.N, "%s: sel_stride %lld", who, sel_stride);
+  REQUIRE(((uintptr_t)prim_info & 15) == 0 && ((uintptr_t)workspace & 255) == 0,
+          "%s: prim_info must be 16-byte and workspace 256-byte aligned", who);
+  return launch_bin(g, batch, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, sel_stride, tmpl_bbox,
+                    (PrimInfo*)prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
+                    total_and_overflow + 1, 2, host_flags, workspace, workspace_bytes, st);
 }
 
 int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii,
@@ -244,25 +276,72 @@ int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const
   Geom g;
   int rc = make_geom(cv, &g, "dbmp_bin_batch");
   if (rc) return rc;
-  REQUIRE(batch >= 0, "dbmp_bin_batch: batch %d < 0", batch);
+  return bin_checked(g, "dbmp_bin_batch", cv, batch, means2D, radii, rotations, opacities, colors, sel, sel_stride,
+                     tmpl_bbox, prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
+                     nullptr, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii, const float* rotations,
+                const float* opacities, const float* colors, const int32_t* sel, long long sel_stride,
+                const float* tmpl_bbox, const void* atlas, void* prim_info, int32_t* tile_offsets,
+                int32_t* tile_indices, long long index_stride, long long capacity, int32_t* total_and_overflow,
+                int32_t* host_flags, const float* colors_orig, long long colors_orig_stride, float c_blend,
+                float* out_color, float* out_alpha, float* T_last, int32_t* last_pos, void* workspace,
+                size_t workspace_bytes, void* stream) {
+  Geom g;
+  int rc = make_geom(cv, &g, "dbmp_render");
+  if (rc) return rc;
   if (batch == 0) return DBMP_OK;
-  REQUIRE(cv->bin_mode == DBMP_BIN_CONTENT || cv->bin_mode == DBMP_BIN_CULL || cv->bin_mode == DBMP_BIN_CONTENT_REF,
-          "dbmp_bin_batch: bin_mode %d unknown", cv->bin_mode);
-  REQUIRE(g.N == 0 || (means2D && radii && rotations && opacities && colors && sel && prim_info),
-          "dbmp_bin_batch: null pointer");
-  REQUIRE(cv->bin_mode == DBMP_BIN_CULL || tmpl_bbox,
-          "dbmp_bin_batch: tmpl_bbox is required in the DBMP_BIN_CONTENT modes");
-  REQUIRE(tile_offsets && total_and_overflow && workspace, "dbmp_bin_batch: null output or workspace");
-  REQUIRE(capacity >= 0 && capacity <= 0x7fffffffll, "dbmp_bin_batch: capacity %lld outside [0, 2^31)", capacity);
-  REQUIRE(capacity <= index_stride || batch == 1, "dbmp_bin_batch: index_stride %lld below the capacity %lld",
-          index_stride, capacity);
-  REQUIRE(capacity == 0 || tile_indices, "dbmp_bin_batch: tile_indices is null");
-  REQUIRE(sel_stride == 0 || sel_stride >= g.N, "dbmp_bin_batch: sel_stride %lld", sel_stride);
-  REQUIRE(((uintptr_t)prim_info & 15) == 0 && ((uintptr_t)workspace & 255) == 0,
-          "dbmp_bin_batch: prim_info must be 16-byte and workspace 256-byte aligned");
-  return launch_bin(g, batch, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, sel_stride, tmpl_bbox,
-                    (PrimInfo*)prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
-                    total_and_overflow + 1, 2, workspace, workspace_bytes, (cudaStream_t)stream);
+  REQUIRE(atlas && out_color && out_alpha && T_last && last_pos && host_flags, "dbmp_render: null pointer");
+  REQUIRE(colors_orig_stride >= 0, "dbmp_render: negative stride");
+  REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_render: c_blend %g outside [0, 1]", (double)c_blend);
+  REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_render: colors_orig is null with c_blend > 0");
+  REQUIRE((long long)batch * g.T * 4 <= 0x7fffffffll, "dbmp_render: %d candidates x %d tiles exceed one grid", batch, g.T);
+  // the host waits for the flags, which a captured launch would never write
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing((cudaStream_t)stream, &cap);
+  if (e != cudaSuccess) return cuda_status(e, "dbmp_render: cudaStreamIsCapturing");
+  REQUIRE(cap == cudaStreamCaptureStatusNone, "dbmp_render: cannot be captured in a CUDA graph (the list length is "
+          "read on the host)");
+  for (int b = 0; b < batch; ++b) host_flags[2 * b + 1] = -1;
+  rc = bin_checked(g, "dbmp_render", cv, batch, means2D, radii, rotations, opacities, colors, sel, sel_stride,
+                   tmpl_bbox, prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
+                   host_flags, workspace, workspace_bytes, (cudaStream_t)stream);
+  if (rc) return rc;
+  // the forward runs behind the binning without waiting for the host; a
+  // candidate whose lists overflowed renders nothing
+  return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
+                              out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream,
+                              batch, index_stride, colors_orig_stride, total_and_overflow);
+}
+
+int dbmp_convert_half(int n, const void* const* src, void* const* dst, const long long* counts, int to_half,
+                      void* stream) {
+  REQUIRE(n >= 0 && n <= 8, "dbmp_convert_half: %d arrays outside [0, 8]", n);
+  REQUIRE(n == 0 || (src && dst && counts), "dbmp_convert_half: null pointer");
+  for (int k = 0; k < n; ++k) {
+    REQUIRE(counts[k] >= 0, "dbmp_convert_half: negative count");
+    REQUIRE(counts[k] == 0 || (src[k] && dst[k]), "dbmp_convert_half: null array");
+  }
+  return launch_convert(n, src, dst, counts, to_half != 0, (cudaStream_t)stream);
+}
+
+int dbmp_render_wait(const int32_t* host_flags, int batch, void* stream) {
+  REQUIRE(host_flags && batch >= 0, "dbmp_render_wait: null pointer");
+  const volatile int32_t* f = host_flags;
+  const auto t0 = std::chrono::steady_clock::now();
+  for (int b = 0; b < batch; ++b) {
+    for (unsigned spin = 1; f[2 * b + 1] < 0; ++spin) {
+      if (spin % 4096 != 0) continue;
+      // a launch that failed, or a stream busy for long: wait for it as usual
+      if (std::chrono::steady_clock::now() - t0 < std::chrono::seconds(2)) continue;
+      const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+      if (e != cudaSuccess) return cuda_status(e, "dbmp_render_wait: cudaStreamSynchronize");
+      REQUIRE(f[2 * b + 1] >= 0, "dbmp_render_wait: the binning did not report");
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return DBMP_OK;
 }
 
 int dbmp_forward(const dbmp_canvas* cv, const void* prim_info, const void* atlas, const int32_t* tile_offsets,
@@ -327,7 +406,7 @@ int dbmp_forward_blend(const dbmp_canvas* cv, const void* prim_info, const void*
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_forward_blend: colors_orig is null with c_blend > 0");
   return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream, 1,
-                              0, 0);
+                              0, 0, nullptr);
 }
 
 int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void* atlas, const int32_t* tile_offsets,
@@ -373,7 +452,7 @@ int dbmp_forward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, 
   REQUIRE(((uintptr_t)prim_info & 15) == 0, "dbmp_forward_batch: prim_info must be 16-byte aligned");
   return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream,
-                              batch, index_stride, colors_orig_stride);
+                              batch, index_stride, colors_orig_stride, nullptr);
 }
 
 int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, const void* atlas,

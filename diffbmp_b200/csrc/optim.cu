@@ -135,6 +135,42 @@ __global__ void step_increment_kernel(int* __restrict__ step_count, const int* _
 }
 
 // ---------------------------------------------------------------------------
+// Half <-> float conversion of several arrays in one launch (blockIdx.y: the
+// array), for callers that hold a job's tensors in FP16.
+struct ConvertArgs {
+  const void* src[8];
+  void* dst[8];
+  long long count[8];
+};
+
+template <bool TO_HALF>
+__global__ void __launch_bounds__(256) convert_kernel(ConvertArgs a) {
+  grid_dependency();
+  const int k = blockIdx.y;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.count[k]; i += (long long)gridDim.x * blockDim.x) {
+    if (TO_HALF) static_cast<__half*>(a.dst[k])[i] = __float2half_rn(static_cast<const float*>(a.src[k])[i]);
+    else static_cast<float*>(a.dst[k])[i] = __half2float(static_cast<const __half*>(a.src[k])[i]);
+  }
+}
+
+int launch_convert(int n, const void* const* src, void* const* dst, const long long* counts, bool to_half,
+                   cudaStream_t st) {
+  ConvertArgs a{};
+  long long most = 0;
+  for (int k = 0; k < n; ++k) {
+    a.src[k] = src[k];
+    a.dst[k] = dst[k];
+    a.count[k] = counts[k];
+    most = counts[k] > most ? counts[k] : most;
+  }
+  if (most == 0) return DBMP_OK;
+  const long long ctas = (most + 255) / 256;
+  const dim3 grid((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8), n);
+  return to_half ? launch_chained("convert_kernel", convert_kernel<true>, grid, 256, 0, st, a)
+                 : launch_chained("convert_kernel", convert_kernel<false>, grid, 256, 0, st, a);
+}
+
+// ---------------------------------------------------------------------------
 // Pruning (restart) of low-opacity primitives: the reference's do_prune
 // (simple_tile_renderer.py:1007-1013 schedule, :1236-1270 selection and
 // replacement) as one CTA.  Primitives with sigmoid(v) < threshold, in

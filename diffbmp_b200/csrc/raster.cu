@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
-    long long idx_stride, long long cmap_stride) {
+    long long idx_stride, long long cmap_stride, const int* __restrict__ flags) {
   grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
@@ -843,6 +843,9 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
   // records, lists and images follow candidate b-1's
   const int gt = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;
+  // binning overflowed for a candidate: its lists do not exist, and the caller
+  // bins again (flags: list length and overflow per candidate)
+  if (flags != nullptr && flags[2 * b + 1] != 0) return;
   const size_t pix = (size_t)b * g.H * g.W;
   prims += (size_t)b * g.N;
   offs += (size_t)b * (g.T + 1);
@@ -1064,25 +1067,26 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fu
 // images at b H W (x3 for colour), colour maps at cmap + b cmap_stride.
 int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                          const int* idx, float* color, float* alpha, float* T_last, int* last_pos, const float* cmap,
-                         float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride) {
+                         float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride,
+                         const int* flags) {
   if (g.T == 0 || batch == 0) return DBMP_OK;
   const long long ctas = (long long)batch * g.T * kParts<32>();
   if (ctas > 0x7fffffffll) { set_error("forward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
   if (cmap != nullptr && cblend > 0.f) {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
         "forward_kernel", forward_kernel<TSV, KD, true>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
-        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride)));
+        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride, flags)));
   } else {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
         "forward_kernel", forward_kernel<TSV, KD, false>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
-        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll)));
+        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll, flags)));
   }
 }
 
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                    const int* idx, float* color, float* alpha, float* T_last, int* last_pos, cudaStream_t st) {
   return launch_forward_blend(g, kind, prims, atlas, offs, idx, color, alpha, T_last, last_pos, nullptr, 0.f, st, 1,
-                              0, 0);
+                              0, 0, nullptr);
 }
 
 int launch_count(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs, const int* idx,

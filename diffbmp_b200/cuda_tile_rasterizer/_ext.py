@@ -9,6 +9,7 @@ Every computation runs in the library's CUDA kernels; there is no fallback.
 """
 from __future__ import annotations
 
+import ctypes
 import time
 
 import torch
@@ -63,13 +64,40 @@ def _f(t):
     return t.detach().to(torch.float32).contiguous()
 
 
+def _convert(ts, dtype):
+    """Contiguous CUDA tensors of one device and one dtype to the other of float16
+    / float32, in one launch per eight."""
+    out = [torch.empty(t.shape, dtype=dtype, device=t.device) for t in ts]
+    for k in range(0, len(ts), 8):
+        a, b = ts[k:k + 8], out[k:k + 8]
+        n = len(a)
+        R.call("dbmp_convert_half", n, (ctypes.c_void_p * n)(*[t.data_ptr() for t in a]),
+               (ctypes.c_void_p * n)(*[t.data_ptr() for t in b]), (ctypes.c_longlong * n)(*[t.numel() for t in a]),
+               int(dtype is torch.float16), R._stream())
+    return out
+
+
+def _floats(*ts):
+    """Each tensor (or None) as contiguous f32, the half ones converted together."""
+    out = [t if t is None else t.detach() for t in ts]
+    todo = [k for k, t in enumerate(out) if t is not None and t.dtype is torch.float16 and t.is_cuda
+            and t.is_contiguous()]
+    for k, t in zip(todo, _convert([out[k] for k in todo], torch.float32)):
+        out[k] = t
+    return [t if t is None else R._operand(t) for t in out]
+
+
+def _halves(ts):
+    return tuple(_convert([t.contiguous() for t in ts], torch.float16))
+
+
 def forward(fp16, means2D, radii, rotations, opacities, colors, colors_orig, templates, sel, c_blend, mapping,
             keep=True):
     g = _get(fp16)
     t0 = time.perf_counter()
     atlas = g.get_atlas(templates)
-    m, r, th, v, c = _f(means2D).view(-1, 2), _f(radii).view(-1), _f(rotations).view(-1), _f(opacities).view(-1), \
-        _f(colors).view(-1, 3)
+    m, r, th, v, c = _floats(means2D, radii, rotations, opacities, colors)
+    m, r, th, v, c = m.view(-1, 2), r.view(-1), th.view(-1), v.view(-1), c.view(-1, 3)
     s = sel.to(torch.int32).contiguous().view(-1)
     has_map = mapping is not None and isinstance(mapping, torch.Tensor) and mapping.numel() > 0
     rz = g.rz_map if has_map else g.rz_cull
@@ -83,7 +111,7 @@ def forward(fp16, means2D, radii, rotations, opacities, colors, colors_orig, tem
     g.t_fwd += (time.perf_counter() - t0) * 1e3
     g.n_fwd += 1
     if fp16:
-        return color.half(), alpha.half()
+        return _halves((color, alpha))
     return color, alpha, (state, rz, atlas)
 
 
@@ -95,14 +123,12 @@ def backward(fp16, grad_color, grad_alpha, radii, rotations, opacities, colors, 
         saved = g.states[-1]
     state, rz, atlas = saved
     t0 = time.perf_counter()
-    gm, gr, gth, gv, gc = rz.backward(state, _f(grad_color), None if grad_alpha is None else _f(grad_alpha),
-                                      _f(radii).view(-1), _f(rotations).view(-1), _f(opacities).view(-1),
-                                      _f(colors).view(-1, 3), atlas)
+    gcol, galp, r, th, v, c = _floats(grad_color, grad_alpha, radii, rotations, opacities, colors)
+    out = rz.backward(state, gcol, galp, r.view(-1), th.view(-1), v.view(-1), c.view(-1, 3), atlas)
+    if fp16:
+        out = _halves(out)
     g.t_bwd += (time.perf_counter() - t0) * 1e3
     g.n_bwd += 1
-    out = (gm, gr, gth, gv, gc)
-    if fp16:
-        out = tuple(x.half() for x in out)
     return out
 
 
@@ -117,9 +143,8 @@ def forward_batch(fp16, means2D, radii, rotations, opacities, colors, colors_ori
     t0 = time.perf_counter()
     atlas = g.get_atlas(templates)
     B = int(radii.shape[0])
-    m = _f(means2D).view(B, -1, 2)
-    r, th, v = _f(radii).view(B, -1), _f(rotations).view(B, -1), _f(opacities).view(B, -1)
-    c = _f(colors).view(B, -1, 3)
+    m, r, th, v, c = _floats(means2D, radii, rotations, opacities, colors)
+    m, r, th, v, c = m.view(B, -1, 2), r.view(B, -1), th.view(B, -1), v.view(B, -1), c.view(B, -1, 3)
     s = sel.to(torch.int32).contiguous()
     if isinstance(mappings, torch.Tensor):
         mappings = [mappings] * B if mappings.numel() > 0 else None
@@ -134,7 +159,7 @@ def forward_batch(fp16, means2D, radii, rotations, opacities, colors, colors_ori
     g.t_fwd += (time.perf_counter() - t0) * 1e3
     g.n_fwd += 1
     if fp16:
-        return color.half(), alpha.half()
+        return _halves((color, alpha))
     return color, alpha
 
 
@@ -149,13 +174,12 @@ def backward_batch(fp16, grad_color, grad_alpha, radii, rotations, opacities, co
     if state.batch != B:
         raise RuntimeError(f"backward_batch of {B} candidates after a forward_batch of {state.batch}")
     t0 = time.perf_counter()
-    out = rz.backward_batch(state, _f(grad_color), None if grad_alpha is None else _f(grad_alpha),
-                            _f(radii).view(B, -1), _f(rotations).view(B, -1), _f(opacities).view(B, -1),
-                            _f(colors).view(B, -1, 3), atlas)
+    gcol, galp, r, th, v, c = _floats(grad_color, grad_alpha, radii, rotations, opacities, colors)
+    out = rz.backward_batch(state, gcol, galp, r.view(B, -1), th.view(B, -1), v.view(B, -1), c.view(B, -1, 3), atlas)
+    if fp16:
+        out = _halves(out)
     g.t_bwd += (time.perf_counter() - t0) * 1e3
     g.n_bwd += 1
-    if fp16:
-        out = tuple(x.half() for x in out)
     return out
 
 

@@ -119,7 +119,8 @@ def encode_channel_blocks(buf, sizes, offsets, host_sizes, order, select, width_
     Returns (blob, block_bytes, chosen): the device uint8 blob of PSD channel
     blocks (4 per chosen image, slots in ``order``, each = compression word,
     big-endian row sizes, PackBits rows), the (len(chosen), 4) block sizes and
-    the chosen indices.  The host reads back only per-group sizes and flags.
+    the chosen indices.  The host reads back only the block sizes and flags; the
+    groups' destinations are summed on the device.
     """
     dev = buf.device
     hs = np.asarray(host_sizes, dtype=np.int64).reshape(-1, 2)
@@ -130,30 +131,40 @@ def encode_channel_blocks(buf, sizes, offsets, host_sizes, order, select, width_
     group_base[1:] = np.cumsum(ngroups)
     G = int(group_base[-1])
     st = _stream(stream)
-    gb = torch.from_numpy(group_base).to(dev)
+    # group_base, then heights and group counts for the plan, in one copy
+    meta = torch.from_numpy(np.concatenate([group_base, h, ngroups])).to(dev)
+    gb, hd, ng = meta[:n + 1], meta[n + 1:2 * n + 1], meta[2 * n + 1:]
     row_bytes = torch.empty(max(G, 1) * 32 * 4, dtype=torch.int16, device=dev)
     group_tot = torch.empty((max(G, 1), 4), dtype=torch.int32, device=dev)
     alpha_any = torch.zeros(max(n, 1), dtype=torch.int32, device=dev)
     call("dbmp_psd_rle_count", _ptr(buf), _ptr(sizes), _ptr(offsets), _ptr(gb), n, G, _check_order(order),
          int(width_limit), _ptr(row_bytes), _ptr(group_tot), _ptr(alpha_any), st)
-    gt = group_tot[:G].cpu().numpy().astype(np.int64)
-    chosen = np.asarray(select(alpha_any[:n].cpu().numpy()), dtype=np.int64).reshape(-1)
-    if len(np.unique(chosen)) != len(chosen) or (len(chosen) and (chosen.min() < 0 or chosen.max() >= n)):
+    # encoded bytes before each group (one running sum over the four slots in turn)
+    # and of each image's four blocks; the host reads the blocks and the alpha
+    # flags in one copy
+    cs = torch.zeros(4 * G + 1, dtype=torch.int64, device=dev)
+    torch.cumsum(group_tot[:G].t().reshape(-1), 0, dtype=torch.int64, out=cs[1:])
+    slot = torch.arange(4, device=dev)[:, None] * G
+    edge = cs[slot + gb]                                                         # (4,n+1) before each image
+    head = 2 + 2 * hd
+    host = torch.cat([head + edge[:, 1:] - edge[:, :-1], alpha_any[None, :n].to(torch.int64)]).cpu().numpy().T
+    block = host[:, :4]                                                          # (n,4) bytes per block
+    chosen = np.asarray(select(host[:, 4].astype(np.int32)), dtype=np.int64).reshape(-1)
+    seen = np.zeros(n, bool)
+    if len(chosen) and chosen.min() >= 0 and chosen.max() < n:
+        seen[chosen] = True
+    if int(seen.sum()) != len(chosen):
         raise ValueError("select must return distinct image indices")
-    cs = np.zeros((G + 1, 4), np.int64)
-    cs[1:] = np.cumsum(gt, axis=0)
-    block = 2 + 2 * h[:, None] + (cs[group_base[1:]] - cs[group_base[:-1]])      # (n,4) bytes per block
     chan_off = np.full((n, 4), -1, np.int64)
     flat = block[chosen].reshape(-1)
     starts = np.concatenate([[0], np.cumsum(flat)[:-1]]) if len(flat) else flat
     chan_off[chosen] = starts.reshape(-1, 4)
     total = int(flat.sum())
-    layer_of = np.repeat(np.arange(n), ngroups)
-    gdst = chan_off[layer_of] + 2 + 2 * h[layer_of, None] + (cs[:-1] - cs[group_base[layer_of]])
-    gdst[chan_off[layer_of] < 0] = -1
     out = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
     co = torch.from_numpy(chan_off).to(dev)
-    gd = torch.from_numpy(np.ascontiguousarray(gdst)).to(dev)
+    # where each group's first row goes: its block, the block's header, the groups before it
+    dst = torch.where(co.t() >= 0, co.t() + head - edge[:, :-1], -1 << 62)
+    gd = (torch.repeat_interleave(dst, ng, 1, output_size=G) + cs[:-1].view(4, G)).clamp_(min=-1).t().contiguous()
     call("dbmp_psd_rle_write", _ptr(buf), _ptr(sizes), _ptr(offsets), _ptr(gb), n, G, _check_order(order),
          int(width_limit), _ptr(row_bytes), _ptr(co), _ptr(gd), _ptr(out), total, st)
     return out[:total], block[chosen], chosen

@@ -76,14 +76,18 @@ class SimpleTileRenderer:
         self.primitive_bboxes = [tuple(b) for b in self._atlas.bbox.tolist()]
         self._rz = Rasterizer(self.H, self.W, self.tile_size, self.alpha_upper_bound, device=self.device)
         self.cuda_rasterizer = self._rz
+        self._sel = None
 
     # -- helpers -------------------------------------------------------------
     def _num_templates(self) -> int:
         return self._atlas.P
 
     def _global_bmp_sel(self, N: int) -> torch.Tensor:
-        """Template of primitive i: (N-1-i) % p (simple_tile_renderer.py:221-224)."""
-        return (torch.arange(N, device=self.device, dtype=torch.int32) % self._num_templates()).flip(0).contiguous()
+        """Template of primitive i: (N-1-i) % p (simple_tile_renderer.py:221-224); the
+        last N's assignment is kept."""
+        if self._sel is None or self._sel.numel() != N:
+            self._sel = (torch.arange(N, device=self.device, dtype=torch.int32) % self._num_templates()).flip(0).contiguous()
+        return self._sel
 
     def _atlas_for(self, is_final: bool) -> Atlas:
         return self._atlas_blurred if (self._atlas_blurred is not None and not is_final) else self._atlas
@@ -199,8 +203,11 @@ class SimpleTileRenderer:
                           c.detach().float(), sel, atlas, target_image.to(self.device).float(), bg, cfg,
                           device=self.device)
         for k in range(cfg.num_iterations):
-            if k == 1:
-                job.capture()           # iteration 0 ran eagerly; the rest replay one graph
+            # iteration 0 runs eagerly; a longer fit replays one graph for the rest
+            # (capturing and instantiating it takes about 1.1 ms, an eager step of
+            # the host about 80 us)
+            if k == 1 and cfg.num_iterations > 16:
+                job.capture()
             job.step()
         job.sync()
         self.last_loss = job.loss()

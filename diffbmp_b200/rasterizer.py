@@ -43,12 +43,13 @@ DEFAULT_T_STOP = 1e-6   # image error <= t_stop * max colour, well inside the 1e
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need_cuda(*ts):
@@ -59,6 +60,11 @@ def _need_cuda(*ts):
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
     return t.detach().to(torch.float32).contiguous()
+
+
+def _operand(t: torch.Tensor) -> torch.Tensor:
+    """t as a kernel operand: itself where it is contiguous f32 already."""
+    return t if t.dtype is torch.float32 and t.is_contiguous() else _f32(t)
 
 
 class Atlas:
@@ -217,10 +223,15 @@ class Rasterizer:
         self.tiles_x = (self.W + self.ts - 1) // self.ts
         self.tiles_y = (self.H + self.ts - 1) // self.ts
         self.T = self.tiles_x * self.tiles_y
+        # a fit job's persistent lists and binning workspace (_ensure); the
+        # renders allocate theirs per call, so that calls on other streams or
+        # threads never share them
         self.capacity = 0
         self._ws = None
         self._idx = None
-        self._small = torch.zeros(2, dtype=torch.int32, device=self.device)   # total L, overflow flag
+        self._hint = None          # list capacity of the next render
+        self._ws_need = (None, 0)  # workspace bytes of the last (batch, N)
+        self._pins = []            # pinned flag buffers not in use
 
     def canvas(self, N: int, atlas: Atlas) -> Canvas:
         atlas.refresh()
@@ -228,18 +239,50 @@ class Rasterizer:
                       self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.extended else 0)
 
     # -- binning -----------------------------------------------------------
-    def _ensure(self, cv: Canvas, cap: int, nbytes: int = 0):
-        """Scratch for lists of `cap` entries, and nbytes of workspace at least."""
+    def _ensure(self, cv: Canvas, cap: int):
         if cap > self.capacity or self._ws is None:
             self.capacity = int(cap)
             self._idx = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=self.device)
-        nbytes = max(nbytes, int(lib.dbmp_bin_workspace_bytes(ctypes.byref(cv), self.capacity)))
+        nbytes = int(lib.dbmp_bin_workspace_bytes(ctypes.byref(cv), self.capacity))
         if self._ws is None or self._ws.numel() < nbytes + 256:
             self._ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=self.device)
 
     def _ws_ptr(self):
         base = self._ws.data_ptr()
         return ctypes.c_void_p((base + 255) & ~255), self._ws.numel() - 256
+
+    def _scratch(self, cv: Canvas, B: int, N: int, stream):
+        """(tensor, workspace bytes): a binning's workspace, followed by two ints
+        per candidate for its flags."""
+        if self._ws_need[0] != (B, N):
+            need = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), B))
+            self._ws_need = ((B, N), (need + 255) & ~255)
+        nbytes = self._ws_need[1]
+        t = torch.empty(nbytes + 8 * B, dtype=torch.uint8, device=self.device)
+        if stream is not None:      # freed while that stream may still use it
+            t.record_stream(stream)
+        return t, nbytes
+
+    @staticmethod
+    def _flat_batch(ts, stream):
+        """The tensors contiguous: the batch calls step from candidate to candidate
+        by N, but candidates may come strided or expanded."""
+        out = [t.contiguous() for t in ts]
+        if stream is not None:
+            for t, o in zip(ts, out):
+                if o is not t:
+                    o.record_stream(stream)
+        return out
+
+    def _capacity(self, N: int) -> int:
+        """List entries to provide per candidate: 1.25 times the longest lists so
+        far, at first an eighth of all (tile, primitive) pairs up to 16 MB."""
+        if self._hint is None:
+            self._hint = min(N * self.T, max(N * self.T // 8, 1024) + 4096, 4 << 20)
+        return self._hint
+
+    def _grow_hint(self, L: int):
+        self._hint = min(max(self._hint, int(L * 1.25) + 4096), 0x7fffffff)
 
     def bin(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None):
         """Device binning.  Returns (prim_info, TileLists).  Synchronises once
@@ -249,20 +292,59 @@ class Rasterizer:
         st = _stream(stream)
         prim_info = torch.empty((max(N, 1), 16), dtype=torch.float32, device=self.device)
         offsets = torch.empty(self.T + 1, dtype=torch.int32, device=self.device)
-        args = [_ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities), _ptr(colors), _ptr(sel),
-                _ptr(atlas.bbox), _ptr(prim_info), _ptr(offsets)]
+        ws, nbytes = self._scratch(cv, 1, N, stream)
+        flags = ws[nbytes:].view(torch.int32)
         for _ in range(3):
-            self._ensure(cv, self.capacity)
-            ws, wsb = self._ws_ptr()
             # each binning owns its index list: a ForwardState must stay valid
             # while later forwards on this canvas run (batch APIs keep several)
-            indices = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=self.device)
-            call("dbmp_bin", ctypes.byref(cv), *args, _ptr(indices), ctypes.c_longlong(self.capacity),
-                 _ptr(self._small), ctypes.c_void_p(self._small.data_ptr() + 4), ws, ctypes.c_size_t(wsb), st)
-            L, overflow = self._small.tolist()
+            cap = self._capacity(N)
+            indices = torch.empty(max(cap, 1), dtype=torch.int32, device=self.device)
+            call("dbmp_bin", ctypes.byref(cv), _ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities),
+                 _ptr(colors), _ptr(sel), _ptr(atlas.bbox), _ptr(prim_info), _ptr(offsets), _ptr(indices), cap,
+                 _ptr(flags), flags.data_ptr() + 4, _ptr(ws), nbytes, st)
+            L, overflow = flags.tolist()
             if not overflow:
                 return prim_info, TileLists(offsets, indices, int(L))
-            self._ensure(cv, int(L * 1.25) + 4096)
+            self._grow_hint(L)
+        raise DbmpError("binning capacity did not converge")
+
+    def _render(self, lead: tuple, means2D, radii, rotations, opacities, colors, sel, sel_stride: int, atlas: Atlas,
+                stream, cmap=None, cmap_stride: int = 0, c_blend: float = 0.0):
+        """Binning and forward of B candidates (lead: () for one, else (B,)) in one
+        call; the host waits for the list lengths while the forward runs, and
+        repeats the call if they exceed the capacity.  Returns (color, alpha,
+        T_last, last_pos, prim_info, offsets, indices, longest list)."""
+        B = lead[0] if lead else 1
+        N = int(radii.shape[-1])
+        cv = self.canvas(N, atlas)
+        dev, H, W = self.device, self.H, self.W
+        color = torch.empty((*lead, H, W, 3), dtype=torch.float32, device=dev)
+        alpha = torch.empty((*lead, H, W), dtype=torch.float32, device=dev)
+        T_last = torch.empty((*lead, H, W), dtype=torch.float32, device=dev)
+        last_pos = torch.empty((*lead, H, W), dtype=torch.int32, device=dev)
+        prim = torch.empty((max(B * N, 1), 16), dtype=torch.float32, device=dev)
+        offsets = torch.empty((*lead, self.T + 1), dtype=torch.int32, device=dev)
+        ws, nbytes = self._scratch(cv, B, N, stream)
+        st = _stream(stream)
+        pin = self._pins.pop() if self._pins else torch.empty(2 * B, dtype=torch.int32).pin_memory()
+        if pin.numel() < 2 * B:
+            pin = torch.empty(2 * B, dtype=torch.int32).pin_memory()
+        flags = pin.numpy()
+        for _ in range(3):
+            cap = self._capacity(N)
+            stride = max(cap, 1)
+            indices = torch.empty((*lead, stride), dtype=torch.int32, device=dev)
+            call("dbmp_render", ctypes.byref(cv), B, _ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities),
+                 _ptr(colors), _ptr(sel), sel_stride, _ptr(atlas.bbox), _ptr(atlas.data), _ptr(prim), _ptr(offsets),
+                 _ptr(indices), stride, cap, ws.data_ptr() + nbytes, _ptr(pin), _ptr(cmap), cmap_stride,
+                 float(c_blend) if cmap is not None else 0.0, _ptr(color), _ptr(alpha), _ptr(T_last), _ptr(last_pos),
+                 _ptr(ws), nbytes, st)
+            call("dbmp_render_wait", _ptr(pin), B, st)
+            if not flags[1:2 * B:2].any():
+                L = int(flags[0:2 * B:2].max())
+                self._pins.append(pin)
+                return color, alpha, T_last, last_pos, prim, offsets, indices, L
+            self._grow_hint(int(flags[0:2 * B:2].max()))
         raise DbmpError("binning capacity did not converge")
 
     def prepare(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None):
@@ -283,11 +365,13 @@ class Rasterizer:
         _need_cuda(means2D, radii, rotations, opacities, colors, sel)
         N = int(radii.shape[0])
         cmap = self._colour_maps(colors_orig, c_blend, N, atlas)
-        if mapping is not None and mapping.numel() > 0:
-            lists = lists_from_mapping(mapping, self.T, N)
-            prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
-        else:
-            prim_info, lists = self.bin(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
+        if mapping is None or mapping.numel() == 0:
+            color, alpha, T_last, last_pos, prim_info, offsets, indices, L = self._render(
+                (), means2D, radii, rotations, opacities, colors, sel, 0, atlas, stream, cmap, 0, c_blend)
+            return color, alpha, ForwardState(prim_info, TileLists(offsets, indices, L), T_last, last_pos, cmap,
+                                              float(c_blend) if cmap is not None else 0.0)
+        lists = lists_from_mapping(mapping, self.T, N)
+        prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
         cv = self.canvas(N, atlas)
         color = torch.empty((self.H, self.W, 3), dtype=torch.float32, device=self.device)
         alpha = torch.empty((self.H, self.W), dtype=torch.float32, device=self.device)
@@ -316,28 +400,25 @@ class Rasterizer:
         small = torch.empty((B, 2), dtype=torch.int32, device=self.device)    # per candidate: L, overflow
         sel_stride = N if sel.dim() == 2 else 0
         if B == 0:
-            return prim, offsets, torch.empty((0, max(self.capacity, 1)), dtype=torch.int32, device=self.device)
-        # the call steps from candidate to candidate by N (candidates may come strided or expanded)
-        means2D, radii, rotations, opacities, colors, sel = (
-            t.contiguous() for t in (means2D, radii, rotations, opacities, colors, sel))
+            return prim, offsets, torch.empty((0, 1), dtype=torch.int32, device=self.device)
+        means2D, radii, rotations, opacities, colors, sel = self._flat_batch(
+            (means2D, radii, rotations, opacities, colors, sel), stream)
         n = min(B, 65535)                       # candidates of one call
-        nbytes = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), n))
+        ws, nbytes = self._scratch(cv, n, N, stream)
         for _ in range(3):
-            self._ensure(cv, self.capacity, nbytes)
-            ws, wsb = self._ws_ptr()
-            cap = max(self.capacity, 1)
-            indices = torch.empty((B, cap), dtype=torch.int32, device=self.device)
+            cap = self._capacity(N)
+            stride = max(cap, 1)
+            indices = torch.empty((B, stride), dtype=torch.int32, device=self.device)
             for b in range(0, B, n):
                 call("dbmp_bin_batch", ctypes.byref(cv), min(n, B - b), _ptr(means2D[b]), _ptr(radii[b]),
                      _ptr(rotations[b]), _ptr(opacities[b]), _ptr(colors[b]),
-                     _ptr(sel[b]) if sel_stride else _ptr(sel), ctypes.c_longlong(sel_stride), _ptr(atlas.bbox),
-                     ctypes.c_void_p(prim.data_ptr() + b * N * 64), _ptr(offsets[b]), _ptr(indices[b]),
-                     ctypes.c_longlong(cap), ctypes.c_longlong(self.capacity), _ptr(small[b]), ws,
-                     ctypes.c_size_t(wsb), st)
+                     _ptr(sel[b]) if sel_stride else _ptr(sel), sel_stride, _ptr(atlas.bbox),
+                     prim.data_ptr() + b * N * 64, _ptr(offsets[b]), _ptr(indices[b]), stride, cap, _ptr(small[b]),
+                     _ptr(ws), nbytes, st)
             Ls = small.cpu()
             if not bool(Ls[:, 1].any()):
                 return prim, offsets, indices
-            self._ensure(cv, int(int(Ls[:, 0].max()) * 1.25) + 4096)
+            self._grow_hint(int(Ls[:, 0].max()))
         raise DbmpError("binning capacity did not converge")
 
     def forward_batch(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, mappings=None,
@@ -350,7 +431,21 @@ class Rasterizer:
         _need_cuda(means2D, radii, rotations, opacities, colors, sel)
         B, N = int(radii.shape[0]), int(radii.shape[1])
         st = _stream(stream)
-        if mappings is not None and len(mappings) > 0:
+        cmap, cstride = None, 0
+        if colors_orig is not None and colors_orig.numel() > 0 and float(c_blend) > 0.0:
+            if colors_orig.dim() == 5:
+                cmap = self._colour_maps(colors_orig.reshape(B * N, *colors_orig.shape[2:]), c_blend, B * N, atlas)
+                cstride = N * atlas.Ht * atlas.Wt * 3
+            else:
+                cmap = self._colour_maps(colors_orig, c_blend, N, atlas)
+        has_maps = mappings is not None and len(mappings) > 0
+        if not has_maps and 0 < B <= 65535:
+            params = self._flat_batch((means2D, radii, rotations, opacities, colors, sel), stream)
+            color, alpha, T_last, last_pos, prim, offsets, indices, _ = self._render(
+                (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend)
+            return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
+                                            float(c_blend) if cmap is not None else 0.0)
+        if has_maps:
             if len(mappings) != B:
                 raise ValueError(f"{len(mappings)} mappings for {B} candidates")
             lists = [lists_from_mapping(m, self.T, N) for m in mappings]
@@ -368,13 +463,6 @@ class Rasterizer:
                      ctypes.c_void_p(prim.data_ptr() + b * N * 64), st)
         else:
             prim, offsets, indices = self.bin_batch(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
-        cmap, cstride = None, 0
-        if colors_orig is not None and colors_orig.numel() > 0 and float(c_blend) > 0.0:
-            if colors_orig.dim() == 5:
-                cmap = self._colour_maps(colors_orig.reshape(B * N, *colors_orig.shape[2:]), c_blend, B * N, atlas)
-                cstride = N * atlas.Ht * atlas.Wt * 3
-            else:
-                cmap = self._colour_maps(colors_orig, c_blend, N, atlas)
         cv = self.canvas(N, atlas)
         dev = self.device
         color = torch.empty((B, self.H, self.W, 3), dtype=torch.float32, device=dev)
@@ -395,8 +483,8 @@ class Rasterizer:
         B, N = int(radii.shape[0]), int(radii.shape[1])
         cv = self.canvas(N, atlas)
         dev = self.device
-        gc = _f32(grad_color)
-        ga = _f32(grad_alpha) if grad_alpha is not None else None
+        gc = _operand(grad_color)
+        ga = _operand(grad_alpha) if grad_alpha is not None else None
         acc = torch.empty((max(B * N, 1), 8), dtype=torch.float64, device=dev)
         outs = [torch.empty(sh, dtype=torch.float32, device=dev)
                 for sh in ((B, N, 2), (B, N), (B, N), (B, N), (B, N, 3))]
@@ -428,8 +516,8 @@ class Rasterizer:
         N = int(radii.shape[0])
         cv = self.canvas(N, atlas)
         dev = self.device
-        gc = _f32(grad_color)
-        ga = _f32(grad_alpha) if grad_alpha is not None else None
+        gc = _operand(grad_color)
+        ga = _operand(grad_alpha) if grad_alpha is not None else None
         acc = torch.empty((max(N, 1), 8), dtype=torch.float64, device=dev)
         g_means = torch.empty((N, 2), dtype=torch.float32, device=dev)
         g_r = torch.empty(N, dtype=torch.float32, device=dev)
@@ -450,6 +538,14 @@ class Rasterizer:
         return g_means, g_r, g_rot, g_op, g_col
 
 
+def _flat(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dim() == 1 else t.view(-1)
+
+
+def _shaped(t: torch.Tensor, k: int) -> torch.Tensor:
+    return t if t.dim() == 2 and t.shape[1] == k else t.view(-1, k)
+
+
 class RasterizeFunction(torch.autograd.Function):
     """Differentiable render of bitmap primitives (hand-written backward).
 
@@ -464,10 +560,10 @@ class RasterizeFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, means2D, radii, rotations, opacities, colors, sel, atlas, rasterizer, mapping=None,
                 colors_orig=None, c_blend=0.0):
-        m, r, th, v, c = (_f32(t) for t in (means2D, radii, rotations, opacities, colors))
+        m, r, th, v, c = (_operand(t) for t in (means2D, radii, rotations, opacities, colors))
         s = sel.detach().to(torch.int32).contiguous()
-        color, alpha, state = rasterizer.forward(m.view(-1, 2), r.view(-1), th.view(-1), v.view(-1),
-                                                 c.view(-1, 3), s.view(-1), atlas, mapping, None,
+        color, alpha, state = rasterizer.forward(_shaped(m, 2), _flat(r), _flat(th), _flat(v), _shaped(c, 3),
+                                                 _flat(s), atlas, mapping, None,
                                                  None if colors_orig is None else colors_orig.detach(),
                                                  float(c_blend))
         ctx.state = state
@@ -483,10 +579,8 @@ class RasterizeFunction(torch.autograd.Function):
         rz: Rasterizer = ctx.rasterizer
         if grad_color is None:
             grad_color = torch.zeros((rz.H, rz.W, 3), dtype=torch.float32, device=r.device)
-        gm, gr, gth, gv, gc = rz.backward(ctx.state, grad_color, grad_alpha, r.view(-1), th.view(-1), v.view(-1),
-                                          c.view(-1, 3), ctx.atlas)
-        sh = ctx.shapes
-        return (gm.view(sh[0]), gr.view(sh[1]), gth.view(sh[2]), gv.view(sh[3]), gc.view(sh[4]),
+        g = rz.backward(ctx.state, grad_color, grad_alpha, _flat(r), _flat(th), _flat(v), _shaped(c, 3), ctx.atlas)
+        return (*(x if x.shape == sh else x.view(sh) for x, sh in zip(g, ctx.shapes)),
                 None, None, None, None, None, None)
 
 
@@ -505,7 +599,7 @@ class RasterizeBatchFunction(torch.autograd.Function):
     def forward(ctx, means2D, radii, rotations, opacities, colors, sel, atlas, rasterizer, mappings=None,
                 colors_orig=None, c_blend=0.0):
         B = int(radii.shape[0])
-        m, r, th, v, c = (_f32(t) for t in (means2D, radii, rotations, opacities, colors))
+        m, r, th, v, c = (_operand(t) for t in (means2D, radii, rotations, opacities, colors))
         s = sel.detach().to(torch.int32).contiguous()
         color, alpha, state = rasterizer.forward_batch(m.view(B, -1, 2), r.view(B, -1), th.view(B, -1),
                                                        v.view(B, -1), c.view(B, -1, 3), s, atlas, mappings, None,

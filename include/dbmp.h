@@ -3,8 +3,9 @@
  *
  * Plain pointers and sizes only: every array argument is a device pointer
  * (CUDA global memory of the current device) unless the comment says "host".
- * `stream` is a cudaStream_t passed as void*.  No entry point synchronises the
- * device or reads device memory from the host; all work is stream-ordered.
+ * `stream` is a cudaStream_t passed as void*.  No entry point but
+ * dbmp_render_wait synchronises with the device or reads device memory from
+ * the host; all work is stream-ordered.
  * Every call returns a dbmp_status; on failure dbmp_last_error() describes it
  * (thread-local string).  There is no fallback path: a failed call leaves its
  * outputs undefined.
@@ -181,6 +182,23 @@ int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const
                    long long capacity, int32_t* total_and_overflow, void* workspace,
                    size_t workspace_bytes, void* stream);
 
+/* dbmp_bin_batch followed by dbmp_forward_batch (blending when c_blend > 0)
+ * of the same candidates, without the host in between.  The binning also
+ * writes each candidate's two flags to host_flags (pinned host memory, 2 ints
+ * per candidate), which dbmp_render_wait polls; a candidate whose lists
+ * exceed the capacity is not rendered, and the caller calls again with more.
+ * Not capturable in a CUDA graph.  dbmp_render_wait(host_flags, batch, stream)
+ * returns once the flags are there (spinning, then synchronising the stream):
+ * the one call of this library that waits for the device. */
+int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii,
+                const float* rotations, const float* opacities, const float* colors, const int32_t* sel,
+                long long sel_stride, const float* tmpl_bbox, const void* atlas, void* prim_info,
+                int32_t* tile_offsets, int32_t* tile_indices, long long index_stride, long long capacity,
+                int32_t* total_and_overflow, int32_t* host_flags, const float* colors_orig,
+                long long colors_orig_stride, float c_blend, float* out_color, float* out_alpha,
+                float* T_last, int32_t* last_pos, void* workspace, size_t workspace_bytes, void* stream);
+int dbmp_render_wait(const int32_t* host_flags, int batch, void* stream);
+
 /* Forward compositing.  out_color (H,W,3) f32 = sum_k T_k a_k c_k and
  * out_alpha (H,W) f32 = 1 - T_final, front to back over each tile's list,
  * stopping a pixel once T < t_stop.  Per pixel it also stores the
@@ -194,6 +212,13 @@ int dbmp_forward(const dbmp_canvas* cv, const void* prim_info, const void* atlas
                  const int32_t* tile_offsets, const int32_t* tile_indices,
                  float* out_color, float* out_alpha, float* T_last, int32_t* last_pos,
                  void* stream);
+
+/* Converts n <= 8 arrays between IEEE half and f32 (to_half: f32 -> half) in
+ * one launch; src, dst and counts are host arrays of n device pointers and
+ * element counts.  For callers that hold a job's tensors in FP16, as the
+ * reference's FP16 extension takes them (cuda_tile_rasterizer/__init__.py:342-436). */
+int dbmp_convert_half(int n, const void* const* src, void* const* dst, const long long* counts,
+                      int to_half, void* stream);
 
 /* Backward.  Reverse traversal from each pixel's last contributor,
  * recovering T_k from T_last; per-primitive sums are warp/CTA reduced and

@@ -59,6 +59,7 @@ def test_overflow_leaves_lists_and_reports_length_gpu():
     rz = R.Rasterizer(H, W)
     L = rz.bin(*p, atlas)[1].length
     cv = rz.canvas(N, atlas)
+    rz._ensure(cv, L)
     ws, wsb = rz._ws_ptr()
     prim = torch.empty((N, 16), device="cuda")
     offsets = torch.full((rz.T + 1,), -7, dtype=torch.int32, device="cuda")
