@@ -331,7 +331,7 @@ struct TileWalker {
   }
 
   // tile: the CTA's tile; part: which group of warps of the tile the CTA runs
-  // (a CTA holds kCtaWarps of the tile's NW warps).
+  // (a CTA holds cta_warps of the tile's NW warps).
   __device__ __forceinline__ void init(const Geom& g, int tile, int part, int cta_warps,
                                        const int* __restrict__ offs) {
     lw = threadIdx.x >> 5;
@@ -559,9 +559,11 @@ struct TileWalker {
     return pair_over(g, r, m, f0, f1, p.tx, p.ty, f, vote);
   }
 
-  // Forward walk.  Entries that are sampled go two at a time: the texel loads
+  // Forward walk.  Two sampled entries in a row go together: the texel loads
   // of both are issued before either is composited, so their latencies
-  // overlap.  Solid entries (mask 1 on the whole footprint) are composited
+  // overlap (a lone one on its own path: issuing a copy of it as the second
+  // took 221 against 204 us at 2048x2048, N=20000, FP16 quads; three or four
+  // together spill, as do two in the backward walk).  Solid entries (mask 1 on the whole footprint) are composited
   // straight from their record: they need a third of the instructions of a
   // sampled one, and at 2048x2048, N=20000, 256x256 bitmaps with soft rims they
   // are 44 % of the entries (forward walk 244 -> 218 us, backward 432 -> 361,
@@ -590,16 +592,21 @@ struct TileWalker {
           ++j;
           continue;
         }
-        const bool two = j + 1 < c.n && !((c.solid >> (j + 1)) & 1u);
-        const int j2 = two ? j + 1 : j;   // j again when no sampled entry follows it
-        PairPre<KIND> p1, p2;
-        pair_issue(g, atlas, w[j], (c.inside >> j) & 1u, (c.fast >> j) & 1u, f.live, p1);
-        pair_issue(g, atlas, w[j2], (c.inside >> j2) & 1u, (c.fast >> j2) & 1u, f.live, p2);
-        // one termination vote per pair: a pixel that stops at the first has live
-        // false, so the second composites nothing for it
-        if (pair_composite(g, w[j], p1, f, !two)) { warp_done = true; break; }
-        if (two && pair_composite(g, w[j2], p2, f, true)) { warp_done = true; break; }
-        j = j2 + 1;
+        if (j + 1 < c.n && !((c.solid >> (j + 1)) & 1u)) {
+          // one termination vote per pair: a pixel that stops at the first has live
+          // false, so the second composites nothing for it
+          PairPre<KIND> p1, p2;
+          pair_issue(g, atlas, w[j], (c.inside >> j) & 1u, (c.fast >> j) & 1u, f.live, p1);
+          pair_issue(g, atlas, w[j + 1], (c.inside >> (j + 1)) & 1u, (c.fast >> (j + 1)) & 1u, f.live, p2);
+          pair_composite(g, w[j], p1, f, false);
+          if (pair_composite(g, w[j + 1], p2, f, true)) { warp_done = true; break; }
+          j += 2;
+        } else {
+          PairPre<KIND> p1;
+          pair_issue(g, atlas, w[j], (c.inside >> j) & 1u, (c.fast >> j) & 1u, f.live, p1);
+          if (pair_composite(g, w[j], p1, f, true)) { warp_done = true; break; }
+          ++j;
+        }
       }
     }
     C[0][0] = f.cr.x; C[0][1] = f.cg.x; C[0][2] = f.cb.x;
@@ -800,14 +807,15 @@ struct TileWalker {
   }
 };
 
-// CTA shape of the walk kernels: a CTA runs kCtaWarps warps of one tile (the
-// warps walk independently, so a tile may be split over several CTAs, which
-// lets an SM refill as soon as a few warps finish); kParts CTAs per tile.
-// Registers are bounded for a number of resident warps per SM, tuned on B200
-// per atlas kind: 36 (56 registers a thread, a few bytes of spills) for the
-// packed atlases, whose walk waits mostly on texel loads and gains from the
-// extra warps; 32 (64 registers) for the reference layout and the
-// colour-map walks.
+// CTA shape of the walk kernels.  The warps of a tile walk independently, so a
+// tile may be split over several CTAs, which lets an SM refill as soon as a few
+// warps finish: kFwdWarps per CTA in the forward walk, one in the walks with a
+// backward part, whose warps differ more in length (2048x2048, N=20000, FP16
+// quads, one / four warps: backward 325 / 339 us, fused 498 / 503; forward 208 /
+// 204).  Registers are bounded for a number of resident warps per SM, tuned on
+// B200 per atlas kind: 36 (56 registers a thread) for the packed atlases, whose
+// walk waits mostly on texel loads and gains from the extra warps; 32 (64
+// registers) for the reference layout and the colour-map walks.
 #ifndef DBMP_CTA_WARPS
 #define DBMP_CTA_WARPS 4
 #endif
@@ -818,19 +826,17 @@ struct TileWalker {
 #define DBMP_WARPS_PER_SM_F32 32
 #endif
 template <int TS> constexpr int kTileWarps() { return Layout<TS>::NW; }
-template <int TS> constexpr int kCtaWarps() {
+template <int TS> constexpr int kFwdWarps() {
   return kTileWarps<TS>() < DBMP_CTA_WARPS ? kTileWarps<TS>() : DBMP_CTA_WARPS;
 }
-template <int TS> constexpr int kParts() { return kTileWarps<TS>() / kCtaWarps<TS>(); }
-template <int TS> constexpr int kThreadsOf() { return kCtaWarps<TS>() * 32; }
-template <int TS, int KIND, bool CB = false> constexpr int kBlocksPerSM() {
-  constexpr int w = (KIND == ATLAS_F32 || CB) ? DBMP_WARPS_PER_SM_F32 : DBMP_WARPS_PER_SM;
-  return w / kCtaWarps<TS>() > 0 ? w / kCtaWarps<TS>() : 1;
+template <int TS> constexpr int kFwdParts() { return kTileWarps<TS>() / kFwdWarps<TS>(); }
+template <int KIND, bool CB = false> constexpr int kBlocksPerSM(int cta_warps) {
+  return ((KIND == ATLAS_F32 || CB) ? DBMP_WARPS_PER_SM_F32 : DBMP_WARPS_PER_SM) / cta_warps;
 }
 
 // ---------------------------------------------------------------------------
 template <int TS, int KIND, bool CB>
-__global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()) forward_kernel(
+__global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(kFwdWarps<TS>())) forward_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
@@ -838,10 +844,10 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
   grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
-  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
+  __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
   // a batch of candidates is one grid over all their tiles: candidate b's
   // records, lists and images follow candidate b-1's
-  const int gt = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
+  const int gt = blockIdx.x / kFwdParts<TS>(), part = blockIdx.x % kFwdParts<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;
   // binning overflowed for a candidate: its lists do not exist, and the caller
   // bins again (flags: list length and overflow per candidate)
@@ -854,7 +860,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
   TW tw;
   tw.cmap = CB ? cmap + (size_t)b * cmap_stride : cmap;
   tw.cblend = cblend;
-  tw.init(g, tile, part, kCtaWarps<TS>(), offs);
+  tw.init(g, tile, part, kFwdWarps<TS>(), offs);
   float C[NP][3], T[NP], Tl[NP];
   int lp[NP];
   tw.forward(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp);
@@ -874,22 +880,22 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
 // Counting pass (diagnostics / roofline accounting): same walk as the
 // forward, no outputs except the counters.
 template <int TS, int KIND>
-__global__ void __launch_bounds__(kThreadsOf<TS>()) count_kernel(Geom g, const PrimInfo* __restrict__ prims,
-                                                                 const void* __restrict__ atlas,
-                                                                 const int* __restrict__ offs,
-                                                                 const int* __restrict__ idx,
-                                                                 unsigned long long* __restrict__ cnt) {
+__global__ void __launch_bounds__(kFwdWarps<TS>() * 32) count_kernel(Geom g, const PrimInfo* __restrict__ prims,
+                                                                     const void* __restrict__ atlas,
+                                                                     const int* __restrict__ offs,
+                                                                     const int* __restrict__ idx,
+                                                                     unsigned long long* __restrict__ cnt) {
   using TW = TileWalker<TS, KIND>;
-  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
+  __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
   TW tw;
-  const int tile = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
-  tw.init(g, tile, part, kCtaWarps<TS>(), offs);
+  const int tile = blockIdx.x / kFwdParts<TS>(), part = blockIdx.x % kFwdParts<TS>();
+  tw.init(g, tile, part, kFwdWarps<TS>(), offs);
   tw.count(g, prims, atlas, idx, s_pi[tw.lw], cnt);
   if (threadIdx.x == 0 && part == 0) atomicAdd(cnt + 2, (unsigned long long)(tw.end - tw.start));
 }
 
 template <int TS, int KIND, bool CB>
-__global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()) backward_kernel(
+__global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
     const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
@@ -897,8 +903,8 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
   grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
-  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
-  const int gt = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
+  __shared__ Rec s_pi[kChunk];
+  const int gt = blockIdx.x / kTileWarps<TS>(), part = blockIdx.x % kTileWarps<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;     // candidate and tile (see forward_kernel)
   const size_t pix = (size_t)b * g.H * g.W;
   prims += (size_t)b * g.N;
@@ -910,7 +916,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
   TW tw;
   tw.cmap = CB ? cmap + (size_t)b * cmap_stride : cmap;
   tw.cblend = cblend;
-  tw.init(g, tile, part, kCtaWarps<TS>(), offs);
+  tw.init(g, tile, part, 1, offs);
   float gC[NP][3], gA[NP], Ts[NP];
   int lp[NP];
 #pragma unroll
@@ -928,7 +934,7 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND, CB>()
       gA[p] = 0.f; Ts[p] = 1.f; lp[p] = -1;
     }
   }
-  tw.backward(g, prims, atlas, idx, s_pi[tw.lw], gC, gA, Ts, lp, gacc);
+  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc);
 }
 
 __device__ __forceinline__ double sigmoid_d(double x) {
@@ -981,11 +987,10 @@ __global__ void finalize_kernel(Geom g, const float* __restrict__ radii, const f
 // reference's mse_loss(rendered, target) (pydiffbmp/util/loss_functions.py:20-40)
 // on rendered = C + (1 - A) * background (simple_tile_renderer.py:704-707):
 //   dL/dC = 2 (rendered - target) / (3HW),  dL/dA = -sum_c dL/dC_c * bg_c.
-// loss_out (f64, may be null) receives sum((rendered - target)^2) / (3HW):
-// each warp leaves its partial in shared memory and the CTA's last warp to
-// finish its forward walk adds the CTA's sum (no barrier between the walks).
+// loss_out (f64, may be null) receives sum((rendered - target)^2) / (3HW),
+// one add per warp.
 template <int TS, int KIND>
-__global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fused_kernel(
+__global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, const float* __restrict__ target, const float* __restrict__ background,
     float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
@@ -994,17 +999,13 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fu
   if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND>;
-  __shared__ Rec s_pi[kCtaWarps<TS>()][kChunk];
-  __shared__ float s_loss[kCtaWarps<TS>()];
-  __shared__ unsigned s_arrived;
-  if (threadIdx.x == 0) s_arrived = 0u;
-  __syncthreads();
+  __shared__ Rec s_pi[kChunk];
   TW tw;
-  const int tile = blockIdx.x / kParts<TS>(), part = blockIdx.x % kParts<TS>();
-  tw.init(g, tile, part, kCtaWarps<TS>(), offs);
+  const int tile = blockIdx.x / kTileWarps<TS>(), part = blockIdx.x % kTileWarps<TS>();
+  tw.init(g, tile, part, 1, offs);
   float C[NP][3], T[NP], Tl[NP], gC[NP][3], gA[NP];
   int lp[NP];
-  tw.forward(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp);
+  tw.forward(g, prims, atlas, idx, s_pi, C, T, Tl, lp);
   const float inv = 1.f / (3.f * (float)g.H * (float)g.W);
   float lsum = 0.f;
 #pragma unroll
@@ -1030,19 +1031,9 @@ __global__ void __launch_bounds__(kThreadsOf<TS>(), kBlocksPerSM<TS, KIND>()) fu
     lsum += __shfl_xor_sync(kFull, lsum, 4);
     lsum += __shfl_xor_sync(kFull, lsum, 2);
     lsum += __shfl_xor_sync(kFull, lsum, 1);
-    if (tw.lane == 0) {
-      s_loss[tw.lw] = lsum;
-      __threadfence_block();
-      if (atomicAdd(&s_arrived, 1u) == (unsigned)(kCtaWarps<TS>() - 1)) {
-        __threadfence_block();
-        const volatile float* sl = s_loss;
-        double t = 0.0;
-        for (int w = 0; w < kCtaWarps<TS>(); ++w) t += sl[w];
-        atomicAdd(loss_out, t * (double)inv);
-      }
-    }
+    if (tw.lane == 0) atomicAdd(loss_out, (double)lsum * (double)inv);
   }
-  tw.backward(g, prims, atlas, idx, s_pi[tw.lw], gC, gA, Tl, lp, gacc);
+  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Tl, lp, gacc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1070,15 +1061,15 @@ int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const v
                          float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride,
                          const int* flags) {
   if (g.T == 0 || batch == 0) return DBMP_OK;
-  const long long ctas = (long long)batch * g.T * kParts<32>();
+  const long long ctas = (long long)batch * g.T * kFwdParts<32>();
   if (ctas > 0x7fffffffll) { set_error("forward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
   if (cmap != nullptr && cblend > 0.f) {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "forward_kernel", forward_kernel<TSV, KD, true>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        "forward_kernel", forward_kernel<TSV, KD, true>, dim3(batch * g.T * kFwdParts<TSV>()), kFwdWarps<TSV>() * 32, 0, st,
         g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride, flags)));
   } else {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "forward_kernel", forward_kernel<TSV, KD, false>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        "forward_kernel", forward_kernel<TSV, KD, false>, dim3(batch * g.T * kFwdParts<TSV>()), kFwdWarps<TSV>() * 32, 0, st,
         g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll, flags)));
   }
 }
@@ -1092,7 +1083,7 @@ int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* a
 int launch_count(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs, const int* idx,
                  unsigned long long* cnt, cudaStream_t st) {
   if (g.T == 0) return DBMP_OK;
-  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (count_kernel<TSV, KD><<<g.T * kParts<TSV>(), kThreadsOf<TSV>(), 0, st>>>(
+  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (count_kernel<TSV, KD><<<g.T * kFwdParts<TSV>(), kFwdWarps<TSV>() * 32, 0, st>>>(
                                                    g, prims, atlas, offs, idx, cnt))));
   DBMP_CHECK_LAUNCH("count_kernel");
   return DBMP_OK;
@@ -1103,16 +1094,16 @@ int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const 
                           const float* grad_alpha, double* gacc, const float* cmap, float cblend, cudaStream_t st,
                           int batch, long long idx_stride, long long cmap_stride) {
   if (g.T == 0 || batch == 0) return DBMP_OK;
-  const long long ctas = (long long)batch * g.T * kParts<32>();
+  const long long ctas = (long long)batch * g.T * kTileWarps<32>();
   if (ctas > 0x7fffffffll) { set_error("backward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
   if (cmap != nullptr && cblend > 0.f) {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "backward_kernel", backward_kernel<TSV, KD, true>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        "backward_kernel", backward_kernel<TSV, KD, true>, dim3((unsigned)(batch * g.T * kTileWarps<TSV>())), 32, 0, st,
         g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, cmap, cblend, idx_stride,
         cmap_stride)));
   } else {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "backward_kernel", backward_kernel<TSV, KD, false>, dim3(batch * g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st,
+        "backward_kernel", backward_kernel<TSV, KD, false>, dim3((unsigned)(batch * g.T * kTileWarps<TSV>())), 32, 0, st,
         g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, (const float*)nullptr, 0.f,
         idx_stride, 0ll)));
   }
@@ -1153,7 +1144,7 @@ int launch_fused(const Geom& g, int kind, const PrimInfo* prims, const void* atl
                  const int* skip_flag, cudaStream_t st) {
   if (g.T == 0) return DBMP_OK;
   DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-      "fused_kernel", fused_kernel<TSV, KD>, dim3(g.T * kParts<TSV>()), kThreadsOf<TSV>(), 0, st, g, prims, atlas, offs,
+      "fused_kernel", fused_kernel<TSV, KD>, dim3((unsigned)(g.T * kTileWarps<TSV>())), 32, 0, st, g, prims, atlas, offs,
       idx, target, background, out_image, gacc, loss, skip_flag)));
 }
 
