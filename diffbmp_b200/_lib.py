@@ -66,8 +66,10 @@ SIGNATURES = {
     "dbmp_bin_workspace_bytes": (_sz, [_CP, _ll]),
     "dbmp_bin_batch_workspace_bytes": (_sz, [_CP, _i]),
     "dbmp_bin_batch": (_i, [_CP, _i] + [_vp] * 6 + [_ll] + [_vp] * 4 + [_ll, _ll, _vp, _vp, _sz, _vp]),
-    "dbmp_render": (_i, [_CP, _i] + [_vp] * 6 + [_ll] + [_vp] * 5 + [_ll, _ll] + [_vp] * 3 + [_ll, _f] + [_vp] * 5
+    "dbmp_render": (_i, [_CP, _i] + [_vp] * 6 + [_ll] + [_vp] * 5 + [_ll, _ll] + [_vp] * 3 + [_ll, _f] + [_vp] * 6
                     + [_sz, _vp]),
+    "dbmp_walk_mask_bytes": (_sz, [_CP, _i]),
+    "dbmp_backward_masked": (_i, [_CP, _i] + [_vp] * 5 + [_ll, _vp, _ll, _f] + [_vp] * 15),
     "dbmp_convert_half": (_i, [_i, _vp, _vp, _vp, _i, _vp]),
     "dbmp_render_wait": (_i, [_vp, _i, _vp]),
     "dbmp_prim_info_bytes": (_sz, [_i]),

@@ -45,11 +45,13 @@ int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* a
 int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                          const int* idx, float* color, float* alpha, float* T_last, int* last_pos, const float* cmap,
                          float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride,
-                         const int* flags);
+                         const int* flags, void* masks);
 int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                           const int* idx, const float* T_last, const int* last_pos, const float* grad_color,
                           const float* grad_alpha, double* gacc, const float* cmap, float cblend, cudaStream_t st,
-                          int batch, long long idx_stride, long long cmap_stride);
+                          int batch, long long idx_stride, long long cmap_stride,
+                          const void* masks);
+size_t walk_mask_bytes(const Geom& g, int batch);
 int launch_count(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs, const int* idx,
                  unsigned long long* cnt, cudaStream_t st);
 int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
@@ -286,14 +288,15 @@ int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const fl
                 const float* tmpl_bbox, const void* atlas, void* prim_info, int32_t* tile_offsets,
                 int32_t* tile_indices, long long index_stride, long long capacity, int32_t* total_and_overflow,
                 int32_t* host_flags, const float* colors_orig, long long colors_orig_stride, float c_blend,
-                float* out_color, float* out_alpha, float* T_last, int32_t* last_pos, void* workspace,
-                size_t workspace_bytes, void* stream) {
+                float* out_color, float* out_alpha, float* T_last, int32_t* last_pos, void* walk_masks,
+                void* workspace, size_t workspace_bytes, void* stream) {
   Geom g;
   int rc = make_geom(cv, &g, "dbmp_render");
   if (rc) return rc;
   if (batch == 0) return DBMP_OK;
   REQUIRE(atlas && out_color && out_alpha && T_last && last_pos && host_flags, "dbmp_render: null pointer");
   REQUIRE(colors_orig_stride >= 0, "dbmp_render: negative stride");
+  REQUIRE(((uintptr_t)walk_masks & 15) == 0, "dbmp_render: walk_masks must be 16-byte aligned");
   REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_render: c_blend %g outside [0, 1]", (double)c_blend);
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_render: colors_orig is null with c_blend > 0");
   REQUIRE((long long)batch * g.T * 4 <= 0x7fffffffll, "dbmp_render: %d candidates x %d tiles exceed one grid", batch, g.T);
@@ -312,7 +315,7 @@ int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const fl
   // candidate whose lists overflowed renders nothing
   return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream,
-                              batch, index_stride, colors_orig_stride, total_and_overflow);
+                              batch, index_stride, colors_orig_stride, total_and_overflow, walk_masks);
 }
 
 int dbmp_convert_half(int n, const void* const* src, void* const* dst, const long long* counts, int to_half,
@@ -406,7 +409,7 @@ int dbmp_forward_blend(const dbmp_canvas* cv, const void* prim_info, const void*
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_forward_blend: colors_orig is null with c_blend > 0");
   return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream, 1,
-                              0, 0, nullptr);
+                              0, 0, nullptr, nullptr);
 }
 
 int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void* atlas, const int32_t* tile_offsets,
@@ -429,7 +432,7 @@ int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void
   rc = launch_zero(grad_accum, 8ll * g.N, nullptr, st);
   if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
-                             T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0);
+                             T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0, nullptr);
   if (rc) return rc;
   return launch_finalize(g, radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii,
                          grad_rotations, grad_opacities, grad_colors, st);
@@ -452,7 +455,42 @@ int dbmp_forward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, 
   REQUIRE(((uintptr_t)prim_info & 15) == 0, "dbmp_forward_batch: prim_info must be 16-byte aligned");
   return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream,
-                              batch, index_stride, colors_orig_stride, nullptr);
+                              batch, index_stride, colors_orig_stride, nullptr, nullptr);
+}
+
+static int backward_batch(const char* who, const void* walk_masks, const dbmp_canvas* cv, int batch, const void* prim_info, const void* atlas,
+                        const int32_t* tile_offsets, const int32_t* tile_indices, long long index_stride,
+                        const float* colors_orig, long long colors_orig_stride, float c_blend, const float* T_last,
+                        const int32_t* last_pos, const float* grad_color, const float* grad_alpha,
+                        const float* radii, const float* rotations, const float* opacities, const float* colors,
+                        double* grad_accum, float* grad_means2D, float* grad_radii, float* grad_rotations,
+                        float* grad_opacities, float* grad_colors, void* stream) {
+  Geom g;
+  int rc = make_geom(cv, &g, who);
+  if (rc) return rc;
+  REQUIRE(batch >= 0, "%s: batch %d < 0", who, batch);
+  REQUIRE(index_stride >= 0 && colors_orig_stride >= 0, "%s: negative stride", who);
+  REQUIRE(batch == 0 || (atlas && tile_offsets && tile_indices && T_last && last_pos && grad_color),
+          "%s: null input", who);
+  const bool work = batch > 0 && g.N > 0;
+  REQUIRE(!work || (prim_info && radii && rotations && opacities && colors), "%s: null parameter", who);
+  REQUIRE(!work || (grad_accum && grad_means2D && grad_radii && grad_rotations && grad_opacities && grad_colors),
+          "%s: null output", who);
+  REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "%s: c_blend %g outside [0, 1]", who, (double)c_blend);
+  REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "%s: colors_orig is null with c_blend > 0", who);
+  if (!work) return DBMP_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, st);
+  if (rc) return rc;
+  rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
+                             T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, batch,
+                             index_stride, colors_orig_stride, walk_masks);
+  if (rc) return rc;
+  // the chain rule is per primitive: the batch's (B, N) primitives are one flat array
+  Geom gb = g;
+  gb.N = g.N * batch;
+  return launch_finalize(gb, radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii,
+                         grad_rotations, grad_opacities, grad_colors, st);
 }
 
 int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, const void* atlas,
@@ -462,32 +500,28 @@ int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info,
                         const float* radii, const float* rotations, const float* opacities, const float* colors,
                         double* grad_accum, float* grad_means2D, float* grad_radii, float* grad_rotations,
                         float* grad_opacities, float* grad_colors, void* stream) {
+  return backward_batch("dbmp_backward_batch", nullptr, cv, batch, prim_info, atlas, tile_offsets, tile_indices, index_stride, colors_orig, colors_orig_stride, c_blend,
+                        T_last, last_pos, grad_color, grad_alpha, radii, rotations, opacities, colors, grad_accum,
+                        grad_means2D, grad_radii, grad_rotations, grad_opacities, grad_colors, stream);
+}
+
+int dbmp_backward_masked(const dbmp_canvas* cv, int batch, const void* walk_masks, const void* prim_info, const void* atlas,
+                        const int32_t* tile_offsets, const int32_t* tile_indices, long long index_stride,
+                        const float* colors_orig, long long colors_orig_stride, float c_blend, const float* T_last,
+                        const int32_t* last_pos, const float* grad_color, const float* grad_alpha,
+                        const float* radii, const float* rotations, const float* opacities, const float* colors,
+                        double* grad_accum, float* grad_means2D, float* grad_radii, float* grad_rotations,
+                        float* grad_opacities, float* grad_colors, void* stream) {
+  REQUIRE(((uintptr_t)walk_masks & 15) == 0, "dbmp_backward_masked: walk_masks must be 16-byte aligned");
+  return backward_batch("dbmp_backward_masked", walk_masks, cv, batch, prim_info, atlas, tile_offsets, tile_indices, index_stride, colors_orig, colors_orig_stride, c_blend,
+                        T_last, last_pos, grad_color, grad_alpha, radii, rotations, opacities, colors, grad_accum,
+                        grad_means2D, grad_radii, grad_rotations, grad_opacities, grad_colors, stream);
+}
+
+size_t dbmp_walk_mask_bytes(const dbmp_canvas* cv, int batch) {
   Geom g;
-  int rc = make_geom(cv, &g, "dbmp_backward_batch");
-  if (rc) return rc;
-  REQUIRE(batch >= 0, "dbmp_backward_batch: batch %d < 0", batch);
-  REQUIRE(index_stride >= 0 && colors_orig_stride >= 0, "dbmp_backward_batch: negative stride");
-  REQUIRE(batch == 0 || (atlas && tile_offsets && tile_indices && T_last && last_pos && grad_color),
-          "dbmp_backward_batch: null input");
-  const bool work = batch > 0 && g.N > 0;
-  REQUIRE(!work || (prim_info && radii && rotations && opacities && colors), "dbmp_backward_batch: null parameter");
-  REQUIRE(!work || (grad_accum && grad_means2D && grad_radii && grad_rotations && grad_opacities && grad_colors),
-          "dbmp_backward_batch: null output");
-  REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_backward_batch: c_blend %g outside [0, 1]", (double)c_blend);
-  REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_backward_batch: colors_orig is null with c_blend > 0");
-  if (!work) return DBMP_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, st);
-  if (rc) return rc;
-  rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
-                             T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, batch,
-                             index_stride, colors_orig_stride);
-  if (rc) return rc;
-  // the chain rule is per primitive: the batch's (B, N) primitives are one flat array
-  Geom gb = g;
-  gb.N = g.N * batch;
-  return launch_finalize(gb, radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii,
-                         grad_rotations, grad_opacities, grad_colors, st);
+  if (make_geom(cv, &g, "dbmp_walk_mask_bytes") != DBMP_OK || batch < 0) return 0;
+  return walk_mask_bytes(g, batch);
 }
 
 int dbmp_count(const dbmp_canvas* cv, const void* prim_info, const void* atlas, const int32_t* tile_offsets,

@@ -153,6 +153,11 @@ struct Layout {
   static constexpr bool kDirect = TS == 16;
 };
 
+// Chunks of 32 list entries whose staging masks a warp's forward walk keeps.
+#ifndef DBMP_KEPT_CHUNKS
+#define DBMP_KEPT_CHUNKS 8
+#endif
+
 struct Geom {
   // operand pairs of the packed pixel-pair arithmetic (both halves equal)
   float2 k23;          // 2^23

@@ -279,16 +279,18 @@ struct Chunk {
 };
 constexpr unsigned kInside = 1u, kFast = 2u, kSolid = 4u, kClear = 8u;
 
-// What the fused kernel's forward walk leaves for its backward walk, in shared
-// memory: the masks of the first kKeptChunks chunks, so that the backward walk
-// stages them without the tests (of a chunk's 32 entries: which survived; of the
-// survivors: inside, fast, solid), and which chunk's records the buffer holds
-// (fused kernel at 2048x2048, N=20000, FP16 quads, where a walk stages 2.5 chunks:
-// 492 -> 466 us).
-constexpr int kKeptChunks = 8;
+// What a forward walk leaves for the backward walk of the same warp: the masks of
+// its first kKeptChunks chunks (of a chunk's 32 entries: which survived; of the
+// survivors: inside, fast, solid), so that the backward walk stages them without
+// the tests.  The fused kernel keeps them in shared memory, with which chunk's
+// records the buffer holds (2048x2048, N=20000, FP16 quads, where a walk stages 2.5
+// chunks: 492 -> 466 us); a forward call can leave them in global memory for the
+// backward call (2048x2048, N=20000, FP16 quads: backward call 355 -> 330 us;
+// 1024x1024, N=5000, FP32: 168 -> 158; 4096x4096, N=100000: 2146 -> 2058).
+constexpr int kKeptChunks = DBMP_KEPT_CHUNKS;
 struct Kept {
   uint4 masks[kKeptChunks];
-  int in_buffer;   // index of the last staged chunk
+  int in_buffer;   // index of the last staged chunk (-1: none)
 };
 
 // Staged record: [0] (mx, my, hw, hh)  [1] A  [2] (op, r, g, b)
@@ -461,8 +463,9 @@ struct TileWalker {
   // stage() for a chunk whose masks the forward walk kept: only the survivors
   // up to list position `last` (relative to the tile's) are needed, and no test.
   // in_buffer: their records are still in w.
-  __device__ __forceinline__ Chunk restage(const PrimInfo* __restrict__ prims, const int* __restrict__ idx, int base,
-                                           int last, const uint4& m, bool in_buffer, Rec* w) const {
+  __device__ __forceinline__ Chunk restage(const PrimInfo* __restrict__ prims, int num_prims,
+                                           const int* __restrict__ idx, int base, int last, const uint4& m,
+                                           bool in_buffer, Rec* w) const {
     Chunk c;
     c.todo = m.x;
     if (last - base < kChunk - 1) c.todo &= (2u << (last - base)) - 1u;
@@ -473,7 +476,8 @@ struct TileWalker {
     if (in_buffer) return c;
     __syncwarp();   // every lane is done with the previous chunk's records
     if ((c.todo >> lane) & 1u) {
-      const int id = __ldg(idx + start + base + lane);
+      int id = __ldg(idx + start + base + lane);
+      if ((unsigned)id >= (unsigned)num_prims) id = 0;   // (a list changed since the forward stays in bounds)
       const float4* r = reinterpret_cast<const float4*>(prims + id);
       float4* d = w[__popc(c.todo & ((1u << lane) - 1u))];
       float4 g2 = __ldg(r + 2);
@@ -617,7 +621,7 @@ struct TileWalker {
   __device__ __forceinline__ void forward(const Geom& g, const PrimInfo* __restrict__ prims,
                                           const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
                                           float (&C)[2][3], float (&T)[2], float (&Tl)[2], int (&lp)[2],
-                                          Kept* kept = nullptr) const {
+                                          uint4* masks, int* in_buffer) const {
     const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
     PairFwd f;
     f.cr = f.cg = f.cb = make_float2(0.f, 0.f);
@@ -628,10 +632,10 @@ struct TileWalker {
     bool warp_done = __all_sync(kFull, !f.live[0] && !f.live[1]);
     for (int base = start; base < end && !warp_done; base += kChunk) {
       const Chunk c = stage<false>(g, prims, idx, grid, base, end, w);
-      if (kept && lane == 0) {
+      if (masks && lane == 0) {
         const int k = (base - start) / kChunk;
-        kept->in_buffer = k;
-        if (k < kKeptChunks) kept->masks[k] = make_uint4(c.todo, c.inside, c.fast, c.solid);
+        if (in_buffer) *in_buffer = k;
+        if (k < kKeptChunks) masks[k] = make_uint4(c.todo, c.inside, c.fast, c.solid);
       }
       for (int j = 0; j < c.n;) {
         if ((c.solid >> j) & 1u) {   // every live pixel of the warp has mask 1: nothing to sample
@@ -688,7 +692,7 @@ struct TileWalker {
                                            const void* __restrict__ atlas, const int* __restrict__ idx, Rec* w,
                                            const float (&gC)[2][3], const float (&gA)[2], const float (&Ts)[2],
                                            const int (&lp)[2], double* __restrict__ gacc,
-                                           const Kept* kept = nullptr) const {
+                                           const Kept* kept) const {
     const int warp_max = __reduce_max_sync(kFull, max(lp[0], lp[1]));
     if (warp_max < 0) return;
     const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
@@ -700,7 +704,7 @@ struct TileWalker {
     for (int cb = (warp_max / kChunk) * kChunk; cb >= 0; cb -= kChunk) {
       Chunk c;
       const int k = cb / kChunk;
-      if (kept && k < kKeptChunks) c = restage(prims, idx, cb, warp_max, kept->masks[k], k == kept->in_buffer, w);
+      if (kept && k < kKeptChunks) c = restage(prims, g.N, idx, cb, warp_max, kept->masks[k], k == kept->in_buffer, w);
       else c = stage<false>(g, prims, idx, grid, start + cb, start + warp_max + 1, w);
       for (int j = c.n - 1; j >= 0; --j) {
         const Rec& r = w[j];
@@ -896,7 +900,7 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(k
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
     float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
-    long long idx_stride, long long cmap_stride, const int* __restrict__ flags) {
+    long long idx_stride, long long cmap_stride, const int* __restrict__ flags, uint4* __restrict__ masks) {
   grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
@@ -919,7 +923,8 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(k
   tw.init(g, tile, part, kFwdWarps<TS>(), offs);
   float C[NP][3], T[NP], Tl[NP];
   int lp[NP];
-  tw.forward(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp);
+  if (masks) masks += ((size_t)gt * kTileWarps<TS>() + tw.warp) * kKeptChunks;
+  tw.forward(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp, masks, nullptr);
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     if (!tw.valid[p]) continue;
@@ -955,11 +960,13 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
     const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
-    const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride) {
+    const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride,
+    const uint4* __restrict__ masks) {
   grid_dependency();
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
   __shared__ Rec s_pi[kChunk];
+  __shared__ Kept s_kept;
   const int gt = blockIdx.x / kTileWarps<TS>(), part = blockIdx.x % kTileWarps<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;     // candidate and tile (see forward_kernel)
   const size_t pix = (size_t)b * g.H * g.W;
@@ -990,7 +997,13 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel
       gA[p] = 0.f; Ts[p] = 1.f; lp[p] = -1;
     }
   }
-  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc);
+  if (masks) {
+    const size_t at = ((size_t)gt * kTileWarps<TS>() + tw.warp) * kKeptChunks;
+    if (tw.lane < kKeptChunks) s_kept.masks[tw.lane] = masks[at + tw.lane];   // (those never written are never used)
+    if (tw.lane == 0) s_kept.in_buffer = -1;
+    __syncwarp();
+  }
+  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc, masks ? &s_kept : nullptr);
 }
 
 __device__ __forceinline__ double sigmoid_d(double x) {
@@ -1062,7 +1075,7 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
   tw.init(g, tile, part, 1, offs);
   float C[NP][3], T[NP], Tl[NP], gC[NP][3], gA[NP];
   int lp[NP];
-  tw.forward(g, prims, atlas, idx, s_pi, C, T, Tl, lp, &s_kept);
+  tw.forward(g, prims, atlas, idx, s_pi, C, T, Tl, lp, s_kept.masks, &s_kept.in_buffer);
   const float inv = 1.f / (3.f * (float)g.H * (float)g.W);
   float lsum = 0.f;
 #pragma unroll
@@ -1114,28 +1127,33 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
 // batch > 1: `batch` candidates of the same canvas in one grid, candidate b's
 // records at prims + b N, lists at offs + b (T+1) / idx + b idx_stride,
 // images at b H W (x3 for colour), colour maps at cmap + b cmap_stride.
+size_t walk_mask_bytes(const Geom& g, int batch) {
+  const size_t warps = (size_t)batch * g.T * (g.TS == 32 ? kTileWarps<32>() : kTileWarps<16>());
+  return warps * kKeptChunks * sizeof(uint4);
+}
+
 int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                          const int* idx, float* color, float* alpha, float* T_last, int* last_pos, const float* cmap,
                          float cblend, cudaStream_t st, int batch, long long idx_stride, long long cmap_stride,
-                         const int* flags) {
+                         const int* flags, void* masks) {
   if (g.T == 0 || batch == 0) return DBMP_OK;
   const long long ctas = (long long)batch * g.T * kFwdParts<32>();
   if (ctas > 0x7fffffffll) { set_error("forward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
   if (cmap != nullptr && cblend > 0.f) {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
         "forward_kernel", forward_kernel<TSV, KD, true>, dim3(batch * g.T * kFwdParts<TSV>()), kFwdWarps<TSV>() * 32, 0, st,
-        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride, flags)));
+        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride, flags, (uint4*)masks)));
   } else {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
         "forward_kernel", forward_kernel<TSV, KD, false>, dim3(batch * g.T * kFwdParts<TSV>()), kFwdWarps<TSV>() * 32, 0, st,
-        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll, flags)));
+        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll, flags, (uint4*)masks)));
   }
 }
 
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                    const int* idx, float* color, float* alpha, float* T_last, int* last_pos, cudaStream_t st) {
   return launch_forward_blend(g, kind, prims, atlas, offs, idx, color, alpha, T_last, last_pos, nullptr, 0.f, st, 1,
-                              0, 0, nullptr);
+                              0, 0, nullptr, nullptr);
 }
 
 int launch_count(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs, const int* idx,
@@ -1150,7 +1168,7 @@ int launch_count(const Geom& g, int kind, const PrimInfo* prims, const void* atl
 int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                           const int* idx, const float* T_last, const int* last_pos, const float* grad_color,
                           const float* grad_alpha, double* gacc, const float* cmap, float cblend, cudaStream_t st,
-                          int batch, long long idx_stride, long long cmap_stride) {
+                          int batch, long long idx_stride, long long cmap_stride, const void* masks) {
   if (g.T == 0 || batch == 0) return DBMP_OK;
   const long long ctas = (long long)batch * g.T * kTileWarps<32>();
   if (ctas > 0x7fffffffll) { set_error("backward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
@@ -1158,12 +1176,12 @@ int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const 
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
         "backward_kernel", backward_kernel<TSV, KD, true>, dim3((unsigned)(batch * g.T * kTileWarps<TSV>())), 32, 0, st,
         g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, cmap, cblend, idx_stride,
-        cmap_stride)));
+        cmap_stride, (const uint4*)masks)));
   } else {
     DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
         "backward_kernel", backward_kernel<TSV, KD, false>, dim3((unsigned)(batch * g.T * kTileWarps<TSV>())), 32, 0, st,
         g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, (const float*)nullptr, 0.f,
-        idx_stride, 0ll)));
+        idx_stride, 0ll, (const uint4*)masks)));
   }
 }
 
@@ -1171,7 +1189,7 @@ int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* 
                     const int* idx, const float* T_last, const int* last_pos, const float* grad_color,
                     const float* grad_alpha, double* gacc, cudaStream_t st) {
   return launch_backward_blend(g, kind, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc,
-                               nullptr, 0.f, st, 1, 0, 0);
+                               nullptr, 0.f, st, 1, 0, 0, nullptr);
 }
 
 // Zeroes n doubles at a and, when given, one at b: a kernel rather than

@@ -173,6 +173,7 @@ class BatchState:
     colors_orig: Optional[torch.Tensor] = None
     cmap_stride: int = 0
     c_blend: float = 0.0
+    walk_masks: Optional[torch.Tensor] = None    # what the forward's tests found (dbmp_render)
 
     @property
     def batch(self) -> int:
@@ -187,6 +188,7 @@ class ForwardState:
     last_pos: torch.Tensor
     colors_orig: Optional[torch.Tensor] = None   # colour maps of a blended render
     c_blend: float = 0.0
+    walk_masks: Optional[torch.Tensor] = None    # what the forward's tests found (dbmp_render)
 
 
 def lists_from_mapping(mapping: torch.Tensor, num_tiles: int, num_prims: int) -> TileLists:
@@ -231,6 +233,7 @@ class Rasterizer:
         self._idx = None
         self._hint = None          # list capacity of the next render
         self._ws_need = (None, 0)  # workspace bytes of the last (batch, N)
+        self._mask_bytes = None    # walk masks of one candidate
         self._pins = []            # pinned flag buffers not in use
 
     def canvas(self, N: int, atlas: Atlas) -> Canvas:
@@ -309,11 +312,12 @@ class Rasterizer:
         raise DbmpError("binning capacity did not converge")
 
     def _render(self, lead: tuple, means2D, radii, rotations, opacities, colors, sel, sel_stride: int, atlas: Atlas,
-                stream, cmap=None, cmap_stride: int = 0, c_blend: float = 0.0):
+                stream, cmap=None, cmap_stride: int = 0, c_blend: float = 0.0, masks: bool = True):
         """Binning and forward of B candidates (lead: () for one, else (B,)) in one
         call; the host waits for the list lengths while the forward runs, and
         repeats the call if they exceed the capacity.  Returns (color, alpha,
-        T_last, last_pos, prim_info, offsets, indices, longest list)."""
+        T_last, last_pos, prim_info, offsets, indices, longest list, walk_masks);
+        masks: the render's backward will be wanted."""
         B = lead[0] if lead else 1
         N = int(radii.shape[-1])
         cv = self.canvas(N, atlas)
@@ -324,6 +328,11 @@ class Rasterizer:
         last_pos = torch.empty((*lead, H, W), dtype=torch.int32, device=dev)
         prim = torch.empty((max(B * N, 1), 16), dtype=torch.float32, device=dev)
         offsets = torch.empty((*lead, self.T + 1), dtype=torch.int32, device=dev)
+        walk = None
+        if masks:
+            if self._mask_bytes is None:
+                self._mask_bytes = int(lib.dbmp_walk_mask_bytes(ctypes.byref(cv), 1))
+            walk = torch.empty(self._mask_bytes * B, dtype=torch.uint8, device=dev)
         ws, nbytes = self._scratch(cv, B, N, stream)
         st = _stream(stream)
         pin = self._pins.pop() if self._pins else torch.empty(2 * B, dtype=torch.int32).pin_memory()
@@ -338,12 +347,12 @@ class Rasterizer:
                  _ptr(colors), _ptr(sel), sel_stride, _ptr(atlas.bbox), _ptr(atlas.data), _ptr(prim), _ptr(offsets),
                  _ptr(indices), stride, cap, ws.data_ptr() + nbytes, _ptr(pin), _ptr(cmap), cmap_stride,
                  float(c_blend) if cmap is not None else 0.0, _ptr(color), _ptr(alpha), _ptr(T_last), _ptr(last_pos),
-                 _ptr(ws), nbytes, st)
+                 _ptr(walk), _ptr(ws), nbytes, st)
             call("dbmp_render_wait", _ptr(pin), B, st)
             if not flags[1:2 * B:2].any():
                 L = int(flags[0:2 * B:2].max())
                 self._pins.append(pin)
-                return color, alpha, T_last, last_pos, prim, offsets, indices, L
+                return color, alpha, T_last, last_pos, prim, offsets, indices, L, walk
             self._grow_hint(int(flags[0:2 * B:2].max()))
         raise DbmpError("binning capacity did not converge")
 
@@ -358,18 +367,19 @@ class Rasterizer:
     # -- forward / backward -------------------------------------------------
     def forward(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas,
                 mapping: Optional[torch.Tensor] = None, stream=None, colors_orig: Optional[torch.Tensor] = None,
-                c_blend: float = 0.0):
-        """Returns (color (H,W,3), alpha (H,W), ForwardState).  With
+                c_blend: float = 0.0, for_backward: bool = True):
+        """Returns (color (H,W,3), alpha (H,W), ForwardState).  for_backward: the
+        state also keeps what speeds up its backward.  With
         colors_orig (N,Ht,Wt,3) and c_blend in (0, 1], fragment colours blend
         the per-primitive colour maps (dbmp_forward_blend)."""
         _need_cuda(means2D, radii, rotations, opacities, colors, sel)
         N = int(radii.shape[0])
         cmap = self._colour_maps(colors_orig, c_blend, N, atlas)
         if mapping is None or mapping.numel() == 0:
-            color, alpha, T_last, last_pos, prim_info, offsets, indices, L = self._render(
-                (), means2D, radii, rotations, opacities, colors, sel, 0, atlas, stream, cmap, 0, c_blend)
+            color, alpha, T_last, last_pos, prim_info, offsets, indices, L, walk = self._render(
+                (), means2D, radii, rotations, opacities, colors, sel, 0, atlas, stream, cmap, 0, c_blend, for_backward)
             return color, alpha, ForwardState(prim_info, TileLists(offsets, indices, L), T_last, last_pos, cmap,
-                                              float(c_blend) if cmap is not None else 0.0)
+                                              float(c_blend) if cmap is not None else 0.0, walk)
         lists = lists_from_mapping(mapping, self.T, N)
         prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
         cv = self.canvas(N, atlas)
@@ -422,7 +432,8 @@ class Rasterizer:
         raise DbmpError("binning capacity did not converge")
 
     def forward_batch(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, mappings=None,
-                      stream=None, colors_orig: Optional[torch.Tensor] = None, c_blend: float = 0.0):
+                      stream=None, colors_orig: Optional[torch.Tensor] = None, c_blend: float = 0.0,
+                      for_backward: bool = True):
         """B candidates of this canvas in one launch.  means2D (B,N,2), radii /
         rotations / opacities (B,N), colors (B,N,3), sel (N) or (B,N);
         mappings: None (device binning) or B reference mapping tensors;
@@ -441,10 +452,10 @@ class Rasterizer:
         has_maps = mappings is not None and len(mappings) > 0
         if not has_maps and 0 < B <= 65535:
             params = self._flat_batch((means2D, radii, rotations, opacities, colors, sel), stream)
-            color, alpha, T_last, last_pos, prim, offsets, indices, _ = self._render(
-                (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend)
+            color, alpha, T_last, last_pos, prim, offsets, indices, _, walk = self._render(
+                (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend, for_backward)
             return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
-                                            float(c_blend) if cmap is not None else 0.0)
+                                            float(c_blend) if cmap is not None else 0.0, walk)
         if has_maps:
             if len(mappings) != B:
                 raise ValueError(f"{len(mappings)} mappings for {B} candidates")
@@ -488,9 +499,9 @@ class Rasterizer:
         acc = torch.empty((max(B * N, 1), 8), dtype=torch.float64, device=dev)
         outs = [torch.empty(sh, dtype=torch.float32, device=dev)
                 for sh in ((B, N, 2), (B, N), (B, N), (B, N), (B, N, 3))]
-        call("dbmp_backward_batch", ctypes.byref(cv), B, _ptr(state.prim_info), _ptr(atlas.data),
-             _ptr(state.offsets), _ptr(state.indices), ctypes.c_longlong(state.indices.shape[1]),
-             _ptr(state.colors_orig), ctypes.c_longlong(state.cmap_stride), ctypes.c_float(state.c_blend),
+        call("dbmp_backward_masked", ctypes.byref(cv), B, _ptr(state.walk_masks), _ptr(state.prim_info),
+             _ptr(atlas.data), _ptr(state.offsets), _ptr(state.indices), state.indices.shape[1],
+             _ptr(state.colors_orig), state.cmap_stride, float(state.c_blend),
              _ptr(state.T_last), _ptr(state.last_pos), _ptr(gc), _ptr(ga), _ptr(radii), _ptr(rotations),
              _ptr(opacities), _ptr(colors), _ptr(acc), *[_ptr(o) for o in outs], _stream(stream))
         return tuple(outs)
@@ -524,17 +535,12 @@ class Rasterizer:
         g_rot = torch.empty(N, dtype=torch.float32, device=dev)
         g_op = torch.empty(N, dtype=torch.float32, device=dev)
         g_col = torch.empty((N, 3), dtype=torch.float32, device=dev)
-        if state.colors_orig is None:
-            call("dbmp_backward", ctypes.byref(cv), _ptr(state.prim_info), _ptr(atlas.data),
-                 _ptr(state.lists.offsets), _ptr(state.lists.indices), _ptr(state.T_last), _ptr(state.last_pos),
-                 _ptr(gc), _ptr(ga), _ptr(radii), _ptr(rotations), _ptr(opacities), _ptr(colors), _ptr(acc),
-                 _ptr(g_means), _ptr(g_r), _ptr(g_rot), _ptr(g_op), _ptr(g_col), _stream(stream))
-        else:
-            call("dbmp_backward_blend", ctypes.byref(cv), _ptr(state.prim_info), _ptr(atlas.data),
-                 _ptr(state.lists.offsets), _ptr(state.lists.indices), _ptr(state.colors_orig),
-                 ctypes.c_float(state.c_blend), _ptr(state.T_last), _ptr(state.last_pos),
-                 _ptr(gc), _ptr(ga), _ptr(radii), _ptr(rotations), _ptr(opacities), _ptr(colors), _ptr(acc),
-                 _ptr(g_means), _ptr(g_r), _ptr(g_rot), _ptr(g_op), _ptr(g_col), _stream(stream))
+        call("dbmp_backward_masked", ctypes.byref(cv), 1, _ptr(state.walk_masks), _ptr(state.prim_info),
+             _ptr(atlas.data), _ptr(state.lists.offsets), _ptr(state.lists.indices), state.lists.indices.numel(),
+             _ptr(state.colors_orig), 0, float(state.c_blend) if state.colors_orig is not None else 0.0,
+             _ptr(state.T_last), _ptr(state.last_pos), _ptr(gc), _ptr(ga), _ptr(radii), _ptr(rotations),
+             _ptr(opacities), _ptr(colors), _ptr(acc), _ptr(g_means), _ptr(g_r), _ptr(g_rot), _ptr(g_op), _ptr(g_col),
+             _stream(stream))
         return g_means, g_r, g_rot, g_op, g_col
 
 
@@ -565,7 +571,7 @@ class RasterizeFunction(torch.autograd.Function):
         color, alpha, state = rasterizer.forward(_shaped(m, 2), _flat(r), _flat(th), _flat(v), _shaped(c, 3),
                                                  _flat(s), atlas, mapping, None,
                                                  None if colors_orig is None else colors_orig.detach(),
-                                                 float(c_blend))
+                                                 float(c_blend), any(ctx.needs_input_grad[:5]))
         ctx.state = state
         ctx.atlas = atlas
         ctx.rasterizer = rasterizer
@@ -604,7 +610,7 @@ class RasterizeBatchFunction(torch.autograd.Function):
         color, alpha, state = rasterizer.forward_batch(m.view(B, -1, 2), r.view(B, -1), th.view(B, -1),
                                                        v.view(B, -1), c.view(B, -1, 3), s, atlas, mappings, None,
                                                        None if colors_orig is None else colors_orig.detach(),
-                                                       float(c_blend))
+                                                       float(c_blend), any(ctx.needs_input_grad[:5]))
         ctx.state, ctx.atlas, ctx.rasterizer = state, atlas, rasterizer
         ctx.shapes = (means2D.shape, radii.shape, rotations.shape, opacities.shape, colors.shape)
         ctx.save_for_backward(r, th, v, c)

@@ -189,14 +189,20 @@ int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const
  * exceed the capacity is not rendered, and the caller calls again with more.
  * Not capturable in a CUDA graph.  dbmp_render_wait(host_flags, batch, stream)
  * returns once the flags are there (spinning, then synchronising the stream):
- * the one call of this library that waits for the device. */
+ * the one call of this library that waits for the device.
+ * walk_masks (may be null): dbmp_walk_mask_bytes of scratch in which the forward
+ * leaves the outcome of its per-warp tests; dbmp_backward_masked is
+ * dbmp_backward_batch reading them instead of testing again (same canvas,
+ * records and lists; null: it tests). */
+size_t dbmp_walk_mask_bytes(const dbmp_canvas* cv, int batch);
 int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii,
                 const float* rotations, const float* opacities, const float* colors, const int32_t* sel,
                 long long sel_stride, const float* tmpl_bbox, const void* atlas, void* prim_info,
                 int32_t* tile_offsets, int32_t* tile_indices, long long index_stride, long long capacity,
                 int32_t* total_and_overflow, int32_t* host_flags, const float* colors_orig,
                 long long colors_orig_stride, float c_blend, float* out_color, float* out_alpha,
-                float* T_last, int32_t* last_pos, void* workspace, size_t workspace_bytes, void* stream);
+                float* T_last, int32_t* last_pos, void* walk_masks, void* workspace,
+                size_t workspace_bytes, void* stream);
 int dbmp_render_wait(const int32_t* host_flags, int batch, void* stream);
 
 /* Forward compositing.  out_color (H,W,3) f32 = sum_k T_k a_k c_k and
@@ -305,6 +311,14 @@ int dbmp_forward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, 
                        const float* colors_orig, long long colors_orig_stride, float c_blend, float* out_color,
                        float* out_alpha, float* T_last, int32_t* last_pos, void* stream);
 int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, const void* atlas,
+                        const int32_t* tile_offsets, const int32_t* tile_indices, long long index_stride,
+                        const float* colors_orig, long long colors_orig_stride, float c_blend,
+                        const float* T_last, const int32_t* last_pos, const float* grad_color,
+                        const float* grad_alpha, const float* radii, const float* rotations,
+                        const float* opacities, const float* colors, double* grad_accum,
+                        float* grad_means2D, float* grad_radii, float* grad_rotations,
+                        float* grad_opacities, float* grad_colors, void* stream);
+int dbmp_backward_masked(const dbmp_canvas* cv, int batch, const void* walk_masks, const void* prim_info, const void* atlas,
                         const int32_t* tile_offsets, const int32_t* tile_indices, long long index_stride,
                         const float* colors_orig, long long colors_orig_stride, float c_blend,
                         const float* T_last, const int32_t* last_pos, const float* grad_color,

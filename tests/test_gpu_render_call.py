@@ -48,6 +48,29 @@ def test_render_grows_its_lists_gpu(N, hint):
     assert torch.equal(st.lists.mapping_tensor(), lists.mapping_tensor())
 
 
+@pytest.mark.parametrize("kind,ts,N,opac,blend", [
+    ("f32", 32, 40, 0.0, 0.0), ("f16q", 16, 700, -5.0, 0.0),     # 700 faint layers: beyond the chunks whose masks are kept
+    ("bf16", 32, 700, -5.0, 0.0), ("f32", 32, 300, -3.0, 0.5)])
+def test_backward_with_the_forwards_masks_gpu(kind, ts, N, opac, blend):
+    """The backward that stages from the forward's masks against the one that tests
+    again: the same terms in the same order per warp (FP64 sums over warps are
+    unordered: 1e-6 of the block's norm)."""
+    W, H = 75, 61
+    rng = np.random.default_rng(5)
+    at = R.Atlas(torch.from_numpy(rng.uniform(0, 1, (2, 20, 24)).astype(np.float32)).cuda(), kind)
+    p = params(3, N, W, H, 60.0)
+    p[3] += opac
+    maps = torch.rand(N, 20, 24, 3, device="cuda") if blend else None
+    rz = R.Rasterizer(H, W, ts)
+    c, a, st = rz.forward(*p, at, None, None, maps, blend)
+    assert int(st.last_pos.max()) >= (8 * 32 if N == 700 else 1)
+    gc, ga = torch.randn_like(c), torch.randn_like(a)
+    with_masks = rz.backward(st, gc, ga, *p[1:5], at)
+    st.walk_masks = None
+    for x, y in zip(with_masks, rz.backward(st, gc, ga, *p[1:5], at)):
+        assert (x - y).norm() <= 1e-6 * y.norm()
+
+
 def test_renders_on_several_streams_gpu():
     at, rz = atlas(), R.Rasterizer(300, 500)
     sets = [params(k, 300 + 200 * k, 500, 300) for k in range(3)]
