@@ -285,8 +285,8 @@ constexpr unsigned kInside = 1u, kFast = 2u, kSolid = 4u, kClear = 8u;
 // the tests.  The fused kernel keeps them in shared memory, with which chunk's
 // records the buffer holds (2048x2048, N=20000, FP16 quads, where a walk stages 2.5
 // chunks: 492 -> 466 us); a forward call can leave them in global memory for the
-// backward call (2048x2048, N=20000, FP16 quads: backward call 355 -> 330 us;
-// 1024x1024, N=5000, FP32: 168 -> 158; 4096x4096, N=100000: 2146 -> 2058).
+// backward call (2048x2048, N=20000, FP16 quads: backward call 339 -> 332 us;
+// 1024x1024, N=5000, FP32: 163 -> 156; 4096x4096, N=100000: 2058 -> 2041).
 constexpr int kKeptChunks = DBMP_KEPT_CHUNKS;
 struct Kept {
   uint4 masks[kKeptChunks];
@@ -873,9 +873,13 @@ struct TileWalker {
 // backward part, whose warps differ more in length (2048x2048, N=20000, FP16
 // quads, one / four warps: backward 325 / 339 us, fused 498 / 503; forward 208 /
 // 204).  Registers are bounded for a number of resident warps per SM, tuned on
-// B200 per atlas kind: 36 (56 registers a thread) for the packed atlases, whose
-// walk waits mostly on texel loads and gains from the extra warps; 32 (64
-// registers) for the reference layout and the colour-map walks.
+// B200 per atlas kind: 36 (56 registers a thread) for the packed atlases' forward
+// walk, which waits mostly on texel loads and gains from the extra warps; 32 (64
+// registers) for the reference layout and the colour-map walks.  One-warp CTAs
+// have 64 registers in any case: an SM holds 32 CTAs.  Forward and backward come
+// with and without kept masks as kernels of their own: a pointer tested in the
+// walk costs registers (2048x2048, N=20000, FP16 quads: forward 207 -> 204 us,
+// backward without masks 354 -> 339; 4096x4096, N=100000: 2133 -> 2058).
 #ifndef DBMP_CTA_WARPS
 #define DBMP_CTA_WARPS 4
 #endif
@@ -895,7 +899,7 @@ template <int KIND, bool CB = false> constexpr int kBlocksPerSM(int cta_warps) {
 }
 
 // ---------------------------------------------------------------------------
-template <int TS, int KIND, bool CB>
+template <int TS, int KIND, bool CB, bool MASKED>
 __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(kFwdWarps<TS>())) forward_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
@@ -923,8 +927,9 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(k
   tw.init(g, tile, part, kFwdWarps<TS>(), offs);
   float C[NP][3], T[NP], Tl[NP];
   int lp[NP];
-  if (masks) masks += ((size_t)gt * kTileWarps<TS>() + tw.warp) * kKeptChunks;
-  tw.forward(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp, masks, nullptr);
+  uint4* kept = nullptr;   // MASKED: this warp's masks for the backward
+  if (MASKED) kept = masks + ((size_t)gt * kTileWarps<TS>() + tw.warp) * kKeptChunks;
+  tw.forward(g, prims, atlas, idx, s_pi[tw.lw], C, T, Tl, lp, kept, nullptr);
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
     if (!tw.valid[p]) continue;
@@ -955,7 +960,7 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32) count_kernel(Geom g, con
   if (threadIdx.x == 0 && part == 0) atomicAdd(cnt + 2, (unsigned long long)(tw.end - tw.start));
 }
 
-template <int TS, int KIND, bool CB>
+template <int TS, int KIND, bool CB, bool MASKED>
 __global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
@@ -997,13 +1002,13 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel
       gA[p] = 0.f; Ts[p] = 1.f; lp[p] = -1;
     }
   }
-  if (masks) {
+  if constexpr (MASKED) {
     const size_t at = ((size_t)gt * kTileWarps<TS>() + tw.warp) * kKeptChunks;
     if (tw.lane < kKeptChunks) s_kept.masks[tw.lane] = masks[at + tw.lane];   // (those never written are never used)
     if (tw.lane == 0) s_kept.in_buffer = -1;
     __syncwarp();
   }
-  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc, masks ? &s_kept : nullptr);
+  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc, MASKED ? &s_kept : nullptr);
 }
 
 __device__ __forceinline__ double sigmoid_d(double x) {
@@ -1139,15 +1144,18 @@ int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const v
   if (g.T == 0 || batch == 0) return DBMP_OK;
   const long long ctas = (long long)batch * g.T * kFwdParts<32>();
   if (ctas > 0x7fffffffll) { set_error("forward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
-  if (cmap != nullptr && cblend > 0.f) {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "forward_kernel", forward_kernel<TSV, KD, true>, dim3(batch * g.T * kFwdParts<TSV>()), kFwdWarps<TSV>() * 32, 0, st,
-        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, cmap, cblend, idx_stride, cmap_stride, flags, (uint4*)masks)));
-  } else {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "forward_kernel", forward_kernel<TSV, KD, false>, dim3(batch * g.T * kFwdParts<TSV>()), kFwdWarps<TSV>() * 32, 0, st,
-        g, prims, atlas, offs, idx, color, alpha, T_last, last_pos, (const float*)nullptr, 0.f, idx_stride, 0ll, flags, (uint4*)masks)));
-  }
+  const bool blend = cmap != nullptr && cblend > 0.f;
+  auto go = [&](auto kernel, int parts, int threads) {
+    return launch_chained("forward_kernel", kernel, dim3((unsigned)(batch * g.T * parts)), threads, 0, st, g, prims,
+                          atlas, offs, idx, color, alpha, T_last, last_pos, blend ? cmap : nullptr,
+                          blend ? cblend : 0.f, idx_stride, blend ? cmap_stride : 0ll, flags, (uint4*)masks);
+  };
+  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, constexpr int parts = kFwdParts<TSV>(), threads = kFwdWarps<TSV>() * 32;
+      if (blend) return masks ? go(forward_kernel<TSV, KD, true, true>, parts, threads)
+                              : go(forward_kernel<TSV, KD, true, false>, parts, threads);
+      return masks ? go(forward_kernel<TSV, KD, false, true>, parts, threads)
+                   : go(forward_kernel<TSV, KD, false, false>, parts, threads)));
+  return DBMP_OK;
 }
 
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
@@ -1172,17 +1180,18 @@ int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const 
   if (g.T == 0 || batch == 0) return DBMP_OK;
   const long long ctas = (long long)batch * g.T * kTileWarps<32>();
   if (ctas > 0x7fffffffll) { set_error("backward: %d candidates x %d tiles exceed one grid", batch, g.T); return DBMP_ERR_INVALID; }
-  if (cmap != nullptr && cblend > 0.f) {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "backward_kernel", backward_kernel<TSV, KD, true>, dim3((unsigned)(batch * g.T * kTileWarps<TSV>())), 32, 0, st,
-        g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, cmap, cblend, idx_stride,
-        cmap_stride, (const uint4*)masks)));
-  } else {
-    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-        "backward_kernel", backward_kernel<TSV, KD, false>, dim3((unsigned)(batch * g.T * kTileWarps<TSV>())), 32, 0, st,
-        g, prims, atlas, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, (const float*)nullptr, 0.f,
-        idx_stride, 0ll, (const uint4*)masks)));
-  }
+  const bool blend = cmap != nullptr && cblend > 0.f;
+  auto go = [&](auto kernel, int warps) {
+    return launch_chained("backward_kernel", kernel, dim3((unsigned)(batch * g.T * warps)), 32, 0, st, g, prims, atlas,
+                          offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, blend ? cmap : nullptr,
+                          blend ? cblend : 0.f, idx_stride, blend ? cmap_stride : 0ll, (const uint4*)masks);
+  };
+  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind,
+      if (blend) return masks ? go(backward_kernel<TSV, KD, true, true>, kTileWarps<TSV>())
+                              : go(backward_kernel<TSV, KD, true, false>, kTileWarps<TSV>());
+      return masks ? go(backward_kernel<TSV, KD, false, true>, kTileWarps<TSV>())
+                   : go(backward_kernel<TSV, KD, false, false>, kTileWarps<TSV>())));
+  return DBMP_OK;
 }
 
 int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
