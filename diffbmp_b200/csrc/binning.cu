@@ -259,9 +259,9 @@ __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const 
 // The write loop is bound by its instructions: write positions are pointers and
 // the compaction buffer is padded, so that it holds neither 64-bit index sums nor
 // bounds tests.  Replayed from a graph: 16.5 -> 10.5 us at 256x256, N=512;
-// 20.5 -> 14.1 at 1024x1024, N=5000; 49.0 -> 45.3 at 2048x2048, N=20000; 487 ->
-// 439 at 4096x4096, N=100000 (against a memset, a difference array in global
-// memory and a library scan of all counts, six launches).
+// 20.5 -> 14.1 at 1024x1024, N=5000 (against a memset, a difference array in global
+// memory and a library scan of all counts, six launches); with the masks of
+// use_masks 49.0 -> 36.6 at 2048x2048, N=20000 and 487 -> 281 at 4096x4096, N=100000.
 constexpr int kBinThreads = 512;
 constexpr int kBinWarps = kBinThreads / 32;
 constexpr int kBinTPW = 2;                       // tiles per warp
@@ -273,16 +273,39 @@ struct BinGrid {
   int span;     // primitives per slice (multiple of kBinThreads)
   int subs;     // counting slices per slice
   int cspan;    // primitives per counting slice
+  int words;    // 32-bit words of a cell's primitive mask (0: lists written without masks)
   long long ctas;
 };
 
-// Enough slices to give every SM several CTAs, never a slice below one chunk.
+constexpr size_t kCountsSmem = 200 * 1024;
+// A masking CTA: its primitives, their words, and its words of shared memory
+// (an odd stride, so that a cell's words lie in different banks).
+constexpr int kMaskPrims = kBinThreads, kMaskWords = kMaskPrims / 32;
+__host__ __device__ static inline size_t mask_stride(int cells) { return (size_t)cells | 1; }
+
+// Whether lists are written from primitive masks of the cells (tile row, group of
+// kBinGroup tiles).  Testing every rectangle in every cell costs cells x chunks,
+// marking the masks about as much as the lists are long.  By cells x chunks, without
+// and with masks (whole binning, us): 1280 (1024x1024, N=20000) 22.9 / 24.3; 1536
+// (2048x2048, N=6000) 25.1 / 25.6; 1760 (1024x1024, N=28000) 28.7 / 27.7; 5120
+// (2048x2048, N=20000) 45.1 / 36.6; 100352 (4096x4096, N=100000) 437 / 281.  The
+// marks of a masking CTA have to fit its shared memory (cells up to 3200, canvases
+// to about 10000x10000 at tile 32), and the masks 64 MB of workspace.
+static inline bool use_masks(long long cells, int chunks) {
+  return cells * chunks >= 1600 && cells * chunks <= (1ll << 20) && cells <= INT_MAX &&
+         mask_stride((int)cells) * kMaskWords * sizeof(unsigned) <= kCountsSmem;
+}
+
+// Enough slices to give every SM several CTAs (with masks, where a CTA has little
+// to do per primitive, half as many: 36.6 us against 39.1 at 2048x2048, N=20000),
+// never a slice below one chunk.
 static inline BinGrid bin_grid(int N, int tilesX, int tilesY) {
   BinGrid b;
   b.groups = (tilesX + kBinGroup - 1) / kBinGroup;
   const long long base = (long long)b.groups * tilesY;
   const int chunks = N > 0 ? (N + kBinThreads - 1) / kBinThreads : 1;
-  const long long want = (148 * 8 + base - 1) / base;
+  b.words = use_masks(base, chunks) ? chunks * kMaskWords : 0;
+  const long long want = (148 * (b.words ? 4 : 8) + base - 1) / base;
   b.slices = (int)(want < chunks ? want : chunks);
   if (b.slices < 1) b.slices = 1;
   const int per = (chunks + b.slices - 1) / b.slices;
@@ -299,6 +322,39 @@ static inline BinGrid bin_grid(int N, int tilesX, int tilesY) {
   return b;
 }
 
+// The part of the counting launch that marks, for each cell (tile row, group of
+// kBinGroup tiles), which of kMaskPrims primitives touch it, and writes the cells'
+// words of masks[cell][word].  Two threads per primitive, one for every other row
+// of its rectangle, each lane of a warp starting at another row, so that lanes with
+// tall rectangles rarely meet in a word.
+__device__ __forceinline__ void mask_rects(const Geom& g, const BinGrid& bg, const int4* __restrict__ rects,
+                                           unsigned* s, int block, unsigned* __restrict__ masks) {
+  const int cells = bg.groups * g.tilesY;
+  const int stride = (int)mask_stride(cells);
+  for (int i = threadIdx.x; i < stride * kMaskWords; i += blockDim.x) s[i] = 0u;
+  __syncthreads();
+  const int own = threadIdx.x % kMaskPrims, n = block * kMaskPrims + own;
+  if (n < g.N) {
+    const int4 rc = rects[n];
+    if (rc.x <= rc.y && rc.z <= rc.w) {
+      const int g0 = rc.x / kBinGroup, g1 = rc.y / kBinGroup, h = rc.w - rc.z + 1;
+      unsigned* mine = s + (own >> 5) * stride;
+      const unsigned bit = 1u << (own & 31);
+      int y = (own & 31) % h;
+      for (int i = 0; i < h; ++i) {
+        if ((i & 1) == threadIdx.x / kMaskPrims)
+          for (int q = g0; q <= g1; ++q) atomicOr(mine + (rc.z + y) * bg.groups + q, bit);
+        y = y + 1 == h ? 0 : y + 1;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < cells * kMaskWords; i += blockDim.x) {
+    const int cell = i / kMaskWords, w = i % kMaskWords;
+    masks[(size_t)cell * bg.words + block * kMaskWords + w] = s[w * stride + cell];
+  }
+}
+
 // One CTA per (counting slice, candidate); slice s has counting slices s subs to
 // s subs + subs - 1.  The difference array of (tilesY+1) x
 // (tilesX+1) counters sits in dynamic shared memory, or, for canvases beyond
@@ -307,11 +363,17 @@ static inline BinGrid bin_grid(int N, int tilesX, int tilesY) {
 // columns the same way.
 __global__ void __launch_bounds__(1024) counts_kernel(Geom g, BinGrid bg, const int4* __restrict__ rects,
                                                       int* __restrict__ scratch, int* __restrict__ counts,
-                                                      unsigned long long* __restrict__ row_total) {
+                                                      unsigned long long* __restrict__ row_total,
+                                                      unsigned* __restrict__ masks) {
   extern __shared__ int s_diff[];
   grid_dependency();
-  const int part = blockIdx.x, parts = gridDim.x;   // counting slice
+  const int part = blockIdx.x, parts = bg.slices * bg.subs;   // counting slice
   const size_t b = blockIdx.y;
+  if (part >= parts) {
+    mask_rects(g, bg, rects + b * g.N, (unsigned*)s_diff, part - parts,
+               masks + b * ((size_t)bg.groups * g.tilesY * bg.words));
+    return;
+  }
   const int gw = g.tilesX + 1;
   const int cells = (g.tilesY + 1) * gw;
   int* d = scratch ? scratch + (b * parts + part) * cells : s_diff;
@@ -424,6 +486,146 @@ __global__ void __launch_bounds__(kOffsThreads) offsets_kernel(Geom g, BinGrid b
   }
 }
 
+// What the writing kernels share.  A CTA's cell and slice, and of its warps' tiles
+// gx0 + warp + k kBinWarps: the column a rectangle must reach (INT_MAX for a tile
+// past the canvas, which no rectangle contains) and the next write position.
+struct BinTiles {
+  int slice, ty, gx0, gx1;
+  int col[kBinTPW];
+  int* cur[kBinTPW];
+
+  // Publishes tile_offsets, L and the overflow flag; false when the lists do not fit.
+  __device__ __forceinline__ bool open(const Geom& g, const BinGrid& bg, const long long* __restrict__ offs,
+                                       long long cap, int* __restrict__ indices, long long index_stride,
+                                       int* __restrict__ tile_offsets, int* __restrict__ total_out,
+                                       int* __restrict__ overflow_out, long long flag_stride,
+                                       volatile int* host_flags) {
+    const size_t cand = blockIdx.y;   // candidate of a batch
+    const long long nslots = (long long)g.T * bg.slices;
+    offs += cand * (nslots + 1);
+    indices += cand * index_stride;
+    tile_offsets += cand * (g.T + 1);
+    slice = blockIdx.x % bg.slices;
+    const int rg = blockIdx.x / bg.slices;
+    ty = rg / bg.groups;
+    gx0 = (rg - ty * bg.groups) * kBinGroup;
+    gx1 = min(gx0 + kBinGroup - 1, g.tilesX - 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long L = offs[nslots];
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (first) {
+      if (total_out) total_out[cand * flag_stride] = (int)min(L, (long long)INT_MAX);
+      if (overflow_out) overflow_out[cand * flag_stride] = (L > cap) ? 1 : 0;
+      if (host_flags) {   // the host polls the second word
+        host_flags[2 * cand] = (int)min(L, (long long)INT_MAX);
+        __threadfence_system();
+        host_flags[2 * cand + 1] = (L > cap) ? 1 : 0;
+        __threadfence_system();
+      }
+    }
+    if (L > cap) return false;   // uniform over the CTA
+    if (first) tile_offsets[g.T] = (int)L;
+#pragma unroll
+    for (int k = 0; k < kBinTPW; ++k) {
+      const int tx = gx0 + warp + k * kBinWarps;
+      col[k] = INT_MAX;
+      cur[k] = indices;
+      if (tx <= gx1) {
+        const int t = ty * g.tilesX + tx;
+        const long long at = offs[(long long)t * bg.slices + slice];
+        col[k] = tx;
+        cur[k] = indices + at;
+        if (lane == 0 && slice == 0) tile_offsets[t] = (int)at;
+      }
+    }
+    return true;
+  }
+
+  // Appends the ids of those of the compacted rectangles (padded to a multiple of
+  // 32 with empty ones) that contain each of the warp's tiles.
+  __device__ __forceinline__ void append(const int* s_id, const int2* s_xr, int padded) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int j = lane; j < padded; j += 32) {
+      const int2 xr = s_xr[j];
+      const int id = s_id[j];   // (not set in the padding, nor used there)
+#pragma unroll
+      for (int k = 0; k < kBinTPW; ++k) {
+        const bool in = xr.x <= col[k] && col[k] <= xr.y;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) cur[k][__popc(m & lt)] = id;
+        cur[k] += __popc(m);
+      }
+    }
+  }
+};
+
+// The lists from the cells' primitive masks: a thread expands the bits of a word of
+// its CTA's slice into the compaction buffer, so that a chunk is kBinThreads words,
+// 16384 primitives, where testing every rectangle of the canvas in every cell takes
+// a chunk per kBinThreads rectangles (4096x4096, N=100000, L=167e6: binning 437 ->
+// 281 us, of which writing the lists takes 103 at the copy rate).  What is left is
+// mostly the write loop's population counts.  Not faster: their sums as byte
+// counters of four tiles in a shuffle scan (321 us), four tiles per warp (329).
+constexpr int kMaskBuffer = 2048;
+
+__global__ void __launch_bounds__(kBinThreads, 3) bin_masks_kernel(
+    Geom g, BinGrid bg, const int4* __restrict__ rects, const unsigned* __restrict__ masks,
+    const long long* __restrict__ offs, long long cap, int* __restrict__ indices, long long index_stride,
+    int* __restrict__ tile_offsets, int* __restrict__ total_out, int* __restrict__ overflow_out, long long flag_stride,
+    volatile int* host_flags) {
+  __shared__ int s_id[kMaskBuffer];
+  __shared__ int2 s_xr[kMaskBuffer];   // the rectangle's tile columns x0, x1
+  __shared__ int s_wcnt[kBinWarps];
+  grid_dependency();
+  BinTiles bt;
+  if (!bt.open(g, bg, offs, cap, indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride, host_flags))
+    return;
+  rects += (size_t)blockIdx.y * g.N;
+  const int cell = blockIdx.x / bg.slices, cells = bg.groups * g.tilesY;
+  masks += ((size_t)blockIdx.y * cells + cell) * bg.words;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lo = bt.slice * (bg.span / 32), hi = min(bg.words, lo + bg.span / 32);
+  for (int w0 = lo; w0 < hi; w0 += kBinThreads) {
+    const int w = w0 + (int)threadIdx.x;
+    unsigned word = w < hi ? masks[w] : 0u;
+    int inc = __popc(word);
+    const int own = inc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) s_wcnt[warp] = inc;
+    __syncthreads();
+    int sum = lane < kBinWarps ? s_wcnt[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < kBinWarps; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += u;
+    }
+    const int total = __shfl_sync(0xffffffffu, sum, kBinWarps - 1);
+    int at = inc - own + (warp == 0 ? 0 : __shfl_sync(0xffffffffu, sum, warp - 1));   // this word's first entry
+    for (int base = 0; base < total; base += kMaskBuffer) {
+      const int count = min(kMaskBuffer, total - base), padded = (count + 31) & ~31;
+      while (word != 0u && at < base + kMaskBuffer) {
+        s_id[at++ - base] = (w << 5) + __ffs(word) - 1;
+        word &= word - 1u;
+      }
+      __syncthreads();
+      for (int j = threadIdx.x; j < padded; j += kBinThreads) {
+        int2 xr = make_int2(1, 0);   // contains no column
+        if (j < count) xr = *reinterpret_cast<const int2*>(rects + s_id[j]);
+        s_xr[j] = xr;
+      }
+      __syncthreads();
+      bt.append(s_id, s_xr, padded);
+      __syncthreads();
+    }
+    __syncthreads();   // s_wcnt is rewritten by the next round
+  }
+}
+
 __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGrid bg,
                                                                   const int4* __restrict__ rects,
                                                                   const long long* __restrict__ offs, long long cap,
@@ -440,52 +642,13 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
   __shared__ int2 s_xr[2][kBinThreads];   // the rectangle's tile columns x0, x1
   __shared__ int s_wcnt[2][kBinWarps];
   grid_dependency();
-  const size_t cand = blockIdx.y;   // candidate of a batch
-  const long long nslots = (long long)g.T * bg.slices;
-  rects += cand * g.N;
-  offs += cand * (nslots + 1);
-  indices += cand * index_stride;
-  tile_offsets += cand * (g.T + 1);
-  const int slice = blockIdx.x % bg.slices;
-  const int rg = blockIdx.x / bg.slices;
-  const int ty = rg / bg.groups;
-  const int gx0 = (rg - ty * bg.groups) * kBinGroup, gx1 = min(gx0 + kBinGroup - 1, g.tilesX - 1);
+  BinTiles bt;
+  if (!bt.open(g, bg, offs, cap, indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride, host_flags))
+    return;
+  rects += (size_t)blockIdx.y * g.N;
+  const int slice = bt.slice, ty = bt.ty, gx0 = bt.gx0, gx1 = bt.gx1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  // this warp's tiles gx0 + warp + k kBinWarps: the column a rectangle must
-  // reach (INT_MAX for a tile past the canvas, which no rectangle contains)
-  // and the next write position of each
-  int col[kBinTPW];
-  int* cur[kBinTPW];
-  {
-    const long long L = offs[nslots];
-    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
-    if (first) {
-      if (total_out) total_out[cand * flag_stride] = (int)min(L, (long long)INT_MAX);
-      if (overflow_out) overflow_out[cand * flag_stride] = (L > cap) ? 1 : 0;
-      if (host_flags) {   // the host polls the second word
-        host_flags[2 * cand] = (int)min(L, (long long)INT_MAX);
-        __threadfence_system();
-        host_flags[2 * cand + 1] = (L > cap) ? 1 : 0;
-        __threadfence_system();
-      }
-    }
-    if (L > cap) return;   // uniform over the CTA
-    if (first) tile_offsets[g.T] = (int)L;
-#pragma unroll
-    for (int k = 0; k < kBinTPW; ++k) {
-      const int tx = gx0 + warp + k * kBinWarps;
-      col[k] = INT_MAX;
-      cur[k] = indices;
-      if (tx <= gx1) {
-        const int t = ty * g.tilesX + tx;
-        const long long at = offs[(long long)t * bg.slices + slice];
-        col[k] = tx;
-        cur[k] = indices + at;
-        if (lane == 0 && slice == 0) tile_offsets[t] = (int)at;
-      }
-    }
-  }
   const int lo = slice * bg.span, hi = min(g.N, lo + bg.span);
   const int4 none = make_int4(1, 0, 1, 0);
   // a rectangle survives the CTA's test when it covers row ty and overlaps the tile group
@@ -531,17 +694,7 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
     // barrier), and s_wcnt[buf], last read in (1) above (before this barrier).
     __syncthreads();
     // (3) each warp writes the compacted rectangles that contain its tiles
-    for (int j = lane; j < padded; j += 32) {
-      const int2 xr = s_xr[buf][j];
-      const int id = s_id[buf][j];   // (not set in the padding, nor used there)
-#pragma unroll
-      for (int k = 0; k < kBinTPW; ++k) {
-        const bool in = xr.x <= col[k] && col[k] <= xr.y;
-        const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (in) cur[k][__popc(m & lt)] = id;
-        cur[k] += __popc(m);
-      }
-    }
+    bt.append(s_id[buf], s_xr[buf], padded);
   }
 }
 
@@ -551,12 +704,11 @@ struct BinWorkspace {
   int* counts;                     // (tile, counting slice) entries per candidate
   long long* offs;                 // list positions per (tile, writing slice), and L, per candidate
   unsigned long long* row_total;   // tilesY list lengths of the tile rows per candidate
+  unsigned* masks;                 // primitive masks of the cells per candidate (null without)
   int* scratch;                    // difference arrays that do not fit shared memory (null otherwise)
 };
 
 static inline size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
-
-constexpr size_t kCountsSmem = 200 * 1024;
 
 static inline size_t diff_cells_bytes(int tilesX, int tilesY) {
   return sizeof(int) * (size_t)(tilesY + 1) * (tilesX + 1);
@@ -572,6 +724,8 @@ static size_t layout_ws(void* base, int batch, int N, int T, int tilesX, int til
   const size_t o_counts = take(sizeof(int) * 2 * (B * T * parts + 1));
   const size_t o_offs = take(sizeof(long long) * B * ((size_t)T * bg.slices + 1));
   const size_t o_rows = take(sizeof(unsigned long long) * B * tilesY);
+  const size_t mask_words = (size_t)bg.groups * tilesY * bg.words;
+  const size_t o_masks = mask_words ? take(sizeof(unsigned) * B * mask_words) : 0;
   const size_t cells = diff_cells_bytes(tilesX, tilesY);
   const size_t o_scratch = cells > kCountsSmem ? take(cells * B * parts) : 0;
   if (w) {
@@ -580,6 +734,7 @@ static size_t layout_ws(void* base, int batch, int N, int T, int tilesX, int til
     w->counts = reinterpret_cast<int*>(b + o_counts);
     w->offs = reinterpret_cast<long long*>(b + o_offs);
     w->row_total = reinterpret_cast<unsigned long long*>(b + o_rows);
+    w->masks = mask_words ? reinterpret_cast<unsigned*>(b + o_masks) : nullptr;
     w->scratch = cells > kCountsSmem ? reinterpret_cast<int*>(b + o_scratch) : nullptr;
   }
   return off;
@@ -932,17 +1087,23 @@ int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, con
   int rc = launch_chained("prepare_kernel", prepare_kernel, prep, kPrepThreads, 0, st, g, means2D, radii, rot, opac,
                           colors, sel, sel_stride, tbbox, bin_mode, prim_info, w.rects, w.row_total);
   if (rc) return rc;
-  const size_t smem = w.scratch ? 0 : diff_cells_bytes(g.tilesX, g.tilesY);
+  size_t smem = w.scratch ? 0 : diff_cells_bytes(g.tilesX, g.tilesY);
+  if (bg.words) smem = std::max(smem, mask_stride(bg.groups * g.tilesY) * kMaskWords * sizeof(unsigned));
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(counts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountsSmem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(counts_kernel)");
   }
-  rc = launch_chained("counts_kernel", counts_kernel, dim3(bg.slices * bg.subs, batch), 1024, smem, st, g, bg,
-                      (const int4*)w.rects, w.scratch, w.counts, w.row_total);
+  rc = launch_chained("counts_kernel", counts_kernel, dim3(bg.slices * bg.subs + bg.words / kMaskWords, batch), 1024, smem, st,
+                      g, bg, (const int4*)w.rects, w.scratch, w.counts, w.row_total, w.masks);
   if (rc) return rc;
   rc = launch_chained("offsets_kernel", offsets_kernel, dim3(g.tilesY, batch), kOffsThreads, 0, st, g, bg,
                       (const int*)w.counts, (const unsigned long long*)w.row_total, w.offs);
   if (rc) return rc;
+  if (bg.words)
+    return launch_chained("bin_masks_kernel", bin_masks_kernel, dim3((unsigned)bg.ctas, batch), kBinThreads, 0, st, g,
+                          bg, (const int4*)w.rects, (const unsigned*)w.masks, (const long long*)w.offs, cap,
+                          tile_indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride,
+                          (volatile int*)host_flags);
   return launch_chained("bin_rows_kernel", bin_rows_kernel, dim3((unsigned)bg.ctas, batch), kBinThreads, 0, st, g, bg,
                         (const int4*)w.rects, (const long long*)w.offs, cap, tile_indices, index_stride, tile_offsets,
                         total_out, overflow_out, flag_stride, (volatile int*)host_flags);

@@ -20,6 +20,13 @@ CASES = [  # H, W, tile, N, largest radius
     (2081, 64, 32, 1300, 200.0),
     (64, 65, 32, 40000, 40.0),
     (3713, 3712, 16, 700, 60.0),
+    # lists from primitive masks: few primitives per word; more than a buffer of them
+    # in a cell; more than a chunk of words in the only slice; just below the rule
+    (33 * 32 + 1, 65 * 32, 32, 8200, 30.0),
+    (1100, 1050, 32, 26000, 900.0),
+    (16 * 790, 16 * 100, 16, 17000, 20.0),
+    (1024, 1024, 32, 25088, 40.0),
+    (1024, 1024, 32, 25089, 40.0),
 ]
 
 
