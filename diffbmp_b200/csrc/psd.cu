@@ -160,8 +160,15 @@ struct PsdArgs {
 // with its cosine and sine, opacity and colour once per layer, broadcast to
 // the lanes.  Each thread then computes its pixels with the reference's
 // per-pixel operations on the same values, so the bytes are the ones a
-// per-pixel evaluation gives.
-__global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float* __restrict__ means2D,
+// per-pixel evaluation gives.  Bound by its instructions: without a colour map the
+// colour bytes of a layer are converted once, since a pixel's mask factor is 1
+// wherever its template value is above 0, and stores step a pointer.  Many short
+// ranges (96 CTAs of four warps per SM) keep the SMs filled to the end, where ranges
+// of cheap outside blocks finish early.  1024x1024, N=1500: 289 -> 212 us (ranges
+// alone 258, one kernel with and without colour map 219); N=5000 913 -> 642;
+// 2048x2048, N=20000: 11.7 -> 9.7 ms.
+template <bool MAPPED>
+__global__ void __launch_bounds__(128, 8) psd_layers_kernel(PsdArgs a, const float* __restrict__ means2D,
                                                          const float* __restrict__ radii,
                                                          const float* __restrict__ rot,
                                                          const float* __restrict__ colors,
@@ -183,6 +190,7 @@ __global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float*
   long long next = 0;              // blk[n + 1]
   int4 bb = make_int4(0, 0, 0, 0);
   float x = 0.f, y = 0.f, r = 0.f, theta = 0.f, cos_t = 0.f, sin_t = 0.f, vs = 0.f, cr = 0.f, cg = 0.f, cb = 0.f;
+  unsigned rgb8 = 0u;              // the layer's colour bytes
   int t_idx = 0, bx_n = 1;
   long long off = 0, first = 0;    // the layer's byte offset and first block
   int bx = 0, by = 0;              // the current block's first pixel within the crop
@@ -226,6 +234,7 @@ __global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float*
       cos_t = __shfl_sync(0xffffffffu, cos_t, 0); sin_t = __shfl_sync(0xffffffffu, sin_t, 0);
       vs = __shfl_sync(0xffffffffu, vs, 0);
       cr = __shfl_sync(0xffffffffu, cr, 0); cg = __shfl_sync(0xffffffffu, cg, 0); cb = __shfl_sync(0xffffffffu, cb, 0);
+      rgb8 = to_u8(cr) | to_u8(cg) << 8 | to_u8(cb) << 16;
       t_idx = __shfl_sync(0xffffffffu, t_idx, 0);
       off = __shfl_sync(0xffffffffu, off, 0);
       first = __shfl_sync(0xffffffffu, first, 0);
@@ -265,14 +274,14 @@ __global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float*
     if (lpx >= bw) continue;
     const int px = bb.x + lpx;
     const int rows = min(kPsdBlock, bh - by);   // rows of this block inside the crop
+    uint8_t* dst = out + off + ((long long)(by + ly0) * bw + lpx) * 4;   // this thread's pixel of the row
+    const long long step = (long long)bw * 8;
     if (outside) {
-      for (int ly = ly0; ly < rows; ly += 2)
-        *reinterpret_cast<uchar4*>(out + off + ((long long)(by + ly) * bw + lpx) * 4) = make_uchar4(0, 0, 0, 0);
+      for (int ly = ly0; ly < rows; ly += 2, dst += step) *reinterpret_cast<uchar4*>(dst) = make_uchar4(0, 0, 0, 0);
       continue;
     }
-    for (int ly = ly0; ly < rows; ly += 2) {
-      const int lpy = by + ly;
-      const int py = bb.y + lpy;
+    for (int ly = ly0; ly < rows; ly += 2, dst += step) {
+      const int py = bb.y + by + ly;
       // The column is hidden from the optimiser in every row, so no part of
       // the pixel's expression is hoisted out of the loop: a hoisted cos*u
       // lets the compiler fuse the other product instead, which changes the
@@ -281,23 +290,28 @@ __global__ void __launch_bounds__(256) psd_layers_kernel(PsdArgs a, const float*
       asm volatile("" : "+r"(pxr));
       const float tv = psd_template_value(tmpl, t_idx, a.P, a.Ht, a.Wt, pxr, py, x, y, r, cos_t, sin_t);
       const float alpha_val = tv * vs * a.alpha_max;
-      uchar4 px4 = make_uchar4(0, 0, 0, 0);
+      unsigned px4 = 0u;
       if (!(alpha_val < 0.001f)) {
-        float rgb_r = cr, rgb_g = cg, rgb_b = cb;
-        if (colors_orig != nullptr && a.c_blend > 0.0f) {
-          const float* cm = colors_orig + (size_t)n * a.Ht * a.Wt * 3;
-          const float ux = x / a.scale, uy = y / a.scale;
-          const float upx = (float)pxr / a.scale, upy = (float)py / a.scale;
-          const float ur = r / a.scale;
-          const float3 co = psd_color_map(cm, a.Ht, a.Wt, upx - ux, upy - uy, ur, theta);
-          rgb_r = (1.0f - a.c_blend) * rgb_r + a.c_blend * co.x;
-          rgb_g = (1.0f - a.c_blend) * rgb_g + a.c_blend * co.y;
-          rgb_b = (1.0f - a.c_blend) * rgb_b + a.c_blend * co.z;
+        if (!MAPPED && tv > 0.0f) {
+          px4 = rgb8 | (unsigned)to_u8(alpha_val) << 24;
+        } else {
+          float rgb_r = cr, rgb_g = cg, rgb_b = cb;
+          if constexpr (MAPPED) {
+            const float* cm = colors_orig + (size_t)n * a.Ht * a.Wt * 3;
+            const float ux = x / a.scale, uy = y / a.scale;
+            const float upx = (float)pxr / a.scale, upy = (float)py / a.scale;
+            const float ur = r / a.scale;
+            const float3 co = psd_color_map(cm, a.Ht, a.Wt, upx - ux, upy - uy, ur, theta);
+            rgb_r = (1.0f - a.c_blend) * rgb_r + a.c_blend * co.x;
+            rgb_g = (1.0f - a.c_blend) * rgb_g + a.c_blend * co.y;
+            rgb_b = (1.0f - a.c_blend) * rgb_b + a.c_blend * co.z;
+          }
+          const float mask = tv > 0.0f ? 1.0f : 0.0f;
+          px4 = to_u8(mask * rgb_r) | to_u8(mask * rgb_g) << 8 | to_u8(mask * rgb_b) << 16 |
+                (unsigned)to_u8(alpha_val) << 24;
         }
-        const float mask = tv > 0.0f ? 1.0f : 0.0f;
-        px4 = make_uchar4(to_u8(mask * rgb_r), to_u8(mask * rgb_g), to_u8(mask * rgb_b), to_u8(alpha_val));
       }
-      *reinterpret_cast<uchar4*>(out + off + ((long long)lpy * bw + lpx) * 4) = px4;
+      *reinterpret_cast<unsigned*>(dst) = px4;
     }
   }
 }
@@ -672,8 +686,10 @@ int launch_psd_layers(int N, int P, int Ht, int Wt, float scale, float alpha_max
                       cudaStream_t st) {
   if (N == 0) return DBMP_OK;
   PsdArgs a{N, P, Ht, Wt, scale, alpha_max, c_blend};
-  psd_layers_kernel<<<148 * 8, 256, 0, st>>>(a, means2D, radii, rot, colors, vis, tmpl, sel, bbox, layer_offsets,
-                                             blk, colors_orig, out);
+  const bool mapped = colors_orig != nullptr && c_blend > 0.0f;
+  auto* kernel = mapped ? psd_layers_kernel<true> : psd_layers_kernel<false>;
+  kernel<<<148 * 96, 128, 0, st>>>(a, means2D, radii, rot, colors, vis, tmpl, sel, bbox, layer_offsets, blk,
+                                        colors_orig, out);
   DBMP_CHECK_LAUNCH("psd_layers_kernel");
   return DBMP_OK;
 }
