@@ -261,7 +261,7 @@ __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const 
 // bounds tests.  Replayed from a graph: 16.5 -> 10.5 us at 256x256, N=512;
 // 20.5 -> 14.1 at 1024x1024, N=5000 (against a memset, a difference array in global
 // memory and a library scan of all counts, six launches); with the masks of
-// use_masks 49.0 -> 36.6 at 2048x2048, N=20000 and 487 -> 281 at 4096x4096, N=100000.
+// use_masks 49.0 -> 34.2 at 2048x2048, N=20000 and 487 -> 268 at 4096x4096, N=100000.
 constexpr int kBinThreads = 512;
 constexpr int kBinWarps = kBinThreads / 32;
 constexpr int kBinTPW = 2;                       // tiles per warp
@@ -434,8 +434,13 @@ __global__ void __launch_bounds__(1024) counts_kernel(Geom g, BinGrid bg, const 
 // slice) of the row, offs[t * S + slice] (tile-major, slice-minor over the
 // canvas), from the totals of the rows above and a scan over the row's counts.
 // The last row's CTA also writes offs[T * S] = L.
+// PER counts per thread and round: as few as a round needs to take the whole row, up
+// to eight (whole binning with 1 / 4 / 8: 14.1 / 14.7 / 15.3 us at 1024x1024, N=5000,
+// 320 counts in a row; 36.5 / 34.9 / 34.1 at 2048x2048, N=20000, 2560 counts; 282 /
+// 272 / 268 at 4096x4096, N=100000, 8192).
 constexpr int kOffsThreads = 512;
 
+template <int PER>
 __global__ void __launch_bounds__(kOffsThreads) offsets_kernel(Geom g, BinGrid bg, const int* __restrict__ counts,
                                                                const unsigned long long* __restrict__ row_total,
                                                                long long* __restrict__ offs) {
@@ -461,10 +466,15 @@ __global__ void __launch_bounds__(kOffsThreads) offsets_kernel(Geom g, BinGrid b
   }
   const int len = g.tilesX * parts;
   long long carry = 0;
-  for (int i0 = 0; i0 < len; i0 += kOffsThreads) {
-    const int i = i0 + threadIdx.x;
-    const int own = i < len ? counts[i] : 0;
-    int v = own;
+  for (int i0 = 0; i0 < len; i0 += kOffsThreads * PER) {
+    const int first = i0 + threadIdx.x * PER;
+    int own[PER], v = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      own[k] = first + k < len ? counts[first + k] : 0;
+      v += own[k];
+    }
+    const int mine = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, v, o);
@@ -480,7 +490,13 @@ __global__ void __launch_bounds__(kOffsThreads) offsets_kernel(Geom g, BinGrid b
     }
     const int before = warp > 0 ? __shfl_sync(0xffffffffu, w, warp - 1) : 0;
     const int total = __shfl_sync(0xffffffffu, w, kOffsThreads / 32 - 1);
-    if (i < len && i % bg.subs == 0) offs[i / bg.subs] = s_base + carry + before + v - own;
+    long long at = s_base + carry + before + v - mine;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int i = first + k;
+      if (i < len && i % bg.subs == 0) offs[i / bg.subs] = at;
+      at += own[k];
+    }
     carry += total;
     __syncthreads();   // s_warp is rewritten by the next round
   }
@@ -1096,7 +1112,9 @@ int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, con
   rc = launch_chained("counts_kernel", counts_kernel, dim3(bg.slices * bg.subs + bg.words / kMaskWords, batch), 1024, smem, st,
                       g, bg, (const int4*)w.rects, w.scratch, w.counts, w.row_total, w.masks);
   if (rc) return rc;
-  rc = launch_chained("offsets_kernel", offsets_kernel, dim3(g.tilesY, batch), kOffsThreads, 0, st, g, bg,
+  const long long row = (long long)g.tilesX * bg.slices * bg.subs;   // counts of a tile row
+  auto* offsets = row > 4 * kOffsThreads ? offsets_kernel<8> : row > kOffsThreads ? offsets_kernel<4> : offsets_kernel<1>;
+  rc = launch_chained("offsets_kernel", offsets, dim3(g.tilesY, batch), kOffsThreads, 0, st, g, bg,
                       (const int*)w.counts, (const unsigned long long*)w.row_total, w.offs);
   if (rc) return rc;
   if (bg.words)
