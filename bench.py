@@ -8,8 +8,8 @@ N=20000 primitives drawn from a 16-bitmap 256x256 atlas, one image-fitting
 iteration per step (device binning + forward + L2 loss + backward + Adam).
 ``value`` is iterations/s of the FP16-storage fused step (half-precision
 bilinear-quad atlas), replayed from a CUDA graph with every input resident in
-HBM; the plain FP32 kernels (unfused forward / backward, FP32 atlas in the
-reference layout) and the FP16 pair-layout atlas are timed beside it on the
+HBM; the plain FP32 kernels (unfused forward / backward, FP32 atlas) and the
+FP16 pair-layout atlas are timed beside it on the
 same scene.  ``e2e`` is the same iteration through the public Python API with the
 primitive parameters uploaded from pinned host memory before each step and
 each step's loss read back by the host (one step in flight: the host reads
@@ -45,8 +45,8 @@ METRIC = "fwd+bwd iters/s at 2048^2 N=20k (FP16-storage fused vs plain FP32)"
 HEADLINE_KIND = "f16q"          # FP16 bilinear-quad atlas
 HEADLINE_KERNEL = "fused_kernel<32, F16_QUAD>"
 # DRAM bytes of one fused_kernel launch (FP16 quad atlas) on the 2048^2 / N=20k
-# scene, from one ncu capture (read 108.3 MB + write 3.8 MB); null for other configs.
-FUSED_DRAM_BYTES_C2 = 112.057e6
+# scene, from one ncu capture (read 107.5 MB + write 3.9 MB); null for other configs.
+FUSED_DRAM_BYTES_C2 = 111.441e6
 
 
 def parse():
@@ -739,7 +739,7 @@ def main():
         "plain_fp32": {"iters_per_s": world * args.steps / t_plain, "ms_per_step": t_plain / args.steps * 1e3,
                        "what": "unfused forward + torch L2 gradient + backward, FP32 atlas, graph replay"},
         "fused_fp32": {"iters_per_s": world * args.steps / t_fused32, "ms_per_step": t_fused32 / args.steps * 1e3,
-                       "what": "fused kernel, FP32 atlas in the reference layout"},
+                       "what": "fused kernel, FP32 atlas (walked as bilinear quads)"},
         "fused_f16_pair": {"iters_per_s": world * args.steps / t_pair, "ms_per_step": t_pair / args.steps * 1e3,
                            "what": "fused kernel, FP16 atlas as horizontal texel pairs (half the FP32 bytes)"},
         "fused_bf16_quad": {"iters_per_s": world * args.steps / t_bf16["bf16q"],
@@ -766,10 +766,8 @@ def main():
                 "what": "public API: every step's parameters H2D from pinned host (ImageFitter.upload_params: copy "
                         "stream, two staging buffers), ImageFitter.step(), loss D2H read by the host every step, "
                         "one step in flight"},
-        "gpu_launches": 6 * args.steps,
-        "gpu_launches_note": "ours per step: prepare, counts, bin_rows, fused, adam, step_increment "
-                             "(+ three memsets -- the binning difference arrays, the loss and the gradient "
-                             "sums -- and the two kernels of one CUB exclusive scan over the tile counts)",
+        "gpu_launches": 8 * args.steps,
+        "gpu_launches_note": "ours per step: prepare, counts, offsets, bin_masks, zero, fused, adam, step_increment",
         "clocks": clocks,
     }
     if args.serving_jobs > 0 and world == 1:   # the serving stream is a single-GPU measurement

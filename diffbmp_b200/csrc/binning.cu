@@ -1,10 +1,10 @@
 // Device binning: per-primitive preparation, primitive -> tile rectangles,
-// then CSR tile lists built row by row without a sort: for each tile row a
-// group of CTAs walks the primitives in index order, compacts those whose
-// rectangle touches the group's tiles, and each warp counts (first pass) or
-// writes (second pass) the entries of its own tile.  Lists therefore come out
-// in ascending primitive order per tile, as the reference's per-tile nonzero()
-// gives them, with no host round trip.
+// then CSR tile lists built row by row without a sort: the tiles' entries are
+// counted from difference arrays of rectangle corners, and for each tile row a
+// group of CTAs takes the primitives in index order, compacts those whose
+// rectangle touches the group's tiles, and each warp writes the entries of its
+// own tiles.  Lists therefore come out in ascending primitive order per tile,
+// as the reference's per-tile nonzero() gives them, with no host round trip.
 //
 // This translation unit is compiled WITHOUT fast-math: the world-space bbox
 // must reproduce the reference's float32 torch element-wise arithmetic
