@@ -290,7 +290,8 @@ __host__ __device__ static inline size_t mask_stride(int cells) { return (size_t
 // (2048x2048, N=6000) 25.1 / 25.6; 1760 (1024x1024, N=28000) 28.7 / 27.7; 5120
 // (2048x2048, N=20000) 45.1 / 36.6; 100352 (4096x4096, N=100000) 437 / 281.  With
 // few chunks there is less to skip: 512 x 4 (4096x4096, N=2000) 33.3 / 35.3; 1128 x 4
-// (6000x6000, N=2000) 58.8 / 50.1; 2538 x 1 (9000x9000, N=500) even.  The marks of a masking CTA have to fit its shared memory (cells up to 3200, canvases
+// (6000x6000, N=2000) 58.8 / 50.1; 2538 x 1 (9000x9000, N=500) even.  The
+// marks of a masking CTA have to fit its shared memory (cells up to 3200, canvases
 // to about 10000x10000 at tile 32), and the masks 64 MB of workspace.
 static inline bool use_masks(long long cells, int chunks) {
   return chunks >= 3 && cells * chunks >= (chunks < 8 ? 2560 : 1600) && cells * chunks <= (1ll << 20) &&
