@@ -18,6 +18,7 @@ DBMP_OK, DBMP_ERR_INVALID, DBMP_ERR_CUDA, DBMP_ERR_CAPACITY, DBMP_ERR_UNSUPPORTE
 ATLAS_F32, ATLAS_F32_QUAD, ATLAS_F16_QUAD, ATLAS_BF16_QUAD, ATLAS_F16_PAIR, ATLAS_BF16_PAIR = range(6)
 BIN_CONTENT, BIN_CULL, BIN_CONTENT_REF = 0, 1, 2
 EXTENDED_ATLAS = 0x41545845    # Canvas.reserved of calls that pass an extended atlas
+FOLLOWED_ATLAS = 0x46545845    # ... and of a FollowedCanvas
 
 # Every symbol include/dbmp.h declares, with (restype, argtypes).
 _vp, _i, _ll, _sz, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_size_t, ctypes.c_float
@@ -50,6 +51,11 @@ class Canvas(ctypes.Structure):
                 ("tmpl_h", ctypes.c_int32), ("tmpl_w", ctypes.c_int32), ("atlas_kind", ctypes.c_int32),
                 ("bin_mode", ctypes.c_int32), ("alpha_max", ctypes.c_float), ("t_stop", ctypes.c_float),
                 ("reserved", ctypes.c_int32)]
+
+
+class FollowedCanvas(Canvas):
+    """Mirror of dbmp_followed_canvas (a canvas in front)."""
+    _fields_ = [("templates", ctypes.c_void_p), ("changed", ctypes.c_void_p)]
 
 
 _CP = ctypes.POINTER(Canvas)

@@ -149,13 +149,14 @@ __device__ __forceinline__ int2 tile_span_cull(float m, float h, int ts, int ext
 
 // blockIdx.y: the candidate of a batch, whose inputs and outputs follow those
 // of the one before (sel: sel_stride apart).  row_total (tilesY per candidate)
-// is zeroed for counts_kernel.
+// is zeroed for counts_kernel, and the flag of a followed atlas for the walk behind.
 __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const float* __restrict__ radii,
                                const float* __restrict__ rot, const float* __restrict__ opac,
                                const float* __restrict__ colors, const int* __restrict__ sel, long long sel_stride,
                                const float* __restrict__ tbbox, int bin_mode, PrimInfo* __restrict__ out,
                                int4* __restrict__ rects, unsigned long long* __restrict__ row_total) {
   grid_dependency();
+  if (g.changed != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *g.changed = 0;
   const size_t b = blockIdx.y, bn = b * g.N;
   means2D += 2 * bn; radii += bn; rot += bn; opac += bn; colors += 3 * bn;
   sel += b * sel_stride;
@@ -947,9 +948,12 @@ int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* 
 int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st) {
   if (P == 0) return DBMP_OK;
   const AtlasExt x = atlas_ext(P, Ht, Wt, kind);
-  if (x.rec_off != 0 && tmpl != out) {   // DBMP_ATLAS_F32: the plain templates come first
-    const cudaError_t e = cudaMemcpyAsync(out, tmpl, sizeof(float) * (size_t)P * Ht * Wt, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMemcpyAsync(templates)");
+  if (x.rec_off != 0) {   // DBMP_ATLAS_F32: the plain templates come first
+    if (tmpl != out) {
+      const cudaError_t e = cudaMemcpyAsync(out, tmpl, sizeof(float) * (size_t)P * Ht * Wt, cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return cuda_status(e, "cudaMemcpyAsync(templates)");
+    }
+    tmpl = static_cast<const float*>(out);   // quads and grids are those of the copy, whatever happens to the original
   }
   return pack_records(tmpl, P, Ht, Wt, x.kind, static_cast<unsigned char*>(out) + x.rec_off, x.solid_off, st);
 }

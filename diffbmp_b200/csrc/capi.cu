@@ -32,7 +32,7 @@ int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* 
 int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
 int launch_convert(int n, const void* const* src, void* const* dst, const long long* counts, bool to_half,
                    cudaStream_t st);
-int launch_zero(double* a, long long n, double* b, cudaStream_t st);
+int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st);
 int launch_prepare(const Geom& g, const float* means2D, const float* radii, const float* rot, const float* opac,
                    const float* colors, const int* sel, PrimInfo* out, cudaStream_t st);
 int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
@@ -130,7 +130,18 @@ int make_geom(const dbmp_canvas* cv, Geom* g, const char* who) {
   grid_shape(cv->tmpl_h, &g->gsy, &g->gGy);
   g->solid_delta = 0;
   g->rec_off = 0;
-  if (cv->reserved == DBMP_CANVAS_EXTENDED_ATLAS) {
+  g->live = nullptr;
+  g->changed = nullptr;
+  if (cv->reserved == DBMP_CANVAS_FOLLOWED_ATLAS) {
+    const dbmp_followed_canvas* f = reinterpret_cast<const dbmp_followed_canvas*>(cv);
+    if (cv->atlas_kind != DBMP_ATLAS_F32 || !f->templates || !f->changed) {
+      set_error("%s: a followed atlas is DBMP_ATLAS_F32 and comes with its templates and a flag", who);
+      return DBMP_ERR_INVALID;
+    }
+    g->live = f->templates;
+    g->changed = f->changed;
+  }
+  if (cv->reserved == DBMP_CANVAS_EXTENDED_ATLAS || g->live) {
     const AtlasExt x = atlas_ext(g->P, g->Ht, g->Wt, g->kind);
     g->kind = x.kind;
     g->rec_off = (long long)x.rec_off;
@@ -373,7 +384,7 @@ int dbmp_backward(const dbmp_canvas* cv, const void* prim_info, const void* atla
   REQUIRE(g.N == 0 || (grad_accum && grad_means2D && grad_radii && grad_rotations && grad_opacities && grad_colors),
           "dbmp_backward: null output");
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, st);
+  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, g.changed, st);
   if (rc) return rc;
   rc = launch_backward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, T_last,
                        last_pos, grad_color, grad_alpha, grad_accum, st);
@@ -429,7 +440,7 @@ int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void
   REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_backward_blend: c_blend %g outside [0, 1]", (double)c_blend);
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_backward_blend: colors_orig is null with c_blend > 0");
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, st);
+  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, g.changed, st);
   if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0, nullptr);
@@ -480,7 +491,7 @@ static int backward_batch(const char* who, const void* walk_masks, const dbmp_ca
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "%s: colors_orig is null with c_blend > 0", who);
   if (!work) return DBMP_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, st);
+  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, g.changed, st);
   if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, batch,
@@ -551,7 +562,7 @@ int dbmp_fused_fwd_bwd(const dbmp_canvas* cv, const void* prim_info, const void*
   REQUIRE(atlas && tile_offsets && tile_indices && target && loss_out, "dbmp_fused_fwd_bwd: null input");
   REQUIRE(g.N == 0 || (prim_info && grad_accum), "dbmp_fused_fwd_bwd: null prim_info / grad_accum");
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N, loss_out, st);
+  rc = launch_zero(grad_accum, 8ll * g.N, loss_out, g.changed, st);
   if (rc) return rc;
   return launch_fused(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, target,
                       background, out_image, grad_accum, loss_out, skip_flag, st);

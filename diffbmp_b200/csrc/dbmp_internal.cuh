@@ -181,6 +181,10 @@ struct Geom {
   long long grid_off;  // byte offset of the clearance grid in a packed atlas
   int solid_delta;     // solid grid minus clearance grid, in bytes (0: no extended atlas)
   long long rec_off;   // byte offset of the records the walks read (host side only)
+  // followed atlases (dbmp_followed_canvas): the templates, and whether they differ
+  // from the packed ones (null otherwise)
+  const float* live;
+  int* changed;
   // the walks' atlas: the caller's pointer advanced to the records they read
   const void* records(const void* atlas) const {
     return atlas ? static_cast<const char*>(atlas) + rec_off : nullptr;

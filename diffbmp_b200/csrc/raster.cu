@@ -898,20 +898,26 @@ template <int KIND, bool CB = false> constexpr int kBlocksPerSM(int cta_warps) {
   return ((KIND == ATLAS_F32 || CB) ? DBMP_WARPS_PER_SM_F32 : DBMP_WARPS_PER_SM) / cta_warps;
 }
 
+// True where a followed atlas's templates differ from the packed ones that this walk
+// would read: its *_changed_kernel then walks the templates.
+template <int KIND> __device__ __forceinline__ bool packed_is_stale(const Geom& g) {
+  return KIND == ATLAS_F32_QUAD && g.changed != nullptr && *g.changed != 0;
+}
+
 // ---------------------------------------------------------------------------
+// One block of a forward launch: kFwdWarps warps of a tile.
 template <int TS, int KIND, bool CB, bool MASKED>
-__global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(kFwdWarps<TS>())) forward_kernel(
-    Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
-    const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
-    float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
-    long long idx_stride, long long cmap_stride, const int* __restrict__ flags, uint4* __restrict__ masks) {
-  grid_dependency();
+__device__ __forceinline__ void forward_block(
+    const Geom& g, int block, Rec (*s_pi)[kChunk], const PrimInfo* __restrict__ prims, const void* __restrict__ atlas,
+    const int* __restrict__ offs, const int* __restrict__ idx, float* __restrict__ out_color,
+    float* __restrict__ out_alpha, float* __restrict__ T_last, int* __restrict__ last_pos,
+    const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride,
+    const int* __restrict__ flags, uint4* __restrict__ masks) {
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
-  __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
   // a batch of candidates is one grid over all their tiles: candidate b's
   // records, lists and images follow candidate b-1's
-  const int gt = blockIdx.x / kFwdParts<TS>(), part = blockIdx.x % kFwdParts<TS>();
+  const int gt = block / kFwdParts<TS>(), part = block % kFwdParts<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;
   // binning overflowed for a candidate: its lists do not exist, and the caller
   // bins again (flags: list length and overflow per candidate)
@@ -943,6 +949,41 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(k
   }
 }
 
+template <int TS, int KIND, bool CB, bool MASKED>
+__global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(kFwdWarps<TS>())) forward_kernel(
+    Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
+    const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
+    float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap, float cblend,
+    long long idx_stride, long long cmap_stride, const int* __restrict__ flags, uint4* __restrict__ masks) {
+  __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
+  grid_dependency();
+  if (packed_is_stale<KIND>(g)) return;
+  forward_block<TS, KIND, CB, MASKED>(g, blockIdx.x, s_pi, prims, atlas, offs, idx, out_color, out_alpha, T_last,
+                                      last_pos, cmap, cblend, idx_stride, cmap_stride, flags, masks);
+}
+
+// The walks of a followed atlas whose templates have changed, on the templates.  They
+// nearly always find nothing to do, so a grid of at most the resident blocks loops
+// over the tiles: it starts and ends in 1 to 2 us, where a block per tile would take
+// 0.2 ns a pixel.  What following costs a job with unchanged templates, the
+// comparison included (1024x1024, N=6000, 8 of 128x128, us): forward 90.7 against 87,
+// backward 138.6 against 136; the walks on the templates themselves take 164.9 and
+// 241.3.
+template <int TS, bool CB, bool MASKED>
+__global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<ATLAS_F32, CB>(kFwdWarps<TS>()))
+    forward_changed_kernel(Geom g, unsigned blocks, const PrimInfo* __restrict__ prims, const int* __restrict__ offs,
+                           const int* __restrict__ idx, float* __restrict__ out_color, float* __restrict__ out_alpha,
+                           float* __restrict__ T_last, int* __restrict__ last_pos, const float* __restrict__ cmap,
+                           float cblend, long long idx_stride, long long cmap_stride, const int* __restrict__ flags,
+                           uint4* __restrict__ masks) {
+  __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
+  grid_dependency();
+  if (*g.changed == 0) return;
+  for (unsigned b = blockIdx.x; b < blocks; b += gridDim.x)
+    forward_block<TS, ATLAS_F32, CB, MASKED>(g, (int)b, s_pi, prims, g.live, offs, idx, out_color, out_alpha, T_last,
+                                             last_pos, cmap, cblend, idx_stride, cmap_stride, flags, masks);
+}
+
 // Counting pass (diagnostics / roofline accounting): same walk as the
 // forward, no outputs except the counters.
 template <int TS, int KIND>
@@ -960,19 +1001,17 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32) count_kernel(Geom g, con
   if (threadIdx.x == 0 && part == 0) atomicAdd(cnt + 2, (unsigned long long)(tw.end - tw.start));
 }
 
+// One block of a backward launch: a warp of a tile.  kept: null without masks.
 template <int TS, int KIND, bool CB, bool MASKED>
-__global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel(
-    Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
-    const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
-    const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
-    const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride,
-    const uint4* __restrict__ masks) {
-  grid_dependency();
+__device__ __forceinline__ void backward_block(
+    const Geom& g, int block, Rec* s_pi, Kept* s_kept, const PrimInfo* __restrict__ prims,
+    const void* __restrict__ atlas, const int* __restrict__ offs, const int* __restrict__ idx,
+    const float* __restrict__ T_last, const int* __restrict__ last_pos, const float* __restrict__ grad_color,
+    const float* __restrict__ grad_alpha, double* __restrict__ gacc, const float* __restrict__ cmap, float cblend,
+    long long idx_stride, long long cmap_stride, const uint4* __restrict__ masks) {
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND, CB>;
-  __shared__ Rec s_pi[kChunk];
-  __shared__ Kept s_kept;
-  const int gt = blockIdx.x / kTileWarps<TS>(), part = blockIdx.x % kTileWarps<TS>();
+  const int gt = block / kTileWarps<TS>(), part = block % kTileWarps<TS>();
   const int b = gt / g.T, tile = gt - b * g.T;     // candidate and tile (see forward_kernel)
   const size_t pix = (size_t)b * g.H * g.W;
   prims += (size_t)b * g.N;
@@ -1004,11 +1043,42 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel
   }
   if constexpr (MASKED) {
     const size_t at = ((size_t)gt * kTileWarps<TS>() + tw.warp) * kKeptChunks;
-    if (tw.lane < kKeptChunks) s_kept.masks[tw.lane] = masks[at + tw.lane];   // (those never written are never used)
-    if (tw.lane == 0) s_kept.in_buffer = -1;
+    if (tw.lane < kKeptChunks) s_kept->masks[tw.lane] = masks[at + tw.lane];   // (those never written are never used)
+    if (tw.lane == 0) s_kept->in_buffer = -1;
     __syncwarp();
   }
-  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc, MASKED ? &s_kept : nullptr);
+  tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc, MASKED ? s_kept : nullptr);
+}
+
+template <int TS, int KIND, bool CB, bool MASKED>
+__global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel(
+    Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
+    const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
+    const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
+    const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride,
+    const uint4* __restrict__ masks) {
+  __shared__ Rec s_pi[kChunk];
+  __shared__ Kept s_kept;
+  grid_dependency();
+  if (packed_is_stale<KIND>(g)) return;
+  backward_block<TS, KIND, CB, MASKED>(g, blockIdx.x, s_pi, &s_kept, prims, atlas, offs, idx, T_last, last_pos,
+                                       grad_color, grad_alpha, gacc, cmap, cblend, idx_stride, cmap_stride, masks);
+}
+
+// (see forward_changed_kernel; the forward's masks belong to the packed templates)
+template <int TS, bool CB>
+__global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32, CB>(1)) backward_changed_kernel(
+    Geom g, unsigned blocks, const PrimInfo* __restrict__ prims, const int* __restrict__ offs,
+    const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
+    const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
+    const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride) {
+  __shared__ Rec s_pi[kChunk];
+  grid_dependency();
+  if (*g.changed == 0) return;
+  for (unsigned b = blockIdx.x; b < blocks; b += gridDim.x)
+    backward_block<TS, ATLAS_F32, CB, false>(g, (int)b, s_pi, nullptr, prims, g.live, offs, idx, T_last, last_pos,
+                                             grad_color, grad_alpha, gacc, cmap, cblend, idx_stride, cmap_stride,
+                                             nullptr);
 }
 
 __device__ __forceinline__ double sigmoid_d(double x) {
@@ -1064,19 +1134,16 @@ __global__ void finalize_kernel(Geom g, const float* __restrict__ radii, const f
 // loss_out (f64, may be null) receives sum((rendered - target)^2) / (3HW),
 // one add per warp.
 template <int TS, int KIND>
-__global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
-    Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
-    const int* __restrict__ idx, const float* __restrict__ target, const float* __restrict__ background,
-    float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
-    const int* __restrict__ skip_flag) {
-  grid_dependency();
-  if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
+__device__ __forceinline__ void fused_block(const Geom& g, int block, Rec* s_pi, Kept& s_kept,
+                                            const PrimInfo* __restrict__ prims, const void* __restrict__ atlas,
+                                            const int* __restrict__ offs, const int* __restrict__ idx,
+                                            const float* __restrict__ target, const float* __restrict__ background,
+                                            float* __restrict__ out_image, double* __restrict__ gacc,
+                                            double* __restrict__ loss_out) {
   constexpr int NP = 2;
   using TW = TileWalker<TS, KIND>;
-  __shared__ Rec s_pi[kChunk];
-  __shared__ Kept s_kept;
   TW tw;
-  const int tile = blockIdx.x / kTileWarps<TS>(), part = blockIdx.x % kTileWarps<TS>();
+  const int tile = block / kTileWarps<TS>(), part = block % kTileWarps<TS>();
   tw.init(g, tile, part, 1, offs);
   float C[NP][3], T[NP], Tl[NP], gC[NP][3], gA[NP];
   int lp[NP];
@@ -1112,6 +1179,60 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
   tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Tl, lp, gacc, &s_kept);
 }
 
+template <int TS, int KIND>
+__global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
+    Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
+    const int* __restrict__ idx, const float* __restrict__ target, const float* __restrict__ background,
+    float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
+    const int* __restrict__ skip_flag) {
+  __shared__ Rec s_pi[kChunk];
+  __shared__ Kept s_kept;
+  grid_dependency();
+  if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
+  if (packed_is_stale<KIND>(g)) return;
+  fused_block<TS, KIND>(g, blockIdx.x, s_pi, s_kept, prims, atlas, offs, idx, target, background, out_image, gacc,
+                        loss_out);
+}
+
+// (see forward_changed_kernel)
+template <int TS>
+__global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32>(1)) fused_changed_kernel(
+    Geom g, unsigned blocks, const PrimInfo* __restrict__ prims, const int* __restrict__ offs,
+    const int* __restrict__ idx, const float* __restrict__ target, const float* __restrict__ background,
+    float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
+    const int* __restrict__ skip_flag) {
+  __shared__ Rec s_pi[kChunk];
+  __shared__ Kept s_kept;
+  grid_dependency();
+  if ((skip_flag != nullptr && *skip_flag != 0) || *g.changed == 0) return;
+  for (unsigned b = blockIdx.x; b < blocks; b += gridDim.x) {
+    __syncwarp();   // every lane is done with the previous block's masks
+    fused_block<TS, ATLAS_F32>(g, (int)b, s_pi, s_kept, prims, g.live, offs, idx, target, background, out_image, gacc,
+                               loss_out);
+  }
+}
+
+// Whether a followed atlas's templates still hold the texels packed from them (the
+// first part of an extended DBMP_ATLAS_F32 atlas), bit by bit; *changed was zeroed
+// before.  16-byte loads where both sides allow them.  8 bytes a texel: 2 us up to
+// 256k texels, at the copy rate beyond the L2.
+template <typename V>
+__global__ void __launch_bounds__(256) templates_changed_kernel(const V* __restrict__ a, const V* __restrict__ b,
+                                                                long long n, int* __restrict__ changed) {
+  grid_dependency();
+  unsigned diff = 0u;
+#pragma unroll 4
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    if constexpr (sizeof(V) == 16) {
+      const uint4 x = a[i], y = b[i];
+      diff |= (x.x ^ y.x) | (x.y ^ y.y) | (x.z ^ y.z) | (x.w ^ y.w);
+    } else {
+      diff |= a[i] ^ b[i];
+    }
+  }
+  if (__any_sync(kFull, diff != 0u) && (threadIdx.x & 31) == 0) atomicOr(changed, 1);
+}
+
 // ---------------------------------------------------------------------------
 #define DBMP_KIND_SWITCH(kind, ...)                                                   \
   switch (kind) {                                                                     \
@@ -1132,6 +1253,31 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
 // batch > 1: `batch` candidates of the same canvas in one grid, candidate b's
 // records at prims + b N, lists at offs + b (T+1) / idx + b idx_stride,
 // images at b H W (x3 for colour), colour maps at cmap + b cmap_stride.
+int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st);
+
+// Compares a followed atlas's templates with the packed records at `atlas` (zero: the
+// flag is not zeroed yet).
+static int launch_changed(const Geom& g, const void* atlas, bool zero, cudaStream_t st) {
+  if (zero) {
+    const int rc = launch_zero(nullptr, 0, nullptr, g.changed, st);
+    if (rc) return rc;
+  }
+  const char* packed = static_cast<const char*>(atlas) - g.rec_off;
+  const long long n = (long long)g.P * g.Ht * g.Wt;
+  const bool wide = n % 4 == 0 && ((uintptr_t)packed & 15) == 0 && ((uintptr_t)g.live & 15) == 0;
+  const long long items = wide ? n / 4 : n, ctas = (items + 255) / 256;
+  const dim3 grid((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8));
+  return wide ? launch_chained("templates_changed_kernel", templates_changed_kernel<uint4>, grid, 256, 0, st,
+                               (const uint4*)g.live, (const uint4*)packed, items, g.changed)
+              : launch_chained("templates_changed_kernel", templates_changed_kernel<unsigned>, grid, 256, 0, st,
+                               (const unsigned*)g.live, (const unsigned*)packed, items, g.changed);
+}
+
+// Grid of a *_changed_kernel: at most what is resident at once.
+static dim3 changed_grid(long long blocks, int per_sm) {
+  return dim3((unsigned)(blocks < 148ll * per_sm ? blocks : 148ll * per_sm));
+}
+
 size_t walk_mask_bytes(const Geom& g, int batch) {
   const size_t warps = (size_t)batch * g.T * (g.TS == 32 ? kTileWarps<32>() : kTileWarps<16>());
   return warps * kKeptChunks * sizeof(uint4);
@@ -1150,11 +1296,31 @@ int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const v
                           atlas, offs, idx, color, alpha, T_last, last_pos, blend ? cmap : nullptr,
                           blend ? cblend : 0.f, idx_stride, blend ? cmap_stride : 0ll, flags, (uint4*)masks);
   };
-  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, constexpr int parts = kFwdParts<TSV>(), threads = kFwdWarps<TSV>() * 32;
-      if (blend) return masks ? go(forward_kernel<TSV, KD, true, true>, parts, threads)
-                              : go(forward_kernel<TSV, KD, true, false>, parts, threads);
-      return masks ? go(forward_kernel<TSV, KD, false, true>, parts, threads)
-                   : go(forward_kernel<TSV, KD, false, false>, parts, threads)));
+  auto walk = [&]() -> int {
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, constexpr int parts = kFwdParts<TSV>(), threads = kFwdWarps<TSV>() * 32;
+        if (blend) return masks ? go(forward_kernel<TSV, KD, true, true>, parts, threads)
+                                : go(forward_kernel<TSV, KD, true, false>, parts, threads);
+        return masks ? go(forward_kernel<TSV, KD, false, true>, parts, threads)
+                     : go(forward_kernel<TSV, KD, false, false>, parts, threads)));
+    return DBMP_OK;
+  };
+  if (!g.live) return walk();
+  // flags: behind a binning, whose first kernel zeroed the flag of the comparison
+  int rc = launch_changed(g, atlas, flags == nullptr, st);
+  if (!rc) rc = walk();
+  if (rc) return rc;
+  auto again = [&](auto kernel, int parts, int threads) {
+    const long long blocks = (long long)batch * g.T * parts;
+    return launch_chained("forward_changed_kernel", kernel, changed_grid(blocks, DBMP_WARPS_PER_SM_F32 * 32 / threads),
+                          threads, 0, st, g, (unsigned)blocks, prims, offs, idx, color, alpha, T_last, last_pos,
+                          blend ? cmap : nullptr, blend ? cblend : 0.f, idx_stride, blend ? cmap_stride : 0ll, flags,
+                          (uint4*)masks);
+  };
+  DBMP_TS_SWITCH(g.TS, constexpr int parts = kFwdParts<TSV>(), threads = kFwdWarps<TSV>() * 32;
+      if (blend) return masks ? again(forward_changed_kernel<TSV, true, true>, parts, threads)
+                              : again(forward_changed_kernel<TSV, true, false>, parts, threads);
+      return masks ? again(forward_changed_kernel<TSV, false, true>, parts, threads)
+                   : again(forward_changed_kernel<TSV, false, false>, parts, threads));
   return DBMP_OK;
 }
 
@@ -1167,6 +1333,10 @@ int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* a
 int launch_count(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs, const int* idx,
                  unsigned long long* cnt, cudaStream_t st) {
   if (g.T == 0) return DBMP_OK;
+  if (g.live) {   // counts what the reference layout's walk does
+    kind = ATLAS_F32;
+    atlas = g.live;
+  }
   DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, (count_kernel<TSV, KD><<<g.T * kFwdParts<TSV>(), kFwdWarps<TSV>() * 32, 0, st>>>(
                                                    g, prims, atlas, offs, idx, cnt))));
   DBMP_CHECK_LAUNCH("count_kernel");
@@ -1186,11 +1356,26 @@ int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const 
                           offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc, blend ? cmap : nullptr,
                           blend ? cblend : 0.f, idx_stride, blend ? cmap_stride : 0ll, (const uint4*)masks);
   };
-  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind,
-      if (blend) return masks ? go(backward_kernel<TSV, KD, true, true>, kTileWarps<TSV>())
-                              : go(backward_kernel<TSV, KD, true, false>, kTileWarps<TSV>());
-      return masks ? go(backward_kernel<TSV, KD, false, true>, kTileWarps<TSV>())
-                   : go(backward_kernel<TSV, KD, false, false>, kTileWarps<TSV>())));
+  auto walk = [&]() -> int {
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind,
+        if (blend) return masks ? go(backward_kernel<TSV, KD, true, true>, kTileWarps<TSV>())
+                                : go(backward_kernel<TSV, KD, true, false>, kTileWarps<TSV>());
+        return masks ? go(backward_kernel<TSV, KD, false, true>, kTileWarps<TSV>())
+                     : go(backward_kernel<TSV, KD, false, false>, kTileWarps<TSV>())));
+    return DBMP_OK;
+  };
+  if (!g.live) return walk();
+  int rc = launch_changed(g, atlas, false, st);   // launch_zero came before
+  if (!rc) rc = walk();
+  if (rc) return rc;
+  auto again = [&](auto kernel, int warps) {
+    const long long blocks = (long long)batch * g.T * warps;
+    return launch_chained("backward_changed_kernel", kernel, changed_grid(blocks, DBMP_WARPS_PER_SM_F32), 32, 0, st, g,
+                          (unsigned)blocks, prims, offs, idx, T_last, last_pos, grad_color, grad_alpha, gacc,
+                          blend ? cmap : nullptr, blend ? cblend : 0.f, idx_stride, blend ? cmap_stride : 0ll);
+  };
+  DBMP_TS_SWITCH(g.TS, return blend ? again(backward_changed_kernel<TSV, true>, kTileWarps<TSV>())
+                                    : again(backward_changed_kernel<TSV, false>, kTileWarps<TSV>()));
   return DBMP_OK;
 }
 
@@ -1201,20 +1386,21 @@ int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* 
                                nullptr, 0.f, st, 1, 0, 0, nullptr);
 }
 
-// Zeroes n doubles at a and, when given, one at b: a kernel rather than
+// Zeroes n doubles at a and, when given, one at b and an int: a kernel rather than
 // memsets, so that the launches around it stay chained.
-__global__ void zero_kernel(double* __restrict__ a, long long n, double* __restrict__ b) {
+__global__ void zero_kernel(double* __restrict__ a, long long n, double* __restrict__ b, int* __restrict__ flag) {
   grid_dependency();
   const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (long long i = i0; i < n; i += (long long)gridDim.x * blockDim.x) a[i] = 0.0;
   if (b != nullptr && i0 == 0) *b = 0.0;
+  if (flag != nullptr && i0 == 0) *flag = 0;
 }
 
-int launch_zero(double* a, long long n, double* b, cudaStream_t st) {
-  if (n == 0 && b == nullptr) return DBMP_OK;
+int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st) {
+  if (n == 0 && b == nullptr && flag == nullptr) return DBMP_OK;
   const long long ctas = (n + 255) / 256;
   return launch_chained("zero_kernel", zero_kernel, dim3((unsigned)(ctas < 1 ? 1 : ctas < 1184 ? ctas : 1184)), 256, 0,
-                        st, a, n, b);
+                        st, a, n, b, flag);
 }
 
 int launch_finalize(const Geom& g, const float* radii, const float* rot, const float* opac, const float* colors,
@@ -1228,9 +1414,19 @@ int launch_fused(const Geom& g, int kind, const PrimInfo* prims, const void* atl
                  const float* target, const float* background, float* out_image, double* gacc, double* loss,
                  const int* skip_flag, cudaStream_t st) {
   if (g.T == 0) return DBMP_OK;
-  DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
-      "fused_kernel", fused_kernel<TSV, KD>, dim3((unsigned)(g.T * kTileWarps<TSV>())), 32, 0, st, g, prims, atlas, offs,
-      idx, target, background, out_image, gacc, loss, skip_flag)));
+  auto walk = [&]() -> int {
+    DBMP_TS_SWITCH(g.TS, DBMP_KIND_SWITCH(kind, return launch_chained(
+        "fused_kernel", fused_kernel<TSV, KD>, dim3((unsigned)(g.T * kTileWarps<TSV>())), 32, 0, st, g, prims, atlas,
+        offs, idx, target, background, out_image, gacc, loss, skip_flag)));
+    return DBMP_OK;
+  };
+  if (!g.live) return walk();
+  int rc = launch_changed(g, atlas, false, st);   // launch_zero came before
+  if (!rc) rc = walk();
+  if (rc) return rc;
+  DBMP_TS_SWITCH(g.TS, const long long blocks = (long long)g.T * kTileWarps<TSV>(); return launch_chained(
+      "fused_changed_kernel", fused_changed_kernel<TSV>, changed_grid(blocks, DBMP_WARPS_PER_SM_F32), 32, 0, st, g,
+      (unsigned)blocks, prims, offs, idx, target, background, out_image, gacc, loss, skip_flag));
 }
 
 }  // namespace dbmp

@@ -207,7 +207,12 @@ class ImageFitter:
         self.background = _dev_f32(background, dev, copy=False) if background is not None else None
         self.atlas = atlas
         self.rz = Rasterizer(self.H, self.W, cfg.tile_size, cfg.alpha_max, cfg.t_stop, device=dev)
-        self.cv = self.rz.canvas(self.N, atlas)
+        self.cv = self.rz.canvas(self.N, atlas)      # (of calls that pass atlas.data)
+        # the walks' canvas and atlas pointer: an "f32" job's steps keep the packed
+        # copy that they started with
+        self._changed = torch.zeros(1, dtype=torch.int32, device=dev)
+        self._quads = atlas.quads() if cfg.blur == "none" else None
+        self._walk_cv, self._walk_atlas = self.rz.walk_canvas(self.N, atlas, self._quads, _ptr(self._changed))
         N8 = (max(self.N, 1), 8)
         self.adam_m = torch.zeros(N8, dtype=torch.float32, device=dev)
         self.adam_v = torch.zeros(N8, dtype=torch.float32, device=dev)
@@ -242,6 +247,7 @@ class ImageFitter:
                 raise ValueError("the adaptive blur schedule needs FitConfig.num_iterations")
             self.atlas = atlas.private_copy(self.H * self.W)
             self.cv = self.rz.canvas(self.N, self.atlas)
+            self._walk_cv, self._walk_atlas = self.rz.walk_canvas(self.N, self.atlas, None, 0)
             self.blur = _lib.BlurSchedule(BLUR_MODES[cfg.blur], cfg.blur_sigma, cfg.blur_sigma_start,
                                           cfg.blur_sigma_end, int(cfg.num_iterations))
             self._blurred = (self.atlas.data if self.atlas.kind == _lib.ATLAS_F32
@@ -294,12 +300,12 @@ class ImageFitter:
         a = self.atlas
         call("dbmp_template_blur_scheduled", _ptr(a.templates), a.P, a.Ht, a.Wt, ctypes.byref(self.blur),
              _ptr(self.step_count), _ptr(self._blurred), st)
-        if a.extended:
+        if a.own:
             a.pack(self._blurred, st)
 
     def _enqueue(self):
         st = _stream()
-        cv = self.cv
+        cv, texels = self._walk_cv, self._walk_atlas
         rz = self.rz
         ws, wsb = rz._ws_ptr()
         skip = ctypes.c_void_p(self.flags.data_ptr() + 4)
@@ -315,7 +321,7 @@ class ImageFitter:
              _ptr(self.offsets), _ptr(rz._idx), ctypes.c_longlong(rz.capacity), _ptr(self.flags), skip, ws,
              ctypes.c_size_t(wsb), st)
         if self.cfg.fused:
-            call("dbmp_fused_fwd_bwd", ctypes.byref(cv), _ptr(self.prim_info), _ptr(self.atlas.data),
+            call("dbmp_fused_fwd_bwd", ctypes.byref(cv), _ptr(self.prim_info), texels,
                  _ptr(self.offsets), _ptr(rz._idx), _ptr(self.target), _ptr(self.background), None,
                  _ptr(self.gacc), _ptr(self.loss_dev), skip, st)
         else:
@@ -323,14 +329,14 @@ class ImageFitter:
             # gradient (simple_tile_renderer.py:704-707, loss_functions.py:20-40),
             # backward kernel.  An overflowed bin leaves stale lists, but the
             # Adam step below is skipped and the step replayed, as in fused form.
-            call("dbmp_forward", ctypes.byref(cv), _ptr(self.prim_info), _ptr(self.atlas.data), _ptr(self.offsets),
+            call("dbmp_forward", ctypes.byref(cv), _ptr(self.prim_info), texels, _ptr(self.offsets),
                  _ptr(rz._idx), _ptr(self.color), _ptr(self.alpha), _ptr(self.T_last), _ptr(self.last_pos), st)
             img = self.color if self.background is None else self.color + (1 - self.alpha).unsqueeze(-1) * self.background
             d = img - self.target
             self.loss_dev.copy_((d * d).mean().double().view(1))
             gC = d * (2.0 / d.numel())
             gA = -(gC * self.background).sum(-1) if self.background is not None else None
-            call("dbmp_backward", ctypes.byref(cv), _ptr(self.prim_info), _ptr(self.atlas.data), _ptr(self.offsets),
+            call("dbmp_backward", ctypes.byref(cv), _ptr(self.prim_info), texels, _ptr(self.offsets),
                  _ptr(rz._idx), _ptr(self.T_last), _ptr(self.last_pos), _ptr(gC), _ptr(gA), _ptr(self.radii),
                  _ptr(self.rotations), _ptr(self.opacities), _ptr(self.colors), _ptr(self.gacc),
                  *[_ptr(g) for g in self.grads], st)
@@ -370,7 +376,6 @@ class ImageFitter:
 
     def step(self):
         """Enqueues one fit iteration (no host synchronisation)."""
-        self.atlas.refresh()
         if self.graph is not None:
             self.graph.replay()
         else:

@@ -23,7 +23,8 @@ import torch
 
 from . import _lib
 from ._lib import (ATLAS_BF16_PAIR, ATLAS_BF16_QUAD, ATLAS_F16_PAIR, ATLAS_F16_QUAD, ATLAS_F32, ATLAS_F32_QUAD,
-                   BIN_CONTENT, BIN_CONTENT_REF, BIN_CULL, EXTENDED_ATLAS, Canvas, DbmpError, call, lib)
+                   BIN_CONTENT, BIN_CONTENT_REF, BIN_CULL, EXTENDED_ATLAS, FOLLOWED_ATLAS, Canvas, DbmpError,
+                   FollowedCanvas, call, lib)
 
 # Atlas storage kinds: "f32" is the reference layout; the precision form
 # stores half / bfloat16 texels as horizontal pairs ("f16", "bf16", two 4-byte
@@ -31,9 +32,9 @@ from ._lib import (ATLAS_BF16_PAIR, ATLAS_BF16_QUAD, ATLAS_F16_PAIR, ATLAS_F16_Q
 KIND_NAMES = {"f32": ATLAS_F32, "f32q": ATLAS_F32_QUAD, "f16q": ATLAS_F16_QUAD, "bf16q": ATLAS_BF16_QUAD,
               "f16": ATLAS_F16_PAIR, "bf16": ATLAS_BF16_PAIR}
 
-# An "f32" atlas also holds its templates as f32 quads (16 bytes a texel) up to
-# this many bytes.  The walks are as fast on quads far beyond the L2 as inside it
-# (2048x2048, N=20000, 1024 templates of 256x256, 1 GiB of quads: forward 257 us,
+# The renders of an "f32" atlas walk a copy of its templates packed as f32 quads (16
+# bytes a texel) up to this many bytes.  The walks are as fast on quads far beyond
+# the L2 as inside it (2048x2048, N=20000, 1024 templates of 256x256, 1 GiB of quads: forward 257 us,
 # backward 384, against 549 and 810 on the reference layout; with 16 templates 239
 # and 363 against 537 and 800), so the limit only bounds their memory and the time
 # to pack them (1.6 ms per GiB).
@@ -67,11 +68,45 @@ def _operand(t: torch.Tensor) -> torch.Tensor:
     return t if t.dtype is torch.float32 and t.is_contiguous() else _f32(t)
 
 
+class Filled:
+    """Device memory that one stream fills once and calls on any stream then read.
+    Made where the fill has just been enqueued on the current stream."""
+
+    def __init__(self, tensor: torch.Tensor):
+        self.tensor = tensor
+        s = torch.cuda.current_stream(tensor.device)
+        self._home = s.cuda_stream
+        self._event = torch.cuda.Event()
+        self._event.record(s)
+        self._done = False
+
+    def use(self, stream=None) -> torch.Tensor:
+        """The tensor, for work enqueued on `stream` (default: the current one) after
+        this call: behind the fill, and not freed before that work is done.  Under
+        graph capture the caller has waited for the fill, as for the capture's
+        other inputs."""
+        if _stream(stream) != self._home:
+            s = stream if stream is not None else torch.cuda.current_stream(self.tensor.device)
+            if not torch.cuda.is_current_stream_capturing():
+                if not self._done:
+                    self._done = self._event.query()
+                if not self._done:
+                    s.wait_event(self._event)
+            self.tensor.record_stream(s)
+        return self.tensor
+
+
 class Atlas:
     """Template atlas on the device.  ``templates``: (P,Ht,Wt) or (Ht,Wt).
     ``sigma`` > 0 renders with Gaussian-blurred templates while the content
     bboxes (binning) stay those of the unblurred ones, as the reference's
-    VectorRenderer does (vector_renderer.py:80-104)."""
+    VectorRenderer does (vector_renderer.py:80-104).
+
+    An "f32" atlas renders the memory of ``data``, which is the caller's tensor where
+    that is contiguous f32, as it is when a call's turn on its stream comes,
+    whoever has written to it (quads() packs a copy for the walks, and every
+    walk compares it with ``data`` first).  The other kinds hold a packed copy
+    made here."""
 
     def __init__(self, templates: torch.Tensor, kind: str | int = "f32", sigma: float = 0.0):
         t = templates if templates.dim() == 3 else templates.unsqueeze(0)
@@ -92,12 +127,11 @@ class Atlas:
         # "f32" the quads, that let the walks skip work
         self.extended = self.kind != ATLAS_F32 or (self.templates.numel() * 16 <= MAX_F32_QUAD_BYTES
                                                    and not self.templates.is_inference())
-        self._followed = None
-        if self.extended:
+        self.own = self.kind != ATLAS_F32     # data is an extended atlas's buffer
+        self._quads = None                    # ("f32") Filled extended atlas, version of data that it was packed from
+        if self.own:
             self._alloc()
             self.pack(self.templates, st)
-            if self.kind == ATLAS_F32:
-                self._followed = self.templates._version
         else:
             self.data = self.templates
 
@@ -110,11 +144,32 @@ class Atlas:
             self.data = self.data.view(torch.float32).view(self.P, self.Ht, self.Wt)
 
     def refresh(self):
-        """Repacks an "f32" atlas whose templates tensor was changed in place
-        since it was packed: that kind renders the caller's tensor as it is."""
-        if self._followed is not None and self._followed != self.templates._version:
-            self.pack(self.templates)
-            self._followed = self.templates._version
+        """Has an "f32" atlas packed anew by its next render.  Never needed for the
+        result: a walk that finds ``data`` changed reads it in the reference layout,
+        which is slower.  A change that PyTorch counts (``data._version``) is
+        packed anew without this call; writes through ``.data``, of another
+        library's kernel or a replayed graph are not counted."""
+        self._quads = None
+
+    def quads(self, stream=None) -> Optional[Filled]:
+        """An "f32" atlas's extended copy (quads and grids) for work on `stream`, or
+        None where it has none and walks data itself.  A copy never changes once
+        packed: calls in flight on other streams or threads keep the one that they
+        took."""
+        if self.own or not self.extended:
+            return None
+        q, version = self._quads or (None, -1)
+        if version != self.data._version:
+            version = self.data._version
+            with torch.cuda.stream(stream):
+                buf = torch.empty(int(lib.dbmp_atlas_extended_bytes(self.P, self.Ht, self.Wt, self.kind)),
+                                  dtype=torch.uint8, device=self.data.device)
+                call("dbmp_atlas_pack_extended", _ptr(self.data), self.P, self.Ht, self.Wt, self.kind, _ptr(buf),
+                     _stream())
+                q = Filled(buf)
+            self._quads = (q, version)
+        q.use(stream)
+        return q
 
     def pack(self, templates: torch.Tensor, st=None):
         """Fills the buffer from (P,Ht,Wt) f32 templates (extended atlases)."""
@@ -134,7 +189,7 @@ class Atlas:
         a.P, a.Ht, a.Wt, a.kind = self.P, self.Ht, self.Wt, self.kind
         a.extended = self.extended and (a.kind != ATLAS_F32 or pixels is None
                                         or pixels >= max(2 * self.templates.numel(), 1 << 18))
-        a._followed = None
+        a.own, a._quads = a.extended, None
         if a.extended:
             a._alloc()
         else:
@@ -174,6 +229,8 @@ class BatchState:
     cmap_stride: int = 0
     c_blend: float = 0.0
     walk_masks: Optional[torch.Tensor] = None    # what the forward's tests found (dbmp_render)
+    atlas: Optional[Atlas] = None                # the forward's atlas
+    quads: Optional[Filled] = None               # ... and its packed copy, if the forward walked one
 
     @property
     def batch(self) -> int:
@@ -189,6 +246,8 @@ class ForwardState:
     colors_orig: Optional[torch.Tensor] = None   # colour maps of a blended render
     c_blend: float = 0.0
     walk_masks: Optional[torch.Tensor] = None    # what the forward's tests found (dbmp_render)
+    atlas: Optional[Atlas] = None                # the forward's atlas
+    quads: Optional[Filled] = None               # ... and its packed copy, if the forward walked one
 
 
 def lists_from_mapping(mapping: torch.Tensor, num_tiles: int, num_prims: int) -> TileLists:
@@ -237,9 +296,17 @@ class Rasterizer:
         self._pins = []            # pinned flag buffers not in use
 
     def canvas(self, N: int, atlas: Atlas) -> Canvas:
-        atlas.refresh()
+        """The canvas of calls that pass atlas.data."""
         return Canvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
-                      self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.extended else 0)
+                      self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.own else 0)
+
+    def walk_canvas(self, N: int, atlas: Atlas, quads: Optional[Filled], changed: int):
+        """(canvas, atlas pointer) of a walk: on the packed copy `quads` of an "f32"
+        atlas with the flag at `changed` (an int32 of scratch), or on atlas.data."""
+        if quads is None:
+            return self.canvas(N, atlas), _ptr(atlas.data)
+        return FollowedCanvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
+                              self.alpha_max, self.t_stop, FOLLOWED_ATLAS, _ptr(atlas.data), changed), _ptr(quads.tensor)
 
     # -- binning -----------------------------------------------------------
     def _ensure(self, cv: Canvas, cap: int):
@@ -256,12 +323,12 @@ class Rasterizer:
 
     def _scratch(self, cv: Canvas, B: int, N: int, stream):
         """(tensor, workspace bytes): a binning's workspace, followed by two ints
-        per candidate for its flags."""
+        per candidate for its flags and one for the walk's."""
         if self._ws_need[0] != (B, N):
             need = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), B))
             self._ws_need = ((B, N), (need + 255) & ~255)
         nbytes = self._ws_need[1]
-        t = torch.empty(nbytes + 8 * B, dtype=torch.uint8, device=self.device)
+        t = torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device)
         if stream is not None:      # freed while that stream may still use it
             t.record_stream(stream)
         return t, nbytes
@@ -296,7 +363,7 @@ class Rasterizer:
         prim_info = torch.empty((max(N, 1), 16), dtype=torch.float32, device=self.device)
         offsets = torch.empty(self.T + 1, dtype=torch.int32, device=self.device)
         ws, nbytes = self._scratch(cv, 1, N, stream)
-        flags = ws[nbytes:].view(torch.int32)
+        flags = ws[nbytes:nbytes + 8].view(torch.int32)
         for _ in range(3):
             # each binning owns its index list: a ForwardState must stay valid
             # while later forwards on this canvas run (batch APIs keep several)
@@ -316,8 +383,8 @@ class Rasterizer:
         """Binning and forward of B candidates (lead: () for one, else (B,)) in one
         call; the host waits for the list lengths while the forward runs, and
         repeats the call if they exceed the capacity.  Returns (color, alpha,
-        T_last, last_pos, prim_info, offsets, indices, longest list, walk_masks);
-        masks: the render's backward will be wanted."""
+        T_last, last_pos, prim_info, offsets, indices, longest list, walk_masks,
+        the atlas's packed copy); masks: the render's backward will be wanted."""
         B = lead[0] if lead else 1
         N = int(radii.shape[-1])
         cv = self.canvas(N, atlas)
@@ -335,6 +402,8 @@ class Rasterizer:
             walk = torch.empty(self._mask_bytes * B, dtype=torch.uint8, device=dev)
         ws, nbytes = self._scratch(cv, B, N, stream)
         st = _stream(stream)
+        quads = atlas.quads(stream)
+        cv, texels = self.walk_canvas(N, atlas, quads, ws.data_ptr() + nbytes + 8 * B)
         pin = self._pins.pop() if self._pins else torch.empty(2 * B, dtype=torch.int32).pin_memory()
         if pin.numel() < 2 * B:
             pin = torch.empty(2 * B, dtype=torch.int32).pin_memory()
@@ -344,7 +413,7 @@ class Rasterizer:
             stride = max(cap, 1)
             indices = torch.empty((*lead, stride), dtype=torch.int32, device=dev)
             call("dbmp_render", ctypes.byref(cv), B, _ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities),
-                 _ptr(colors), _ptr(sel), sel_stride, _ptr(atlas.bbox), _ptr(atlas.data), _ptr(prim), _ptr(offsets),
+                 _ptr(colors), _ptr(sel), sel_stride, _ptr(atlas.bbox), texels, _ptr(prim), _ptr(offsets),
                  _ptr(indices), stride, cap, ws.data_ptr() + nbytes, _ptr(pin), _ptr(cmap), cmap_stride,
                  float(c_blend) if cmap is not None else 0.0, _ptr(color), _ptr(alpha), _ptr(T_last), _ptr(last_pos),
                  _ptr(walk), _ptr(ws), nbytes, st)
@@ -352,17 +421,33 @@ class Rasterizer:
             if not flags[1:2 * B:2].any():
                 L = int(flags[0:2 * B:2].max())
                 self._pins.append(pin)
-                return color, alpha, T_last, last_pos, prim, offsets, indices, L, walk
+                return color, alpha, T_last, last_pos, prim, offsets, indices, L, walk, quads
             self._grow_hint(int(flags[0:2 * B:2].max()))
         raise DbmpError("binning capacity did not converge")
 
-    def prepare(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None):
+    def _flag(self, stream) -> torch.Tensor:
+        """The flag of a walk that has no other scratch."""
+        with torch.cuda.stream(stream):
+            return torch.empty(1, dtype=torch.int32, device=self.device)
+
+    def prepare(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None,
+                cv: Optional[Canvas] = None):
+        """The records of given lists' walk, for a walk with canvas cv."""
         N = int(radii.shape[0])
-        cv = self.canvas(N, atlas)
+        cv = cv if cv is not None else self.canvas(N, atlas)
         prim_info = torch.empty((max(N, 1), 16), dtype=torch.float32, device=self.device)
         call("dbmp_prepare", ctypes.byref(cv), _ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities),
              _ptr(colors), _ptr(sel), _ptr(prim_info), _stream(stream))
         return prim_info
+
+    def _walk_of(self, state, N: int, atlas: Atlas, changed: int, stream):
+        """(canvas, atlas pointer, masks pointer) of the backward of a forward's
+        state: the forward's packed copy and masks where `atlas` is the forward's."""
+        quads = state.quads if state.atlas is atlas else None
+        if quads is not None:
+            quads.use(stream)
+        cv, texels = self.walk_canvas(N, atlas, quads, changed)
+        return cv, texels, _ptr(state.walk_masks) if state.atlas is atlas else None
 
     # -- forward / backward -------------------------------------------------
     def forward(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas,
@@ -376,25 +461,26 @@ class Rasterizer:
         N = int(radii.shape[0])
         cmap = self._colour_maps(colors_orig, c_blend, N, atlas)
         if mapping is None or mapping.numel() == 0:
-            color, alpha, T_last, last_pos, prim_info, offsets, indices, L, walk = self._render(
+            color, alpha, T_last, last_pos, prim_info, offsets, indices, L, walk, quads = self._render(
                 (), means2D, radii, rotations, opacities, colors, sel, 0, atlas, stream, cmap, 0, c_blend, for_backward)
             return color, alpha, ForwardState(prim_info, TileLists(offsets, indices, L), T_last, last_pos, cmap,
-                                              float(c_blend) if cmap is not None else 0.0, walk)
+                                              float(c_blend) if cmap is not None else 0.0, walk, atlas, quads)
         lists = lists_from_mapping(mapping, self.T, N)
-        prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
-        cv = self.canvas(N, atlas)
+        quads, flag = atlas.quads(stream), self._flag(stream)
+        cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
+        prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream, cv)
         color = torch.empty((self.H, self.W, 3), dtype=torch.float32, device=self.device)
         alpha = torch.empty((self.H, self.W), dtype=torch.float32, device=self.device)
         T_last = torch.empty((self.H, self.W), dtype=torch.float32, device=self.device)
         last_pos = torch.empty((self.H, self.W), dtype=torch.int32, device=self.device)
         if cmap is None:
-            call("dbmp_forward", ctypes.byref(cv), _ptr(prim_info), _ptr(atlas.data), _ptr(lists.offsets),
+            call("dbmp_forward", ctypes.byref(cv), _ptr(prim_info), texels, _ptr(lists.offsets),
                  _ptr(lists.indices), _ptr(color), _ptr(alpha), _ptr(T_last), _ptr(last_pos), _stream(stream))
-            return color, alpha, ForwardState(prim_info, lists, T_last, last_pos)
-        call("dbmp_forward_blend", ctypes.byref(cv), _ptr(prim_info), _ptr(atlas.data), _ptr(lists.offsets),
+            return color, alpha, ForwardState(prim_info, lists, T_last, last_pos, atlas=atlas, quads=quads)
+        call("dbmp_forward_blend", ctypes.byref(cv), _ptr(prim_info), texels, _ptr(lists.offsets),
              _ptr(lists.indices), _ptr(cmap), ctypes.c_float(c_blend), _ptr(color), _ptr(alpha), _ptr(T_last),
              _ptr(last_pos), _stream(stream))
-        return color, alpha, ForwardState(prim_info, lists, T_last, last_pos, cmap, float(c_blend))
+        return color, alpha, ForwardState(prim_info, lists, T_last, last_pos, cmap, float(c_blend), None, atlas, quads)
 
     # -- batches of candidates -------------------------------------------------
     def bin_batch(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None):
@@ -452,10 +538,12 @@ class Rasterizer:
         has_maps = mappings is not None and len(mappings) > 0
         if not has_maps and 0 < B <= 65535:
             params = self._flat_batch((means2D, radii, rotations, opacities, colors, sel), stream)
-            color, alpha, T_last, last_pos, prim, offsets, indices, _, walk = self._render(
+            color, alpha, T_last, last_pos, prim, offsets, indices, _, walk, quads = self._render(
                 (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend, for_backward)
             return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
-                                            float(c_blend) if cmap is not None else 0.0, walk)
+                                            float(c_blend) if cmap is not None else 0.0, walk, atlas, quads)
+        quads, flag = atlas.quads(stream), self._flag(stream)
+        cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
         if has_maps:
             if len(mappings) != B:
                 raise ValueError(f"{len(mappings)} mappings for {B} candidates")
@@ -466,7 +554,6 @@ class Rasterizer:
             for b, l in enumerate(lists):
                 indices[b, :l.length] = l.indices[:l.length]
             prim = torch.empty((max(B * N, 1), 16), dtype=torch.float32, device=self.device)
-            cv = self.canvas(N, atlas)
             sel2 = sel if sel.dim() == 2 else sel.unsqueeze(0).expand(B, -1)
             for b in range(B):
                 call("dbmp_prepare", ctypes.byref(cv), _ptr(means2D[b]), _ptr(radii[b]), _ptr(rotations[b]),
@@ -474,33 +561,32 @@ class Rasterizer:
                      ctypes.c_void_p(prim.data_ptr() + b * N * 64), st)
         else:
             prim, offsets, indices = self.bin_batch(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
-        cv = self.canvas(N, atlas)
         dev = self.device
         color = torch.empty((B, self.H, self.W, 3), dtype=torch.float32, device=dev)
         alpha = torch.empty((B, self.H, self.W), dtype=torch.float32, device=dev)
         T_last = torch.empty((B, self.H, self.W), dtype=torch.float32, device=dev)
         last_pos = torch.empty((B, self.H, self.W), dtype=torch.int32, device=dev)
-        call("dbmp_forward_batch", ctypes.byref(cv), B, _ptr(prim), _ptr(atlas.data), _ptr(offsets), _ptr(indices),
+        call("dbmp_forward_batch", ctypes.byref(cv), B, _ptr(prim), texels, _ptr(offsets), _ptr(indices),
              ctypes.c_longlong(indices.shape[1]), _ptr(cmap), ctypes.c_longlong(cstride),
              ctypes.c_float(c_blend if cmap is not None else 0.0), _ptr(color), _ptr(alpha), _ptr(T_last),
              _ptr(last_pos), st)
         return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
-                                        float(c_blend) if cmap is not None else 0.0)
+                                        float(c_blend) if cmap is not None else 0.0, None, atlas, quads)
 
     def backward_batch(self, state: BatchState, grad_color, grad_alpha, radii, rotations, opacities, colors,
                        atlas: Atlas, stream=None):
         """The five gradients of each candidate, in one launch: (B,N,2),
         (B,N), (B,N), (B,N), (B,N,3)."""
         B, N = int(radii.shape[0]), int(radii.shape[1])
-        cv = self.canvas(N, atlas)
         dev = self.device
         gc = _operand(grad_color)
         ga = _operand(grad_alpha) if grad_alpha is not None else None
-        acc = torch.empty((max(B * N, 1), 8), dtype=torch.float64, device=dev)
+        acc = torch.empty((B * N + 1, 8), dtype=torch.float64, device=dev)    # the last row: the walk's flag
+        cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * B * N, stream)
         outs = [torch.empty(sh, dtype=torch.float32, device=dev)
                 for sh in ((B, N, 2), (B, N), (B, N), (B, N), (B, N, 3))]
-        call("dbmp_backward_masked", ctypes.byref(cv), B, _ptr(state.walk_masks), _ptr(state.prim_info),
-             _ptr(atlas.data), _ptr(state.offsets), _ptr(state.indices), state.indices.shape[1],
+        call("dbmp_backward_masked", ctypes.byref(cv), B, masks, _ptr(state.prim_info),
+             texels, _ptr(state.offsets), _ptr(state.indices), state.indices.shape[1],
              _ptr(state.colors_orig), state.cmap_stride, float(state.c_blend),
              _ptr(state.T_last), _ptr(state.last_pos), _ptr(gc), _ptr(ga), _ptr(radii), _ptr(rotations),
              _ptr(opacities), _ptr(colors), _ptr(acc), *[_ptr(o) for o in outs], _stream(stream))
@@ -525,18 +611,18 @@ class Rasterizer:
         """Returns the reference's five gradients: (means2D (N,2), radii (N),
         rotations (N), opacities (N), colors (N,3)), float32."""
         N = int(radii.shape[0])
-        cv = self.canvas(N, atlas)
         dev = self.device
         gc = _operand(grad_color)
         ga = _operand(grad_alpha) if grad_alpha is not None else None
-        acc = torch.empty((max(N, 1), 8), dtype=torch.float64, device=dev)
+        acc = torch.empty((N + 1, 8), dtype=torch.float64, device=dev)        # the last row: the walk's flag
+        cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * N, stream)
         g_means = torch.empty((N, 2), dtype=torch.float32, device=dev)
         g_r = torch.empty(N, dtype=torch.float32, device=dev)
         g_rot = torch.empty(N, dtype=torch.float32, device=dev)
         g_op = torch.empty(N, dtype=torch.float32, device=dev)
         g_col = torch.empty((N, 3), dtype=torch.float32, device=dev)
-        call("dbmp_backward_masked", ctypes.byref(cv), 1, _ptr(state.walk_masks), _ptr(state.prim_info),
-             _ptr(atlas.data), _ptr(state.lists.offsets), _ptr(state.lists.indices), state.lists.indices.numel(),
+        call("dbmp_backward_masked", ctypes.byref(cv), 1, masks, _ptr(state.prim_info),
+             texels, _ptr(state.lists.offsets), _ptr(state.lists.indices), state.lists.indices.numel(),
              _ptr(state.colors_orig), 0, float(state.c_blend) if state.colors_orig is not None else 0.0,
              _ptr(state.T_last), _ptr(state.last_pos), _ptr(gc), _ptr(ga), _ptr(radii), _ptr(rotations),
              _ptr(opacities), _ptr(colors), _ptr(acc), _ptr(g_means), _ptr(g_r), _ptr(g_rot), _ptr(g_op), _ptr(g_col),

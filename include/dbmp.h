@@ -78,6 +78,21 @@ typedef struct {
  * extended atlases (dbmp_atlas_pack_extended).  Any other value means plain ones. */
 #define DBMP_CANVAS_EXTENDED_ATLAS 0x41545845
 
+/* dbmp_canvas.reserved: the canvas is the first member of a dbmp_followed_canvas
+ * (DBMP_ATLAS_F32 only).  The atlas pointers passed with it are extended atlases packed
+ * from `templates` at some earlier time; every walk first compares the templates, as
+ * they are when the walk's turn on its stream comes, with the packed ones bit by bit,
+ * and where any texel differs it reads the templates in the reference layout instead.
+ * A job can so walk a packed copy of templates that others may write to.  `changed`:
+ * one int32 of device scratch that no other call in flight uses (left nonzero when
+ * the templates differed). */
+#define DBMP_CANVAS_FOLLOWED_ATLAS 0x46545845
+typedef struct {
+  dbmp_canvas canvas;
+  const float* templates;     /* (P,Ht,Wt) f32 */
+  int32_t* changed;
+} dbmp_followed_canvas;
+
 const char* dbmp_last_error(void);
 int dbmp_version(void);
 /* Number of tiles of a canvas: ceil(H/ts)*ceil(W/ts). */
