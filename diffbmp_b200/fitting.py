@@ -25,7 +25,7 @@ import torch
 
 from . import _lib
 from ._lib import AdamCfg, call, lib
-from .rasterizer import Atlas, Rasterizer, _ptr, _stream, DEFAULT_T_STOP
+from .rasterizer import Atlas, Rasterizer, _ptr, _stream, DEFAULT_T_STOP, FIT_QUADS_PRIMS
 
 # Reference defaults (pydiffbmp/util/constants.py:24-38): base lr and gains,
 # ExponentialLR factor, fixed blur sigma.
@@ -211,7 +211,8 @@ class ImageFitter:
         # the walks' canvas and atlas pointer: an "f32" job's steps keep the packed
         # copy that they started with
         self._changed = torch.zeros(1, dtype=torch.int32, device=dev)
-        self._quads = atlas.quads() if cfg.blur == "none" else None
+        follow = cfg.blur == "none" and self.N >= FIT_QUADS_PRIMS
+        self._quads = atlas.quads() if follow else None
         self._walk_cv, self._walk_atlas = self.rz.walk_canvas(self.N, atlas, self._quads, _ptr(self._changed))
         N8 = (max(self.N, 1), 8)
         self.adam_m = torch.zeros(N8, dtype=torch.float32, device=dev)
@@ -245,7 +246,7 @@ class ImageFitter:
                 raise ValueError(f"blur must be one of {sorted(BLUR_MODES)}, not {cfg.blur!r}")
             if cfg.blur == "adaptive" and cfg.num_iterations < 1:
                 raise ValueError("the adaptive blur schedule needs FitConfig.num_iterations")
-            self.atlas = atlas.private_copy(self.H * self.W)
+            self.atlas = atlas.private_copy(self.H * self.W, self.N)
             self.cv = self.rz.canvas(self.N, self.atlas)
             self._walk_cv, self._walk_atlas = self.rz.walk_canvas(self.N, self.atlas, None, 0)
             self.blur = _lib.BlurSchedule(BLUR_MODES[cfg.blur], cfg.blur_sigma, cfg.blur_sigma_start,

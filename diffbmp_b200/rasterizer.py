@@ -40,6 +40,13 @@ KIND_NAMES = {"f32": ATLAS_F32, "f32q": ATLAS_F32_QUAD, "f16q": ATLAS_F16_QUAD, 
 # to pack them (1.6 ms per GiB).
 MAX_F32_QUAD_BYTES = 1 << 30
 
+# Fits (many steps on one packed copy) walk quads from this many primitives on: below,
+# a step's comparison takes what the walks gain.  Gain of a fused step, comparison
+# included, over eight canvases of 64x64 to 1500x1500 and four atlases of 64x64 to
+# 16 of 256x256: -5 to 1 us with N=60 (but 8 at 1500x1500), -3 to 15 up to
+# 1024x1024 with 100, 0.7 to 51 with 200, 4 to 155 with 600.
+FIT_QUADS_PRIMS = 200
+
 DEFAULT_T_STOP = 1e-6   # image error <= t_stop * max colour, well inside the 1e-5 parity bar
 
 
@@ -66,6 +73,24 @@ def _f32(t: torch.Tensor) -> torch.Tensor:
 def _operand(t: torch.Tensor) -> torch.Tensor:
     """t as a kernel operand: itself where it is contiguous f32 already."""
     return t if t.dtype is torch.float32 and t.is_contiguous() else _f32(t)
+
+
+def quads_pay(pixels: int, N: int, texels: int) -> bool:
+    """Whether the walks of one forward and backward, or of one fit step, of N
+    primitives on `pixels` pixels gain more on a packed copy of an "f32" atlas than
+    packing it takes, as a job whose templates change on every call pays for it.
+
+    Packing takes 10 us for 64x64 texels, 23 for 8 of 128x128, 61 for 16 of 256x256 and
+    98 for 16 of 512x512; the walks gain with the pixels and, up to about 500
+    primitives, where a pixel is opaque, with their depth.  Forward and backward's
+    gain in us, the comparison included, on both sides of the line:
+      8 of 128x128 (23):  N=600   384x384 20, 500x512 41, 1024x1024 123;
+                          N=300   600x600 22, 768x768 36;  N=100  1024x1024 8
+      16 of 256x256 (61): N=600   500x512 61, 600x600 77, 768x768 105;
+                          N=300   768x768 56, 1024x1024 93;  N=100  1024x1024 14
+      one 64x64 (10):     N=600   384x384 1, 500x512 9, 768x768 18;
+                          N=6000  256x256 -3, 500x512 10"""
+    return pixels * min(N, 500) >= 500 * (180_000 + texels // 3)
 
 
 class Filled:
@@ -176,19 +201,17 @@ class Atlas:
         call("dbmp_atlas_pack_extended", _ptr(templates), self.P, self.Ht, self.Wt, self.kind, _ptr(self.data),
              st if st is not None else _stream())
 
-    def private_copy(self, pixels: Optional[int] = None) -> "Atlas":
+    def private_copy(self, pixels: Optional[int] = None, N: int = 1 << 30) -> "Atlas":
         """An atlas of the same kind, templates and content bboxes with its own
-        texel buffer (filled by the caller), for a job on a canvas of `pixels`
-        that re-derives its texels every step (the fit loop's blur schedule).
-        Such a job repacks an extended atlas every step, which an "f32" one
-        only does where the walks gain more than that takes: 23 us for 8
-        templates of 128x128 against 33 us of a 512x512 step (N=600), but 50 us
-        for 16 of 256x256 against 10 us of a 300x300 step (N=300)."""
+        texel buffer (filled by the caller), for a job of N primitives on a canvas of
+        `pixels` that re-derives its texels every step (the fit loop's blur
+        schedule).  Such a job repacks an extended atlas every step, which an "f32"
+        one only does where that pays."""
         a = Atlas.__new__(Atlas)
         a.templates, a.sigma, a.bbox = self.templates, self.sigma, self.bbox
         a.P, a.Ht, a.Wt, a.kind = self.P, self.Ht, self.Wt, self.kind
         a.extended = self.extended and (a.kind != ATLAS_F32 or pixels is None
-                                        or pixels >= max(2 * self.templates.numel(), 1 << 18))
+                                        or quads_pay(pixels, N, self.templates.numel()))
         a.own, a._quads = a.extended, None
         if a.extended:
             a._alloc()
@@ -300,6 +323,11 @@ class Rasterizer:
         return Canvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
                       self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.own else 0)
 
+    def _quads(self, atlas: Atlas, N: int, B: int, stream) -> Optional[Filled]:
+        if atlas.own or not quads_pay(B * self.H * self.W, N, atlas.P * atlas.Ht * atlas.Wt):
+            return None
+        return atlas.quads(stream)
+
     def walk_canvas(self, N: int, atlas: Atlas, quads: Optional[Filled], changed: int):
         """(canvas, atlas pointer) of a walk: on the packed copy `quads` of an "f32"
         atlas with the flag at `changed` (an int32 of scratch), or on atlas.data."""
@@ -387,7 +415,8 @@ class Rasterizer:
         the atlas's packed copy); masks: the render's backward will be wanted."""
         B = lead[0] if lead else 1
         N = int(radii.shape[-1])
-        cv = self.canvas(N, atlas)
+        quads = self._quads(atlas, N, B, stream)
+        cv, texels = self.walk_canvas(N, atlas, quads, 1)    # (the flag is set below)
         dev, H, W = self.device, self.H, self.W
         color = torch.empty((*lead, H, W, 3), dtype=torch.float32, device=dev)
         alpha = torch.empty((*lead, H, W), dtype=torch.float32, device=dev)
@@ -402,8 +431,8 @@ class Rasterizer:
             walk = torch.empty(self._mask_bytes * B, dtype=torch.uint8, device=dev)
         ws, nbytes = self._scratch(cv, B, N, stream)
         st = _stream(stream)
-        quads = atlas.quads(stream)
-        cv, texels = self.walk_canvas(N, atlas, quads, ws.data_ptr() + nbytes + 8 * B)
+        if quads is not None:
+            cv.changed = ws.data_ptr() + nbytes + 8 * B
         pin = self._pins.pop() if self._pins else torch.empty(2 * B, dtype=torch.int32).pin_memory()
         if pin.numel() < 2 * B:
             pin = torch.empty(2 * B, dtype=torch.int32).pin_memory()
@@ -443,11 +472,11 @@ class Rasterizer:
     def _walk_of(self, state, N: int, atlas: Atlas, changed: int, stream):
         """(canvas, atlas pointer, masks pointer) of the backward of a forward's
         state: the forward's packed copy and masks where `atlas` is the forward's."""
-        quads = state.quads if state.atlas is atlas else None
-        if quads is not None:
-            quads.use(stream)
-        cv, texels = self.walk_canvas(N, atlas, quads, changed)
-        return cv, texels, _ptr(state.walk_masks) if state.atlas is atlas else None
+        if state.atlas is not atlas:
+            return *self.walk_canvas(N, atlas, None, 0), None
+        if state.quads is not None:
+            state.quads.use(stream)
+        return *self.walk_canvas(N, atlas, state.quads, changed), _ptr(state.walk_masks)
 
     # -- forward / backward -------------------------------------------------
     def forward(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas,
@@ -466,7 +495,7 @@ class Rasterizer:
             return color, alpha, ForwardState(prim_info, TileLists(offsets, indices, L), T_last, last_pos, cmap,
                                               float(c_blend) if cmap is not None else 0.0, walk, atlas, quads)
         lists = lists_from_mapping(mapping, self.T, N)
-        quads, flag = atlas.quads(stream), self._flag(stream)
+        quads, flag = self._quads(atlas, N, 1, stream), self._flag(stream)
         cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
         prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream, cv)
         color = torch.empty((self.H, self.W, 3), dtype=torch.float32, device=self.device)
@@ -542,7 +571,7 @@ class Rasterizer:
                 (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend, for_backward)
             return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
                                             float(c_blend) if cmap is not None else 0.0, walk, atlas, quads)
-        quads, flag = atlas.quads(stream), self._flag(stream)
+        quads, flag = self._quads(atlas, N, B, stream), self._flag(stream)
         cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
         if has_maps:
             if len(mappings) != B:

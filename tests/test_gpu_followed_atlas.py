@@ -9,12 +9,19 @@ import pytest
 import torch
 
 from diffbmp_b200 import cuda_tile_rasterizer as ctr
+from diffbmp_b200 import fitting as F
 from diffbmp_b200 import rasterizer as R
 from diffbmp_b200.fitting import FitConfig, ImageFitter
 
 pytestmark = pytest.mark.gpu
 
 H, W, N = 75, 130, 90
+
+
+@pytest.fixture(autouse=True)
+def packed_at_any_size(monkeypatch):
+    monkeypatch.setattr(R, "quads_pay", lambda pixels, N, texels: True)
+    monkeypatch.setattr(F, "FIT_QUADS_PRIMS", 0)
 
 
 def cu(a, dtype=np.float32):
