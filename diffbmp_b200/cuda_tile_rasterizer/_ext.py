@@ -29,6 +29,7 @@ class _Global:
         self.rz_map = R.Rasterizer(H, W, ts, alpha_ub, bin_mode=R.BIN_CONTENT)
         self.atlas_key = None
         self.atlas = None
+        self.atlas_templates = None    # the keyed tensor: alive, so that no other one gets its address
         self.states = []
         self.batch_state = None     # (BatchState, rasterizer, atlas) of the last forward_batch
         self.t_fwd = self.t_bwd = 0.0
@@ -36,10 +37,10 @@ class _Global:
 
     def get_atlas(self, templates: torch.Tensor) -> R.Atlas:
         t = templates if templates.dim() == 3 else templates.unsqueeze(0)
-        key = (t.data_ptr(), tuple(t.shape), t._version, t.dtype)
+        key = (t.data_ptr(), tuple(t.shape), t.stride(), t._version, t.dtype)
         if key != self.atlas_key:
             self.atlas = R.Atlas(t.float(), self.kind)
-            self.atlas_key = key
+            self.atlas_key, self.atlas_templates = key, t.detach()
         return self.atlas
 
 
