@@ -780,7 +780,7 @@ size_t atlas_bytes(int P, int Ht, int Wt, int kind) {
 }
 
 // Clearance grid and, with SOLID, the solid grid of the same cells (layouts in
-// dbmp_internal.cuh), one CTA per (strip of cell rows, template).
+// dbmp_internal.cuh), one CTA per (template, strip of cell rows).
 // Bounding texels are the support texels, respectively the texels other than
 // exactly 1 (NaN counts as either).  First a warp takes each template row that
 // can matter to the strip (up to kGridCap-1 rows beyond it): ballots turn the
@@ -828,9 +828,10 @@ __global__ void __launch_bounds__(kGridThreads) atlas_grid_kernel(const float* _
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   unsigned* mask = s_mem + (size_t)warp * K * a.words;                             // this warp's row masks
   unsigned char* dist = reinterpret_cast<unsigned char*>(s_mem + (size_t)nwarps * K * a.words);   // K x rows x Gx
-  const int p = blockIdx.y;
+  const int strips = (a.Gy + a.strip - 1) / a.strip;
+  const int p = blockIdx.x / strips;
   const float* t = tmpl + (size_t)p * a.Ht * a.Wt;
-  const int c0 = blockIdx.x * a.strip, c1 = min(c0 + a.strip, a.Gy);
+  const int c0 = (blockIdx.x - p * strips) * a.strip, c1 = min(c0 + a.strip, a.Gy);
   const int y0 = max(0, (c0 << a.gsy) - (kGridCap - 1)), y1 = min(a.Ht - 1, (c1 << a.gsy) + (kGridCap - 1));
   for (int i = lane; i < K * a.words; i += 32) mask[i] = 0u;
   __syncwarp();
@@ -911,14 +912,16 @@ static int launch_grids(const float* tmpl, int P, int Ht, int Wt, int kind, void
     if (e == cudaSuccess && a.solid) e = cudaMemsetAsync(a.solid, 0, atlas_grid_bytes(P, Ht, Wt), st);
     return e == cudaSuccess ? DBMP_OK : cuda_status(e, "cudaMemsetAsync(grid)");
   }
-  const dim3 ctas((a.Gy + a.strip - 1) / a.strip, P);
+  // in one dimension: the others end at 65535
+  const long long ctas = (long long)((a.Gy + a.strip - 1) / a.strip) * P;
+  if (ctas > 0x7fffffffll) { set_error("dbmp_atlas_pack: %d templates of %dx%d exceed one grid", P, Ht, Wt); return DBMP_ERR_INVALID; }
   if (smem > 48 * 1024) {
     const cudaError_t e = a.solid ? cudaFuncSetAttribute(atlas_grid_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem)
                                   : cudaFuncSetAttribute(atlas_grid_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(atlas_grid_kernel)");
   }
-  if (a.solid) atlas_grid_kernel<true><<<ctas, warps * 32, smem, st>>>(tmpl, a);
-  else atlas_grid_kernel<false><<<ctas, warps * 32, smem, st>>>(tmpl, a);
+  if (a.solid) atlas_grid_kernel<true><<<(unsigned)ctas, warps * 32, smem, st>>>(tmpl, a);
+  else atlas_grid_kernel<false><<<(unsigned)ctas, warps * 32, smem, st>>>(tmpl, a);
   DBMP_CHECK_LAUNCH("atlas_grid_kernel");
   return DBMP_OK;
 }
