@@ -310,6 +310,9 @@ template <int TS, int KIND, bool CB = false>
 struct TileWalker {
   static constexpr int NP = 2;      // pixels of a thread
   using L = Layout<TS>;
+  // sets of per-primitive sums of a lane: one over both pixels (32-pixel tiles, FP32
+  // sums over a footprint's 64 pixels), or one for each (16-pixel tiles, over 32)
+  static constexpr int kSumPx = TS == 16 ? 2 : 1;
   static constexpr bool kGrid = KIND != ATLAS_F32;   // packed atlases carry a clearance grid
   static constexpr bool kQuad = KIND == ATLAS_F32_QUAD || KIND == ATLAS_F16_QUAD || KIND == ATLAS_BF16_QUAD;
 
@@ -494,60 +497,61 @@ struct TileWalker {
     return c;
   }
 
-  // Adds the warp's 8 per-primitive sums (acc, one set per lane) to dst[0..7]:
-  // a recursive-halving reduction, 8 sums over 32 lanes in 9 shuffles, after
-  // which lane l < 8 holds sum kidx and adds it in FP64.
-  __device__ __forceinline__ void warp_add(float (&acc)[8], int kidx, double* __restrict__ dst) const {
-    const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+  // Sums of acc[0..K-1] (one set per lane) over the warp by recursive halving: 8 sums
+  // over 32 lanes in 9 shuffles, 16 in 16.  Lane l returns the sum whose index has
+  // the bits of l reversed (in log2 K bits); the lanes beyond K repeat the first K.
+  template <int K>
+  __device__ __forceinline__ float warp_sums(float (&acc)[K]) const {
+    int bit = 1;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float send = b0 ? acc[k] : acc[k + 4];
-      const float keep = b0 ? acc[k + 4] : acc[k];
-      acc[k] = keep + __shfl_xor_sync(kFull, send, 1);
+    for (int n = K / 2; n >= 1; n >>= 1, bit <<= 1) {
+      const bool b = lane & bit;
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        const float send = b ? acc[k] : acc[k + n];
+        const float keep = b ? acc[k + n] : acc[k];
+        acc[k] = keep + __shfl_xor_sync(kFull, send, bit);
+      }
     }
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float send = b1 ? acc[k] : acc[k + 2];
-      const float keep = b1 ? acc[k + 2] : acc[k];
-      acc[k] = keep + __shfl_xor_sync(kFull, send, 2);
+    for (; bit < 32; bit <<= 1) acc[0] += __shfl_xor_sync(kFull, acc[0], bit);
+    return acc[0];
+  }
+
+  // Adds the warp's K per-primitive sums to dst[0..K-1] in FP64.  PX = 1: each lane
+  // gives the sums of its two pixels.  PX = 2: it gives pixel 0's and then pixel
+  // 1's, and the two halves of the footprint (8x4 pixels each) meet in FP64.
+  // Returns the index of the sum that this lane added (-1: none) and its value.
+  template <int K, int PX>
+  __device__ __forceinline__ int add_sums(float (&acc)[PX * K], double* __restrict__ dst, double* value) const {
+    const float sum = warp_sums(acc);
+    double d = (double)sum;
+    int l = lane;
+    if (PX == 2) {
+      d += __shfl_xor_sync(kFull, d, 1);
+      l = (lane & 1) ? 32 : lane >> 1;   // lane bit 0 told the pixels apart
     }
-    {
-      const float send = b2 ? acc[0] : acc[1];
-      const float keep = b2 ? acc[1] : acc[0];
-      acc[0] = keep + __shfl_xor_sync(kFull, send, 4);
-    }
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 8);
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 16);
-    if (lane < 8 && acc[0] != 0.f) atomicAdd(dst + kidx, (double)acc[0]);
+    *value = d;
+    if (l >= K || d == 0.0) return -1;
+    const int k = K == 8 ? 4 * (l & 1) + (l & 2) + ((l >> 2) & 1) : 2 * (l & 1) + ((l >> 1) & 1);
+    atomicAdd(dst + k, d);
+    return k;
+  }
+
+  __device__ __forceinline__ void warp_add(float (&acc)[8 * kSumPx], double* __restrict__ dst) const {
+    double d;
+    add_sums<8, kSumPx>(acc, dst, &d);
   }
 
   // warp_add for a solid entry: acc holds sums 4..7 (the mask-gradient sums
-  // 0..3 are 0), reduced in the same order with 6 shuffles.  A sum that is
-  // not finite (an infinite or NaN gradient or colour) makes 0..3 NaN, as
-  // the product of such a term with the zero mask gradient does.
-  __device__ __forceinline__ void warp_add4(float (&acc)[4], double* __restrict__ dst) const {
-    const bool b0 = lane & 1, b1 = lane & 2;
+  // 0..3 are 0), reduced in the same order.  A sum that is not finite (an infinite
+  // or NaN gradient or colour) makes 0..3 NaN, as the product of such a term with
+  // the zero mask gradient does.
+  __device__ __forceinline__ void warp_add4(float (&acc)[4 * kSumPx], double* __restrict__ dst) const {
+    double d;
+    if (add_sums<4, kSumPx>(acc, dst + 4, &d) == 3 && !(fabs(d) < INFINITY)) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float send = b0 ? acc[k] : acc[k + 2];
-      const float keep = b0 ? acc[k + 2] : acc[k];
-      acc[k] = keep + __shfl_xor_sync(kFull, send, 1);
-    }
-    {
-      const float send = b1 ? acc[0] : acc[1];
-      const float keep = b1 ? acc[1] : acc[0];
-      acc[0] = keep + __shfl_xor_sync(kFull, send, 2);
-    }
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 4);
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 8);
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 16);
-    if (lane < 4 && acc[0] != 0.f) {
-      const int k = 2 * (lane & 1) + ((lane >> 1) & 1);
-      atomicAdd(dst + 4 + k, (double)acc[0]);
-      if (k == 3 && !(fabsf(acc[0]) < INFINITY)) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) atomicAdd(dst + j, (double)NAN);
-      }
+      for (int j = 0; j < 4; ++j) atomicAdd(dst + j, (double)NAN);
     }
   }
 
@@ -672,6 +676,20 @@ struct TileWalker {
     lp[0] = f.lp0; lp[1] = f.lp1;
   }
 
+  // Colour and opacity terms of a lane's pixels: their sum, or one set after the other.
+  __device__ __forceinline__ void colour_sums(float (&acc)[4 * kSumPx], float2 gcr, float2 gcg, float2 gcb, float2 wt,
+                                              float2 dlda, float2 a) const {
+    if constexpr (kSumPx == 2) {
+      acc[0] = gcr.x * wt.x; acc[1] = gcg.x * wt.x; acc[2] = gcb.x * wt.x; acc[3] = dlda.x * a.x;
+      acc[4] = gcr.y * wt.y; acc[5] = gcg.y * wt.y; acc[6] = gcb.y * wt.y; acc[7] = dlda.y * a.y;
+    } else {
+      acc[0] = fmaf(gcr.y, wt.y, gcr.x * wt.x);
+      acc[1] = fmaf(gcg.y, wt.y, gcg.x * wt.x);
+      acc[2] = fmaf(gcb.y, wt.y, gcb.x * wt.x);
+      acc[3] = fmaf(dlda.y, a.y, dlda.x * a.x);
+    }
+  }
+
   // Texel coordinates of the pixel pair alone (solid entries of a colour-map walk).
   __device__ __forceinline__ void pair_coords(const Geom& g, const Rec& r, float2& tx, float2& ty) const {
     const bool live[2] = {true, true};
@@ -696,8 +714,6 @@ struct TileWalker {
     const int warp_max = __reduce_max_sync(kFull, max(lp[0], lp[1]));
     if (warp_max < 0) return;
     const unsigned char* grid = static_cast<const unsigned char*>(atlas) + g.grid_off;
-    // sum index that lane l < 8 holds after the recursive-halving reduction
-    const int kidx = 4 * (lane & 1) + 2 * ((lane >> 1) & 1) + ((lane >> 2) & 1);
     const float2 gcr = make_float2(gC[0][0], gC[1][0]), gcg = make_float2(gC[0][1], gC[1][1]),
                  gcb = make_float2(gC[0][2], gC[1][2]), ga = make_float2(gA[0], gA[1]);
     float2 h = make_float2(0.f, 0.f), bt = make_float2(1.f, 1.f), ts = make_float2(Ts[0], Ts[1]);
@@ -732,11 +748,8 @@ struct TileWalker {
           if (kQuad) dlda = make_float2(tk.x * fmaf(ga.x, bt.x, gcc.x - h.x), tk.y * fmaf(ga.y, bt.y, gcc.y - h.y));
           else dlda = mul2(tk, fma2(ga, bt, sub2(g, gcc, h)));
           const float2 wt = mul2(a, tk);
-          float acc[4];
-          acc[0] = fmaf(gcr.y, wt.y, gcr.x * wt.x);
-          acc[1] = fmaf(gcg.y, wt.y, gcg.x * wt.x);
-          acc[2] = fmaf(gcb.y, wt.y, gcb.x * wt.x);
-          acc[3] = fmaf(dlda.y, a.y, dlda.x * a.x);
+          float acc[4 * kSumPx];
+          colour_sums(acc, gcr, gcg, gcb, wt, dlda, a);
           h = make_float2(fmaf(om.x, h.x, a.x * gcc.x), fmaf(om.y, h.y, a.y * gcc.y));
           bt = make_float2(bt.x * om.x, bt.y * om.y);
           warp_add4(acc, gacc + (size_t)id * 8);
@@ -781,24 +794,31 @@ struct TileWalker {
         }
         const float2 ex = add2(tx, g.nhx), ey = add2(ty, g.nhy);
         const float2 wt = mul2(a, tk);
-        float acc[8];
-        acc[0] = u.x + u.y;
-        acc[1] = v.x + v.y;
-        {
-          const float2 e = fma2(u, ex, mul2(v, ey));
-          acc[2] = e.x + e.y;
+        float acc[8 * kSumPx];
+        const float2 e2 = fma2(u, ex, mul2(v, ey)), e3 = fma2(mul2(u, g.rxy2), ey, mul2(mul2(v, g.nryx2), ex));
+        if constexpr (kSumPx == 2) {
+          acc[0] = u.x; acc[1] = v.x; acc[2] = e2.x; acc[3] = e3.x;
+          acc[8] = u.y; acc[9] = v.y; acc[10] = e2.y; acc[11] = e3.y;
+          float c[8];
+          colour_sums(c, gcr, gcg, gcb, wt, dlda, a);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            acc[4 + k] = c[k];
+            acc[12 + k] = c[4 + k];
+          }
+        } else {
+          acc[0] = u.x + u.y;
+          acc[1] = v.x + v.y;
+          acc[2] = e2.x + e2.y;
+          acc[3] = e3.x + e3.y;
+          float c[4];
+          colour_sums(c, gcr, gcg, gcb, wt, dlda, a);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[4 + k] = c[k];
         }
-        {
-          const float2 e = fma2(mul2(u, g.rxy2), ey, mul2(mul2(v, g.nryx2), ex));
-          acc[3] = e.x + e.y;
-        }
-        acc[4] = fmaf(gcr.y, wt.y, gcr.x * wt.x);
-        acc[5] = fmaf(gcg.y, wt.y, gcg.x * wt.x);
-        acc[6] = fmaf(gcb.y, wt.y, gcb.x * wt.x);
-        acc[7] = fmaf(dlda.y, a.y, dlda.x * a.x);
         h = make_float2(fmaf(om.x, h.x, a.x * gcc.x), fmaf(om.y, h.y, a.y * gcc.y));
         bt = make_float2(bt.x * om.x, bt.y * om.y);
-        if (__any_sync(kFull, f0 || f1)) warp_add(acc, kidx, gacc + (size_t)id * 8);
+        if (__any_sync(kFull, f0 || f1)) warp_add(acc, gacc + (size_t)id * 8);
       }
     }
   }
