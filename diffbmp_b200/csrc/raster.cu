@@ -258,9 +258,9 @@ __device__ __forceinline__ float3 sample_cmap(const float* __restrict__ cm, int 
   float r[3];
 #pragma unroll
   for (int ch = 0; ch < 3; ++ch) {
-    const float c0 = __ldg(p00 + ch) * (1.f - fx) + __ldg(p10 + ch) * fx;
-    const float c1 = __ldg(p01 + ch) * (1.f - fx) + __ldg(p11 + ch) * fx;
-    r[ch] = c0 * (1.f - fy) + c1 * fy;
+    const float c0 = fmaf(__ldg(p00 + ch), 1.f - fx, __ldg(p10 + ch) * fx);
+    const float c1 = fmaf(__ldg(p01 + ch), 1.f - fx, __ldg(p11 + ch) * fx);
+    r[ch] = fmaf(c0, 1.f - fy, c1 * fy);
   }
   return make_float3(r[0], r[1], r[2]);
 }
@@ -324,7 +324,9 @@ struct TileWalker {
   float fcx, fcy;   // centre of the warp footprint
 
   // Colours of the pixel pair for an entry (g2.yzw = sigmoid(c)); with CB, the
-  // map is sampled at the texel coordinates of the pixels with a fragment.
+  // map is sampled at the texel coordinates of the pixels with a fragment.  The
+  // roundings of the map's arithmetic are written out (here, in sample_cmap and in
+  // the backward's sums): left to the compiler they moved with the code around it.
   __device__ __forceinline__ void pair_colour(const Geom& g, const float4& g2, int id, float2 tx, float2 ty, bool f0,
                                               bool f1, float2& r, float2& gr, float2& b) const {
     r = make_float2(g2.y, g2.y);
@@ -333,17 +335,20 @@ struct TileWalker {
     if constexpr (CB) {
       const float* cm = cmap + (size_t)id * g.Ht * g.Wt * 3;
       const float k = 1.f - cblend;
+      auto mix = [&](float c, float co) {   // (16- and 32-pixel tiles differ in which product is rounded)
+        return L::kDirect ? fmaf(k, c, cblend * co) : fmaf(cblend, co, k * c);
+      };
       if (f0) {
         const float3 co = sample_cmap(cm, g.Ht, g.Wt, tx.x, ty.x);
-        r.x = k * g2.y + cblend * co.x;
-        gr.x = k * g2.z + cblend * co.y;
-        b.x = k * g2.w + cblend * co.z;
+        r.x = mix(g2.y, co.x);
+        gr.x = mix(g2.z, co.y);
+        b.x = mix(g2.w, co.z);
       }
       if (f1) {
         const float3 co = sample_cmap(cm, g.Ht, g.Wt, tx.y, ty.y);
-        r.y = k * g2.y + cblend * co.x;
-        gr.y = k * g2.z + cblend * co.y;
-        b.y = k * g2.w + cblend * co.z;
+        r.y = mix(g2.y, co.x);
+        gr.y = mix(g2.z, co.y);
+        b.y = mix(g2.w, co.z);
       }
     }
   }
@@ -809,8 +814,13 @@ struct TileWalker {
         } else {
           acc[0] = u.x + u.y;
           acc[1] = v.x + v.y;
-          acc[2] = e2.x + e2.y;
-          acc[3] = e3.x + e3.y;
+          if constexpr (CB) {
+            acc[2] = fmaf(u.y, ex.y, fmaf(v.y, ey.y, e2.x));
+            acc[3] = fmaf(u.y * g.rxy, ey.y, fmaf(-v.y * g.ryx, ex.y, e3.x));
+          } else {
+            acc[2] = e2.x + e2.y;
+            acc[3] = e3.x + e3.y;
+          }
           float c[4];
           colour_sums(c, gcr, gcg, gcb, wt, dlda, a);
 #pragma unroll
