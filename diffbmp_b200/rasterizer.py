@@ -307,12 +307,14 @@ class Rasterizer:
         self.tiles_x = (self.W + self.ts - 1) // self.ts
         self.tiles_y = (self.H + self.ts - 1) // self.ts
         self.T = self.tiles_x * self.tiles_y
-        # a fit job's persistent lists and binning workspace (_ensure); the
-        # renders allocate theirs per call, so that calls on other streams or
-        # threads never share them
+        # a fit job's persistent lists and binning workspace (_ensure): one job, one
+        # stream at a time
         self.capacity = 0
         self._ws = None
         self._idx = None
+        # the renders allocate their lists and workspace per call, so that calls on
+        # other streams or threads never share them; what they share is sizes, each
+        # read and replaced in one step, and pinned buffers, each held by one call
         self._hint = None          # list capacity of the next render
         self._ws_need = (None, 0)  # workspace bytes of the last (batch, N)
         self._mask_bytes = None    # walk masks of one candidate
@@ -352,10 +354,11 @@ class Rasterizer:
     def _scratch(self, cv: Canvas, B: int, N: int, stream):
         """(tensor, workspace bytes): a binning's workspace, followed by two ints
         per candidate for its flags and one for the walk's."""
-        if self._ws_need[0] != (B, N):
+        size, nbytes = self._ws_need     # read once: another thread may replace it
+        if size != (B, N):
             need = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), B))
-            self._ws_need = ((B, N), (need + 255) & ~255)
-        nbytes = self._ws_need[1]
+            nbytes = (need + 255) & ~255
+            self._ws_need = ((B, N), nbytes)
         t = torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device)
         if stream is not None:      # freed while that stream may still use it
             t.record_stream(stream)
@@ -375,9 +378,10 @@ class Rasterizer:
     def _capacity(self, N: int) -> int:
         """List entries to provide per candidate: 1.25 times the longest lists so
         far, at first an eighth of all (tile, primitive) pairs up to 16 MB."""
-        if self._hint is None:
-            self._hint = min(N * self.T, max(N * self.T // 8, 1024) + 4096, 4 << 20)
-        return self._hint
+        hint = self._hint
+        if hint is None:
+            self._hint = hint = min(N * self.T, max(N * self.T // 8, 1024) + 4096, 4 << 20)
+        return hint
 
     def _grow_hint(self, L: int):
         self._hint = min(max(self._hint, int(L * 1.25) + 4096), 0x7fffffff)
@@ -433,8 +437,11 @@ class Rasterizer:
         st = _stream(stream)
         if quads is not None:
             cv.changed = ws.data_ptr() + nbytes + 8 * B
-        pin = self._pins.pop() if self._pins else torch.empty(2 * B, dtype=torch.int32).pin_memory()
-        if pin.numel() < 2 * B:
+        try:
+            pin = self._pins.pop()       # (one step: another thread may take the last one)
+        except IndexError:
+            pin = None
+        if pin is None or pin.numel() < 2 * B:
             pin = torch.empty(2 * B, dtype=torch.int32).pin_memory()
         flags = pin.numpy()
         for _ in range(3):
