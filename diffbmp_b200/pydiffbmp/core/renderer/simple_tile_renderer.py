@@ -32,7 +32,7 @@ import numpy as np
 import torch
 
 from diffbmp_b200.fitting import FitConfig, ImageFitter, fallback_pool, prune_due
-from diffbmp_b200.rasterizer import Atlas, Rasterizer, rasterize, rasterize_batch
+from diffbmp_b200.rasterizer import Atlas, Filled, Rasterizer, rasterize, rasterize_batch
 
 MAX_PRIMS_PER_PIXEL = 400          # pydiffbmp/util/constants.py:21 (unused: depth is unbounded here)
 
@@ -76,7 +76,7 @@ class SimpleTileRenderer:
         self.primitive_bboxes = [tuple(b) for b in self._atlas.bbox.tolist()]
         self._rz = Rasterizer(self.H, self.W, self.tile_size, self.alpha_upper_bound, device=self.device)
         self.cuda_rasterizer = self._rz
-        self._sel = None
+        self._sel = (None, None)    # (N, its template ids)
 
     # -- helpers -------------------------------------------------------------
     def _num_templates(self) -> int:
@@ -85,9 +85,13 @@ class SimpleTileRenderer:
     def _global_bmp_sel(self, N: int) -> torch.Tensor:
         """Template of primitive i: (N-1-i) % p (simple_tile_renderer.py:221-224); the
         last N's assignment is kept."""
-        if self._sel is None or self._sel.numel() != N:
-            self._sel = (torch.arange(N, device=self.device, dtype=torch.int32) % self._num_templates()).flip(0).contiguous()
-        return self._sel
+        n, sel = self._sel
+        if n != N:
+            with torch.inference_mode(False):      # later calls may be of either mode
+                ids = torch.arange(N, device=self.device, dtype=torch.int32) % self._num_templates()
+                sel = Filled(ids.flip(0).contiguous())
+            self._sel = (N, sel)
+        return sel.use()
 
     def _atlas_for(self, is_final: bool) -> Atlas:
         return self._atlas_blurred if (self._atlas_blurred is not None and not is_final) else self._atlas

@@ -100,7 +100,7 @@ class Filled:
     def __init__(self, tensor: torch.Tensor):
         self.tensor = tensor
         s = torch.cuda.current_stream(tensor.device)
-        self._home = s.cuda_stream
+        self._device, self._home = s.device_index, s.cuda_stream
         self._event = torch.cuda.Event()
         self._event.record(s)
         self._done = False
@@ -110,7 +110,8 @@ class Filled:
         this call: behind the fill, and not freed before that work is done.  Under
         graph capture the caller has waited for the fill, as for the capture's
         other inputs."""
-        if _stream(stream) != self._home:
+        h = stream.cuda_stream if stream is not None else torch._C._cuda_getCurrentRawStream(self._device)
+        if h != self._home:
             s = stream if stream is not None else torch.cuda.current_stream(self.tensor.device)
             if not torch.cuda.is_current_stream_capturing():
                 if not self._done:
