@@ -15,6 +15,7 @@ Main objects:
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from dataclasses import dataclass
 from typing import Optional
@@ -58,6 +59,14 @@ def _stream(stream=None):
     if stream is not None:
         return stream.cuda_stream
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(stream):
+    """The stream as the current one (None: as it is, at none of the cost)."""
+    return _HERE if stream is None else torch.cuda.stream(stream)
 
 
 def _need_cuda(*ts):
@@ -187,7 +196,7 @@ class Atlas:
         q, version = self._quads or (None, -1)
         if version != self.data._version:
             version = self.data._version
-            with torch.cuda.stream(stream):
+            with _on(stream):
                 buf = torch.empty(int(lib.dbmp_atlas_extended_bytes(self.P, self.Ht, self.Wt, self.kind)),
                                   dtype=torch.uint8, device=self.data.device)
                 call("dbmp_atlas_pack_extended", _ptr(self.data), self.P, self.Ht, self.Wt, self.kind, _ptr(buf),
@@ -360,21 +369,16 @@ class Rasterizer:
             need = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), B))
             nbytes = (need + 255) & ~255
             self._ws_need = ((B, N), nbytes)
-        t = torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device)
-        if stream is not None:      # freed while that stream may still use it
-            t.record_stream(stream)
-        return t, nbytes
+        with _on(stream):      # of the call's own stream, which frees it in its order
+            return torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device), nbytes
 
     @staticmethod
     def _flat_batch(ts, stream):
         """The tensors contiguous: the batch calls step from candidate to candidate
-        by N, but candidates may come strided or expanded."""
-        out = [t.contiguous() for t in ts]
-        if stream is not None:
-            for t, o in zip(ts, out):
-                if o is not t:
-                    o.record_stream(stream)
-        return out
+        by N, but candidates may come strided or expanded.  Copied on the call's
+        stream, on which the caller has them ready."""
+        with _on(stream):
+            return [t.contiguous() for t in ts]
 
     def _capacity(self, N: int) -> int:
         """List entries to provide per candidate: 1.25 times the longest lists so
@@ -384,8 +388,12 @@ class Rasterizer:
             self._hint = hint = min(N * self.T, max(N * self.T // 8, 1024) + 4096, 4 << 20)
         return hint
 
-    def _grow_hint(self, L: int):
+    def _grow_hint(self, L: int, indices: torch.Tensor, stream):
+        """After a call on `stream` whose lists of up to L entries `indices` did not
+        hold; the candidates that it did hold may still be walked there."""
         self._hint = min(max(self._hint, int(L * 1.25) + 4096), 0x7fffffff)
+        if stream is not None:
+            indices.record_stream(stream)
 
     def bin(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None):
         """Device binning.  Returns (prim_info, TileLists).  Synchronises once
@@ -405,10 +413,11 @@ class Rasterizer:
             call("dbmp_bin", ctypes.byref(cv), _ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities),
                  _ptr(colors), _ptr(sel), _ptr(atlas.bbox), _ptr(prim_info), _ptr(offsets), _ptr(indices), cap,
                  _ptr(flags), flags.data_ptr() + 4, _ptr(ws), nbytes, st)
-            L, overflow = flags.tolist()
+            with _on(stream):     # behind the binning
+                L, overflow = flags.tolist()
             if not overflow:
                 return prim_info, TileLists(offsets, indices, int(L))
-            self._grow_hint(L)
+            self._grow_hint(L, indices, stream)
         raise DbmpError("binning capacity did not converge")
 
     def _render(self, lead: tuple, means2D, radii, rotations, opacities, colors, sel, sel_stride: int, atlas: Atlas,
@@ -459,12 +468,12 @@ class Rasterizer:
                 L = int(flags[0:2 * B:2].max())
                 self._pins.append(pin)
                 return color, alpha, T_last, last_pos, prim, offsets, indices, L, walk, quads
-            self._grow_hint(int(flags[0:2 * B:2].max()))
+            self._grow_hint(int(flags[0:2 * B:2].max()), indices, stream)
         raise DbmpError("binning capacity did not converge")
 
     def _flag(self, stream) -> torch.Tensor:
         """The flag of a walk that has no other scratch."""
-        with torch.cuda.stream(stream):
+        with _on(stream):
             return torch.empty(1, dtype=torch.int32, device=self.device)
 
     def prepare(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None,
@@ -548,10 +557,11 @@ class Rasterizer:
                      _ptr(sel[b]) if sel_stride else _ptr(sel), sel_stride, _ptr(atlas.bbox),
                      prim.data_ptr() + b * N * 64, _ptr(offsets[b]), _ptr(indices[b]), stride, cap, _ptr(small[b]),
                      _ptr(ws), nbytes, st)
-            Ls = small.cpu()
+            with _on(stream):     # behind the binning
+                Ls = small.cpu()
             if not bool(Ls[:, 1].any()):
                 return prim, offsets, indices
-            self._grow_hint(int(Ls[:, 0].max()))
+            self._grow_hint(int(Ls[:, 0].max()), indices, stream)
         raise DbmpError("binning capacity did not converge")
 
     def forward_batch(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, mappings=None,
@@ -616,9 +626,10 @@ class Rasterizer:
         (B,N), (B,N), (B,N), (B,N,3)."""
         B, N = int(radii.shape[0]), int(radii.shape[1])
         dev = self.device
-        gc = _operand(grad_color)
-        ga = _operand(grad_alpha) if grad_alpha is not None else None
-        acc = torch.empty((B * N + 1, 8), dtype=torch.float64, device=dev)    # the last row: the walk's flag
+        with _on(stream):
+            gc = _operand(grad_color)
+            ga = _operand(grad_alpha) if grad_alpha is not None else None
+            acc = torch.empty((B * N + 1, 8), dtype=torch.float64, device=dev)    # the last row: the walk's flag
         cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * B * N, stream)
         outs = [torch.empty(sh, dtype=torch.float32, device=dev)
                 for sh in ((B, N, 2), (B, N), (B, N), (B, N), (B, N, 3))]
@@ -649,9 +660,10 @@ class Rasterizer:
         rotations (N), opacities (N), colors (N,3)), float32."""
         N = int(radii.shape[0])
         dev = self.device
-        gc = _operand(grad_color)
-        ga = _operand(grad_alpha) if grad_alpha is not None else None
-        acc = torch.empty((N + 1, 8), dtype=torch.float64, device=dev)        # the last row: the walk's flag
+        with _on(stream):
+            gc = _operand(grad_color)
+            ga = _operand(grad_alpha) if grad_alpha is not None else None
+            acc = torch.empty((N + 1, 8), dtype=torch.float64, device=dev)        # the last row: the walk's flag
         cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * N, stream)
         g_means = torch.empty((N, 2), dtype=torch.float32, device=dev)
         g_r = torch.empty(N, dtype=torch.float32, device=dev)
