@@ -164,6 +164,7 @@ class Atlas:
                                                    and not self.templates.is_inference())
         self.own = self.kind != ATLAS_F32     # data is an extended atlas's buffer
         self._quads = None                    # ("f32") Filled extended atlas, version of data that it was packed from
+        self.fills = 0                        # (own) how often pack() has filled the buffer
         if self.own:
             self._alloc()
             self.pack(self.templates, st)
@@ -208,6 +209,7 @@ class Atlas:
 
     def pack(self, templates: torch.Tensor, st=None):
         """Fills the buffer from (P,Ht,Wt) f32 templates (extended atlases)."""
+        self.fills += 1
         call("dbmp_atlas_pack_extended", _ptr(templates), self.P, self.Ht, self.Wt, self.kind, _ptr(self.data),
              st if st is not None else _stream())
 
@@ -222,7 +224,7 @@ class Atlas:
         a.P, a.Ht, a.Wt, a.kind = self.P, self.Ht, self.Wt, self.kind
         a.extended = self.extended and (a.kind != ATLAS_F32 or pixels is None
                                         or quads_pay(pixels, N, self.templates.numel()))
-        a.own, a._quads = a.extended, None
+        a.own, a._quads, a.fills = a.extended, None, 0
         if a.extended:
             a._alloc()
         else:
@@ -263,7 +265,8 @@ class BatchState:
     c_blend: float = 0.0
     walk_masks: Optional[torch.Tensor] = None    # what the forward's tests found (dbmp_render)
     atlas: Optional[Atlas] = None                # the forward's atlas
-    quads: Optional[Filled] = None               # ... and its packed copy, if the forward walked one
+    quads: Optional[Filled] = None               # ... its packed copy, if the forward walked one
+    fills: int = 0                               # ... and its fills
 
     @property
     def batch(self) -> int:
@@ -280,7 +283,8 @@ class ForwardState:
     c_blend: float = 0.0
     walk_masks: Optional[torch.Tensor] = None    # what the forward's tests found (dbmp_render)
     atlas: Optional[Atlas] = None                # the forward's atlas
-    quads: Optional[Filled] = None               # ... and its packed copy, if the forward walked one
+    quads: Optional[Filled] = None               # ... its packed copy, if the forward walked one
+    fills: int = 0                               # ... and its fills
 
 
 def lists_from_mapping(mapping: torch.Tensor, num_tiles: int, num_prims: int) -> TileLists:
@@ -345,8 +349,9 @@ class Rasterizer:
         atlas with the flag at `changed` (an int32 of scratch), or on atlas.data."""
         if quads is None:
             return self.canvas(N, atlas), _ptr(atlas.data)
-        return FollowedCanvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
-                              self.alpha_max, self.t_stop, FOLLOWED_ATLAS, _ptr(atlas.data), changed), _ptr(quads.tensor)
+        cv = FollowedCanvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
+                            self.alpha_max, self.t_stop, FOLLOWED_ATLAS, _ptr(atlas.data), changed)
+        return cv, _ptr(quads.tensor)
 
     # -- binning -----------------------------------------------------------
     def _ensure(self, cv: Canvas, cap: int):
@@ -426,10 +431,10 @@ class Rasterizer:
         call; the host waits for the list lengths while the forward runs, and
         repeats the call if they exceed the capacity.  Returns (color, alpha,
         T_last, last_pos, prim_info, offsets, indices, longest list, walk_masks,
-        the atlas's packed copy); masks: the render's backward will be wanted."""
+        the atlas's packed copy, its fills); masks: the render's backward will be wanted."""
         B = lead[0] if lead else 1
         N = int(radii.shape[-1])
-        quads = self._quads(atlas, N, B, stream)
+        quads, fills = self._quads(atlas, N, B, stream), atlas.fills
         cv, texels = self.walk_canvas(N, atlas, quads, 1)    # (the flag is set below)
         dev, H, W = self.device, self.H, self.W
         color = torch.empty((*lead, H, W, 3), dtype=torch.float32, device=dev)
@@ -467,7 +472,7 @@ class Rasterizer:
             if not flags[1:2 * B:2].any():
                 L = int(flags[0:2 * B:2].max())
                 self._pins.append(pin)
-                return color, alpha, T_last, last_pos, prim, offsets, indices, L, walk, quads
+                return color, alpha, T_last, last_pos, prim, offsets, indices, L, walk, quads, fills
             self._grow_hint(int(flags[0:2 * B:2].max()), indices, stream)
         raise DbmpError("binning capacity did not converge")
 
@@ -488,8 +493,10 @@ class Rasterizer:
 
     def _walk_of(self, state, N: int, atlas: Atlas, changed: int, stream):
         """(canvas, atlas pointer, masks pointer) of the backward of a forward's
-        state: the forward's packed copy and masks where `atlas` is the forward's."""
-        if state.atlas is not atlas:
+        state: the forward's packed copy and masks where `atlas` is the forward's, and
+        filled as it was then.  (Another one may hold anything, sharper or
+        blurred templates, say: its backward tests again.)"""
+        if state.atlas is not atlas or state.fills != atlas.fills:
             return *self.walk_canvas(N, atlas, None, 0), None
         if state.quads is not None:
             state.quads.use(stream)
@@ -507,10 +514,10 @@ class Rasterizer:
         N = int(radii.shape[0])
         cmap = self._colour_maps(colors_orig, c_blend, N, atlas)
         if mapping is None or mapping.numel() == 0:
-            color, alpha, T_last, last_pos, prim_info, offsets, indices, L, walk, quads = self._render(
+            color, alpha, T_last, last_pos, prim_info, offsets, indices, L, walk, quads, fills = self._render(
                 (), means2D, radii, rotations, opacities, colors, sel, 0, atlas, stream, cmap, 0, c_blend, for_backward)
             return color, alpha, ForwardState(prim_info, TileLists(offsets, indices, L), T_last, last_pos, cmap,
-                                              float(c_blend) if cmap is not None else 0.0, walk, atlas, quads)
+                                              float(c_blend) if cmap is not None else 0.0, walk, atlas, quads, fills)
         lists = lists_from_mapping(mapping, self.T, N)
         quads, flag = self._quads(atlas, N, 1, stream), self._flag(stream)
         cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
@@ -585,10 +592,10 @@ class Rasterizer:
         has_maps = mappings is not None and len(mappings) > 0
         if not has_maps and 0 < B <= 65535:
             params = self._flat_batch((means2D, radii, rotations, opacities, colors, sel), stream)
-            color, alpha, T_last, last_pos, prim, offsets, indices, _, walk, quads = self._render(
+            color, alpha, T_last, last_pos, prim, offsets, indices, _, walk, quads, fills = self._render(
                 (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend, for_backward)
             return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
-                                            float(c_blend) if cmap is not None else 0.0, walk, atlas, quads)
+                                            float(c_blend) if cmap is not None else 0.0, walk, atlas, quads, fills)
         quads, flag = self._quads(atlas, N, B, stream), self._flag(stream)
         cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
         if has_maps:
