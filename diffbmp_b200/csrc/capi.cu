@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <thread>
 
 #include "dbmp_internal.cuh"
 
@@ -347,8 +348,15 @@ int dbmp_render_wait(const int32_t* host_flags, int batch, void* stream) {
   for (int b = 0; b < batch; ++b) {
     for (unsigned spin = 1; f[2 * b + 1] < 0; ++spin) {
       if (spin % 4096 != 0) continue;
+      // the binning of an idle stream reports within 0.3 ms (4096x4096, N=100000);
+      // behind a longer queue a core is not held: 50 us more are little there
+      auto waited = std::chrono::steady_clock::now() - t0;
+      while (f[2 * b + 1] < 0 && waited >= std::chrono::milliseconds(1) && waited < std::chrono::seconds(2)) {
+        std::this_thread::sleep_for(std::chrono::microseconds(50));
+        waited = std::chrono::steady_clock::now() - t0;
+      }
       // a launch that failed, or a stream busy for long: wait for it as usual
-      if (std::chrono::steady_clock::now() - t0 < std::chrono::seconds(2)) continue;
+      if (f[2 * b + 1] >= 0 || waited < std::chrono::seconds(2)) continue;
       const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
       if (e != cudaSuccess) return cuda_status(e, "dbmp_render_wait: cudaStreamSynchronize");
       REQUIRE(f[2 * b + 1] >= 0, "dbmp_render_wait: the binning did not report");

@@ -203,7 +203,8 @@ int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const
  * per candidate), which dbmp_render_wait polls; a candidate whose lists
  * exceed the capacity is not rendered, and the caller calls again with more.
  * Not capturable in a CUDA graph.  dbmp_render_wait(host_flags, batch, stream)
- * returns once the flags are there (spinning, then synchronising the stream):
+ * returns once the flags are there (it spins for 1 ms, polls every 50 us for 2 s, then
+ * synchronises the stream):
  * the one call of this library that waits for the device.
  * walk_masks (may be null): dbmp_walk_mask_bytes of scratch in which the forward
  * leaves the outcome of its per-warp tests; dbmp_backward_masked is
