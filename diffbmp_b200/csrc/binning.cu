@@ -740,7 +740,7 @@ static size_t layout_ws(void* base, int batch, int N, int T, int tilesX, int til
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += align_up(bytes); return o; };
   const size_t o_rects = take(sizeof(int4) * B * (N > 0 ? N : 1));
-  const size_t o_counts = take(sizeof(int) * 2 * (B * T * parts + 1));
+  const size_t o_counts = take(sizeof(int) * B * T * parts);
   const size_t o_offs = take(sizeof(long long) * B * ((size_t)T * bg.slices + 1));
   const size_t o_rows = take(sizeof(unsigned long long) * B * tilesY);
   const size_t mask_words = (size_t)bg.groups * tilesY * bg.words;
