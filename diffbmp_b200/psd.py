@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from ._lib import call
-from .rasterizer import _ptr, _stream
+from .rasterizer import _on, _ptr, _stream
 
 
 def _f32(t):
@@ -120,8 +120,14 @@ def encode_channel_blocks(buf, sizes, offsets, host_sizes, order, select, width_
     blocks (4 per chosen image, slots in ``order``, each = compression word,
     big-endian row sizes, PackBits rows), the (len(chosen), 4) block sizes and
     the chosen indices.  The host reads back only the block sizes and flags; the
-    groups' destinations are summed on the device.
+    groups' destinations are summed on the device.  With `stream`, all of that runs
+    on it, where the caller has buf, sizes and offsets ready.
     """
+    with _on(stream):
+        return _encode_channel_blocks(buf, sizes, offsets, host_sizes, order, select, width_limit)
+
+
+def _encode_channel_blocks(buf, sizes, offsets, host_sizes, order, select, width_limit):
     dev = buf.device
     hs = np.asarray(host_sizes, dtype=np.int64).reshape(-1, 2)
     n = hs.shape[0]
@@ -130,7 +136,7 @@ def encode_channel_blocks(buf, sizes, offsets, host_sizes, order, select, width_
     group_base = np.zeros(n + 1, np.int64)
     group_base[1:] = np.cumsum(ngroups)
     G = int(group_base[-1])
-    st = _stream(stream)
+    st = _stream()
     # group_base, then heights and group counts for the plan, in one copy
     meta = torch.from_numpy(np.concatenate([group_base, h, ngroups])).to(dev)
     gb, hd, ng = meta[:n + 1], meta[n + 1:2 * n + 1], meta[2 * n + 1:]
