@@ -712,7 +712,8 @@ def main():
     from diffbmp_b200.rasterizer import _ptr, _stream
 
     def fused_launch():
-        call("dbmp_fused_fwd_bwd", ctypes.byref(job.cv), _ptr(job.prim_info), _ptr(job.atlas.data),
+        cv, texels = job.walk()
+        call("dbmp_fused_fwd_bwd", ctypes.byref(cv), _ptr(job.prim_info), texels,
              _ptr(job.offsets), _ptr(job.rz._idx), _ptr(job.target), _ptr(job.background), None, _ptr(job.gacc),
              _ptr(job.loss_dev), None, _stream())
     job._enqueue(); torch.cuda.synchronize()

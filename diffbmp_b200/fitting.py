@@ -208,12 +208,10 @@ class ImageFitter:
         self.atlas = atlas
         self.rz = Rasterizer(self.H, self.W, cfg.tile_size, cfg.alpha_max, cfg.t_stop, device=dev)
         self.cv = self.rz.canvas(self.N, atlas)      # (of calls that pass atlas.data)
-        # the walks' canvas and atlas pointer: an "f32" job's steps keep the packed
-        # copy that they started with
+        # an "f32" job's steps keep the packed copy that they started with
         self._changed = torch.zeros(1, dtype=torch.int32, device=dev)
         follow = cfg.blur == "none" and self.N >= FIT_QUADS_PRIMS
         self._quads = atlas.quads() if follow else None
-        self._walk_cv, self._walk_atlas = self.rz.walk_canvas(self.N, atlas, self._quads, _ptr(self._changed))
         N8 = (max(self.N, 1), 8)
         self.adam_m = torch.zeros(N8, dtype=torch.float32, device=dev)
         self.adam_v = torch.zeros(N8, dtype=torch.float32, device=dev)
@@ -248,7 +246,6 @@ class ImageFitter:
                 raise ValueError("the adaptive blur schedule needs FitConfig.num_iterations")
             self.atlas = atlas.private_copy(self.H * self.W, self.N)
             self.cv = self.rz.canvas(self.N, self.atlas)
-            self._walk_cv, self._walk_atlas = self.rz.walk_canvas(self.N, self.atlas, None, 0)
             self.blur = _lib.BlurSchedule(BLUR_MODES[cfg.blur], cfg.blur_sigma, cfg.blur_sigma_start,
                                           cfg.blur_sigma_end, int(cfg.num_iterations))
             self._blurred = (self.atlas.data if self.atlas.kind == _lib.ATLAS_F32
@@ -294,6 +291,10 @@ class ImageFitter:
         return [_ptr(self.means2D), _ptr(self.radii), _ptr(self.rotations), _ptr(self.opacities),
                 _ptr(self.colors), _ptr(self.sel)]
 
+    def walk(self):
+        """(canvas, atlas pointer) of the job's walks."""
+        return self.rz.walk_canvas(self.N, self.atlas, self._quads, _ptr(self._changed))
+
     # -- one iteration -------------------------------------------------------
     def _blur_step(self, st=None):
         """This iteration's blurred texels (blur schedule on the device step count)."""
@@ -306,7 +307,7 @@ class ImageFitter:
 
     def _enqueue(self):
         st = _stream()
-        cv, texels = self._walk_cv, self._walk_atlas
+        cv, texels = self.walk()
         rz = self.rz
         ws, wsb = rz._ws_ptr()
         skip = ctypes.c_void_p(self.flags.data_ptr() + 4)

@@ -130,6 +130,9 @@ class Filled:
             self.tensor.record_stream(s)
         return self.tensor
 
+    def __reduce__(self):       # (copied and pickled with its owner)
+        return Filled, (self.use(),)
+
 
 class Atlas:
     """Template atlas on the device.  ``templates``: (P,Ht,Wt) or (Ht,Wt).
@@ -333,6 +336,11 @@ class Rasterizer:
         self._ws_need = (None, 0)  # workspace bytes of the last (batch, N)
         self._mask_bytes = None    # walk masks of one candidate
         self._pins = []            # pinned flag buffers not in use
+
+    def __getstate__(self):
+        # copies and pickles start without flag buffers: a copy of a pinned tensor is
+        # not pinned, and the binning would write to an address the device does not have
+        return {**self.__dict__, "_pins": []}
 
     def canvas(self, N: int, atlas: Atlas) -> Canvas:
         """The canvas of calls that pass atlas.data."""

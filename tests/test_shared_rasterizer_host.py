@@ -30,3 +30,14 @@ def test_workspace_size_of_a_call_is_its_own():
         rz._memo = memo
         t, nbytes = rz._scratch(cv, 2, 20000, None)
         assert nbytes >= need and t.numel() >= nbytes + 8 * 2 and t.device == torch.device("cpu")
+
+
+def test_copies_start_without_pinned_buffers():
+    """A copied pinned tensor is pageable memory, which the device cannot write to."""
+    import copy
+    import pickle
+    rz = R.Rasterizer(64, 96, device="cpu")
+    rz._pins, rz._hint = [torch.zeros(2, dtype=torch.int32)], 77
+    for other in (copy.deepcopy(rz), pickle.loads(pickle.dumps(rz)), copy.copy(rz)):
+        assert other._pins == [] and other._hint == 77 and (other.H, other.W, other.T) == (64, 96, 6)
+    assert len(rz._pins) == 1
