@@ -21,6 +21,7 @@ void set_error(const char* fmt, ...) {
 
 int cuda_status(cudaError_t e, const char* what) {
   set_error("%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
+  (void)cudaGetLastError();   // reported here, not by the next call's check of its launches
   return DBMP_ERR_CUDA;
 }
 
