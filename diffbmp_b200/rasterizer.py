@@ -348,7 +348,7 @@ class Rasterizer:
                       self.alpha_max, self.t_stop, EXTENDED_ATLAS if atlas.own else 0)
 
     def _quads(self, atlas: Atlas, N: int, B: int, stream) -> Optional[Filled]:
-        if atlas.own or not quads_pay(B * self.H * self.W, N, atlas.P * atlas.Ht * atlas.Wt):
+        if atlas.own or not quads_pay(B * self.H * self.W, N, atlas.templates.numel()):
             return None
         return atlas.quads(stream)
 
@@ -382,7 +382,9 @@ class Rasterizer:
             need = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), B))
             nbytes = (need + 255) & ~255
             self._ws_need = ((B, N), nbytes)
-        with _on(stream):      # of the call's own stream, which frees it in its order
+        if stream is None:
+            return torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device), nbytes
+        with torch.cuda.stream(stream):      # of the call's own stream, which frees it in its order
             return torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device), nbytes
 
     @staticmethod
@@ -442,7 +444,7 @@ class Rasterizer:
         the atlas's packed copy, its fills); masks: the render's backward will be wanted."""
         B = lead[0] if lead else 1
         N = int(radii.shape[-1])
-        quads, fills = self._quads(atlas, N, B, stream), atlas.fills
+        fills, quads = atlas.fills, None if atlas.own else self._quads(atlas, N, B, stream)
         cv, texels = self.walk_canvas(N, atlas, quads, 1)    # (the flag is set below)
         dev, H, W = self.device, self.H, self.W
         color = torch.empty((*lead, H, W, 3), dtype=torch.float32, device=dev)
@@ -499,16 +501,27 @@ class Rasterizer:
              _ptr(colors), _ptr(sel), _ptr(prim_info), _stream(stream))
         return prim_info
 
+    def _sums(self, grad_color, grad_alpha, rows: int, stream):
+        """(colour, alpha gradients as operands, accumulator) of a backward, on its
+        stream; the accumulator's last row holds the walk's flag."""
+        if stream is not None:
+            with torch.cuda.stream(stream):
+                return self._sums(grad_color, grad_alpha, rows, None)
+        return (_operand(grad_color), _operand(grad_alpha) if grad_alpha is not None else None,
+                torch.empty((rows + 1, 8), dtype=torch.float64, device=self.device))
+
     def _walk_of(self, state, N: int, atlas: Atlas, changed: int, stream):
         """(canvas, atlas pointer, masks pointer) of the backward of a forward's
         state: the forward's packed copy and masks where `atlas` is the forward's, and
         filled as it was then.  (Another one may hold anything, sharper or
         blurred templates, say: its backward tests again.)"""
         if state.atlas is not atlas or state.fills != atlas.fills:
-            return *self.walk_canvas(N, atlas, None, 0), None
-        if state.quads is not None:
-            state.quads.use(stream)
-        return *self.walk_canvas(N, atlas, state.quads, changed), _ptr(state.walk_masks)
+            return self.canvas(N, atlas), _ptr(atlas.data), None
+        if state.quads is None:
+            return self.canvas(N, atlas), _ptr(atlas.data), _ptr(state.walk_masks)
+        state.quads.use(stream)
+        cv, texels = self.walk_canvas(N, atlas, state.quads, changed)
+        return cv, texels, _ptr(state.walk_masks)
 
     # -- forward / backward -------------------------------------------------
     def forward(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas,
@@ -641,10 +654,7 @@ class Rasterizer:
         (B,N), (B,N), (B,N), (B,N,3)."""
         B, N = int(radii.shape[0]), int(radii.shape[1])
         dev = self.device
-        with _on(stream):
-            gc = _operand(grad_color)
-            ga = _operand(grad_alpha) if grad_alpha is not None else None
-            acc = torch.empty((B * N + 1, 8), dtype=torch.float64, device=dev)    # the last row: the walk's flag
+        gc, ga, acc = self._sums(grad_color, grad_alpha, B * N, stream)
         cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * B * N, stream)
         outs = [torch.empty(sh, dtype=torch.float32, device=dev)
                 for sh in ((B, N, 2), (B, N), (B, N), (B, N), (B, N, 3))]
@@ -675,10 +685,7 @@ class Rasterizer:
         rotations (N), opacities (N), colors (N,3)), float32."""
         N = int(radii.shape[0])
         dev = self.device
-        with _on(stream):
-            gc = _operand(grad_color)
-            ga = _operand(grad_alpha) if grad_alpha is not None else None
-            acc = torch.empty((N + 1, 8), dtype=torch.float64, device=dev)        # the last row: the walk's flag
+        gc, ga, acc = self._sums(grad_color, grad_alpha, N, stream)
         cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * N, stream)
         g_means = torch.empty((N, 2), dtype=torch.float32, device=dev)
         g_r = torch.empty(N, dtype=torch.float32, device=dev)
