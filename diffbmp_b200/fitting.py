@@ -25,7 +25,7 @@ import torch
 
 from . import _lib
 from ._lib import AdamCfg, call, lib
-from .rasterizer import Atlas, Rasterizer, _ptr, _stream, DEFAULT_T_STOP, FIT_QUADS_PRIMS
+from .rasterizer import Atlas, Rasterizer, _ptr, _stream, DEFAULT_T_STOP, fit_quads_pay
 
 # Reference defaults (pydiffbmp/util/constants.py:24-38): base lr and gains,
 # ExponentialLR factor, fixed blur sigma.
@@ -210,7 +210,7 @@ class ImageFitter:
         self.cv = self.rz.canvas(self.N, atlas)      # (of calls that pass atlas.data)
         # an "f32" job's steps keep the packed copy that they started with
         self._changed = torch.zeros(1, dtype=torch.int32, device=dev)
-        follow = cfg.blur == "none" and self.N >= FIT_QUADS_PRIMS
+        follow = cfg.blur == "none" and fit_quads_pay(self.H * self.W, self.N, atlas.templates.numel())
         self._quads = atlas.quads() if follow else None
         N8 = (max(self.N, 1), 8)
         self.adam_m = torch.zeros(N8, dtype=torch.float32, device=dev)

@@ -41,13 +41,6 @@ KIND_NAMES = {"f32": ATLAS_F32, "f32q": ATLAS_F32_QUAD, "f16q": ATLAS_F16_QUAD, 
 # to pack them (1.6 ms per GiB).
 MAX_F32_QUAD_BYTES = 1 << 30
 
-# Fits (many steps on one packed copy) walk quads from this many primitives on: below,
-# a step's comparison takes what the walks gain.  Gain of a fused step, comparison
-# included, over eight canvases of 64x64 to 1500x1500 and four atlases of 64x64 to
-# 16 of 256x256: -5 to 1 us with N=60 (but 8 at 1500x1500), -3 to 15 up to
-# 1024x1024 with 100, 0.7 to 51 with 200, 4 to 155 with 600.
-FIT_QUADS_PRIMS = 200
-
 DEFAULT_T_STOP = 1e-6   # image error <= t_stop * max colour, well inside the 1e-5 parity bar
 
 
@@ -90,16 +83,33 @@ def quads_pay(pixels: int, N: int, texels: int) -> bool:
     packing it takes, as a job whose templates change on every call pays for it.
 
     Packing takes 10 us for 64x64 texels, 23 for 8 of 128x128, 61 for 16 of 256x256 and
-    98 for 16 of 512x512; the walks gain with the pixels and, up to about 500
-    primitives, where a pixel is opaque, with their depth.  Forward and backward's
-    gain in us, the comparison included, on both sides of the line:
+    10 more for each further million; the walks gain with the pixels and, up to about
+    500 primitives, where a pixel is opaque, with their depth.  Forward and
+    backward's gain in us, the comparison included, on both sides of the line:
       8 of 128x128 (23):  N=600   384x384 20, 500x512 41, 1024x1024 123;
                           N=300   600x600 22, 768x768 36;  N=100  1024x1024 8
       16 of 256x256 (61): N=600   500x512 61, 600x600 77, 768x768 105;
                           N=300   768x768 56, 1024x1024 93;  N=100  1024x1024 14
+      16 of 512x512 (101), 1024x1024 (228): N=600  512x512 52 and 30, 1024x1024 211
+                          and 208, 2048x2048 679 and 855
       one 64x64 (10):     N=600   384x384 1, 500x512 9, 768x768 18;
                           N=6000  256x256 -3, 500x512 10"""
-    return pixels * min(N, 500) >= 500 * (180_000 + texels // 3)
+    million = 1 << 20
+    line = 180_000 + min(texels, million) // 3 + max(0, texels - million) // 9
+    return pixels * min(N, 500) >= 500 * line
+
+
+def fit_quads_pay(pixels: int, N: int, texels: int) -> bool:
+    """Whether a fit, whose steps share one packed copy, walks quads of an "f32" atlas.
+
+    From 200 primitives on a step gains more than its comparison takes: -5 to 1 us
+    with N=60 (8 at 1500x1500), -3 to 15 up to 1024x1024 with 100, 0.7 to 51 with 200,
+    4 to 155 with 600, over canvases from 64x64 and atlases from 64x64 to 16 of
+    256x256.  The comparison of larger atlases takes that back on small canvases: with
+    four million texels, N=600, a step gains -34 us at 64x64, 3 at 256x256 and 23 at
+    384x384; with 17 million 5 at 384x384 and 47 at 512x512 (N=200: -17 and -3); with
+    67 million 52 at 512x512 and 191 at 1024x1024 (-36 and 7)."""
+    return N >= 200 and texels <= (1 << 20) + 64 * pixels
 
 
 class Filled:

@@ -21,7 +21,7 @@ COPIES = {"deepcopy": copy.deepcopy, "pickle": lambda x: pickle.loads(pickle.dum
 @pytest.fixture(autouse=True)
 def packed_at_any_size(monkeypatch):
     monkeypatch.setattr(R, "quads_pay", lambda pixels, N, texels: True)
-    monkeypatch.setattr(F, "FIT_QUADS_PRIMS", 0)
+    monkeypatch.setattr(F, "fit_quads_pay", lambda pixels, N, texels: True)
 
 
 def params(seed=0):
