@@ -259,7 +259,7 @@ __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const 
 // overflow flag, and leaves the outputs untouched when L exceeds the capacity.
 // The write loop is bound by its instructions: write positions are pointers and
 // the compaction buffer is padded, so that it holds neither 64-bit index sums nor
-// bounds tests.  Replayed from a graph: 16.5 -> 10.5 us at 256x256, N=512;
+// bounds tests.  Replayed from a graph: 16.5 -> 11.3 us at 256x256, N=512;
 // 20.5 -> 14.1 at 1024x1024, N=5000 (against a memset, a difference array in global
 // memory and a library scan of all counts, six launches); with the masks of
 // use_masks 49.0 -> 34.2 at 2048x2048, N=20000 and 487 -> 268 at 4096x4096, N=100000.

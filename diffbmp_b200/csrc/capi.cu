@@ -452,7 +452,8 @@ int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void
   rc = launch_zero(grad_accum, 8ll * g.N, nullptr, g.changed, st);
   if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
-                             T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0, nullptr);
+                             T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0,
+                             nullptr);
   if (rc) return rc;
   return launch_finalize(g, radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii,
                          grad_rotations, grad_opacities, grad_colors, st);
@@ -478,13 +479,14 @@ int dbmp_forward_batch(const dbmp_canvas* cv, int batch, const void* prim_info, 
                               batch, index_stride, colors_orig_stride, nullptr, nullptr);
 }
 
-static int backward_batch(const char* who, const void* walk_masks, const dbmp_canvas* cv, int batch, const void* prim_info, const void* atlas,
-                        const int32_t* tile_offsets, const int32_t* tile_indices, long long index_stride,
-                        const float* colors_orig, long long colors_orig_stride, float c_blend, const float* T_last,
-                        const int32_t* last_pos, const float* grad_color, const float* grad_alpha,
-                        const float* radii, const float* rotations, const float* opacities, const float* colors,
-                        double* grad_accum, float* grad_means2D, float* grad_radii, float* grad_rotations,
-                        float* grad_opacities, float* grad_colors, void* stream) {
+static int backward_batch(const char* who, const void* walk_masks, const dbmp_canvas* cv, int batch,
+                          const void* prim_info, const void* atlas, const int32_t* tile_offsets,
+                          const int32_t* tile_indices, long long index_stride, const float* colors_orig,
+                          long long colors_orig_stride, float c_blend, const float* T_last, const int32_t* last_pos,
+                          const float* grad_color, const float* grad_alpha, const float* radii,
+                          const float* rotations, const float* opacities, const float* colors, double* grad_accum,
+                          float* grad_means2D, float* grad_radii, float* grad_rotations, float* grad_opacities,
+                          float* grad_colors, void* stream) {
   Geom g;
   int rc = make_geom(cv, &g, who);
   if (rc) return rc;
@@ -520,22 +522,24 @@ int dbmp_backward_batch(const dbmp_canvas* cv, int batch, const void* prim_info,
                         const float* radii, const float* rotations, const float* opacities, const float* colors,
                         double* grad_accum, float* grad_means2D, float* grad_radii, float* grad_rotations,
                         float* grad_opacities, float* grad_colors, void* stream) {
-  return backward_batch("dbmp_backward_batch", nullptr, cv, batch, prim_info, atlas, tile_offsets, tile_indices, index_stride, colors_orig, colors_orig_stride, c_blend,
-                        T_last, last_pos, grad_color, grad_alpha, radii, rotations, opacities, colors, grad_accum,
-                        grad_means2D, grad_radii, grad_rotations, grad_opacities, grad_colors, stream);
+  return backward_batch("dbmp_backward_batch", nullptr, cv, batch, prim_info, atlas, tile_offsets, tile_indices,
+                        index_stride, colors_orig, colors_orig_stride, c_blend, T_last, last_pos, grad_color, grad_alpha,
+                        radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii, grad_rotations,
+                        grad_opacities, grad_colors, stream);
 }
 
-int dbmp_backward_masked(const dbmp_canvas* cv, int batch, const void* walk_masks, const void* prim_info, const void* atlas,
-                        const int32_t* tile_offsets, const int32_t* tile_indices, long long index_stride,
-                        const float* colors_orig, long long colors_orig_stride, float c_blend, const float* T_last,
-                        const int32_t* last_pos, const float* grad_color, const float* grad_alpha,
-                        const float* radii, const float* rotations, const float* opacities, const float* colors,
-                        double* grad_accum, float* grad_means2D, float* grad_radii, float* grad_rotations,
-                        float* grad_opacities, float* grad_colors, void* stream) {
+int dbmp_backward_masked(const dbmp_canvas* cv, int batch, const void* walk_masks, const void* prim_info,
+                         const void* atlas, const int32_t* tile_offsets, const int32_t* tile_indices,
+                         long long index_stride, const float* colors_orig, long long colors_orig_stride,
+                         float c_blend, const float* T_last, const int32_t* last_pos, const float* grad_color,
+                         const float* grad_alpha, const float* radii, const float* rotations, const float* opacities,
+                         const float* colors, double* grad_accum, float* grad_means2D, float* grad_radii,
+                         float* grad_rotations, float* grad_opacities, float* grad_colors, void* stream) {
   REQUIRE(((uintptr_t)walk_masks & 15) == 0, "dbmp_backward_masked: walk_masks must be 16-byte aligned");
-  return backward_batch("dbmp_backward_masked", walk_masks, cv, batch, prim_info, atlas, tile_offsets, tile_indices, index_stride, colors_orig, colors_orig_stride, c_blend,
-                        T_last, last_pos, grad_color, grad_alpha, radii, rotations, opacities, colors, grad_accum,
-                        grad_means2D, grad_radii, grad_rotations, grad_opacities, grad_colors, stream);
+  return backward_batch("dbmp_backward_masked", walk_masks, cv, batch, prim_info, atlas, tile_offsets, tile_indices,
+                        index_stride, colors_orig, colors_orig_stride, c_blend, T_last, last_pos, grad_color, grad_alpha,
+                        radii, rotations, opacities, colors, grad_accum, grad_means2D, grad_radii, grad_rotations,
+                        grad_opacities, grad_colors, stream);
 }
 
 size_t dbmp_walk_mask_bytes(const dbmp_canvas* cv, int batch) {

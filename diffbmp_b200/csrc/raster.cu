@@ -485,7 +485,7 @@ struct TileWalker {
     __syncwarp();   // every lane is done with the previous chunk's records
     if ((c.todo >> lane) & 1u) {
       int id = __ldg(idx + start + base + lane);
-      if ((unsigned)id >= (unsigned)num_prims) id = 0;   // (a list changed since the forward stays in bounds)
+      if ((unsigned)id >= (unsigned)num_prims) id = 0;   // (never in the forward's own list; keeps the record read in bounds)
       const float4* r = reinterpret_cast<const float4*>(prims + id);
       float4* d = w[__popc(c.todo & ((1u << lane) - 1u))];
       float4 g2 = __ldg(r + 2);
@@ -994,11 +994,9 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(k
 
 // The walks of a followed atlas whose templates have changed, on the templates.  They
 // nearly always find nothing to do, so a grid of at most the resident blocks loops
-// over the tiles: it starts and ends in 1 to 2 us, where a block per tile would take
-// 0.2 ns a pixel.  What following costs a job with unchanged templates, the
-// comparison included (1024x1024, N=6000, 8 of 128x128, us): forward 90.7 against 87,
-// backward 138.6 against 136; the walks on the templates themselves take 164.9 and
-// 241.3.
+// over the tiles, rather than a block per tile that starts only to return.  1024x1024,
+// N=600, 8 of 128x128, comparison included (us): forward 107.3 without, 111.0 with
+// following, backward 174.4 and 180.6 (random texels, no solid cores).
 template <int TS, bool CB, bool MASKED>
 __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<ATLAS_F32, CB>(kFwdWarps<TS>()))
     forward_changed_kernel(Geom g, unsigned blocks, const PrimInfo* __restrict__ prims, const int* __restrict__ offs,
@@ -1244,8 +1242,10 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32>(1)) fused_changed_
 
 // Whether a followed atlas's templates still hold the texels packed from them (the
 // first part of an extended DBMP_ATLAS_F32 atlas), bit by bit; *changed was zeroed
-// before.  16-byte loads where both sides allow them.  8 bytes a texel: 2 us up to
-// 256k texels, at the copy rate beyond the L2.
+// before.  16-byte loads where both sides allow them.  8 bytes a texel; with the
+// *_changed_kernel behind the walk it costs a forward and a backward of 1024x1024 4 and
+// 6 us up to a million texels, 11 and 13 with four million, 81 each with 67 million
+// (the copy rate).
 template <typename V>
 __global__ void __launch_bounds__(256) templates_changed_kernel(const V* __restrict__ a, const V* __restrict__ b,
                                                                 long long n, int* __restrict__ changed) {

@@ -12,8 +12,8 @@ Same constructor, attributes and methods on the rasterizer's path:
   all their tiles (and one backward launch), not a loop over candidates;
 * ``optimize_parameters`` / ``_optimize_parameters_whole`` (:913-1228): the
   fit loop -- Adam with the reference's per-parameter gains, ExponentialLR
-  decay, the blur schedule, pruning and the clamp -- as CUDA-graph-replayed
-  device steps (diffbmp_b200.fitting.ImageFitter).
+  decay, the blur schedule, pruning and the clamp -- as device steps, replayed
+  from a CUDA graph beyond 16 iterations (diffbmp_b200.fitting.ImageFitter).
 
 Differences from the reference, by design: no CPU or PyTorch fallback (a
 failing call raises); per-pixel depth is unbounded (``max_prims_per_pixel`` is
@@ -172,10 +172,11 @@ class SimpleTileRenderer:
     def _optimize_parameters_whole(self, x, y, r, v, theta, c, target_image, opt_conf: dict,
                                    target_binary_mask=None, initializer: Optional[Any] = None):
         """The reference's loop (simple_tile_renderer.py:913-1228) on the
-        device: num_iterations graph-replayed steps of binning, fused forward +
-        L2 loss + backward, Adam with the per-group gains and ExponentialLR
-        decay, the blur schedule, pruning and the clamp.  Returns the fitted
-        (x, y, r, v, theta, c), also written into the given tensors.
+        device: num_iterations steps (replayed from one graph where there are more
+        than 16) of binning, fused forward + L2 loss + backward, Adam with the
+        per-group gains and ExponentialLR decay, the blur schedule, pruning and the
+        clamp.  Returns the fitted (x, y, r, v, theta, c), also written into the
+        given tensors.
 
         The L2 loss (loss_config type "mse", loss_functions.py:20-40) is the
         one the device step fuses.  Pruning draws its replacement rows from

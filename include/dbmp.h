@@ -75,7 +75,8 @@ typedef struct {
 } dbmp_canvas;
 
 /* dbmp_canvas.reserved: the atlas pointers passed with this canvas are
- * extended atlases (dbmp_atlas_pack_extended).  Any other value means plain ones. */
+ * extended atlases (dbmp_atlas_pack_extended).  Values other than this and the next mean
+ * plain ones. */
 #define DBMP_CANVAS_EXTENDED_ATLAS 0x41545845
 
 /* dbmp_canvas.reserved: the canvas is the first member of a dbmp_followed_canvas
