@@ -149,14 +149,14 @@ __device__ __forceinline__ int2 tile_span_cull(float m, float h, int ts, int ext
 
 // blockIdx.y: the candidate of a batch, whose inputs and outputs follow those
 // of the one before (sel: sel_stride apart).  row_total (tilesY per candidate)
-// is zeroed for counts_kernel, and the flag of a followed atlas for the walk behind.
+// is zeroed for counts_kernel, and the flags of a followed atlas for the walks.
 __global__ void prepare_kernel(Geom g, const float* __restrict__ means2D, const float* __restrict__ radii,
                                const float* __restrict__ rot, const float* __restrict__ opac,
                                const float* __restrict__ colors, const int* __restrict__ sel, long long sel_stride,
                                const float* __restrict__ tbbox, int bin_mode, PrimInfo* __restrict__ out,
                                int4* __restrict__ rects, unsigned long long* __restrict__ row_total) {
   grid_dependency();
-  if (g.changed != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *g.changed = 0;
+  if (g.changed != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) g.changed[threadIdx.x] = 0;
   const size_t b = blockIdx.y, bn = b * g.N;
   means2D += 2 * bn; radii += bn; rot += bn; opac += bn; colors += 3 * bn;
   sel += b * sel_stride;
@@ -367,11 +367,15 @@ __device__ __forceinline__ void mask_rects(const Geom& g, const BinGrid& bg, con
 __global__ void __launch_bounds__(1024) counts_kernel(Geom g, BinGrid bg, const int4* __restrict__ rects,
                                                       int* __restrict__ scratch, int* __restrict__ counts,
                                                       unsigned long long* __restrict__ row_total,
-                                                      unsigned* __restrict__ masks) {
+                                                      unsigned* __restrict__ masks, Follow follow) {
   extern __shared__ int s_diff[];
   grid_dependency();
   const int part = blockIdx.x, parts = bg.slices * bg.subs;   // counting slice
   const size_t b = blockIdx.y;
+  if (part >= parts + bg.words / kMaskWords) {                // the CTAs behind the marking ones
+    if (b == 0) follow_compare(follow, part - parts - bg.words / kMaskWords);
+    return;
+  }
   if (part >= parts) {
     mask_rects(g, bg, rects + b * g.N, (unsigned*)s_diff, part - parts,
                masks + b * ((size_t)bg.groups * g.tilesY * bg.words));
@@ -518,7 +522,7 @@ struct BinTiles {
                                        long long cap, int* __restrict__ indices, long long index_stride,
                                        int* __restrict__ tile_offsets, int* __restrict__ total_out,
                                        int* __restrict__ overflow_out, long long flag_stride,
-                                       volatile int* host_flags) {
+                                       volatile int* host_flags, const int* changed) {
     const size_t cand = blockIdx.y;   // candidate of a batch
     const long long nslots = (long long)g.T * bg.slices;
     offs += cand * (nslots + 1);
@@ -538,7 +542,8 @@ struct BinTiles {
       if (host_flags) {   // the host polls the second word
         host_flags[2 * cand] = (int)min(L, (long long)INT_MAX);
         __threadfence_system();
-        host_flags[2 * cand + 1] = (L > cap) ? 1 : 0;
+        // (bit 1: a followed atlas's templates have changed, and the host calls again)
+        host_flags[2 * cand + 1] = (L > cap ? 1 : 0) | (changed != nullptr && follow_changed(changed) ? 2 : 0);
         __threadfence_system();
       }
     }
@@ -592,13 +597,14 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_masks_kernel(
     Geom g, BinGrid bg, const int4* __restrict__ rects, const unsigned* __restrict__ masks,
     const long long* __restrict__ offs, long long cap, int* __restrict__ indices, long long index_stride,
     int* __restrict__ tile_offsets, int* __restrict__ total_out, int* __restrict__ overflow_out, long long flag_stride,
-    volatile int* host_flags) {
+    volatile int* host_flags, const int* changed) {
   __shared__ int s_id[kMaskBuffer];
   __shared__ int2 s_xr[kMaskBuffer];   // the rectangle's tile columns x0, x1
   __shared__ int s_wcnt[kBinWarps];
   grid_dependency();
   BinTiles bt;
-  if (!bt.open(g, bg, offs, cap, indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride, host_flags))
+  if (!bt.open(g, bg, offs, cap, indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride, host_flags,
+               changed))
     return;
   rects += (size_t)blockIdx.y * g.N;
   const int cell = blockIdx.x / bg.slices, cells = bg.groups * g.tilesY;
@@ -653,7 +659,8 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
                                                                   int* __restrict__ total_out,
                                                                   int* __restrict__ overflow_out,
                                                                   long long flag_stride,
-                                                                  volatile int* host_flags) {
+                                                                  volatile int* host_flags,
+                                                                  const int* changed) {
   // Two compaction buffers: chunk c is compacted into buffer c & 1 while the
   // warps may still read chunk c - 1 from the other one, so one barrier per
   // chunk orders everything (see the loop).
@@ -662,7 +669,8 @@ __global__ void __launch_bounds__(kBinThreads, 3) bin_rows_kernel(Geom g, BinGri
   __shared__ int s_wcnt[2][kBinWarps];
   grid_dependency();
   BinTiles bt;
-  if (!bt.open(g, bg, offs, cap, indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride, host_flags))
+  if (!bt.open(g, bg, offs, cap, indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride, host_flags,
+               changed))
     return;
   rects += (size_t)blockIdx.y * g.N;
   const int slice = bt.slice, ty = bt.ty, gx0 = bt.gx0, gx1 = bt.gx1;
@@ -1094,8 +1102,8 @@ int launch_prepare(const Geom& g, const float* means2D, const float* radii, cons
 int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
                const float* opac, const float* colors, const int* sel, long long sel_stride, const float* tbbox,
                PrimInfo* prim_info, int* tile_offsets, int* tile_indices, long long index_stride, long long cap,
-               int* total_out, int* overflow_out, long long flag_stride, int* host_flags, void* ws, size_t ws_bytes,
-               cudaStream_t st) {
+               int* total_out, int* overflow_out, long long flag_stride, int* host_flags, const Follow& follow, void* ws,
+               size_t ws_bytes, cudaStream_t st) {
   const BinGrid bg = bin_grid(g.N, g.tilesX, g.tilesY);
   BinWorkspace w{};
   const size_t need = layout_ws(ws, batch, g.N, g.T, g.tilesX, g.tilesY, bg, &w);
@@ -1107,7 +1115,7 @@ int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, con
     set_error("dbmp_bin: canvas, primitive count or batch too large");
     return DBMP_ERR_INVALID;
   }
-  // prepare also runs with N = 0: it zeroes the row totals
+  // prepare also runs with N = 0: it zeroes the row totals and the flags
   const dim3 prep(g.N > 0 ? (g.N + kPrepThreads - 1) / kPrepThreads : 1, batch);
   int rc = launch_chained("prepare_kernel", prepare_kernel, prep, kPrepThreads, 0, st, g, means2D, radii, rot, opac,
                           colors, sel, sel_stride, tbbox, bin_mode, prim_info, w.rects, w.row_total);
@@ -1118,8 +1126,9 @@ int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, con
     const cudaError_t e = cudaFuncSetAttribute(counts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountsSmem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(counts_kernel)");
   }
-  rc = launch_chained("counts_kernel", counts_kernel, dim3(bg.slices * bg.subs + bg.words / kMaskWords, batch), 1024, smem, st,
-                      g, bg, (const int4*)w.rects, w.scratch, w.counts, w.row_total, w.masks);
+  rc = launch_chained("counts_kernel", counts_kernel,
+                      dim3(bg.slices * bg.subs + bg.words / kMaskWords + follow.blocks, batch), 1024, smem, st, g, bg,
+                      (const int4*)w.rects, w.scratch, w.counts, w.row_total, w.masks, follow);
   if (rc) return rc;
   const long long row = (long long)g.tilesX * bg.slices * bg.subs;   // counts of a tile row
   auto* offsets = row > 4 * kOffsThreads ? offsets_kernel<8> : row > kOffsThreads ? offsets_kernel<4> : offsets_kernel<1>;
@@ -1130,10 +1139,10 @@ int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, con
     return launch_chained("bin_masks_kernel", bin_masks_kernel, dim3((unsigned)bg.ctas, batch), kBinThreads, 0, st, g,
                           bg, (const int4*)w.rects, (const unsigned*)w.masks, (const long long*)w.offs, cap,
                           tile_indices, index_stride, tile_offsets, total_out, overflow_out, flag_stride,
-                          (volatile int*)host_flags);
+                          (volatile int*)host_flags, (const int*)follow.changed);
   return launch_chained("bin_rows_kernel", bin_rows_kernel, dim3((unsigned)bg.ctas, batch), kBinThreads, 0, st, g, bg,
                         (const int4*)w.rects, (const long long*)w.offs, cap, tile_indices, index_stride, tile_offsets,
-                        total_out, overflow_out, flag_stride, (volatile int*)host_flags);
+                        total_out, overflow_out, flag_stride, (volatile int*)host_flags, (const int*)follow.changed);
 }
 
 }  // namespace dbmp

@@ -34,14 +34,14 @@ int launch_atlas_pack(const float* tmpl, int P, int Ht, int Wt, int kind, void* 
 int launch_atlas_extended(const float* tmpl, int P, int Ht, int Wt, int kind, void* out, cudaStream_t st);
 int launch_convert(int n, const void* const* src, void* const* dst, const long long* counts, bool to_half,
                    cudaStream_t st);
-int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st);
+int launch_zero(double* a, long long n, double* b, const Follow& f, cudaStream_t st);
 int launch_prepare(const Geom& g, const float* means2D, const float* radii, const float* rot, const float* opac,
                    const float* colors, const int* sel, PrimInfo* out, cudaStream_t st);
 int launch_bin(const Geom& g, int batch, int bin_mode, const float* means2D, const float* radii, const float* rot,
                const float* opac, const float* colors, const int* sel, long long sel_stride, const float* tbbox,
                PrimInfo* prim_info, int* tile_offsets, int* tile_indices, long long index_stride, long long cap,
-               int* total_out, int* overflow_out, long long flag_stride, int* host_flags, void* ws, size_t ws_bytes,
-               cudaStream_t st);
+               int* total_out, int* overflow_out, long long flag_stride, int* host_flags, const Follow& follow, void* ws,
+               size_t ws_bytes, cudaStream_t st);
 int launch_forward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                    const int* idx, float* color, float* alpha, float* T_last, int* last_pos, cudaStream_t st);
 int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
@@ -137,7 +137,7 @@ int make_geom(const dbmp_canvas* cv, Geom* g, const char* who) {
   if (cv->reserved == DBMP_CANVAS_FOLLOWED_ATLAS) {
     const dbmp_followed_canvas* f = reinterpret_cast<const dbmp_followed_canvas*>(cv);
     if (cv->atlas_kind != DBMP_ATLAS_F32 || !f->templates || !f->changed) {
-      set_error("%s: a followed atlas is DBMP_ATLAS_F32 and comes with its templates and a flag", who);
+      set_error("%s: a followed atlas is DBMP_ATLAS_F32 and comes with its templates and two flags", who);
       return DBMP_ERR_INVALID;
     }
     g->live = f->templates;
@@ -254,15 +254,15 @@ int dbmp_bin(const dbmp_canvas* cv, const float* means2D, const float* radii, co
           "dbmp_bin: prim_info must be 16-byte and workspace 256-byte aligned");
   return launch_bin(g, 1, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, 0, tmpl_bbox,
                     (PrimInfo*)prim_info, tile_offsets, tile_indices, 0, capacity, total_out, overflow_out, 0,
-                    nullptr, workspace, workspace_bytes, (cudaStream_t)stream);
+                    nullptr, Follow{}, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 static int bin_checked(const Geom& g, const char* who, const dbmp_canvas* cv, int batch, const float* means2D,
                        const float* radii, const float* rotations, const float* opacities, const float* colors,
                        const int32_t* sel, long long sel_stride, const float* tmpl_bbox, void* prim_info,
                        int32_t* tile_offsets, int32_t* tile_indices, long long index_stride, long long capacity,
-                       int32_t* total_and_overflow, int32_t* host_flags, void* workspace, size_t workspace_bytes,
-                       cudaStream_t st) {
+                       int32_t* total_and_overflow, int32_t* host_flags, const Follow& follow, void* workspace,
+                       size_t workspace_bytes, cudaStream_t st) {
   REQUIRE(batch >= 0, "%s: batch %d < 0", who, batch);
   if (batch == 0) return DBMP_OK;
   REQUIRE(cv->bin_mode == DBMP_BIN_CONTENT || cv->bin_mode == DBMP_BIN_CULL || cv->bin_mode == DBMP_BIN_CONTENT_REF,
@@ -280,7 +280,7 @@ static int bin_checked(const Geom& g, const char* who, const dbmp_canvas* cv, in
           "%s: prim_info must be 16-byte and workspace 256-byte aligned", who);
   return launch_bin(g, batch, cv->bin_mode, means2D, radii, rotations, opacities, colors, sel, sel_stride, tmpl_bbox,
                     (PrimInfo*)prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
-                    total_and_overflow + 1, 2, host_flags, workspace, workspace_bytes, st);
+                    total_and_overflow + 1, 2, host_flags, follow, workspace, workspace_bytes, st);
 }
 
 int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii,
@@ -293,7 +293,7 @@ int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const
   if (rc) return rc;
   return bin_checked(g, "dbmp_bin_batch", cv, batch, means2D, radii, rotations, opacities, colors, sel, sel_stride,
                      tmpl_bbox, prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
-                     nullptr, workspace, workspace_bytes, (cudaStream_t)stream);
+                     nullptr, Follow{}, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const float* radii, const float* rotations,
@@ -322,10 +322,11 @@ int dbmp_render(const dbmp_canvas* cv, int batch, const float* means2D, const fl
   for (int b = 0; b < batch; ++b) host_flags[2 * b + 1] = -1;
   rc = bin_checked(g, "dbmp_render", cv, batch, means2D, radii, rotations, opacities, colors, sel, sel_stride,
                    tmpl_bbox, prim_info, tile_offsets, tile_indices, index_stride, capacity, total_and_overflow,
-                   host_flags, workspace, workspace_bytes, (cudaStream_t)stream);
+                   host_flags, make_follow(g, g.records(atlas), 0), workspace, workspace_bytes, (cudaStream_t)stream);
   if (rc) return rc;
   // the forward runs behind the binning without waiting for the host; a
-  // candidate whose lists overflowed renders nothing
+  // candidate whose lists overflowed renders nothing, and none does when the
+  // templates of a followed atlas have changed
   return launch_forward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                               out_color, out_alpha, T_last, last_pos, colors_orig, c_blend, (cudaStream_t)stream,
                               batch, index_stride, colors_orig_stride, total_and_overflow, walk_masks);
@@ -393,7 +394,7 @@ int dbmp_backward(const dbmp_canvas* cv, const void* prim_info, const void* atla
   REQUIRE(g.N == 0 || (grad_accum && grad_means2D && grad_radii && grad_rotations && grad_opacities && grad_colors),
           "dbmp_backward: null output");
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, g.changed, st);
+  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, make_follow(g, g.records(atlas), 1), st);
   if (rc) return rc;
   rc = launch_backward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, T_last,
                        last_pos, grad_color, grad_alpha, grad_accum, st);
@@ -449,7 +450,7 @@ int dbmp_backward_blend(const dbmp_canvas* cv, const void* prim_info, const void
   REQUIRE(c_blend >= 0.f && c_blend <= 1.f, "dbmp_backward_blend: c_blend %g outside [0, 1]", (double)c_blend);
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "dbmp_backward_blend: colors_orig is null with c_blend > 0");
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, g.changed, st);
+  rc = launch_zero(grad_accum, 8ll * g.N, nullptr, make_follow(g, g.records(atlas), 1), st);
   if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, 1, 0, 0,
@@ -502,7 +503,7 @@ static int backward_batch(const char* who, const void* walk_masks, const dbmp_ca
   REQUIRE(c_blend == 0.f || g.N == 0 || colors_orig, "%s: colors_orig is null with c_blend > 0", who);
   if (!work) return DBMP_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, g.changed, st);
+  rc = launch_zero(grad_accum, 8ll * g.N * batch, nullptr, make_follow(g, g.records(atlas), 1), st);
   if (rc) return rc;
   rc = launch_backward_blend(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices,
                              T_last, last_pos, grad_color, grad_alpha, grad_accum, colors_orig, c_blend, st, batch,
@@ -575,7 +576,7 @@ int dbmp_fused_fwd_bwd(const dbmp_canvas* cv, const void* prim_info, const void*
   REQUIRE(atlas && tile_offsets && tile_indices && target && loss_out, "dbmp_fused_fwd_bwd: null input");
   REQUIRE(g.N == 0 || (prim_info && grad_accum), "dbmp_fused_fwd_bwd: null prim_info / grad_accum");
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(grad_accum, 8ll * g.N, loss_out, g.changed, st);
+  rc = launch_zero(grad_accum, 8ll * g.N, loss_out, make_follow(g, g.records(atlas), 1), st);
   if (rc) return rc;
   return launch_fused(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, target,
                       background, out_image, grad_accum, loss_out, skip_flag, st);

@@ -181,8 +181,8 @@ struct Geom {
   long long grid_off;  // byte offset of the clearance grid in a packed atlas
   int solid_delta;     // solid grid minus clearance grid, in bytes (0: no extended atlas)
   long long rec_off;   // byte offset of the records the walks read (host side only)
-  // followed atlases (dbmp_followed_canvas): the templates, and whether they differ
-  // from the packed ones (null otherwise)
+  // followed atlases (dbmp_followed_canvas): the templates, and whether a forward, and
+  // a backward, found them other than the packed ones (null otherwise)
   const float* live;
   int* changed;
   // the walks' atlas: the caller's pointer advanced to the records they read
@@ -316,6 +316,61 @@ int cuda_status(cudaError_t e, const char* what);
     cudaError_t _e = cudaGetLastError();                         \
     if (_e != cudaSuccess) return ::dbmp::cuda_status(_e, what); \
   } while (0)
+
+// The comparison of a followed atlas's templates with the texels packed from them (the
+// first part of an extended DBMP_ATLAS_F32 atlas), bit by bit, by blocks of a kernel
+// that runs before the walk anyway.  A difference sets the flag, which was zeroed with
+// the records; one that an earlier or concurrent walk of the same records has set stays,
+// and the walk on the templates that it leads to is right in any case.  8 bytes a
+// texel; 16-byte loads where both sides allow them.
+struct Follow {
+  const void* live;     // null: nothing to compare
+  const void* packed;
+  long long items;      // 16-byte items (wide) or texels
+  bool wide;
+  int* changed;
+  int blocks;           // of 1024 threads (a block per SM at most)
+};
+
+// word: 0 for a forward, 1 for a backward; records: where the walk reads them.
+inline Follow make_follow(const Geom& g, const void* records, int word) {
+  Follow f{};
+  if (!g.live) return f;
+  f.live = g.live;
+  f.packed = static_cast<const char*>(records) - g.rec_off;
+  f.items = (long long)g.P * g.Ht * g.Wt;
+  f.wide = f.items % 4 == 0 && (((uintptr_t)f.live | (uintptr_t)f.packed) & 15) == 0;
+  if (f.wide) f.items /= 4;
+  f.changed = g.changed + word;
+  const long long blocks = (f.items + 1023) / 1024;
+  f.blocks = (int)(blocks < 148 ? blocks : 148);
+  return f;
+}
+
+// Block `block` (< f.blocks) of the comparison, by all threads of the CTA.
+__device__ __forceinline__ void follow_compare(const Follow& f, int block) {
+  const long long i0 = (long long)block * blockDim.x + threadIdx.x, step = (long long)f.blocks * blockDim.x;
+  unsigned diff = 0u;
+  if (f.wide) {
+    const uint4* a = static_cast<const uint4*>(f.live);
+    const uint4* b = static_cast<const uint4*>(f.packed);
+#pragma unroll 4
+    for (long long i = i0; i < f.items; i += step) {
+      const uint4 x = a[i], y = b[i];
+      diff |= (x.x ^ y.x) | (x.y ^ y.y) | (x.z ^ y.z) | (x.w ^ y.w);
+    }
+  } else {
+    const unsigned* a = static_cast<const unsigned*>(f.live);
+    const unsigned* b = static_cast<const unsigned*>(f.packed);
+#pragma unroll 4
+    for (long long i = i0; i < f.items; i += step) diff |= a[i] ^ b[i];
+  }
+  if (diff != 0u) atomicOr(f.changed, 1);
+}
+
+__device__ __forceinline__ bool follow_changed(const int* changed) {
+  return *static_cast<const volatile int*>(changed) != 0;
+}
 
 // Chained launches (programmatic dependent launch): a kernel of a chain starts
 // while the one before it on the stream drains, and grid_dependency(), its

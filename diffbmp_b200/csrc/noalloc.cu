@@ -30,7 +30,7 @@ constexpr int kMaxDevices = 64;
 static __device__ __align__(256) double g_noalloc_accum[(size_t)kNoAllocMaxPrims * 8];
 
 int make_geom(const dbmp_canvas* cv, Geom* g, const char* who);
-int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st);
+int launch_zero(double* a, long long n, double* b, const Follow& f, cudaStream_t st);
 int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* atlas, const int* offs,
                     const int* idx, const float* T_last, const int* last_pos, const float* grad_color,
                     const float* grad_alpha, double* gacc, cudaStream_t st);
@@ -127,7 +127,7 @@ extern "C" int dbmp_backward_noalloc(const dbmp_canvas* cv, const void* prim_inf
   rc = noalloc_scratch(&scratch);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_zero(scratch, 8ll * g.N, nullptr, g.changed, st);
+  rc = launch_zero(scratch, 8ll * g.N, nullptr, make_follow(g, g.records(atlas), 1), st);
   if (rc) return rc;
   rc = launch_backward(g, g.kind, (const PrimInfo*)prim_info, g.records(atlas), tile_offsets, tile_indices, T_last,
                        last_pos, grad_color, grad_alpha, scratch, st);

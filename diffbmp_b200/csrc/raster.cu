@@ -930,8 +930,8 @@ template <int KIND, bool CB = false> constexpr int kBlocksPerSM(int cta_warps) {
 
 // True where a followed atlas's templates differ from the packed ones that this walk
 // would read: its *_changed_kernel then walks the templates.
-template <int KIND> __device__ __forceinline__ bool packed_is_stale(const Geom& g) {
-  return KIND == ATLAS_F32_QUAD && g.changed != nullptr && *g.changed != 0;
+template <int KIND> __device__ __forceinline__ bool packed_is_stale(const Geom& g, int word) {
+  return KIND == ATLAS_F32_QUAD && g.changed != nullptr && follow_changed(g.changed + word);
 }
 
 // ---------------------------------------------------------------------------
@@ -987,16 +987,17 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<KIND, CB>(k
     long long idx_stride, long long cmap_stride, const int* __restrict__ flags, uint4* __restrict__ masks) {
   __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
   grid_dependency();
-  if (packed_is_stale<KIND>(g)) return;
+  if (packed_is_stale<KIND>(g, 0)) return;
   forward_block<TS, KIND, CB, MASKED>(g, blockIdx.x, s_pi, prims, atlas, offs, idx, out_color, out_alpha, T_last,
                                       last_pos, cmap, cblend, idx_stride, cmap_stride, flags, masks);
 }
 
-// The walks of a followed atlas whose templates have changed, on the templates.  They
-// nearly always find nothing to do, so a grid of at most the resident blocks loops
-// over the tiles, rather than a block per tile that starts only to return.  1024x1024,
-// N=600, 8 of 128x128, comparison included (us): forward 107.3 without, 111.0 with
-// following, backward 174.4 and 180.6 (random texels, no solid cores).
+// The walks of a followed atlas whose templates have changed, on the templates, behind
+// those on its packed copy that return at once then: for forwards of given lists,
+// backwards and fits.  (A render tells the host to call again, and small masked
+// backwards read the templates themselves.)  They nearly always find nothing to do, so a
+// grid of at most the resident blocks loops over the tiles, rather than a block per
+// tile that starts only to return.
 template <int TS, bool CB, bool MASKED>
 __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<ATLAS_F32, CB>(kFwdWarps<TS>()))
     forward_changed_kernel(Geom g, unsigned blocks, const PrimInfo* __restrict__ prims, const int* __restrict__ offs,
@@ -1006,7 +1007,7 @@ __global__ void __launch_bounds__(kFwdWarps<TS>() * 32, kBlocksPerSM<ATLAS_F32, 
                            uint4* __restrict__ masks) {
   __shared__ Rec s_pi[kFwdWarps<TS>()][kChunk];
   grid_dependency();
-  if (*g.changed == 0) return;
+  if (!follow_changed(g.changed)) return;
   for (unsigned b = blockIdx.x; b < blocks; b += gridDim.x)
     forward_block<TS, ATLAS_F32, CB, MASKED>(g, (int)b, s_pi, prims, g.live, offs, idx, out_color, out_alpha, T_last,
                                              last_pos, cmap, cblend, idx_stride, cmap_stride, flags, masks);
@@ -1078,8 +1079,17 @@ __device__ __forceinline__ void backward_block(
   tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Ts, lp, gacc, MASKED ? s_kept : nullptr);
 }
 
-template <int TS, int KIND, bool CB, bool MASKED>
-__global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel(
+// INNER: the masked walk on FP32 quads with the walk on a followed atlas's templates
+// beside it, for small launches.  Behind it in a launch of its own, that one costs the
+// host 5 us, which small calls wait for; inside, it costs the kernel's code 3 to 4 %
+// (backward at 1024x1024, N=5000: 128.5 -> 132.5 us; 4096x4096, N=100000: 2369 ->
+// 2455), bounded to the 72 registers that leave it its 28 warps per SM.  Forward and
+// backward together, launched apart / inside: 512x512 (host-bound) 224 / 220 us,
+// 1024x1024 243 / 243, 4096x4096 3370 / 3450.
+constexpr long long kInnerWarps = 12288;   // walks of up to about 887x887 pixels
+
+template <int TS, int KIND, bool CB, bool MASKED, bool INNER = false>
+__global__ void __launch_bounds__(32, INNER && !CB ? 28 : kBlocksPerSM<KIND, CB>(1)) backward_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, const float* __restrict__ T_last, const int* __restrict__ last_pos,
     const float* __restrict__ grad_color, const float* __restrict__ grad_alpha, double* __restrict__ gacc,
@@ -1088,7 +1098,13 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND, CB>(1)) backward_kernel
   __shared__ Rec s_pi[kChunk];
   __shared__ Kept s_kept;
   grid_dependency();
-  if (packed_is_stale<KIND>(g)) return;
+  if (packed_is_stale<KIND>(g, 1)) {
+    if constexpr (INNER)   // (the masks belong to the packed templates)
+      backward_block<TS, ATLAS_F32, CB, false>(g, blockIdx.x, s_pi, nullptr, prims, g.live, offs, idx, T_last, last_pos,
+                                               grad_color, grad_alpha, gacc, cmap, cblend, idx_stride, cmap_stride,
+                                               nullptr);
+    return;
+  }
   backward_block<TS, KIND, CB, MASKED>(g, blockIdx.x, s_pi, &s_kept, prims, atlas, offs, idx, T_last, last_pos,
                                        grad_color, grad_alpha, gacc, cmap, cblend, idx_stride, cmap_stride, masks);
 }
@@ -1102,7 +1118,7 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32, CB>(1)) backward_c
     const float* __restrict__ cmap, float cblend, long long idx_stride, long long cmap_stride) {
   __shared__ Rec s_pi[kChunk];
   grid_dependency();
-  if (*g.changed == 0) return;
+  if (!follow_changed(g.changed + 1)) return;
   for (unsigned b = blockIdx.x; b < blocks; b += gridDim.x)
     backward_block<TS, ATLAS_F32, CB, false>(g, (int)b, s_pi, nullptr, prims, g.live, offs, idx, T_last, last_pos,
                                              grad_color, grad_alpha, gacc, cmap, cblend, idx_stride, cmap_stride,
@@ -1217,7 +1233,7 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
   __shared__ Kept s_kept;
   grid_dependency();
   if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
-  if (packed_is_stale<KIND>(g)) return;
+  if (packed_is_stale<KIND>(g, 1)) return;
   fused_block<TS, KIND>(g, blockIdx.x, s_pi, s_kept, prims, atlas, offs, idx, target, background, out_image, gacc,
                         loss_out);
 }
@@ -1232,7 +1248,7 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32>(1)) fused_changed_
   __shared__ Rec s_pi[kChunk];
   __shared__ Kept s_kept;
   grid_dependency();
-  if ((skip_flag != nullptr && *skip_flag != 0) || *g.changed == 0) return;
+  if ((skip_flag != nullptr && *skip_flag != 0) || !follow_changed(g.changed + 1)) return;
   for (unsigned b = blockIdx.x; b < blocks; b += gridDim.x) {
     __syncwarp();   // every lane is done with the previous block's masks
     fused_block<TS, ATLAS_F32>(g, (int)b, s_pi, s_kept, prims, g.live, offs, idx, target, background, out_image, gacc,
@@ -1240,27 +1256,11 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32>(1)) fused_changed_
   }
 }
 
-// Whether a followed atlas's templates still hold the texels packed from them (the
-// first part of an extended DBMP_ATLAS_F32 atlas), bit by bit; *changed was zeroed
-// before.  16-byte loads where both sides allow them.  8 bytes a texel; with the
-// *_changed_kernel behind the walk it costs a forward and a backward of 1024x1024 4 and
-// 6 us up to a million texels, 11 and 13 with four million, 81 each with 67 million
-// (the copy rate).
-template <typename V>
-__global__ void __launch_bounds__(256) templates_changed_kernel(const V* __restrict__ a, const V* __restrict__ b,
-                                                                long long n, int* __restrict__ changed) {
+// The comparison alone, for forwards of given lists (renders compare beside the
+// counting of their binning, backwards and fits beside the zeroing of their sums).
+__global__ void __launch_bounds__(1024) follow_kernel(Follow f) {
   grid_dependency();
-  unsigned diff = 0u;
-#pragma unroll 4
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if constexpr (sizeof(V) == 16) {
-      const uint4 x = a[i], y = b[i];
-      diff |= (x.x ^ y.x) | (x.y ^ y.y) | (x.z ^ y.z) | (x.w ^ y.w);
-    } else {
-      diff |= a[i] ^ b[i];
-    }
-  }
-  if (__any_sync(kFull, diff != 0u) && (threadIdx.x & 31) == 0) atomicOr(changed, 1);
+  follow_compare(f, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1283,26 +1283,6 @@ __global__ void __launch_bounds__(256) templates_changed_kernel(const V* __restr
 // batch > 1: `batch` candidates of the same canvas in one grid, candidate b's
 // records at prims + b N, lists at offs + b (T+1) / idx + b idx_stride,
 // images at b H W (x3 for colour), colour maps at cmap + b cmap_stride.
-int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st);
-
-// Compares a followed atlas's templates with the packed records at `atlas` (zero: the
-// flag is not zeroed yet).
-static int launch_changed(const Geom& g, const void* atlas, bool zero, cudaStream_t st) {
-  if (zero) {
-    const int rc = launch_zero(nullptr, 0, nullptr, g.changed, st);
-    if (rc) return rc;
-  }
-  const char* packed = static_cast<const char*>(atlas) - g.rec_off;
-  const long long n = (long long)g.P * g.Ht * g.Wt;
-  const bool wide = n % 4 == 0 && ((uintptr_t)packed & 15) == 0 && ((uintptr_t)g.live & 15) == 0;
-  const long long items = wide ? n / 4 : n, ctas = (items + 255) / 256;
-  const dim3 grid((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8));
-  return wide ? launch_chained("templates_changed_kernel", templates_changed_kernel<uint4>, grid, 256, 0, st,
-                               (const uint4*)g.live, (const uint4*)packed, items, g.changed)
-              : launch_chained("templates_changed_kernel", templates_changed_kernel<unsigned>, grid, 256, 0, st,
-                               (const unsigned*)g.live, (const unsigned*)packed, items, g.changed);
-}
-
 // Grid of a *_changed_kernel: at most what is resident at once.
 static dim3 changed_grid(long long blocks, int per_sm) {
   return dim3((unsigned)(blocks < 148ll * per_sm ? blocks : 148ll * per_sm));
@@ -1334,9 +1314,10 @@ int launch_forward_blend(const Geom& g, int kind, const PrimInfo* prims, const v
                      : go(forward_kernel<TSV, KD, false, false>, parts, threads)));
     return DBMP_OK;
   };
-  if (!g.live) return walk();
-  // flags: behind a binning, whose first kernel zeroed the flag of the comparison
-  int rc = launch_changed(g, atlas, flags == nullptr, st);
+  // flags: behind a binning, which compared a followed atlas and told the host
+  if (!g.live || flags != nullptr) return walk();
+  const Follow f = make_follow(g, atlas, 0);
+  int rc = launch_chained("follow_kernel", follow_kernel, dim3(f.blocks), 1024, 0, st, f);
   if (!rc) rc = walk();
   if (rc) return rc;
   auto again = [&](auto kernel, int parts, int threads) {
@@ -1395,8 +1376,12 @@ int launch_backward_blend(const Geom& g, int kind, const PrimInfo* prims, const 
     return DBMP_OK;
   };
   if (!g.live) return walk();
-  int rc = launch_changed(g, atlas, false, st);   // launch_zero came before
-  if (!rc) rc = walk();
+  // launch_zero has compared a followed atlas
+  if (masks != nullptr && ctas <= kInnerWarps && kind == ATLAS_F32_QUAD) {
+    DBMP_TS_SWITCH(g.TS, return blend ? go(backward_kernel<TSV, ATLAS_F32_QUAD, true, true, true>, kTileWarps<TSV>())
+                                      : go(backward_kernel<TSV, ATLAS_F32_QUAD, false, true, true>, kTileWarps<TSV>()));
+  }
+  const int rc = walk();
   if (rc) return rc;
   auto again = [&](auto kernel, int warps) {
     const long long blocks = (long long)batch * g.T * warps;
@@ -1416,21 +1401,25 @@ int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* 
                                nullptr, 0.f, st, 1, 0, 0, nullptr);
 }
 
-// Zeroes n doubles at a and, when given, one at b and an int: a kernel rather than
-// memsets, so that the launches around it stay chained.
-__global__ void zero_kernel(double* __restrict__ a, long long n, double* __restrict__ b, int* __restrict__ flag) {
+// Zeroes n doubles at a and, when given, one at b: a kernel rather than memsets, so
+// that the launches around it stay chained.  Its first blocks also compare a followed
+// atlas's templates for the walk behind.
+__global__ void __launch_bounds__(1024) zero_kernel(double* __restrict__ a, long long n, double* __restrict__ b, Follow f) {
   grid_dependency();
+  if (blockIdx.x < f.blocks) follow_compare(f, blockIdx.x);
   const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (long long i = i0; i < n; i += (long long)gridDim.x * blockDim.x) a[i] = 0.0;
   if (b != nullptr && i0 == 0) *b = 0.0;
-  if (flag != nullptr && i0 == 0) *flag = 0;
 }
 
-int launch_zero(double* a, long long n, double* b, int* flag, cudaStream_t st) {
-  if (n == 0 && b == nullptr && flag == nullptr) return DBMP_OK;
-  const long long ctas = (n + 255) / 256;
-  return launch_chained("zero_kernel", zero_kernel, dim3((unsigned)(ctas < 1 ? 1 : ctas < 1184 ? ctas : 1184)), 256, 0,
-                        st, a, n, b, flag);
+int launch_zero(double* a, long long n, double* b, const Follow& f, cudaStream_t st) {
+  if (n == 0 && b == nullptr && f.live == nullptr) return DBMP_OK;
+  const unsigned threads = f.live ? 1024 : 256;
+  long long ctas = (n + threads - 1) / threads;
+  if (ctas < 1) ctas = 1;
+  if (ctas < f.blocks) ctas = f.blocks;
+  if (ctas > 1184) ctas = 1184;
+  return launch_chained("zero_kernel", zero_kernel, dim3((unsigned)ctas), threads, 0, st, a, n, b, f);
 }
 
 int launch_finalize(const Geom& g, const float* radii, const float* rot, const float* opac, const float* colors,
@@ -1451,8 +1440,7 @@ int launch_fused(const Geom& g, int kind, const PrimInfo* prims, const void* atl
     return DBMP_OK;
   };
   if (!g.live) return walk();
-  int rc = launch_changed(g, atlas, false, st);   // launch_zero came before
-  if (!rc) rc = walk();
+  const int rc = walk();   // (launch_zero has compared a followed atlas)
   if (rc) return rc;
   DBMP_TS_SWITCH(g.TS, const long long blocks = (long long)g.T * kTileWarps<TSV>(); return launch_chained(
       "fused_changed_kernel", fused_changed_kernel<TSV>, changed_grid(blocks, DBMP_WARPS_PER_SM_F32), 32, 0, st, g,

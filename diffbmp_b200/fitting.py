@@ -209,9 +209,9 @@ class ImageFitter:
         self.rz = Rasterizer(self.H, self.W, cfg.tile_size, cfg.alpha_max, cfg.t_stop, device=dev)
         self.cv = self.rz.canvas(self.N, atlas)      # (of calls that pass atlas.data)
         # an "f32" job's steps keep the packed copy that they started with
-        self._changed = torch.zeros(1, dtype=torch.int32, device=dev)
         follow = cfg.blur == "none" and fit_quads_pay(self.H * self.W, self.N, atlas.templates.numel())
         self._quads = atlas.quads() if follow else None
+        self._changed = torch.zeros(2, dtype=torch.int32, device=dev) if self._quads is not None else None
         N8 = (max(self.N, 1), 8)
         self.adam_m = torch.zeros(N8, dtype=torch.float32, device=dev)
         self.adam_v = torch.zeros(N8, dtype=torch.float32, device=dev)
@@ -293,6 +293,8 @@ class ImageFitter:
 
     def walk(self):
         """(canvas, atlas pointer) of the job's walks."""
+        if self._quads is None:
+            return self.cv, _ptr(self.atlas.data)
         return self.rz.walk_canvas(self.N, self.atlas, self._quads, _ptr(self._changed))
 
     # -- one iteration -------------------------------------------------------

@@ -83,20 +83,21 @@ def quads_pay(pixels: int, N: int, texels: int) -> bool:
     packing it takes, as a job whose templates change on every call pays for it.
 
     Packing takes 10 us for 64x64 texels, 23 for 8 of 128x128, 61 for 16 of 256x256 and
-    10 more for each further million; the walks gain with the pixels and, up to about
-    500 primitives, where a pixel is opaque, with their depth.  Forward and
-    backward's gain in us, the comparison included, on both sides of the line:
-      8 of 128x128 (23):  N=600   384x384 20, 500x512 41, 1024x1024 123;
-                          N=300   600x600 22, 768x768 36;  N=100  1024x1024 8
-      16 of 256x256 (61): N=600   500x512 61, 600x600 77, 768x768 105;
-                          N=300   768x768 56, 1024x1024 93;  N=100  1024x1024 14
+    10 more for each further million; the walks gain with the pixels and, between 50
+    and about 500 primitives, where a pixel is opaque, with their depth.  Forward and
+    backward's gain in us on both sides of the line, measured with launches of their
+    own for the comparison (5 us more than it takes now):
+      one 64x64 (10):     N=200  500x512 0, 768x768 4;  N=300  384x384 -2, 500x512 6
+      4 of 64x64 (10):    N=200  384x384 0;  N=300  500x512 11
+      8 of 128x128 (23):  N=300  384x384 4, 500x512 15, 600x600 22, 768x768 36;
+                          N=600  300x300 18, 384x384 20, 500x512 41
+      16 of 256x256 (61): N=60   1500x1500 7;  N=300  500x512 29, 768x768 56,
+                          1024x1024 93;  N=600  384x384 29, 600x600 77
       16 of 512x512 (101), 1024x1024 (228): N=600  512x512 52 and 30, 1024x1024 211
-                          and 208, 2048x2048 679 and 855
-      one 64x64 (10):     N=600   384x384 1, 500x512 9, 768x768 18;
-                          N=6000  256x256 -3, 500x512 10"""
+                          and 208, 2048x2048 679 and 855"""
     million = 1 << 20
-    line = 180_000 + min(texels, million) // 3 + max(0, texels - million) // 9
-    return pixels * min(N, 500) >= 500 * line
+    line = 125_000 + min(texels, million) // 8 + max(0, texels - million) // 9
+    return pixels * (min(N, 500) - 50) >= 450 * line
 
 
 def fit_quads_pay(pixels: int, N: int, texels: int) -> bool:
@@ -177,6 +178,7 @@ class Atlas:
                                                    and not self.templates.is_inference())
         self.own = self.kind != ATLAS_F32     # data is an extended atlas's buffer
         self._quads = None                    # ("f32") Filled extended atlas, version of data that it was packed from
+        self._anew = self._anew_next = 0      # calls that pack whatever the version; how many after the next miss
         self.fills = 0                        # (own) how often pack() has filled the buffer
         if self.own:
             self._alloc()
@@ -194,11 +196,18 @@ class Atlas:
 
     def refresh(self):
         """Has an "f32" atlas packed anew by its next render.  Never needed for the
-        result: a walk that finds ``data`` changed reads it in the reference layout,
-        which is slower.  A change that PyTorch counts (``data._version``) is
-        packed anew without this call; writes through ``.data``, of another
-        library's kernel or a replayed graph are not counted."""
+        result: a render that finds ``data`` changed repeats itself on it, and the
+        other walks read it in the reference layout, which is slower.  A change that
+        PyTorch counts (``data._version``) is packed anew without this call; writes
+        through ``.data``, of another library's kernel or a replayed graph are not
+        counted."""
         self._quads = None
+
+    def _missed(self):
+        """A render has found the copy out of date and repeats itself: the next ones
+        pack anew, one after the first such miss, up to 63 when misses go on."""
+        self._quads = None
+        self._anew, self._anew_next = self._anew_next, min(2 * self._anew_next + 1, 63)
 
     def quads(self, stream=None) -> Optional[Filled]:
         """An "f32" atlas's extended copy (quads and grids) for work on `stream`, or
@@ -208,7 +217,8 @@ class Atlas:
         if self.own or not self.extended:
             return None
         q, version = self._quads or (None, -1)
-        if version != self.data._version:
+        if self._anew or version != self.data._version:
+            self._anew = max(0, self._anew - 1)
             version = self.data._version
             with _on(stream):
                 buf = torch.empty(int(lib.dbmp_atlas_extended_bytes(self.P, self.Ht, self.Wt, self.kind)),
@@ -237,7 +247,7 @@ class Atlas:
         a.P, a.Ht, a.Wt, a.kind = self.P, self.Ht, self.Wt, self.kind
         a.extended = self.extended and (a.kind != ATLAS_F32 or pixels is None
                                         or quads_pay(pixels, N, self.templates.numel()))
-        a.own, a._quads, a.fills = a.extended, None, 0
+        a.own, a._quads, a._anew, a._anew_next, a.fills = a.extended, None, 0, 0, 0
         if a.extended:
             a._alloc()
         else:
@@ -364,7 +374,7 @@ class Rasterizer:
 
     def walk_canvas(self, N: int, atlas: Atlas, quads: Optional[Filled], changed: int):
         """(canvas, atlas pointer) of a walk: on the packed copy `quads` of an "f32"
-        atlas with the flag at `changed` (an int32 of scratch), or on atlas.data."""
+        atlas with its flags at `changed` (behind the records), or on atlas.data."""
         if quads is None:
             return self.canvas(N, atlas), _ptr(atlas.data)
         cv = FollowedCanvas(self.H, self.W, self.ts, int(N), atlas.P, atlas.Ht, atlas.Wt, atlas.kind, self.bin_mode,
@@ -386,16 +396,16 @@ class Rasterizer:
 
     def _scratch(self, cv: Canvas, B: int, N: int, stream):
         """(tensor, workspace bytes): a binning's workspace, followed by two ints
-        per candidate for its flags and one for the walk's."""
+        per candidate for its flags."""
         size, nbytes = self._ws_need     # read once: another thread may replace it
         if size != (B, N):
             need = int(lib.dbmp_bin_batch_workspace_bytes(ctypes.byref(cv), B))
             nbytes = (need + 255) & ~255
             self._ws_need = ((B, N), nbytes)
         if stream is None:
-            return torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device), nbytes
+            return torch.empty(nbytes + 8 * B, dtype=torch.uint8, device=self.device), nbytes
         with torch.cuda.stream(stream):      # of the call's own stream, which frees it in its order
-            return torch.empty(nbytes + 8 * B + 4, dtype=torch.uint8, device=self.device), nbytes
+            return torch.empty(nbytes + 8 * B, dtype=torch.uint8, device=self.device), nbytes
 
     @staticmethod
     def _flat_batch(ts, stream):
@@ -455,13 +465,13 @@ class Rasterizer:
         B = lead[0] if lead else 1
         N = int(radii.shape[-1])
         fills, quads = atlas.fills, None if atlas.own else self._quads(atlas, N, B, stream)
-        cv, texels = self.walk_canvas(N, atlas, quads, 1)    # (the flag is set below)
         dev, H, W = self.device, self.H, self.W
         color = torch.empty((*lead, H, W, 3), dtype=torch.float32, device=dev)
         alpha = torch.empty((*lead, H, W), dtype=torch.float32, device=dev)
         T_last = torch.empty((*lead, H, W), dtype=torch.float32, device=dev)
         last_pos = torch.empty((*lead, H, W), dtype=torch.int32, device=dev)
-        prim = torch.empty((max(B * N, 1), 16), dtype=torch.float32, device=dev)
+        prim = torch.empty((B * N + 1, 16), dtype=torch.float32, device=dev)     # (the last one: flags)
+        cv, texels = self.walk_canvas(N, atlas, quads, prim.data_ptr() + 64 * B * N)
         offsets = torch.empty((*lead, self.T + 1), dtype=torch.int32, device=dev)
         walk = None
         if masks:
@@ -470,8 +480,6 @@ class Rasterizer:
             walk = torch.empty(self._mask_bytes * B, dtype=torch.uint8, device=dev)
         ws, nbytes = self._scratch(cv, B, N, stream)
         st = _stream(stream)
-        if quads is not None:
-            cv.changed = ws.data_ptr() + nbytes + 8 * B
         try:
             pin = self._pins.pop()       # (one step: another thread may take the last one)
         except IndexError:
@@ -479,7 +487,7 @@ class Rasterizer:
         if pin is None or pin.numel() < 2 * B:
             pin = torch.empty(2 * B, dtype=torch.int32).pin_memory()
         flags = pin.numpy()
-        for _ in range(3):
+        for _ in range(4):
             cap = self._capacity(N)
             stride = max(cap, 1)
             indices = torch.empty((*lead, stride), dtype=torch.int32, device=dev)
@@ -489,6 +497,13 @@ class Rasterizer:
                  float(c_blend) if cmap is not None else 0.0, _ptr(color), _ptr(alpha), _ptr(T_last), _ptr(last_pos),
                  _ptr(walk), _ptr(ws), nbytes, st)
             call("dbmp_render_wait", _ptr(pin), B, st)
+            if quads is not None and flags[1] & 2:        # the copy is out of date: nothing was rendered
+                atlas._missed()
+                quads = None
+                cv, texels = self.walk_canvas(N, atlas, None, 0)
+                if stream is not None:
+                    indices.record_stream(stream)
+                continue
             if not flags[1:2 * B:2].any():
                 L = int(flags[0:2 * B:2].max())
                 self._pins.append(pin)
@@ -496,31 +511,27 @@ class Rasterizer:
             self._grow_hint(int(flags[0:2 * B:2].max()), indices, stream)
         raise DbmpError("binning capacity did not converge")
 
-    def _flag(self, stream) -> torch.Tensor:
-        """The flag of a walk that has no other scratch."""
-        with _on(stream):
-            return torch.empty(1, dtype=torch.int32, device=self.device)
-
     def prepare(self, means2D, radii, rotations, opacities, colors, sel, atlas: Atlas, stream=None,
-                cv: Optional[Canvas] = None):
-        """The records of given lists' walk, for a walk with canvas cv."""
+                quads: Optional[Filled] = None):
+        """The records of given lists' walk (of the packed copy `quads`: its flags are
+        the last record)."""
         N = int(radii.shape[0])
-        cv = cv if cv is not None else self.canvas(N, atlas)
-        prim_info = torch.empty((max(N, 1), 16), dtype=torch.float32, device=self.device)
+        prim_info = torch.empty((N + 1 if quads is not None else max(N, 1), 16), dtype=torch.float32, device=self.device)
+        cv, _ = self.walk_canvas(N, atlas, quads, prim_info.data_ptr() + 64 * N)
         call("dbmp_prepare", ctypes.byref(cv), _ptr(means2D), _ptr(radii), _ptr(rotations), _ptr(opacities),
              _ptr(colors), _ptr(sel), _ptr(prim_info), _stream(stream))
         return prim_info
 
     def _sums(self, grad_color, grad_alpha, rows: int, stream):
         """(colour, alpha gradients as operands, accumulator) of a backward, on its
-        stream; the accumulator's last row holds the walk's flag."""
+        stream."""
         if stream is not None:
             with torch.cuda.stream(stream):
                 return self._sums(grad_color, grad_alpha, rows, None)
         return (_operand(grad_color), _operand(grad_alpha) if grad_alpha is not None else None,
-                torch.empty((rows + 1, 8), dtype=torch.float64, device=self.device))
+                torch.empty((max(rows, 1), 8), dtype=torch.float64, device=self.device))
 
-    def _walk_of(self, state, N: int, atlas: Atlas, changed: int, stream):
+    def _walk_of(self, state, N: int, rows: int, atlas: Atlas, stream):
         """(canvas, atlas pointer, masks pointer) of the backward of a forward's
         state: the forward's packed copy and masks where `atlas` is the forward's, and
         filled as it was then.  (Another one may hold anything, sharper or
@@ -530,7 +541,7 @@ class Rasterizer:
         if state.quads is None:
             return self.canvas(N, atlas), _ptr(atlas.data), _ptr(state.walk_masks)
         state.quads.use(stream)
-        cv, texels = self.walk_canvas(N, atlas, state.quads, changed)
+        cv, texels = self.walk_canvas(N, atlas, state.quads, state.prim_info.data_ptr() + 64 * rows)
         return cv, texels, _ptr(state.walk_masks)
 
     # -- forward / backward -------------------------------------------------
@@ -550,9 +561,9 @@ class Rasterizer:
             return color, alpha, ForwardState(prim_info, TileLists(offsets, indices, L), T_last, last_pos, cmap,
                                               float(c_blend) if cmap is not None else 0.0, walk, atlas, quads, fills)
         lists = lists_from_mapping(mapping, self.T, N)
-        quads, flag = self._quads(atlas, N, 1, stream), self._flag(stream)
-        cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
-        prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream, cv)
+        quads = self._quads(atlas, N, 1, stream)
+        prim_info = self.prepare(means2D, radii, rotations, opacities, colors, sel, atlas, stream, quads)
+        cv, texels = self.walk_canvas(N, atlas, quads, prim_info.data_ptr() + 64 * N)
         color = torch.empty((self.H, self.W, 3), dtype=torch.float32, device=self.device)
         alpha = torch.empty((self.H, self.W), dtype=torch.float32, device=self.device)
         T_last = torch.empty((self.H, self.W), dtype=torch.float32, device=self.device)
@@ -627,9 +638,9 @@ class Rasterizer:
                 (B,), *params, N if sel.dim() == 2 else 0, atlas, stream, cmap, cstride, c_blend, for_backward)
             return color, alpha, BatchState(prim, offsets, indices, T_last, last_pos, cmap, cstride,
                                             float(c_blend) if cmap is not None else 0.0, walk, atlas, quads, fills)
-        quads, flag = self._quads(atlas, N, B, stream), self._flag(stream)
-        cv, texels = self.walk_canvas(N, atlas, quads, _ptr(flag))
+        quads = None
         if has_maps:
+            quads = self._quads(atlas, N, B, stream)
             if len(mappings) != B:
                 raise ValueError(f"{len(mappings)} mappings for {B} candidates")
             lists = [lists_from_mapping(m, self.T, N) for m in mappings]
@@ -638,7 +649,8 @@ class Rasterizer:
             indices = torch.zeros((B, stride), dtype=torch.int32, device=self.device)
             for b, l in enumerate(lists):
                 indices[b, :l.length] = l.indices[:l.length]
-            prim = torch.empty((max(B * N, 1), 16), dtype=torch.float32, device=self.device)
+            prim = torch.empty((B * N + 1, 16), dtype=torch.float32, device=self.device)    # (the last one: flags)
+            cv, _ = self.walk_canvas(N, atlas, quads, prim.data_ptr() + 64 * B * N)
             sel2 = sel if sel.dim() == 2 else sel.unsqueeze(0).expand(B, -1)
             for b in range(B):
                 call("dbmp_prepare", ctypes.byref(cv), _ptr(means2D[b]), _ptr(radii[b]), _ptr(rotations[b]),
@@ -646,6 +658,7 @@ class Rasterizer:
                      ctypes.c_void_p(prim.data_ptr() + b * N * 64), st)
         else:
             prim, offsets, indices = self.bin_batch(means2D, radii, rotations, opacities, colors, sel, atlas, stream)
+        cv, texels = self.walk_canvas(N, atlas, quads, prim.data_ptr() + 64 * B * N)
         dev = self.device
         color = torch.empty((B, self.H, self.W, 3), dtype=torch.float32, device=dev)
         alpha = torch.empty((B, self.H, self.W), dtype=torch.float32, device=dev)
@@ -665,7 +678,7 @@ class Rasterizer:
         B, N = int(radii.shape[0]), int(radii.shape[1])
         dev = self.device
         gc, ga, acc = self._sums(grad_color, grad_alpha, B * N, stream)
-        cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * B * N, stream)
+        cv, texels, masks = self._walk_of(state, N, B * N, atlas, stream)
         outs = [torch.empty(sh, dtype=torch.float32, device=dev)
                 for sh in ((B, N, 2), (B, N), (B, N), (B, N), (B, N, 3))]
         call("dbmp_backward_masked", ctypes.byref(cv), B, masks, _ptr(state.prim_info),
@@ -696,7 +709,7 @@ class Rasterizer:
         N = int(radii.shape[0])
         dev = self.device
         gc, ga, acc = self._sums(grad_color, grad_alpha, N, stream)
-        cv, texels, masks = self._walk_of(state, N, atlas, acc.data_ptr() + 64 * N, stream)
+        cv, texels, masks = self._walk_of(state, N, N, atlas, stream)
         g_means = torch.empty((N, 2), dtype=torch.float32, device=dev)
         g_r = torch.empty(N, dtype=torch.float32, device=dev)
         g_rot = torch.empty(N, dtype=torch.float32, device=dev)

@@ -83,10 +83,12 @@ typedef struct {
  * (DBMP_ATLAS_F32 only).  The atlas pointers passed with it are extended atlases packed
  * from `templates` at some earlier time; every walk first compares the templates, as
  * they are when the walk's turn on its stream comes, with the packed ones bit by bit,
- * and where any texel differs it reads the templates in the reference layout instead.
- * A job can so walk a packed copy of templates that others may write to.  `changed`:
- * one int32 of device scratch that no other call in flight uses (left nonzero when
- * the templates differed). */
+ * and where any texel differs it reads the templates in the reference layout instead
+ * (dbmp_render tells the caller to: see there).  A job can so walk a packed copy of
+ * templates that others may write to.  `changed`: two int32 on the device that belong
+ * to the job's records: the call that writes these (dbmp_bin, dbmp_bin_batch,
+ * dbmp_prepare, dbmp_render) zeroes them, forwards set the first and backwards (and
+ * dbmp_fused_fwd_bwd) the second when the templates differ. */
 #define DBMP_CANVAS_FOLLOWED_ATLAS 0x46545845
 typedef struct {
   dbmp_canvas canvas;
@@ -202,7 +204,10 @@ int dbmp_bin_batch(const dbmp_canvas* cv, int batch, const float* means2D, const
  * of the same candidates, without the host in between.  The binning also
  * writes each candidate's two flags to host_flags (pinned host memory, 2 ints
  * per candidate), which dbmp_render_wait polls; a candidate whose lists
- * exceed the capacity is not rendered, and the caller calls again with more.
+ * exceed the capacity is not rendered, and the caller calls again with more.  The
+ * second of a candidate's host flags has bit 0 set for that, and bit 1 when the
+ * templates of a followed atlas have changed: nothing is rendered then, and the caller
+ * calls again with a canvas of the templates themselves (or packs them anew).
  * Not capturable in a CUDA graph.  dbmp_render_wait(host_flags, batch, stream)
  * returns once the flags are there (it spins for 1 ms, polls every 50 us for 2 s, then
  * synchronises the stream):

@@ -221,3 +221,19 @@ def test_changed_templates_on_several_streams_gpu(monkeypatch):
         for g in got:
             assert torch.equal(g, want[k])
         torch.cuda.synchronize()
+
+
+def test_a_writer_that_is_never_counted_gpu(monkeypatch):
+    """Templates that change before every call: each render shows them, from copies
+    packed anew after the first few calls that found theirs out of date."""
+    T, p, rz = templates(0), params(11), R.Rasterizer(H, W)
+    atlas = R.Atlas(T, "f32")
+    misses = []
+    monkeypatch.setattr(atlas, "_missed", lambda: (misses.append(1), R.Atlas._missed(atlas)))
+    for k in range(40):
+        T.data.copy_(templates(k % 7))
+        ref = plain(T, atlas, monkeypatch)
+        c, a, st = rz.forward(*p, atlas)
+        c0, a0, _ = R.Rasterizer(H, W).forward(*p, ref)
+        assert torch.equal(c, c0) and torch.equal(a, a0)
+    assert 1 <= len(misses) <= 6
