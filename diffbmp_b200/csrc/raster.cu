@@ -1223,8 +1223,8 @@ __device__ __forceinline__ void fused_block(const Geom& g, int block, Rec* s_pi,
   tw.backward(g, prims, atlas, idx, s_pi, gC, gA, Tl, lp, gacc, &s_kept);
 }
 
-template <int TS, int KIND>
-__global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
+template <int TS, int KIND, bool INNER = false>   // INNER: see backward_kernel
+__global__ void __launch_bounds__(32, INNER ? 28 : kBlocksPerSM<KIND>(1)) fused_kernel(
     Geom g, const PrimInfo* __restrict__ prims, const void* __restrict__ atlas, const int* __restrict__ offs,
     const int* __restrict__ idx, const float* __restrict__ target, const float* __restrict__ background,
     float* __restrict__ out_image, double* __restrict__ gacc, double* __restrict__ loss_out,
@@ -1233,7 +1233,12 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<KIND>(1)) fused_kernel(
   __shared__ Kept s_kept;
   grid_dependency();
   if (skip_flag != nullptr && *skip_flag != 0) return;   // binning overflowed: leave all state untouched
-  if (packed_is_stale<KIND>(g, 1)) return;
+  if (packed_is_stale<KIND>(g, 1)) {
+    if constexpr (INNER)
+      fused_block<TS, ATLAS_F32>(g, blockIdx.x, s_pi, s_kept, prims, g.live, offs, idx, target, background, out_image, gacc,
+                                 loss_out);
+    return;
+  }
   fused_block<TS, KIND>(g, blockIdx.x, s_pi, s_kept, prims, atlas, offs, idx, target, background, out_image, gacc,
                         loss_out);
 }
@@ -1258,8 +1263,11 @@ __global__ void __launch_bounds__(32, kBlocksPerSM<ATLAS_F32>(1)) fused_changed_
 
 // The comparison alone, for forwards of given lists (renders compare beside the
 // counting of their binning, backwards and fits beside the zeroing of their sums).
+// Without a trigger: the walk's CTAs launch as these end.  Launched beside them, they
+// crowd onto the SMs that are free first (fit step of 256x256, N=5000, 16 of 256x256:
+// 125 us, 89 without, 90.5 without a comparison).
 __global__ void __launch_bounds__(1024) follow_kernel(Follow f) {
-  grid_dependency();
+  cudaGridDependencySynchronize();
   follow_compare(f, blockIdx.x);
 }
 
@@ -1405,8 +1413,9 @@ int launch_backward(const Geom& g, int kind, const PrimInfo* prims, const void* 
 // that the launches around it stay chained.  Its first blocks also compare a followed
 // atlas's templates for the walk behind.
 __global__ void __launch_bounds__(1024) zero_kernel(double* __restrict__ a, long long n, double* __restrict__ b, Follow f) {
-  grid_dependency();
-  if (blockIdx.x < f.blocks) follow_compare(f, blockIdx.x);
+  cudaGridDependencySynchronize();
+  if (f.live == nullptr) cudaTriggerProgrammaticLaunchCompletion();   // (see follow_kernel)
+  else if (blockIdx.x < f.blocks) follow_compare(f, blockIdx.x);
   const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (long long i = i0; i < n; i += (long long)gridDim.x * blockDim.x) a[i] = 0.0;
   if (b != nullptr && i0 == 0) *b = 0.0;
@@ -1440,7 +1449,11 @@ int launch_fused(const Geom& g, int kind, const PrimInfo* prims, const void* atl
     return DBMP_OK;
   };
   if (!g.live) return walk();
-  const int rc = walk();   // (launch_zero has compared a followed atlas)
+  // launch_zero has compared a followed atlas
+  DBMP_TS_SWITCH(g.TS, if ((long long)g.T * kTileWarps<TSV>() <= kInnerWarps) return launch_chained(
+      "fused_kernel", fused_kernel<TSV, ATLAS_F32_QUAD, true>, dim3((unsigned)(g.T * kTileWarps<TSV>())), 32, 0, st, g,
+      prims, atlas, offs, idx, target, background, out_image, gacc, loss, skip_flag));
+  const int rc = walk();
   if (rc) return rc;
   DBMP_TS_SWITCH(g.TS, const long long blocks = (long long)g.T * kTileWarps<TSV>(); return launch_chained(
       "fused_changed_kernel", fused_changed_kernel<TSV>, changed_grid(blocks, DBMP_WARPS_PER_SM_F32), 32, 0, st, g,
